@@ -68,6 +68,9 @@
 (defrstq weight-bind-shard*  "rstq_weight_bind_shard" I [P P P P I L L I I I I I]) ; ... split rank nranks
 (defrstq weight-bind-q4k*    "rstq_weight_bind_q4k"   I [P P P P P P P I L L])     ; ctx w** wq da db aq bq dev out in
 (defrstq weight-bind-q6k*    "rstq_weight_bind_q6k"   I [P P P P P I L L])         ; ctx w** wq sc ds dev out in
+(defrstq quantize-weight*    "rstq_quantize_weight"     I [P P P L I])       ; w codes scales n format
+(defrstq quantize-weight-q4k* "rstq_quantize_weight_q4k" I [P P P P P P L])   ; w wq da db aq bq n
+(defrstq quantize-weight-q6k* "rstq_quantize_weight_q6k" I [P P P P L])       ; w wq sc ds n
 (defrstq weight-clone*       "rstq_weight_clone"      I [P P])
 (defrstq weight-free*        "rstq_weight_free"       I [P])
 (defrstq weight-info*        "rstq_weight_info"       I [P P])

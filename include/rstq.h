@@ -232,6 +232,14 @@ RSTQ_API int32_t rstq_weight_bind_q4k(rstq_ctx* ctx, rstq_weight** w, const void
  * Held on the device as two 8-bit rows per matrix row (twice the reference's code bytes). */
 RSTQ_API int32_t rstq_weight_bind_q6k(rstq_ctx* ctx, rstq_weight** w, const void* wq, const int8_t* sc,
                                       const float* ds, int32_t dev, int64_t out, int64_t in);
+/* The host codecs these arrays come from, on the host's cores (no device, no context): quantize-weight
+ * (src/raster/compiler/backend/cpu/quant.clj:42-70; format Q4_0 or Q8_0, codes n/2 or n bytes, scales n/32),
+ * quantize-weight-q4k (:95-150) and quantize-weight-q6k (:222-262), n elements of f32.  Bit for bit the
+ * reference's double arithmetic.  Returns 1, with the outputs undefined, when w holds an infinity or a NaN. */
+RSTQ_API int32_t rstq_quantize_weight(const float* w, void* codes, float* scales, int64_t n, int32_t format);
+RSTQ_API int32_t rstq_quantize_weight_q4k(const float* w, void* wq, float* da, float* db, int8_t* aq, int8_t* bq,
+                                          int64_t n);
+RSTQ_API int32_t rstq_quantize_weight_q6k(const float* w, void* wq, int8_t* sc, float* ds, int64_t n);
 /* Second device copy of a bound weight at a distinct address (cold-cache measurement). */
 RSTQ_API int32_t rstq_weight_clone(rstq_weight* src, rstq_weight** w);
 RSTQ_API int32_t rstq_weight_free(rstq_weight* w);

@@ -293,11 +293,48 @@ int32_t matmul_device(rstq_ctx* ctx, rstq_weight* w, const void* x, void* y, int
     return launch_gemm(ctx, ds, w, x, nullptr, act_dtype == RSTQ_F32 ? 0 : 1, y, out_dtype, M, x16, rowscale, acc);
 }
 
+// f32 values that a K-quant format holds as products: v[i] = d[i / per] * q[i], formed in double and rounded to
+// f32 once, as the reference forms them.  On the device, from the arrays as they are: the products of a matrix
+// were 4 bytes each through a host array before (4096 x 4096: the Q6_K bind 27 ms, 3 ms now).
+struct ProductScales {
+    const float* d;
+    const int8_t* q;
+    int per;
+};
+__global__ void __launch_bounds__(256)
+product_scales_kernel(const float* __restrict__ d, const int8_t* __restrict__ q, float* __restrict__ v, int64_t n, int per) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        v[i] = (float)((double)d[i / per] * (double)q[i]);
+}
+// dst (device) <- the products of `src` (host), through `tmp` (device, 4 * (n / per) + n bytes and alignment)
+static cudaError_t put_products(rstq_ctx* ctx, DeviceState& ds, const ProductScales& src, float* dst, int64_t n, void* tmp) {
+    const int64_t nd = n / src.per, q_off = (nd * 4 + 255) & ~255ll;
+    float* d = (float*)tmp;
+    int8_t* q = (int8_t*)tmp + q_off;
+    cudaError_t e = cudaMemcpyAsync(d, src.d, (size_t)nd * 4, cudaMemcpyHostToDevice, ds.stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(q, src.q, (size_t)n, cudaMemcpyHostToDevice, ds.stream);
+    if (e != cudaSuccess) return e;
+    int64_t ctas = (n + 255) / 256;
+    if (ctas > (int64_t)ds.sm_count * 8) ctas = (int64_t)ds.sm_count * 8;
+    product_scales_kernel<<<(unsigned)ctas, 256, 0, ds.stream>>>(d, q, dst, n, src.per);
+    ctx->launches++;
+    return cudaGetLastError();
+}
+static int64_t products_tmp_bytes(int64_t n, int per) { return ((n / per * 4 + 255) & ~255ll) + ((n + 255) & ~255ll); }
+static void trim_bind_stage(DeviceState& ds) {
+    if (ds.bind_stage_bytes <= kBindStageKeep) return;
+    cudaFree(ds.bind_stage);
+    ds.bind_stage = nullptr;
+    ds.bind_stage_bytes = 0;
+}
+
+// `products`: the block scales as products (whole matrix, row-major; `scales` is then not read); d == nullptr
+// there: no scales at all (the caller keeps its own beside the codes).
 static int32_t bind_impl(rstq_ctx* ctx, rstq_weight** wout, const void* codes,
                          const float* scales, int dev, int64_t out, int64_t in, int format,
-                         int layout, int split, int rank, int nranks) {
+                         int layout, int split, int rank, int nranks, const ProductScales* products = nullptr) {
     CHECK_CTX(ctx);
-    RSTQ_REQUIRE(wout && codes && scales, RSTQ_E_INVALID, "null argument");
+    RSTQ_REQUIRE(wout && codes && (scales || products), RSTQ_E_INVALID, "null argument");
     *wout = nullptr;
     CHECK_DEV(ctx, dev);
     RSTQ_REQUIRE(format >= RSTQ_FMT_Q4_0 && format <= RSTQ_FMT_Q8_S, RSTQ_E_INVALID,
@@ -341,7 +378,7 @@ static int32_t bind_impl(rstq_ctx* ctx, rstq_weight** wout, const void* codes,
     // K range inside the re-tiling kernel).
     const int64_t code_row_bytes = (int64_t)in * bits / 8;
     const uint8_t* hcodes = (const uint8_t*)codes + row0 * code_row_bytes;
-    const float* hscales = scales + row0 * nb_full;
+    const float* hscales = products ? nullptr : scales + row0 * nb_full;
     const int64_t codes_bytes = sh_out * code_row_bytes;
     const int64_t scales_bytes = sh_out * nb_full * 4;
 
@@ -359,31 +396,34 @@ static int32_t bind_impl(rstq_ctx* ctx, rstq_weight** wout, const void* codes,
     w->data_bytes = (w->outp / 32) * w->nb * unit_bytes(bits);
     w->data = nullptr;
     {
-        float mxs = 0.f;
-        const int64_t ns = sh_out * nb_full;
-        for (int64_t i = 0; i < ns; ++i) {
-            const float a = fabsf(hscales[i]);
-            if (a > mxs && a < 3.0e38f) mxs = a;
-        }
+        const float mxs = products ? 0.f : largest_scale(hscales, sh_out * nb_full);   // (only the tensor-core path reads the exponent)
         int ex = 0;
         if (mxs > 0.f) frexpf(mxs, &ex);       // mxs = f * 2^ex, f in [0.5, 1)
         w->gemm_exp = mxs > 0.f ? 7 - ex : 0;  // largest scaled |weight| = 128 * f * 2^7 < 2^14
     }
-    uint8_t *stage_c = nullptr;
-    float* stage_s = nullptr;
+    // The staging block of both arrays stays with the device up to kBindStageKeep: allocating and freeing
+    // it took as long as the copy of a 10 MB matrix.
+    const int64_t scales_off = (codes_bytes + 255) & ~255ll, tmp_off = scales_off + ((scales_bytes + 255) & ~255ll);
+    const int64_t tmp_bytes = products && products->d ? products_tmp_bytes(sh_out * nb_full, products->per) : 0;
+    if ((rc = dev_reserve(ds, &ds.bind_stage, &ds.bind_stage_bytes, tmp_off + tmp_bytes)) != RSTQ_OK) {
+        delete w;
+        return rc;
+    }
+    uint8_t* stage_c = (uint8_t*)ds.bind_stage;
+    float* stage_s = (float*)(stage_c + scales_off);
     cudaError_t e = cudaMalloc((void**)&w->data, (size_t)w->data_bytes);
-    if (e == cudaSuccess) e = cudaMalloc((void**)&stage_c, (size_t)codes_bytes);
-    if (e == cudaSuccess) e = cudaMalloc((void**)&stage_s, (size_t)scales_bytes);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(stage_c, hcodes, (size_t)codes_bytes, cudaMemcpyHostToDevice, ds.stream);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(stage_s, hscales, (size_t)scales_bytes, cudaMemcpyHostToDevice, ds.stream);
+    if (e == cudaSuccess) {
+        if (!products) e = cudaMemcpyAsync(stage_s, hscales, (size_t)scales_bytes, cudaMemcpyHostToDevice, ds.stream);
+        else if (products->d) e = put_products(ctx, ds, *products, stage_s, sh_out * nb_full, stage_c + tmp_off);
+        else e = cudaMemsetAsync(stage_s, 0, (size_t)scales_bytes, ds.stream);
+    }
     if (e == cudaSuccess) {
         rc = launch_repack(ctx, ds, stage_c, stage_s, w->data, format, layout, sh_out, sh_in, in, kb0);
         if (rc == RSTQ_OK) e = cudaStreamSynchronize(ds.stream);
     }
-    if (stage_c) cudaFree(stage_c);
-    if (stage_s) cudaFree(stage_s);
+    trim_bind_stage(ds);
     if (e != cudaSuccess || rc != RSTQ_OK) {
         if (w->data) cudaFree(w->data);
         delete w;
@@ -509,6 +549,7 @@ int32_t rstq_shutdown(rstq_ctx* ctx) {
         if (ds.attn_scratch) cudaFree(ds.attn_scratch);
         if (ds.kq_scratch) cudaFree(ds.kq_scratch);
         if (ds.f_image) cudaFree(ds.f_image);
+        if (ds.bind_stage) cudaFree(ds.bind_stage);
         if (ds.partials) cudaFree(ds.partials);
         if (ds.counters) cudaFree(ds.counters);
         if (ds.status) cudaFree(ds.status);
@@ -800,25 +841,24 @@ int32_t rstq_weight_bind_q4k(rstq_ctx* ctx, rstq_weight** wout, const void* wq, 
     *wout = nullptr;
     RSTQ_REQUIRE(out >= 1 && in >= 256 && in % 256 == 0, RSTQ_E_SHAPE,
                  "in = %lld must be a positive multiple of 256 and out = %lld >= 1", (long long)in, (long long)out);
-    const int64_t nb = in / 32, n = out * nb;
-    // per-sub-block scale da*aq and min db*bq: the products the reference forms (in double) before
-    // it multiplies by the integer dot and the sub-block sum, rounded to f32 once
-    std::vector<float> a((size_t)n), b((size_t)n);
-    for (int64_t i = 0; i < n; ++i) {
-        a[(size_t)i] = (float)((double)da[i >> 3] * (double)aq[i]);
-        b[(size_t)i] = (float)((double)db[i >> 3] * (double)bq[i]);
-    }
+    const int64_t n = out * (in / 32);
+    const ProductScales a{da, aq, 8}, b{db, bq, 8};   // per sub-block: scale da*aq, minimum db*bq
     rstq_weight* w = nullptr;
-    int32_t rc = bind_impl(ctx, &w, wq, a.data(), dev, out, in, RSTQ_FMT_Q4_0, RSTQ_LAYOUT_ROWMAJOR,
-                           RSTQ_SPLIT_NONE, 0, 1);
+    int32_t rc = bind_impl(ctx, &w, wq, nullptr, dev, out, in, RSTQ_FMT_Q4_0, RSTQ_LAYOUT_ROWMAJOR,
+                           RSTQ_SPLIT_NONE, 0, 1, &a);
     if (rc != RSTQ_OK) return rc;
     w->zp = 0;  // codes are 0 .. 15 as they stand; the offset is the min term
     DeviceState& ds = ctx->devs[dev];
+    if ((rc = dev_reserve(ds, &ds.bind_stage, &ds.bind_stage_bytes, products_tmp_bytes(n, 8))) != RSTQ_OK) {
+        rstq_weight_free(w);
+        return rc;
+    }
     cudaError_t e = cudaMalloc((void**)&w->mins, (size_t)n * 4);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(w->mins, b.data(), (size_t)n * 4, cudaMemcpyHostToDevice, ds.stream);
+    if (e != cudaSuccess) w->mins = nullptr;
+    if (e == cudaSuccess) e = put_products(ctx, ds, b, w->mins, n, ds.bind_stage);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ds.stream);
+    trim_bind_stage(ds);
     if (e != cudaSuccess) {
-        w->mins = nullptr;
         rstq_weight_free(w);
         return cuda_fail(e, "Q4_K bind", __FILE__, __LINE__);
     }
@@ -859,26 +899,27 @@ int32_t rstq_weight_bind_q6k(rstq_ctx* ctx, rstq_weight** wout, const void* wq, 
         // go through the 8-bit repack as they are (with scales that are then dropped), the 2 * nb scales
         // per row ds * sc (the product the reference forms in double, rounded to f32 once) behind them.
         const int64_t n16 = out * (in / 16);
-        std::vector<float> s16((size_t)n16), s32((size_t)(out * nb), 0.0f);
-        for (int64_t o = 0; o < out; ++o)
-            for (int64_t j = 0; j < in / 16; ++j)
-                s16[(size_t)(o * (in / 16) + j)] = (float)((double)dsup[o * nsb + j / 16] * (double)sc[o * (in / 16) + j]);
+        const ProductScales none{nullptr, nullptr, 1}, s16{dsup, sc, 16};
         rstq_weight* w = nullptr;
-        int32_t rc = bind_impl(ctx, &w, q, s32.data(), dev, out, in, RSTQ_FMT_Q8_0, RSTQ_LAYOUT_ROWMAJOR,
-                               RSTQ_SPLIT_NONE, 0, 1);
+        int32_t rc = bind_impl(ctx, &w, q, nullptr, dev, out, in, RSTQ_FMT_Q8_0, RSTQ_LAYOUT_ROWMAJOR,
+                               RSTQ_SPLIT_NONE, 0, 1, &none);
         if (rc != RSTQ_OK) return rc;
         DeviceState& ds = ctx->devs[dev];
+        const int64_t d16_bytes = (n16 * 4 + 255) & ~255ll;
+        if ((rc = dev_reserve(ds, &ds.bind_stage, &ds.bind_stage_bytes, d16_bytes + products_tmp_bytes(n16, 16))) != RSTQ_OK) {
+            rstq_weight_free(w);
+            return rc;
+        }
+        float* d16 = (float*)ds.bind_stage;
         const int64_t kbytes = (w->outp / 32) * w->nb * kUnitBytesQ6K;
         uint8_t* kdata = nullptr;
-        float* d16 = nullptr;
         cudaError_t e = cudaMalloc((void**)&kdata, (size_t)kbytes);
-        if (e == cudaSuccess) e = cudaMalloc((void**)&d16, (size_t)n16 * 4);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(d16, s16.data(), (size_t)n16 * 4, cudaMemcpyHostToDevice, ds.stream);
+        if (e == cudaSuccess) e = put_products(ctx, ds, s16, d16, n16, (char*)ds.bind_stage + d16_bytes);
         if (e == cudaSuccess) {
             rc = launch_q6k_units(ctx, ds, w->data, d16, kdata, out, w->nb);
             if (rc == RSTQ_OK) e = cudaStreamSynchronize(ds.stream);
         }
-        if (d16) cudaFree(d16);
+        trim_bind_stage(ds);
         if (e != cudaSuccess || rc != RSTQ_OK) {
             if (kdata) cudaFree(kdata);
             rstq_weight_free(w);

@@ -105,6 +105,8 @@ struct DeviceState {
     int64_t pinned_bytes = 0;
     void* io_dev = nullptr;        // device staging for the host-array entry points
     int64_t io_dev_bytes = 0;
+    void* bind_stage = nullptr;    // the host arrays of the weight being bound, before they are re-tiled (at most
+    int64_t bind_stage_bytes = 0;  // kBindStageKeep bytes are kept between binds)
     int* status = nullptr;         // device status word: nonzero after a bounded wait ran out
     // Instantiated graphs hold the scratch addresses of the launches they recorded.  While any is
     // alive, scratch that has to grow is parked here instead of freed, so a replay never touches
@@ -115,6 +117,8 @@ struct DeviceState {
     unsigned long long* dbg_store = nullptr;
     mutable uint64_t dbg_launch = 0;        // decode launches recorded so far (picks the timeline slot)
 };
+
+constexpr int64_t kBindStageKeep = 64ll << 20;
 
 }  // namespace rstq
 
@@ -228,6 +232,8 @@ int32_t launch_q6k_prep(rstq_ctx* ctx, DeviceState& ds, const float* xs, const i
 int32_t launch_pair_sum(rstq_ctx* ctx, DeviceState& ds, const float* t, float* y, int64_t M, int64_t out);
 int32_t launch_q4k_min(rstq_ctx* ctx, DeviceState& ds, const float* mins, const float* xs32, const int32_t* bsums,
                        float* y, int64_t M, int64_t nb, int64_t out);
+// codec.cu
+float largest_scale(const float* s, int64_t n);
 // actquant.cu
 constexpr int kGemvMaxM = 16;             // widest token tile of the decode kernels
 // bytes of the decode kernel's image of kGemvMaxM tokens' quantized activations (fragments, then the records)

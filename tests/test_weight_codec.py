@@ -1,0 +1,54 @@
+"""The library's host codecs against the numpy form of the same arithmetic: every byte equal."""
+import numpy as np
+import pytest
+
+from raster_b200 import _lib as L
+from raster_b200.quant import cpu_quant as cq
+
+CODECS = {"q4_0": lambda w: cq.quantize_weight(w, cq.q4_0), "q8_0": lambda w: cq.quantize_weight(w, cq.q8_0),
+          "q4_K": cq.quantize_weight_q4k, "q6_K": cq.quantize_weight_q6k}
+
+
+def values(kind, n):
+    rng = np.random.default_rng(3)
+    w = rng.standard_normal(n).astype(np.float32)
+    if kind == "zeros of both signs":
+        w[: n // 2] = -0.0
+    elif kind == "ties":
+        w = np.round(w * 3) / 2
+    elif kind == "subnormal":
+        w *= np.float32(1e-42)
+    elif kind == "wide range":
+        w *= np.exp(rng.uniform(-80, 80, n))
+    elif kind == "far from zero":
+        w = 1000 + w * np.float32(1e-5)
+    elif kind == "not finite":
+        w[5], w[n // 2] = np.nan, np.inf
+    return w.astype(np.float32)
+
+
+@pytest.mark.parametrize("fmt", sorted(CODECS))
+@pytest.mark.parametrize("kind", ["normal", "zeros of both signs", "ties", "subnormal", "wide range", "far from zero", "not finite"])
+@pytest.mark.parametrize("n", [256, 256 * 515])   # one super-block; several threads with a remainder
+def test_native_codec_gives_the_bytes_of_the_numpy_form(monkeypatch, fmt, kind, n):
+    w = values(kind, n)
+    with np.errstate(all="ignore"):
+        got = CODECS[fmt](w)
+        monkeypatch.setattr(cq, "_native", lambda *a, **k: None)
+        want = CODECS[fmt](w)
+    assert sorted(got) == sorted(want)
+    for k in want:
+        assert got[k].dtype == want[k].dtype and got[k].tobytes() == want[k].tobytes(), k
+    with pytest.raises(ValueError):
+        CODECS[fmt](w[:-1])
+
+
+def test_codec_entry_points_check_their_arguments():
+    lib = L.load()
+    a = np.zeros(256, np.float32)
+    p = a.ctypes.data
+    assert lib.rstq_quantize_weight(None, p, p, 256, L.FMT_Q4_0) == L.E_INVALID
+    assert lib.rstq_quantize_weight(p, p, p, 33, L.FMT_Q4_0) == L.E_SHAPE
+    assert lib.rstq_quantize_weight(p, p, p, 32, L.FMT_Q8_S) == L.E_INVALID
+    assert lib.rstq_quantize_weight_q4k(p, p, p, p, p, p, 128) == L.E_SHAPE
+    assert lib.rstq_quantize_weight_q6k(p, p, p, None, 256) == L.E_INVALID
