@@ -60,6 +60,23 @@ int32_t dev_reserve(DeviceState& ds, void** p, int64_t* have, int64_t need) {
     return RSTQ_OK;
 }
 
+// The same for an operator that callers may record without a first call outside the capture: the allocation
+// does not belong to the capture, and an outgrown block is parked like any that a graph may name.
+int32_t dev_reserve_any_time(DeviceState& ds, void** p, int64_t* have, int64_t need) {
+    if (need <= *have || !ds.capturing) return dev_reserve(ds, p, have, need);
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RSTQ_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+    void* fresh = nullptr;
+    need = (need + 0xFFFFF) & ~0xFFFFFll;
+    const cudaError_t e = cudaMalloc(&fresh, (size_t)need);
+    RSTQ_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+    RSTQ_CUDA(e);
+    if (*p) ds.retired.push_back(*p);
+    *p = fresh;
+    *have = need;
+    return RSTQ_OK;
+}
+
 int32_t dev_release_scratch(DeviceState& ds, void* p) {
     if (!p) return RSTQ_OK;
     if (ds.live_graphs > 0) {   // a recorded launch may still name this block
@@ -508,6 +525,7 @@ int32_t rstq_init(const int32_t* devices, rstq_ctx** ctxp, int32_t ndev) {
             int32_t r = gemv_configure(ds);
             if (r != RSTQ_OK) return r;
             if ((r = gemm_configure(ds)) != RSTQ_OK) return r;
+            if ((r = dx_configure()) != RSTQ_OK) return r;
             RSTQ_CUDA(cudaStreamSynchronize(ds.stream));
             return RSTQ_OK;
         };
@@ -550,6 +568,7 @@ int32_t rstq_shutdown(rstq_ctx* ctx) {
         if (ds.kq_scratch) cudaFree(ds.kq_scratch);
         if (ds.f_image) cudaFree(ds.f_image);
         if (ds.bind_stage) cudaFree(ds.bind_stage);
+        if (ds.dx_scratch) cudaFree(ds.dx_scratch);
         if (ds.partials) cudaFree(ds.partials);
         if (ds.counters) cudaFree(ds.counters);
         if (ds.status) cudaFree(ds.status);

@@ -27,12 +27,11 @@
 //    exponents and store y (f32 or bf16) row-major [token, feature].
 // Every mbarrier wait is time-bounded; on expiry the CTA reports through the
 // status word, drains and still frees its tensor memory.
-#include <cuda.h>
-#include <cuda_fp16.h>
 
 #include "internal.h"
 #include "mma_helpers.cuh"
 #include "sync_helpers.cuh"
+#include "tcgen05_helpers.cuh"
 
 namespace rstq {
 
@@ -41,77 +40,6 @@ constexpr int kGemmThreads = (2 + kDqWarps) * 32;  // TMA warp, MMA warp, 16 deq
 constexpr int kKStep = 128;                        // K elements per pipeline stage (4 blocks)
 constexpr int kAStage = 128 * kKStep * 2;          // 32 KB of fp16 weights per stage
 constexpr int kPrefetch = 4;                       // K-steps of packed weights held in registers
-
-// ---- tcgen05 / TMA wrappers -------------------------------------------------------
-__device__ __forceinline__ void tmem_alloc(uint32_t smem_dst, uint32_t ncols) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_dst),
-                 "r"(ncols)
-                 : "memory");
-}
-__device__ __forceinline__ void tmem_relinquish() {
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
-}
-__device__ __forceinline__ void tc_fence_before() {
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-}
-__device__ __forceinline__ void tc_fence_after() {
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-}
-// D[tmem] (+)= A[smem desc] * B[smem desc]
-__device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                         uint32_t accumulate) {
-    asm volatile(
-        "{ .reg .pred p; setp.ne.b32 p, %4, 0; "
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p; }" ::"r"(d_tmem),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-// mbarrier arrives once all tcgen05.mma issued so far by this thread have completed
-__device__ __forceinline__ void umma_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
-                 : "memory");
-}
-__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-                   "=r"(r[7])
-                 : "r"(taddr));
-}
-__device__ __forceinline__ void tmem_ld_wait() {
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, "
-        "%3}], [%4];" ::"r"(dst),
-        "l"(map), "r"(x), "r"(y), "r"(bar)
-        : "memory");
-}
-__device__ __forceinline__ void sts128(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
-    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
-}
-__device__ __forceinline__ void fence_async_smem() {
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
-
-// Shared-memory matrix descriptor: K-major operand, 128-byte swizzle, rows of 128 bytes
-// (64 fp16), 8-row groups 1024 bytes apart.
-__device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t saddr) {
-    uint64_t d = 0;
-    d |= (uint64_t)((saddr & 0x3FFFF) >> 4);  // start address
-    d |= (uint64_t)1 << 16;                   // leading byte offset (unused with swizzle): 16 B
-    d |= (uint64_t)(1024 >> 4) << 32;         // stride byte offset between 8-row groups
-    d |= (uint64_t)1 << 46;                   // descriptor version of sm_100
-    d |= (uint64_t)2 << 61;                   // SWIZZLE_128B
-    return d;
-}
-// Instruction descriptor of kind::f16: fp16 A and B (both K-major), f32 accumulate, M = 128.
-__host__ __device__ constexpr uint32_t idesc_f16(int n) {
-    return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
-}
 
 // ---- activation pre-pass: x (f32 / bf16 / int8 codes + block scales) -> fp16 * 2^-e(row) ---
 // One CTA per token row.  rowscale[m] = 2^e so that max|x| * 2^-e lies in [2^13, 2^14).
@@ -267,16 +195,6 @@ __device__ __forceinline__ uint32_t scale_h2(float s) {
 // scale s, is exact as well, which makes the result the same bits as subtracting the zero point
 // first (exact integers) and multiplying by s afterwards, in half the instructions.  The caller
 // folds the 2^-24 into the scale.
-__device__ __forceinline__ uint32_t hfma2_u32(uint32_t a, uint32_t b, uint32_t c) {
-    uint32_t d;
-    asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
-    return d;
-}
-__device__ __forceinline__ uint32_t hmul2_u32(uint32_t a, uint32_t b) {
-    uint32_t d;
-    asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-    return d;
-}
 // bytes 0..3 of `bytes` (other bits of each byte pair must be zero) -> four halves v * scale + add
 __device__ __forceinline__ uint2 bytes_fma_h4(uint32_t bytes, uint32_t scale2, uint32_t add2) {
     uint2 r;
@@ -543,24 +461,6 @@ __host__ __device__ constexpr int gemm_issuers(int ntok) { return ntok > 128 ? 1
 constexpr int kAColsPerStage = kKStep / 2;
 constexpr int kWeightPfSteps = 8;  // K-steps of packed weights requested into L2 ahead of the loads
 
-__device__ __forceinline__ void tmem_st_16x256b_x2(uint32_t taddr, const uint32_t (&r)[8]) {
-    asm volatile("tcgen05.st.sync.aligned.16x256b.x2.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr),
-                 "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
-                 : "memory");
-}
-__device__ __forceinline__ void tmem_st_wait() {
-    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-}
-// D[tmem] (+)= A[tmem] * B[smem desc], issued by the lanes whose `leader` is non-zero (one lane).
-// The descriptor comes as two words so that stepping through a stage is one 32-bit add.
-__device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint32_t bdesc_lo, uint32_t bdesc_hi,
-                                            uint32_t idesc, uint32_t accumulate, uint32_t leader) {
-    asm volatile(
-        "{ .reg .pred p, q; .reg .b64 bd; setp.ne.b32 p, %5, 0; setp.ne.b32 q, %6, 0; mov.b64 bd, {%2, %3}; "
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], bd, %4, p; }" ::"r"(d_tmem),
-        "r"(a_tmem), "r"(bdesc_lo), "r"(bdesc_hi), "r"(idesc), "r"(accumulate), "r"(leader)
-        : "memory");
-}
 // One 128-element K-step as a single block of instructions, so that nothing but a branch sits
 // between the last MMA of a step and the first of the next: eight MMAs (A columns a0 + 8 kk, B
 // descriptor b_lo + 2 (kk & 3) + BHALF (kk >> 2) in 16-byte units, BHALF = second 64-element half
@@ -614,14 +514,6 @@ __device__ __forceinline__ uint32_t umma_f16_ts_step(uint32_t d_tmem, uint32_t a
         : "memory");
     return next_ready;
 }
-__device__ __forceinline__ void umma_commit_if(uint32_t bar, uint32_t leader) {
-    asm volatile(
-        "{ .reg .pred q; setp.ne.b32 q, %1, 0; "
-        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0]; }" ::"r"(bar),
-        "r"(leader)
-        : "memory");
-}
-
 template <int BITS>
 struct RawT;
 template <>
@@ -1112,23 +1004,6 @@ gemm_tmem_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tmap) {
 }
 
 // ---- host side --------------------------------------------------------------------------
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
-                                  CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion,
-                                  CUtensorMapFloatOOBfill);
-
-static EncodeTiledFn encode_tiled_fn() {
-    static EncodeTiledFn fn = nullptr;
-    if (!fn) {
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            fn = (EncodeTiledFn)p;
-    }
-    return fn;
-}
-
 template <int BITS, int NTOK>
 static int32_t gemm_attr() {
     if constexpr (NTOK <= 128)
@@ -1151,22 +1026,6 @@ int32_t gemm_configure(DeviceState& ds) {
     if ((rc = gemm_attr<4, 256>()) != RSTQ_OK) return rc;
     if ((rc = gemm_attr<8, 256>()) != RSTQ_OK) return rc;
     return RSTQ_OK;
-}
-
-template <typename K, typename... Args>
-static cudaError_t launch_pdl(K kernel, dim3 grid, dim3 block, size_t smem, const DeviceState& ds,
-                              Args... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = ds.stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = ds.pdl ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
 // x (src 0 = f32, 1 = bf16, 2 = int8 codes with per-block scales xs) -> fp16 rows x16 and 2^e per row

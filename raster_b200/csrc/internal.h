@@ -105,6 +105,8 @@ struct DeviceState {
     int64_t pinned_bytes = 0;
     void* io_dev = nullptr;        // device staging for the host-array entry points
     int64_t io_dev_bytes = 0;
+    void* dx_scratch = nullptr;    // backward-data: its f32 factors as fp16 pairs
+    int64_t dx_scratch_bytes = 0;
     void* bind_stage = nullptr;    // the host arrays of the weight being bound, before they are re-tiled (at most
     int64_t bind_stage_bytes = 0;  // kBindStageKeep bytes are kept between binds)
     int* status = nullptr;         // device status word: nonzero after a bounded wait ran out
@@ -331,6 +333,7 @@ int32_t launch_gemm(rstq_ctx* ctx, DeviceState& ds, const rstq_weight* w, const 
                     float* acc32 = nullptr);
 int32_t gemm_configure(DeviceState& ds);
 // dx.cu
+int32_t dx_configure();  // shared-memory attributes, once per device
 int32_t launch_qlinear_q8_dx(rstq_ctx* ctx, DeviceState& ds, const float* dy, const int8_t* codes,
                              const float* scales, float* dx, int64_t m, int64_t in, int64_t out);
 // capi.cu
@@ -340,6 +343,7 @@ int32_t matmul_device(rstq_ctx* ctx, rstq_weight* w, const void* x, void* y, int
 // capi.cu: grow-only device scratch (refuses to grow during graph capture; the outgrown block is
 // freed at once, or parked until the last live graph of the device is destroyed)
 int32_t dev_reserve(DeviceState& ds, void** p, int64_t* have, int64_t need);
+int32_t dev_reserve_any_time(DeviceState& ds, void** p, int64_t* have, int64_t need);
 int32_t dev_release_scratch(DeviceState& ds, void* p);
 constexpr int64_t kFusedQuantMaxIn = 12288; // longest row the decode kernel quantizes itself (3 passes of 512 threads x 8)
 

@@ -1,0 +1,89 @@
+"""The backward-data GEMM at the edges of its tiles, stages and clusters, against the f64 product."""
+import numpy as np
+import pytest
+
+from raster_b200 import Context
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    c = Context(("cuda:0",))
+    yield c
+    c.close()
+
+
+def run(ctx, m, in_, out, dy, codes, scales):
+    bufs = [ctx.array_to_buffer(a) for a in (dy, codes, scales)] + [ctx.make_buffer(m * in_, np.float32)]
+    bufs[3].fill_bytes(0xFF)
+    ctx.qlinear_q8_dx_device(*bufs, m, in_, out)
+    ctx.sync()
+    dx = bufs[3].download().reshape(m, in_).astype(np.float64)
+    for b in bufs:
+        b.free()
+    return dx
+
+
+def check(ctx, m, in_, out, dy, codes, scales):
+    dx = run(ctx, m, in_, out, dy, codes, scales)
+    w = codes.reshape(out, in_).astype(np.float64) * np.repeat(scales.reshape(out, in_ // 32).astype(np.float64), 32, axis=1)
+    d = dy.reshape(m, out).astype(np.float64)
+    # Per product: two halves of 11 bits each hold a factor to 2^-22 of it, and the product of the two low
+    # halves (2^-22 at most) is left out.  Per sum: 16 products at a time are added to an f32, each addition
+    # off by at most 2^-23 of the sum of magnitudes; up to 8 partial sums and two scalings follow.
+    bound = (3 * 2.0 ** -22 + (out / 16 + 12) * 2.0 ** -23) * (np.abs(d) @ np.abs(w))
+    assert np.all(np.abs(dx - d @ w) <= bound)
+    assert np.abs(dx - d @ w).max() <= 2e-5 * np.abs(d @ w).max() + 1e-300
+
+
+# m: around the 32 / 64 / 128-token tiles; in: one block, a ragged tile of 128 columns; out: one row, ragged
+# groups of 16 and 64 rows, split over 1, 2, 4 and 8 blocks of a cluster
+@pytest.mark.parametrize("m,in_,out", [(1, 32, 1), (3, 96, 15), (15, 160, 65), (32, 128, 64), (33, 128, 200), (64, 288, 1024),
+                                       (65, 256, 1000), (128, 512, 513), (129, 4096, 640), (300, 1056, 2048), (257, 2048, 129),
+                                       (16, 4096, 4096), (20, 96, 9001)])
+def test_dx_at_the_edges(ctx, m, in_, out):
+    rng = np.random.default_rng(m * in_ + out)
+    check(ctx, m, in_, out, rng.standard_normal(m * out).astype(np.float32),
+          rng.integers(-128, 128, out * in_).astype(np.int8),
+          (rng.standard_normal(out * in_ // 32) * 0.01).astype(np.float32))
+
+
+@pytest.mark.parametrize("row,col", [(1e-41, 1.0), (1e30, 1e-30), (1e-20, 1e15), (1e34, 1e-36)])
+def test_dx_keeps_rows_and_column_blocks_of_any_magnitude(ctx, row, col):
+    """A token row and a column block far below the rest keep their own relative precision."""
+    m, in_, out = 40, 256, 320
+    rng = np.random.default_rng(5)
+    dy = (rng.uniform(0.5, 1, (m, out)) * rng.choice([-1, 1], (m, out))).astype(np.float32)
+    dy[7] *= np.float32(row)
+    scales = rng.uniform(0.5, 1, (out, in_ // 32)).astype(np.float32)
+    scales[:, 3] *= np.float32(col)
+    codes = rng.integers(-127, 128, (out, in_)).astype(np.int8)
+    dx = run(ctx, m, in_, out, dy.ravel(), codes.ravel(), scales.ravel())
+    w = codes.astype(np.float64) * np.repeat(scales.astype(np.float64), 32, axis=1)
+    want = dy.astype(np.float64) @ w
+    for rows in (slice(7, 8), slice(8, None)):
+        for cols in (slice(96, 128), slice(128, None)):
+            a, b = dx[rows, cols], want[rows, cols]
+            # 2e-5 as above, and half a step of the subnormal grid of the result
+            assert np.abs(a - b).max() <= 2e-5 * np.abs(b).max() + 1.5e-45 * (1 if np.abs(b).max() < 1e-37 else 0)
+
+
+def test_dx_recorded_without_a_first_call(ctx):
+    m, in_, out = 700, 640, 2560      # more scratch than any call before it
+    rng = np.random.default_rng(9)
+    dy, codes = rng.standard_normal(m * out).astype(np.float32), rng.integers(-127, 128, out * in_).astype(np.int8)
+    scales = np.full(out * in_ // 32, 0.01, np.float32)
+    bufs = [ctx.array_to_buffer(a) for a in (dy, codes, scales)] + [ctx.make_buffer(m * in_, np.float32)]
+    ctx.graph_begin()
+    ctx.qlinear_q8_dx_device(*bufs, m, in_, out)
+    g = ctx.graph_end()
+    g.replay()
+    ctx.sync()
+    got = bufs[3].download()
+    ctx.qlinear_q8_dx_device(*bufs, m, in_, out)
+    ctx.sync()
+    assert np.array_equal(got, bufs[3].download())
+    g.destroy()
+    for b in bufs:
+        b.free()
