@@ -30,6 +30,8 @@
 //    are resident together (one per SM, G <= #SM); every wait -- mbarrier or
 //    hand-over flag -- is time-bounded and reports through a status word
 //    instead of hanging.
+#include <string.h>
+
 #include "internal.h"
 #include "mma_helpers.cuh"
 #include "sync_helpers.cuh"
@@ -122,6 +124,15 @@ struct StreamParams {
     int tp_tail;          // fused exchange: thread blocks that wait for the peers' results and write y (0 = all)
     TpFuse tp;            // tp.nranks == 0: no exchange, results go to y
 };
+
+// One token from a host array: the f32 activations travel in the launch's own parameters (of which a kernel takes
+// 32 764 bytes) and every thread block quantizes them from there -- no copy, no second launch and no read over PCIe.
+template <int N>
+struct StreamParamsX : StreamParams {
+    float xv[N];
+};
+constexpr int kParamXSmall = 4096, kParamXLarge = kParamXMax;
+static_assert(sizeof(StreamParamsX<kParamXLarge>) <= 32764, "kernel parameter limit");
 
 __device__ __forceinline__ void consumer_bar() {
     asm volatile("bar.sync 1, %0;" ::"n"(kConsumers) : "memory");
@@ -299,11 +310,18 @@ __device__ __forceinline__ int quant_exact(float x, double id) {
     const int q = (int)f + ((v - f) >= 0.5 ? 1 : 0);
     return max(-127, min(127, q));
 }
-template <int BITS>
-__device__ __forceinline__ void stage_a8_quant(const StreamParams& p, uint8_t* smem, int tid) {
+// PARAM: x lies in the parameter block.  Its lanes read different words, which the constant path would serve one
+// address at a time; through the generic address they are ordinary cached loads.
+__device__ __forceinline__ uint4 ldgen_u4(const void* p) {
+    uint4 v;
+    asm volatile("ld.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+template <int BITS, bool PARAM>
+__device__ __forceinline__ void stage_a8_quant(const StreamParams& p, const void* x, uint8_t* smem, int tid) {
     uint4* srec = reinterpret_cast<uint4*>(smem + p.act_off);
     const int items = p.nb * 4;   // a multiple of 4: the lanes of a block are active together
-    const bool bf = p.act_dtype == RSTQ_BF16;
+    const bool bf = !PARAM && p.act_dtype == RSTQ_BF16;
     // every load of the thread is issued before the first use (one trip to L2, not one per pass):
     // kQuantPasses passes of kConsumers items cover in <= kQuantMaxIn
     uint4 raw[kQuantPasses][2];
@@ -314,14 +332,14 @@ __device__ __forceinline__ void stage_a8_quant(const StreamParams& p, uint8_t* s
         if (i < items) {
             const int b = i >> 2, tg = i & 3;
             if (bf) {
-                const uint16_t* xb = reinterpret_cast<const uint16_t*>(p.x) + b * 32 + tg * 4;
+                const uint16_t* xb = reinterpret_cast<const uint16_t*>(x) + b * 32 + tg * 4;
                 const uint2 lo = *reinterpret_cast<const uint2*>(xb), hi = *reinterpret_cast<const uint2*>(xb + 16);
                 raw[it][0] = make_uint4(lo.x << 16, lo.x & 0xFFFF0000u, lo.y << 16, lo.y & 0xFFFF0000u);
                 raw[it][1] = make_uint4(hi.x << 16, hi.x & 0xFFFF0000u, hi.y << 16, hi.y & 0xFFFF0000u);
             } else {
-                const uint4* xf = reinterpret_cast<const uint4*>(reinterpret_cast<const float*>(p.x) + b * 32 + tg * 4);
-                raw[it][0] = xf[0];
-                raw[it][1] = xf[4];
+                const uint4* xf = reinterpret_cast<const uint4*>(reinterpret_cast<const float*>(x) + b * 32 + tg * 4);
+                raw[it][0] = PARAM ? ldgen_u4(xf) : xf[0];
+                raw[it][1] = PARAM ? ldgen_u4(xf + 4) : xf[4];
             }
         }
     }
@@ -831,8 +849,9 @@ __device__ __forceinline__ float stream_reduce_rc(const float* red, int row, int
 
 // ---- the kernel ---------------------------------------------------------------------
 // QF: M == 1 only, the kernel quantizes the raw activations p.x itself while staging.
-template <int BITS, int NT, int MODE, bool ONECOL, bool TP, bool QF = false, int UK = 0>
-__global__ void __launch_bounds__(kStreamThreads, 1) gemv_stream_kernel(const StreamParams p) {
+// P: StreamParams, or StreamParamsX with the raw activations inside.
+template <int BITS, int NT, int MODE, bool ONECOL, bool TP, bool QF = false, int UK = 0, typename P = StreamParams>
+__global__ void __launch_bounds__(kStreamThreads, 1) gemv_stream_kernel(const __grid_constant__ P p) {
     constexpr int UNIT = BITS == 4 ? (UK == 1 ? kUnitBytesQ4K : kUnitBytesQ4) : (UK == 2 ? kUnitBytesQ6K : kUnitBytesQ8);
     constexpr int REC = UK == 2 ? 32 : 16;   // bytes of a staged (block, tig) record at M = 1
     constexpr int kUPW = upw_of(BITS), kChunkUnits = chunk_units_of(BITS);
@@ -1062,8 +1081,10 @@ __global__ void __launch_bounds__(kStreamThreads, 1) gemv_stream_kernel(const St
                                  : "memory");
         }
     };
-    if (QF) {
-        stage_a8_quant<BITS>(p, smem, tid);
+    if constexpr (sizeof(P) > sizeof(StreamParams)) {
+        stage_a8_quant<BITS, true>(p, p.xv, smem, tid);
+    } else if (QF) {
+        stage_a8_quant<BITS, false>(p, p.x, smem, tid);
     } else if (MODE == MODE_A8) {
         if (!ONECOL && p.ring) {
             // the slices arrive with the weight chunks
@@ -1639,6 +1660,11 @@ int32_t gemv_configure(DeviceState& ds) {
     if ((rc = set_stream_attr(gemv_stream_kernel<4, 1, MODE_A8, true, true, true>)) != RSTQ_OK) return rc;
     if ((rc = set_stream_attr(gemv_stream_kernel<8, 1, MODE_A8, true, false, true>)) != RSTQ_OK) return rc;
     if ((rc = set_stream_attr(gemv_stream_kernel<8, 1, MODE_A8, true, true, true>)) != RSTQ_OK) return rc;
+    // ... and its activations among the parameters
+    if ((rc = set_stream_attr(gemv_stream_kernel<4, 1, MODE_A8, true, false, true, 0, StreamParamsX<kParamXSmall>>)) != RSTQ_OK) return rc;
+    if ((rc = set_stream_attr(gemv_stream_kernel<4, 1, MODE_A8, true, false, true, 0, StreamParamsX<kParamXLarge>>)) != RSTQ_OK) return rc;
+    if ((rc = set_stream_attr(gemv_stream_kernel<8, 1, MODE_A8, true, false, true, 0, StreamParamsX<kParamXSmall>>)) != RSTQ_OK) return rc;
+    if ((rc = set_stream_attr(gemv_stream_kernel<8, 1, MODE_A8, true, false, true, 0, StreamParamsX<kParamXLarge>>)) != RSTQ_OK) return rc;
     // Q4_K units (minima inside)
     if ((rc = set_stream_attr(gemv_stream_kernel<4, 1, MODE_A8, true, false, false, 1>)) != RSTQ_OK) return rc;
     if ((rc = set_stream_attr(gemv_stream_kernel<4, 1, MODE_A8, false, false, false, 1>)) != RSTQ_OK) return rc;
@@ -1695,9 +1721,8 @@ static void fill_next(StreamParams& p, const DeviceState& ds, const NextWeight& 
     p.nx_pf_units = per_cta < 1 ? 1 : per_cta;
 }
 
-template <typename K>
-static cudaError_t launch_stream(K kernel, const DeviceState& ds, const StreamPlan& pl,
-                                 const StreamParams& p) {
+template <typename K, typename P>
+static cudaError_t launch_stream(K kernel, const DeviceState& ds, const StreamPlan& pl, const P& p) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)pl.G);
     cfg.blockDim = dim3(kStreamThreads);
@@ -1709,6 +1734,14 @@ static cudaError_t launch_stream(K kernel, const DeviceState& ds, const StreamPl
     cfg.attrs = attr;
     cfg.numAttrs = ds.pdl ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, p);
+}
+
+template <int BITS, int N>
+static cudaError_t launch_stream_x(const DeviceState& ds, const StreamPlan& pl, const StreamParams& p, const float* x) {
+    StreamParamsX<N> px;
+    static_cast<StreamParams&>(px) = p;
+    memcpy(px.xv, x, (size_t)p.in * 4);
+    return launch_stream(gemv_stream_kernel<BITS, 1, MODE_A8, true, false, true, 0, StreamParamsX<N>>, ds, pl, px);
 }
 
 // Largest token count <= want whose staged activations fit next to a ring of >= 2 chunks.
@@ -1820,7 +1853,7 @@ int32_t launch_gemv_a8(rstq_ctx* ctx, DeviceState& ds, const GemvA8Args& a) {
     const bool k6 = a.uk == 2;
     // unit kind for the size helpers: Q4_K units carry 128 more bytes than 4-bit ones, Q6_K units 128 more than 8-bit ones
     const int ukind = a.uk == 1 ? 5 : (k6 ? 6 : a.bits);
-    RSTQ_REQUIRE(a.uk == 0 || (a.bits == (k6 ? 8 : 4) && !a.tp && !a.x), RSTQ_E_INVALID,
+    RSTQ_REQUIRE(a.uk == 0 || (a.bits == (k6 ? 8 : 4) && !a.tp && !a.x && !a.x_host), RSTQ_E_INVALID,
                  "K-quant units: one device, pre-quantized activations");
     for (int64_t m0 = 0; m0 < a.M;) {
         const int want = (int)(a.M - m0 < kGemvMaxM ? a.M - m0 : kGemvMaxM);
@@ -1841,7 +1874,8 @@ int32_t launch_gemv_a8(rstq_ctx* ctx, DeviceState& ds, const GemvA8Args& a) {
         RSTQ_REQUIRE(M >= 1, RSTQ_E_LIMIT, "in = %lld: one row of activations exceeds shared memory",
                      (long long)a.in);
         if (a.tp && (M < a.M || a.out % 4 != 0)) return kNotFused;  // the exchange fuses into ONE launch
-        const bool qf = a.x != nullptr;
+        const bool qf = a.x != nullptr || a.x_host != nullptr;
+        RSTQ_REQUIRE(!a.x_host || (a.in <= kParamXMax && !a.tp && a.uk == 0), RSTQ_E_INVALID, "activations as parameters: in <= %d", kParamXMax);
         RSTQ_REQUIRE(!qf || (a.M == 1 && a.in <= kQuantMaxIn), RSTQ_E_INVALID,
                      "the in-kernel quantizer serves M = 1 and in <= %d", kQuantMaxIn);
         int32_t rc = stream_scratch_ok(ds, groups, pl.G, M);
@@ -1879,7 +1913,10 @@ int32_t launch_gemv_a8(rstq_ctx* ctx, DeviceState& ds, const GemvA8Args& a) {
               : launch_stream(gemv_stream_kernel<__VA_ARGS__, false>, ds, pl, p)
 #define LAUNCH1(B)                                                                                       \
     do {                                                                                                 \
-        if (a.tp) le = qf ? launch_stream(gemv_stream_kernel<B, 1, MODE_A8, true, true, true>, ds, pl, p)  \
+        if (a.x_host)                                                                                    \
+            le = a.in <= kParamXSmall ? launch_stream_x<B, kParamXSmall>(ds, pl, p, a.x_host)            \
+                                      : launch_stream_x<B, kParamXLarge>(ds, pl, p, a.x_host);           \
+        else if (a.tp) le = qf ? launch_stream(gemv_stream_kernel<B, 1, MODE_A8, true, true, true>, ds, pl, p)  \
                           : launch_stream(gemv_stream_kernel<B, 1, MODE_A8, true, true, false>, ds, pl, p);\
         else le = qf ? launch_stream(gemv_stream_kernel<B, 1, MODE_A8, true, false, true>, ds, pl, p)      \
                      : launch_stream(gemv_stream_kernel<B, 1, MODE_A8, true, false, false>, ds, pl, p);    \

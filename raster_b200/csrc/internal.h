@@ -84,6 +84,7 @@ struct DeviceState {
     int tp_tail_ctas = 32;         // fused exchange: fewest thread blocks of the decode kernel that stay for the exchange's tail (0 = all)
     int act_ring = 0;              // MODE_A8, M > 1: 0 = the plan with most weight bytes in flight, 1 = activations resident + full chunks, 2 / 3 = activations ride the ring (full / half chunks), 4 = resident + half chunks
     bool act_image = true;         // MODE_A8, 2 <= M <= 16: the quantizer also writes the decode kernel's staged form, taken by bulk copy
+    const float* x_params = nullptr;   // the current host-array call hands x (host memory) to the decode kernel as parameters
     bool x_on_host = false;        // the current host-array call lets its first kernel read x from pinned host memory
     bool fuse_quant = true;        // M = 1 operator: quantize the activations inside the decode kernel
     // scratch owned by the context
@@ -296,6 +297,7 @@ struct GemvA8Args {
     int64_t M, in, out;   // y is [M, out] f32
     int bits, zp;
     const TpFuse* tp = nullptr;
+    const float* x_host = nullptr;   // M == 1, in <= kParamXMax: the same from a host array, passed to the kernel by value
     const void* x = nullptr;     // M == 1 only: raw activations (f32 or bf16), quantized by the kernel
     int act_dtype = RSTQ_F32;    // itself while staging; xq / xs / xsum are then not read
     NextWeight next;
@@ -345,6 +347,7 @@ int32_t matmul_device(rstq_ctx* ctx, rstq_weight* w, const void* x, void* y, int
 int32_t dev_reserve(DeviceState& ds, void** p, int64_t* have, int64_t need);
 int32_t dev_reserve_any_time(DeviceState& ds, void** p, int64_t* have, int64_t need);
 int32_t dev_release_scratch(DeviceState& ds, void* p);
+constexpr int kParamXMax = 7936;            // longest row of f32 activations that fits a launch's parameters beside the rest
 constexpr int64_t kFusedQuantMaxIn = 12288; // longest row the decode kernel quantizes itself (3 passes of 512 threads x 8)
 
 }  // namespace rstq

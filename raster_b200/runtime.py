@@ -427,6 +427,9 @@ _default_lock = threading.Lock()
 def default_context() -> Context:
     """The process-wide context the reference-named operators run on (cuda:0)."""
     global _default
+    ctx = _default
+    if ctx is not None:
+        return ctx
     with _default_lock:
         if _default is None:
             _default = Context(("cuda:0",))
