@@ -221,6 +221,19 @@ static int32_t gemm_scratch(DeviceState& ds, int64_t M, int64_t in, int64_t out,
     return RSTQ_OK;
 }
 
+// One token of a K-quant: the decode kernel quantizes the activations itself, as for the plain formats (7B-class
+// MLP, Q4_K + Q6_K: 22.5 us for its two calls with a quantizer launch each).  From 1 MB of weights up; smaller
+// matrices keep the quantizer and the decode kernel as two launches.
+static bool kquant_fuses(const DeviceState& ds, const rstq_weight* w, int64_t M) {
+    return M == 1 && ds.fuse_quant && !ds.x_on_host && w->in <= kFusedQuantMaxIn && w->data_bytes >= (1ll << 20);
+}
+static int32_t run_kquant_fused(rstq_ctx* ctx, DeviceState& ds, rstq_weight* w, const void* x, void* y) {
+    GemvA8Args a{w->data, nullptr, nullptr, nullptr, (float*)y, 1, w->in, w->out, w->bits, w->zp, nullptr, nullptr, x, RSTQ_F32};
+    a.uk = w->kq ? 1 : 2;
+    a.next = note_decode_launch(ctx, ds, w);
+    return launch_gemv_a8(ctx, ds, a);
+}
+
 int32_t matmul_device(rstq_ctx* ctx, rstq_weight* w, const void* x, void* y, int64_t M, int act_dtype,
                       int out_dtype, int mode, const TpFuse* tp) {
     DeviceState& ds = ctx->devs[w->dev];
@@ -230,6 +243,7 @@ int32_t matmul_device(rstq_ctx* ctx, rstq_weight* w, const void* x, void* y, int
         RSTQ_REQUIRE(mode == RSTQ_MODE_A8 && act_dtype == RSTQ_F32 && out_dtype == RSTQ_F32, RSTQ_E_INVALID,
                      "a Q6_K weight takes f32 activations in MODE_A8 and writes f32");
         if (tp) return kNotFused;   // the exchange is fused into the per-32-block kernels only
+        if (w->k6 && kquant_fuses(ds, w, M)) return run_kquant_fused(ctx, ds, w, x, y);
         ActScratch s;
         int32_t rc = act_scratch(ds, M, w->in, &s);
         if (rc != RSTQ_OK) return rc;
@@ -251,6 +265,7 @@ int32_t matmul_device(rstq_ctx* ctx, rstq_weight* w, const void* x, void* y, int
         RSTQ_REQUIRE(mode == RSTQ_MODE_A8 && act_dtype == RSTQ_F32 && out_dtype == RSTQ_F32, RSTQ_E_INVALID,
                      "a Q4_K weight takes f32 activations in MODE_A8 and writes f32");
         if (tp) return kNotFused;
+        if (w->kq && kquant_fuses(ds, w, M)) return run_kquant_fused(ctx, ds, w, x, y);
         ActScratch s;
         int32_t rc = act_scratch(ds, M, w->in, &s);
         if (rc != RSTQ_OK) return rc;

@@ -317,7 +317,10 @@ __device__ __forceinline__ uint4 ldgen_u4(const void* p) {
     asm volatile("ld.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
     return v;
 }
-template <int BITS, bool PARAM>
+// K-quant units (UK 1, 2): the same with the scale taken per 256-element super-block (quantize-act-q8k, quant.clj:172-193).
+// A super-block is 8 blocks x 4 threads: exactly a warp, so its maximum is five shuffles; nb is a multiple of 8.
+// Records as stage_a8 lays them out: Q4_K t = xs * code sum, Q6_K a constant per half of the block.
+template <int BITS, bool PARAM, int UK = 0>
 __device__ __forceinline__ void stage_a8_quant(const StreamParams& p, const void* x, uint8_t* smem, int tid) {
     uint4* srec = reinterpret_cast<uint4*>(smem + p.act_off);
     const int items = p.nb * 4;   // a multiple of 4: the lanes of a block are active together
@@ -356,6 +359,11 @@ __device__ __forceinline__ void stage_a8_quant(const StreamParams& p, const void
         for (int k = 0; k < 8; ++k) mx = fmaxf(mx, fabsf(f[k]));
         mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
         mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+        if (UK != 0) {
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
+        }
         // f32 shortcut: u = fma(x, 127 / max, 1.5 * 2^23) holds round-to-nearest(x * 127 / max) in its low
         // mantissa bits (two's complement in the low byte); the quotient is 2 ulp accurate, so the
         // product is within 4e-5 of the double one and every element whose remainder is further than
@@ -392,6 +400,18 @@ __device__ __forceinline__ void stage_a8_quant(const StreamParams& p, const void
             wb = (uint32_t)(q[4] & 0xFF) | ((uint32_t)(q[5] & 0xFF) << 8) | ((uint32_t)(q[6] & 0xFF) << 16) |
                  ((uint32_t)(q[7] & 0xFF) << 24);
         }
+        if (UK == 2) {   // sums of elements 0 .. 15 and 16 .. 31
+            int sa = __dp4a((int)wa, 0x01010101, 0), sb = __dp4a((int)wb, 0x01010101, 0);
+            sa += __shfl_xor_sync(0xffffffffu, sa, 1);
+            sb += __shfl_xor_sync(0xffffffffu, sb, 1);
+            sa += __shfl_xor_sync(0xffffffffu, sa, 2);
+            sb += __shfl_xor_sync(0xffffffffu, sb, 2);
+            if (act) {
+                srec[2 * i] = make_uint4(wa, wb, __float_as_uint(xs), (uint32_t)(kMagicInt - p.zp * sa));
+                srec[2 * i + 1] = make_uint4((uint32_t)(kMagicInt - p.zp * sb), 0u, 0u, 0u);
+            }
+            continue;
+        }
         sum = __dp4a((int)wa, 0x01010101, __dp4a((int)wb, 0x01010101, 0));
         sum += __shfl_xor_sync(0xffffffffu, sum, 1);
         sum += __shfl_xor_sync(0xffffffffu, sum, 2);
@@ -401,7 +421,7 @@ __device__ __forceinline__ void stage_a8_quant(const StreamParams& p, const void
             r.x = wa;
             r.y = wb;
             r.z = __float_as_uint(hi ? xs * 0.0625f : xs);
-            r.w = (uint32_t)(kMagicInt - (p.zp * sum) * (hi ? 16 : 1));
+            r.w = UK == 1 ? __float_as_uint(xs * (float)sum) : (uint32_t)(kMagicInt - (p.zp * sum) * (hi ? 16 : 1));
             srec[i] = r;
         }
     }
@@ -1084,7 +1104,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) gemv_stream_kernel(const __
     if constexpr (sizeof(P) > sizeof(StreamParams)) {
         stage_a8_quant<BITS, true>(p, p.xv, smem, tid);
     } else if (QF) {
-        stage_a8_quant<BITS, false>(p, p.x, smem, tid);
+        stage_a8_quant<BITS, false, UK>(p, p.x, smem, tid);
     } else if (MODE == MODE_A8) {
         if (!ONECOL && p.ring) {
             // the slices arrive with the weight chunks
@@ -1667,10 +1687,12 @@ int32_t gemv_configure(DeviceState& ds) {
     if ((rc = set_stream_attr(gemv_stream_kernel<8, 1, MODE_A8, true, false, true, 0, StreamParamsX<kParamXLarge>>)) != RSTQ_OK) return rc;
     // Q4_K units (minima inside)
     if ((rc = set_stream_attr(gemv_stream_kernel<4, 1, MODE_A8, true, false, false, 1>)) != RSTQ_OK) return rc;
+    if ((rc = set_stream_attr(gemv_stream_kernel<4, 1, MODE_A8, true, false, true, 1>)) != RSTQ_OK) return rc;
     if ((rc = set_stream_attr(gemv_stream_kernel<4, 1, MODE_A8, false, false, false, 1>)) != RSTQ_OK) return rc;
     if ((rc = set_stream_attr(gemv_stream_kernel<4, 2, MODE_A8, false, false, false, 1>)) != RSTQ_OK) return rc;
     // Q6_K units (8-bit codes, a scale per 16 elements)
     if ((rc = set_stream_attr(gemv_stream_kernel<8, 1, MODE_A8, true, false, false, 2>)) != RSTQ_OK) return rc;
+    if ((rc = set_stream_attr(gemv_stream_kernel<8, 1, MODE_A8, true, false, true, 2>)) != RSTQ_OK) return rc;
     if ((rc = set_stream_attr(gemv_stream_kernel<8, 1, MODE_A8, false, false, false, 2>)) != RSTQ_OK) return rc;
     if ((rc = set_stream_attr(gemv_stream_kernel<8, 2, MODE_A8, false, false, false, 2>)) != RSTQ_OK) return rc;
     return RSTQ_OK;
@@ -1853,8 +1875,8 @@ int32_t launch_gemv_a8(rstq_ctx* ctx, DeviceState& ds, const GemvA8Args& a) {
     const bool k6 = a.uk == 2;
     // unit kind for the size helpers: Q4_K units carry 128 more bytes than 4-bit ones, Q6_K units 128 more than 8-bit ones
     const int ukind = a.uk == 1 ? 5 : (k6 ? 6 : a.bits);
-    RSTQ_REQUIRE(a.uk == 0 || (a.bits == (k6 ? 8 : 4) && !a.tp && !a.x && !a.x_host), RSTQ_E_INVALID,
-                 "K-quant units: one device, pre-quantized activations");
+    RSTQ_REQUIRE(a.uk == 0 || (a.bits == (k6 ? 8 : 4) && !a.tp && !a.x_host), RSTQ_E_INVALID,
+                 "K-quant units: one device");
     for (int64_t m0 = 0; m0 < a.M;) {
         const int want = (int)(a.M - m0 < kGemvMaxM ? a.M - m0 : kGemvMaxM);
         StreamPlan pl;
@@ -1923,11 +1945,13 @@ int32_t launch_gemv_a8(rstq_ctx* ctx, DeviceState& ds, const GemvA8Args& a) {
     } while (0)
         if (k6) {
             if (NT == 2) le = launch_stream(gemv_stream_kernel<8, 2, MODE_A8, false, false, false, 2>, ds, pl, p);
-            else if (M == 1 && !pl.ring) le = launch_stream(gemv_stream_kernel<8, 1, MODE_A8, true, false, false, 2>, ds, pl, p);
+            else if (M == 1 && !pl.ring) le = qf ? launch_stream(gemv_stream_kernel<8, 1, MODE_A8, true, false, true, 2>, ds, pl, p)
+                                                 : launch_stream(gemv_stream_kernel<8, 1, MODE_A8, true, false, false, 2>, ds, pl, p);
             else le = launch_stream(gemv_stream_kernel<8, 1, MODE_A8, false, false, false, 2>, ds, pl, p);
         } else if (a.uk == 1) {
             if (NT == 2) le = launch_stream(gemv_stream_kernel<4, 2, MODE_A8, false, false, false, 1>, ds, pl, p);
-            else if (M == 1 && !pl.ring) le = launch_stream(gemv_stream_kernel<4, 1, MODE_A8, true, false, false, 1>, ds, pl, p);
+            else if (M == 1 && !pl.ring) le = qf ? launch_stream(gemv_stream_kernel<4, 1, MODE_A8, true, false, true, 1>, ds, pl, p)
+                                                 : launch_stream(gemv_stream_kernel<4, 1, MODE_A8, true, false, false, 1>, ds, pl, p);
             else le = launch_stream(gemv_stream_kernel<4, 1, MODE_A8, false, false, false, 1>, ds, pl, p);
         } else if (a.bits == 4) {
             if (NT == 2) LAUNCH(4, 2, MODE_A8, false);
