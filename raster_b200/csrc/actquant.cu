@@ -8,13 +8,9 @@
 // The scale and the rounding are carried in double so the codes are bit-exact
 // with the JVM's (Java Math.round = nearest, ties toward +infinity).
 #include "internal.h"
+#include "quant_helpers.cuh"
 
 namespace rstq {
-
-__device__ __forceinline__ int round_half_up(double v) {
-    double f = floor(v);
-    return (int)f + ((v - f) >= 0.5 ? 1 : 0);
-}
 
 // One warp per block; lane k owns element k.  Bytes are gathered so that each
 // of eight lanes stores one 32-bit word.
@@ -35,16 +31,9 @@ quant_act_i8_kernel(const void* __restrict__ xv, int8_t* __restrict__ xq, float*
     for (int64_t blk = warp; blk < nblocks; blk += nwarps) {
         const float v = BF16IN ? __uint_as_float((uint32_t)reinterpret_cast<const uint16_t*>(xv)[blk * 32 + lane] << 16)
                                : reinterpret_cast<const float*>(xv)[blk * 32 + lane];
-        float mx = fabsf(v);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        const double d = (double)mx / 127.0;
-        const double id = d == 0.0 ? 0.0 : 1.0 / d;
-        int q = round_half_up((double)v * id);
-        q = max(-127, min(127, q));
-        int s = q;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        int q, s;
+        float scale;
+        quant_block32(v, &q, &s, &scale);
         // pack four neighbouring codes into the word lane (lane & ~3) stores
         uint32_t b = (uint32_t)(q & 0xFF);
         uint32_t w = b << (8 * (lane & 3));
@@ -52,7 +41,7 @@ quant_act_i8_kernel(const void* __restrict__ xv, int8_t* __restrict__ xq, float*
         w |= __shfl_xor_sync(0xffffffffu, w, 2);
         if ((lane & 3) == 0) reinterpret_cast<uint32_t*>(xq)[blk * 8 + (lane >> 2)] = w;
         if (lane == 0) {
-            xs[blk] = (float)d;
+            xs[blk] = scale;
             if (xsum) xsum[blk] = s;
         }
         if (img) {
@@ -69,7 +58,7 @@ quant_act_i8_kernel(const void* __restrict__ xv, int8_t* __restrict__ xq, float*
                 reinterpret_cast<uint32_t*>(im)[((int64_t)(b * Mp + c) * 4 + (j & 3)) * 2 + (j >> 2)] = w;
             const int Mz = (Mp + 1) & ~1;
             uint8_t* recs = im + (((int64_t)nb * Mp * 32 + 127) & ~127ll);
-            if (lane == 0) put_act_record(recs, b, Mz, c, (float)d, zp * s, four_bit);
+            if (lane == 0) put_act_record(recs, b, Mz, c, scale, zp * s, four_bit);
             if (lane == 1 && c == Mp - 1 && Mz > Mp) put_act_record(recs, b, Mz, Mp, 0.f, 0, four_bit);
         }
     }

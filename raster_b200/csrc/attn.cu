@@ -18,6 +18,7 @@
 // warp step); every other head_dim % 4 == 0 up to 256 takes the general gqa_decode_kernel (a
 // warp per position).
 #include "internal.h"
+#include "quant_helpers.cuh"
 
 namespace rstq {
 
@@ -105,11 +106,6 @@ struct AttnParams {
     int32_t* xsum;
 };
 
-__device__ __forceinline__ int attn_round_half_up(double v) {
-    const double f = floor(v);
-    return (int)f + ((v - f) >= 0.5 ? 1 : 0);
-}
-
 // Second half of both attention kernels: the per-warp states in shared memory ([warps][gc][row]:
 // weighted V, max, sum) are merged per CTA, then per KV head across the slices of the cache.
 // GS = query heads per CTA (the stride of the scratch).
@@ -118,23 +114,16 @@ __device__ __forceinline__ int attn_round_half_up(double v) {
 __device__ __forceinline__ void attn_store(const AttnParams& p, int64_t e, float v, int lane) {
     p.out[e] = v;
     if (p.xq) {
-        float mx = fabsf(v);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        const double dq = (double)mx / 127.0;
-        const double id = dq == 0.0 ? 0.0 : 1.0 / dq;
-        int q = attn_round_half_up((double)v * id);
-        q = max(-127, min(127, q));
-        int sm = q;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) sm += __shfl_xor_sync(0xffffffffu, sm, o);
+        int q, sm;
+        float scale;
+        quant_block32(v, &q, &sm, &scale);
         uint32_t word = (uint32_t)(q & 0xFF) << (8 * (lane & 3));
         word |= __shfl_xor_sync(0xffffffffu, word, 1);
         word |= __shfl_xor_sync(0xffffffffu, word, 2);
         const int64_t blk = e >> 5;
         if ((lane & 3) == 0) reinterpret_cast<uint32_t*>(p.xq)[blk * 8 + (lane >> 2)] = word;
         if (lane == 0) {
-            p.xs[blk] = (float)dq;
+            p.xs[blk] = scale;
             if (p.xsum) p.xsum[blk] = sm;
         }
     }

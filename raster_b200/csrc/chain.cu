@@ -9,15 +9,11 @@
 // kernel (the normalized row never goes to memory; codes, scales and block sums are exactly what
 // quant_act_i8_kernel would produce from rms_norm's f32 output).
 #include "internal.h"
+#include "quant_helpers.cuh"
 
 namespace rstq {
 
 constexpr int kRowThreads = 1024;
-
-__device__ __forceinline__ int chain_round_half_up(double v) {
-    const double f = floor(v);
-    return (int)f + ((v - f) >= 0.5 ? 1 : 0);
-}
 
 // sum over the CTA; every thread gets the result
 __device__ __forceinline__ float cta_sum(float v, float* s_red) {
@@ -45,22 +41,15 @@ constexpr int kRowKeep = 8;
 
 __device__ __forceinline__ void quant_block_store(float v, int lane, int64_t blk, int8_t* __restrict__ xq,
                                                   float* __restrict__ xs, int32_t* __restrict__ xsum) {
-    float mx = fabsf(v);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    const double d = (double)mx / 127.0;
-    const double id = d == 0.0 ? 0.0 : 1.0 / d;
-    int q = chain_round_half_up((double)v * id);
-    q = max(-127, min(127, q));
-    int s = q;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    int q, s;
+    float scale;
+    quant_block32(v, &q, &s, &scale);
     uint32_t word = (uint32_t)(q & 0xFF) << (8 * (lane & 3));
     word |= __shfl_xor_sync(0xffffffffu, word, 1);
     word |= __shfl_xor_sync(0xffffffffu, word, 2);
     if ((lane & 3) == 0) reinterpret_cast<uint32_t*>(xq)[blk * 8 + (lane >> 2)] = word;
     if (lane == 0) {
-        xs[blk] = (float)d;
+        xs[blk] = scale;
         if (xsum) xsum[blk] = s;
     }
 }
@@ -157,24 +146,7 @@ gated_quant_kernel(const float* __restrict__ gate, const float* __restrict__ up,
         float v;
         if (OP == 0) v = g * (1.0f / (1.0f + expf(-g))) * u;
         else v = 0.5f * g * (1.0f + tanhf(0.7978845608028654f * (g + 0.044715f * g * g * g))) * u;
-        float mx = fabsf(v);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        const double d = (double)mx / 127.0;
-        const double id = d == 0.0 ? 0.0 : 1.0 / d;
-        int q = chain_round_half_up((double)v * id);
-        q = max(-127, min(127, q));
-        int sm = q;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) sm += __shfl_xor_sync(0xffffffffu, sm, o);
-        uint32_t word = (uint32_t)(q & 0xFF) << (8 * (lane & 3));
-        word |= __shfl_xor_sync(0xffffffffu, word, 1);
-        word |= __shfl_xor_sync(0xffffffffu, word, 2);
-        if ((lane & 3) == 0) reinterpret_cast<uint32_t*>(xq)[blk * 8 + (lane >> 2)] = word;
-        if (lane == 0) {
-            xs[blk] = (float)d;
-            if (xsum) xsum[blk] = sm;
-        }
+        quant_block_store(v, lane, blk, xq, xs, xsum);
     }
 }
 
