@@ -169,37 +169,59 @@ __device__ __forceinline__ void attn_finish(const AttnParams& p, float* s_part, 
         mine[threadIdx.x * row + hd + 1] = s_cL[threadIdx.x];
     }
     if (p.S == 1) return;
-    __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) {
+        __threadfence();
         const int prev = atomicAdd(p.counters + hkv * gridDim.z + gz, 1);
         *s_last_p = prev == p.S - 1;
         if (*s_last_p) p.counters[hkv * gridDim.z + gz] = 0;   // ready for the next launch / graph replay
+        __threadfence();
     }
     __syncthreads();
     if (!*s_last_p) return;
-    __threadfence();
-    // The last CTA of this KV head merges the S slices.  Slice weights exp(m_s - M) and the sums L go
-    // through shared memory (the per-warp states are dead by now; the host keeps S + 1 <= 8 * row),
-    // so that the loop over the slices below is independent loads the compiler can batch.
+    // The last CTA of this KV head merges the S slices.  What it reads -- maxima, sums, weighted V -- lies a trip to L2
+    // away, and three such trips in a row were most of this tail: warp g takes the (max, sum) pairs of head g, up
+    // to kPairs per lane at once, while every thread requests its first kHold weighted values; then the slice weights
+    // exp(m_s - M) go round through shared memory (the per-warp states are dead by now; the host keeps
+    // S + 1 <= 8 * row).
     const float* all = p.part + (((int64_t)hkv * gridDim.z + gz) * p.S * GS) * row;
     const int S = p.S;
-    float* s_w = s_part;            // [gc][S] maxima, then weights
+    float* s_w = s_part;            // [gc][S] weights
     float* s_L = s_part + gc * S;   // [gc]
-    for (int i = threadIdx.x; i < gc * S; i += blockDim.x) {
-        const int g = i / S, sl = i - g * S;
-        s_w[i] = __ldcg(all + ((int64_t)sl * GS + g) * row + hd);
+    constexpr int kPairs = 4, kHold = 20;
+    float held[kHold];
+    {
+        const int i = threadIdx.x, g = i / hd, d = i - g * hd;
+        const float* col = all + (int64_t)g * row + d;
+#pragma unroll
+        for (int k = 0; k < kHold; ++k) held[k] = i < gc * hd && k < S ? __ldcg(col + (int64_t)k * GS * row) : 0.f;
     }
-    __syncthreads();
     if (warp < gc) {
-        float M = kNegInf;
-        for (int sl = lane; sl < S; sl += 32) M = fmaxf(M, s_w[warp * S + sl]);
+        const float* st = all + (int64_t)warp * row + hd;
+        float M = kNegInf, Lsum = 0.f, mv[kPairs], lv[kPairs];
+#pragma unroll
+        for (int k = 0; k < kPairs; ++k) {
+            const int sl = lane + 32 * k;
+            mv[k] = sl < S ? __ldcg(st + (int64_t)sl * GS * row) : kNegInf;
+            lv[k] = sl < S ? __ldcg(st + (int64_t)sl * GS * row + 1) : 0.f;
+        }
+#pragma unroll
+        for (int k = 0; k < kPairs; ++k) M = fmaxf(M, mv[k]);
+        for (int sl = lane + 32 * kPairs; sl < S; sl += 32) M = fmaxf(M, __ldcg(st + (int64_t)sl * GS * row));
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
-        float Lsum = 0.f;
-        for (int sl = lane; sl < S; sl += 32) {
-            const float e = expf(s_w[warp * S + sl] - M);
-            Lsum = fmaf(__ldcg(all + ((int64_t)sl * GS + warp) * row + hd + 1), e, Lsum);
+#pragma unroll
+        for (int k = 0; k < kPairs; ++k) {
+            const int sl = lane + 32 * k;
+            if (sl < S) {
+                const float e = expf(mv[k] - M);
+                Lsum = fmaf(lv[k], e, Lsum);
+                s_w[warp * S + sl] = e;
+            }
+        }
+        for (int sl = lane + 32 * kPairs; sl < S; sl += 32) {
+            const float e = expf(__ldcg(st + (int64_t)sl * GS * row) - M);
+            Lsum = fmaf(__ldcg(st + (int64_t)sl * GS * row + 1), e, Lsum);
             s_w[warp * S + sl] = e;
         }
 #pragma unroll
@@ -211,8 +233,15 @@ __device__ __forceinline__ void attn_finish(const AttnParams& p, float* s_part, 
         const int g = i / hd, d = i - g * hd;
         const float* col = all + (int64_t)g * row + d;
         float O = 0.f;
+        int sl = 0;
+        if (i == (int)threadIdx.x) {
+#pragma unroll
+            for (int k = 0; k < kHold; ++k)
+                if (k < S) O = fmaf(held[k], s_w[g * S + k], O);
+            sl = kHold;
+        }
 #pragma unroll 8
-        for (int sl = 0; sl < S; ++sl) O = fmaf(__ldcg(col + (int64_t)sl * GS * row), s_w[g * S + sl], O);
+        for (; sl < S; ++sl) O = fmaf(__ldcg(col + (int64_t)sl * GS * row), s_w[g * S + sl], O);
         attn_store(p, (int64_t)(hkv * p.group + g0 + g) * hd + d, O * (1.0f / s_L[g]), lane);
     }
 }
@@ -325,18 +354,28 @@ gqa_decode_fast_kernel(const AttnParams p) {
     const int hkv = blockIdx.x, split = blockIdx.y, gz = blockIdx.z;
     const int g0 = gz * GC;
     const int gc = min(GC, p.group - g0);
-    float4* s_q = reinterpret_cast<float4*>(s_part + kAttnWarps * gc * row);
-    for (int i = threadIdx.x; i < gc * hd4; i += blockDim.x) {
-        const float4 t = reinterpret_cast<const float4*>(p.q + (int64_t)(hkv * p.group + g0) * hd)[i];
-        s_q[i] = make_float4(t.x * p.scale, t.y * p.scale, t.z * p.scale, t.w * p.scale);
-    }
-    __syncthreads();
     const int64_t clen = p.clenbuf ? p.clenbuf[0] : p.cache_len;
     const int64_t chunk = (clen + p.S - 1) / p.S;
     const int64_t j0 = split * chunk, j1 = min(clen, j0 + chunk);
     const int64_t kv4 = ((int64_t)p.n_kv * hd) >> 2;
     const float4* kb = reinterpret_cast<const float4*>(p.k + (int64_t)hkv * hd) + sub;
     const float4* vb = reinterpret_cast<const float4*>(p.v + (int64_t)hkv * hd) + sub;
+    // the rows of this lane group's first position are on their way while the query heads are staged (with the merge
+    // at the end in fewer trips: 32 q / 8 kv heads x 4096 14.5 -> 13.2 us, x 128 7.5 -> 6.6; 32 / 32 x 1024 9.6 -> 8.9)
+    const int64_t jf = j0 + warp * 4 + grp;
+    float4 kk[VEC], vv[VEC];
+    if (jf < j1) {
+#pragma unroll
+        for (int u = 0; u < VEC; ++u) kk[u] = __ldg(kb + jf * kv4 + 8 * u);
+#pragma unroll
+        for (int u = 0; u < VEC; ++u) vv[u] = __ldg(vb + jf * kv4 + 8 * u);
+    }
+    float4* s_q = reinterpret_cast<float4*>(s_part + kAttnWarps * gc * row);
+    for (int i = threadIdx.x; i < gc * hd4; i += blockDim.x) {
+        const float4 t = reinterpret_cast<const float4*>(p.q + (int64_t)(hkv * p.group + g0) * hd)[i];
+        s_q[i] = make_float4(t.x * p.scale, t.y * p.scale, t.z * p.scale, t.w * p.scale);
+    }
+    __syncthreads();
     const unsigned gmask = 0xFFu << (grp * 8);
     float4 acc[GC][VEC];
     float m[GC], l[GC];
@@ -351,31 +390,10 @@ gqa_decode_fast_kernel(const AttnParams p) {
     // a few positions per lane group, so an exposed load latency per step is most of the kernel
     // (not with one head per CTA, where four CTAs per SM hide the latency already: measured)
     constexpr bool PF = GC > 1;
-    float4 kk[VEC], vv[VEC], kn[VEC], vn[VEC];
-    {
-        const int64_t jf = j0 + warp * 4 + grp;
-        if (PF && jf < j1) {
-#pragma unroll
-            for (int u = 0; u < VEC; ++u) kn[u] = __ldg(kb + jf * kv4 + 8 * u);
-#pragma unroll
-            for (int u = 0; u < VEC; ++u) vn[u] = __ldg(vb + jf * kv4 + 8 * u);
-        }
-    }
-    for (int64_t j = j0 + warp * 4 + grp; j < j1; j += kAttnWarps * 4) {
-        if (PF) {
-#pragma unroll
-            for (int u = 0; u < VEC; ++u) {
-                kk[u] = kn[u];
-                vv[u] = vn[u];
-            }
-        }
+    float4 kn[VEC], vn[VEC];
+    for (int64_t j = jf; j < j1; j += kAttnWarps * 4) {
         const int64_t jn = j + kAttnWarps * 4;
-        if (!PF) {   // fetch this position's rows now
-#pragma unroll
-            for (int u = 0; u < VEC; ++u) kk[u] = __ldg(kb + j * kv4 + 8 * u);
-#pragma unroll
-            for (int u = 0; u < VEC; ++u) vv[u] = __ldg(vb + j * kv4 + 8 * u);
-        } else if (jn < j1) {
+        if (PF && jn < j1) {
 #pragma unroll
             for (int u = 0; u < VEC; ++u) kn[u] = __ldg(kb + jn * kv4 + 8 * u);
 #pragma unroll
@@ -405,6 +423,18 @@ gqa_decode_fast_kernel(const AttnParams p) {
                     acc[g][u].w = fmaf(acc[g][u].w, corr, pj * vv[u].w);
                 }
             }
+        }
+        if (PF) {
+#pragma unroll
+            for (int u = 0; u < VEC; ++u) {
+                kk[u] = kn[u];
+                vv[u] = vn[u];
+            }
+        } else if (jn < j1) {   // fetch the next position's rows now
+#pragma unroll
+            for (int u = 0; u < VEC; ++u) kk[u] = __ldg(kb + jn * kv4 + 8 * u);
+#pragma unroll
+            for (int u = 0; u < VEC; ++u) vv[u] = __ldg(vb + jn * kv4 + 8 * u);
         }
     }
     // the four position groups of the warp -> one state (every lane ends with the merged values)
