@@ -287,8 +287,8 @@ int32_t matmul_device(rstq_ctx* ctx, rstq_weight* w, const void* x, void* y, int
         const int pieces = gemv_f_pieces(ds, w->bits, w->out, w->in, M, act_dtype);
         if (pieces >= (act_dtype == RSTQ_F32 ? 2 : 3)) tc = true;
     }
-    // The same for MODE_A8 when not even 8 tokens of codes fit (K > 16 K): the codes and scales the
-    // quantizer produced feed the tensor-core path instead (<= 1e-3, no longer the exact integer dots).
+    // The same for MODE_A8 when not even 8 tokens of codes fit (K > 16 K): the quantized
+    // activations feed the tensor-core path instead (<= 1e-3, no longer the exact integer dots).
     // Up to 16 tokens this does not arise: their activations ride the weight ring, whatever K is.
     const bool rides = M <= 16 && ds.act_image && ds.act_ring != 1 && ds.act_ring != 4;
     if (mode == RSTQ_MODE_A8 && !tc && M >= 9 && !rides && ctx->tune_gemm_min_m == 17 && w->in * 8 > 128 * 1024) tc = true;
@@ -296,25 +296,27 @@ int32_t matmul_device(rstq_ctx* ctx, rstq_weight* w, const void* x, void* y, int
     if (mode == RSTQ_MODE_A8) {
         RSTQ_REQUIRE(act_dtype == RSTQ_F32 || act_dtype == RSTQ_BF16, RSTQ_E_INVALID, "unknown activation type");
         RSTQ_REQUIRE(out_dtype == RSTQ_F32 || tc, RSTQ_E_INVALID, "MODE_A8 decode writes f32");
-        if (M == 1 && !tc && ds.fuse_quant && !ds.x_on_host && w->in <= kFusedQuantMaxIn) {   // (x_params: same kernel)
+        if (M == 1 && ds.fuse_quant && !ds.x_on_host && w->in <= kFusedQuantMaxIn) {   // (x_params: same kernel)
             // one token: every CTA of the decode kernel quantizes x (16 - 112 KB, in L2) while it
             // stages it, bit for bit as the quantizer kernel would -- one launch, no scratch
             GemvA8Args a{w->data, nullptr, nullptr, nullptr, (float*)y, 1, w->in, w->out, w->bits, w->zp, tp, ds.x_params, ds.x_params ? nullptr : x, act_dtype};
             a.next = note_decode_launch(ctx, ds, w);
             return launch_gemv_a8(ctx, ds, a);
         }
+        if (tc) {   // prefill: the pre-pass of the GEMM quantizes
+            void* x16;
+            float *rowscale, *acc;
+            const int32_t rs = gemm_scratch(ds, M, w->in, w->out, &x16, &rowscale, &acc);
+            if (rs != RSTQ_OK) return rs;
+            return launch_gemm(ctx, ds, w, x, act_dtype == RSTQ_F32 ? 2 : 3, y, out_dtype, M, x16, rowscale, acc);
+        }
         ActScratch s;
         int32_t rc = act_scratch(ds, M, w->in, &s);
         if (rc != RSTQ_OK) return rc;
-        uint8_t* img = (!tc && ds.act_image) ? s.img : nullptr;
+        uint8_t* img = ds.act_image ? s.img : nullptr;
         rc = launch_quant_act_i8(ctx, ds, x, s.xq, s.xs, s.xsum, M, w->in, act_dtype, img, w->zp, w->bits);
         if (rc != RSTQ_OK) return rc;
-        if (!tc) return run_a8(ctx, w, s.xq, s.xs, s.xsum, (float*)y, M, tp, img);
-        void* x16;
-        float* rowscale;
-        float* acc;
-        if ((rc = gemm_scratch(ds, M, w->in, w->out, &x16, &rowscale, &acc)) != RSTQ_OK) return rc;
-        return launch_gemm(ctx, ds, w, s.xq, s.xs, 2, y, out_dtype, M, x16, rowscale, acc);
+        return run_a8(ctx, w, s.xq, s.xs, s.xsum, (float*)y, M, tp, img);
     }
     if (!tc) return run_f(ctx, w, x, y, M, act_dtype, out_dtype, tp);
     void* x16;
@@ -322,7 +324,7 @@ int32_t matmul_device(rstq_ctx* ctx, rstq_weight* w, const void* x, void* y, int
     float* acc;
     int32_t rc = gemm_scratch(ds, M, w->in, w->out, &x16, &rowscale, &acc);
     if (rc != RSTQ_OK) return rc;
-    return launch_gemm(ctx, ds, w, x, nullptr, act_dtype == RSTQ_F32 ? 0 : 1, y, out_dtype, M, x16, rowscale, acc);
+    return launch_gemm(ctx, ds, w, x, act_dtype == RSTQ_F32 ? 0 : 1, y, out_dtype, M, x16, rowscale, acc);
 }
 
 // f32 values that a K-quant format holds as products: v[i] = d[i / per] * q[i], formed in double and rounded to

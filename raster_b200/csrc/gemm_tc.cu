@@ -30,6 +30,7 @@
 
 #include "internal.h"
 #include "mma_helpers.cuh"
+#include "quant_helpers.cuh"
 #include "sync_helpers.cuh"
 #include "tcgen05_helpers.cuh"
 
@@ -41,22 +42,56 @@ constexpr int kKStep = 128;                        // K elements per pipeline st
 constexpr int kAStage = 128 * kKStep * 2;          // 32 KB of fp16 weights per stage
 constexpr int kPrefetch = 4;                       // K-steps of packed weights held in registers
 
-// ---- activation pre-pass: x (f32 / bf16 / int8 codes + block scales) -> fp16 * 2^-e(row) ---
+// Eight elements of a 32-element block, the block's other three eighths in the neighbouring lanes (lane & ~3):
+// replaced by code * scale of the int8 quantizer, as quant_block32 (quant_helpers.cuh) forms them.
+__device__ __forceinline__ void quant_dequant8(float (&v)[8]) {
+    constexpr float kMagic = 12582912.0f;   // 2^23 + 2^22
+    const unsigned mask = 0xFu << (threadIdx.x & 28);
+    float mx = fabsf(v[0]);
+#pragma unroll
+    for (int j = 1; j < 8; ++j) mx = fmaxf(mx, fabsf(v[j]));
+    mx = fmaxf(mx, __shfl_xor_sync(mask, mx, 1));
+    mx = fmaxf(mx, __shfl_xor_sync(mask, mx, 2));
+    bool exact = !(mx >= 1e-30f && mx <= 1e37f);
+    if (!exact) {
+        const float id = __fdividef(127.f, mx), xs = __fdiv_rn(mx, 127.f);
+        float code[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            code[j] = fmaf(v[j], id, kMagic) - kMagic;
+            exact |= !(fabsf(fmaf(v[j], id, -code[j])) <= 0.5f - 2e-4f);
+        }
+        if (!exact) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v[j] = code[j] * xs;
+            return;
+        }
+    }
+    const double d = (double)mx / 127.0;
+    const double id = d == 0.0 ? 0.0 : 1.0 / d;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = (float)max(-127, min(127, quant_round_half_up((double)v[j] * id))) * (float)d;
+}
+
+// ---- activation pre-pass: x (f32 / bf16, as it is or int8-quantized) -> fp16 * 2^-e(row) ---
 // One CTA per token row.  rowscale[m] = 2^e so that max|x| * 2^-e lies in [2^13, 2^14).
-template <int SRC>  // 0 = f32, 1 = bf16, 2 = int8 codes with per-32-block f32 scales
+// SRC 2, 3: the int8 quantizer on the way (MODE_A8): code * scale of every element, without the quantizer's own
+// launch and its arrays' trip through memory (int4, 11000 x 4128, M = 100: 26.9 us a call with both kernels, 23.1
+// with one; 14336 x 4096, M = 64: 22.4 -> 19.9).
+template <int SRC>  // 0 = f32, 1 = bf16, 2 = f32 quantized here, 3 = bf16 quantized here
 __global__ void __launch_bounds__(256)
-act_to_f16_kernel(const void* __restrict__ x, const float* __restrict__ xs, __half* __restrict__ x16,
+act_to_f16_kernel(const void* __restrict__ x, __half* __restrict__ x16,
                   float* __restrict__ rowscale, int64_t in) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const int64_t m = blockIdx.x;
     // eight consecutive elements (one 16-byte fp16 store) per thread and step
     auto load8 = [&](int64_t k, float (&v)[8]) {
-        if (SRC == 0) {
+        if (SRC == 0 || SRC == 2) {
             const float4* q = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(x) + m * in + k);
             const float4 a = __ldg(q), b = __ldg(q + 1);
             v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-        } else if (SRC == 1) {
+        } else {
             const uint4 a = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(x) + m * in + k));
             const uint32_t w[4] = {a.x, a.y, a.z, a.w};
 #pragma unroll
@@ -64,13 +99,8 @@ act_to_f16_kernel(const void* __restrict__ x, const float* __restrict__ xs, __ha
                 v[2 * j] = __uint_as_float(w[j] << 16);
                 v[2 * j + 1] = __uint_as_float(w[j] & 0xFFFF0000u);
             }
-        } else {
-            const uint2 a = __ldg(reinterpret_cast<const uint2*>(reinterpret_cast<const int8_t*>(x) + m * in + k));
-            const float sc = __ldg(xs + m * (in >> 5) + (k >> 5));
-            const uint32_t w[2] = {a.x, a.y};
-#pragma unroll
-            for (int j = 0; j < 8; ++j) v[j] = (float)(int8_t)(w[j >> 2] >> (8 * (j & 3))) * sc;
         }
+        if (SRC >= 2) quant_dequant8(v);
     };
     // Rows of up to 8192 elements stay in registers between the two passes (max, convert);
     // longer rows are read twice.
@@ -1028,17 +1058,17 @@ int32_t gemm_configure(DeviceState& ds) {
     return RSTQ_OK;
 }
 
-// x (src 0 = f32, 1 = bf16, 2 = int8 codes with per-block scales xs) -> fp16 rows x16 and 2^e per row
-static int32_t launch_act_to_f16(rstq_ctx* ctx, DeviceState& ds, const void* x, const float* xs, int src, void* x16,
+// x (src 0 = f32, 1 = bf16, 2 / 3 = f32 / bf16 through the int8 quantizer) -> fp16 rows x16 and 2^e per row
+static int32_t launch_act_to_f16(rstq_ctx* ctx, DeviceState& ds, const void* x, int src, void* x16,
                                  float* rowscale, int64_t M, int64_t in) {
     cudaError_t le;
     const dim3 grid((unsigned)M), block(256);
-    if (src == 0)
-        le = launch_pdl(act_to_f16_kernel<0>, grid, block, 0, ds, x, xs, (__half*)x16, rowscale, in);
-    else if (src == 1)
-        le = launch_pdl(act_to_f16_kernel<1>, grid, block, 0, ds, x, xs, (__half*)x16, rowscale, in);
-    else
-        le = launch_pdl(act_to_f16_kernel<2>, grid, block, 0, ds, x, xs, (__half*)x16, rowscale, in);
+    switch (src) {
+        case 0: le = launch_pdl(act_to_f16_kernel<0>, grid, block, 0, ds, x, (__half*)x16, rowscale, in); break;
+        case 1: le = launch_pdl(act_to_f16_kernel<1>, grid, block, 0, ds, x, (__half*)x16, rowscale, in); break;
+        case 2: le = launch_pdl(act_to_f16_kernel<2>, grid, block, 0, ds, x, (__half*)x16, rowscale, in); break;
+        default: le = launch_pdl(act_to_f16_kernel<3>, grid, block, 0, ds, x, (__half*)x16, rowscale, in);
+    }
     ctx->launches++;
     RSTQ_CUDA(le);
     return RSTQ_OK;
@@ -1079,10 +1109,10 @@ void gemm_plan(int64_t out, int64_t in, int64_t M, int sm_count, bool tmem_kerne
 }
 
 // y[M, out] = x[M, in] . dequant(W)^T on the tensor cores.  src: 0 = f32 x, 1 = bf16 x,
-// 2 = int8 codes x with per-block scales xs.  x16 / rowscale are caller-provided scratch
+// 2 / 3 = f32 / bf16 x through the int8 quantizer.  x16 / rowscale are caller-provided scratch
 // (M*in fp16, M floats).
-int32_t launch_gemm(rstq_ctx* ctx, DeviceState& ds, const rstq_weight* w, const void* x, const float* xs,
-                    int src, void* y, int out_dtype, int64_t M, void* x16, float* rowscale, float* acc32) {
+int32_t launch_gemm(rstq_ctx* ctx, DeviceState& ds, const rstq_weight* w, const void* x, int src, void* y,
+                    int out_dtype, int64_t M, void* x16, float* rowscale, float* acc32) {
     RSTQ_REQUIRE(M >= 1 && M < (1ll << 30), RSTQ_E_SHAPE, "M = %lld", (long long)M);
     RSTQ_REQUIRE(((uintptr_t)x16 & 15) == 0 && (w->in * 2) % 16 == 0, RSTQ_E_ALIGN,
                  "activation scratch must be 16-byte aligned");
@@ -1105,7 +1135,7 @@ int32_t launch_gemm(rstq_ctx* ctx, DeviceState& ds, const rstq_weight* w, const 
     // pre-pass: activations -> fp16 with one exponent per token row.  kind::f16 wants A and B of
     // one type (fp16 weights against bf16 activations raise "illegal instruction"), and fp16 on
     // both sides keeps three more mantissa bits of the weights than bf16 would.
-    int32_t rc = launch_act_to_f16(ctx, ds, x, xs, src, x16, rowscale, M, w->in);
+    int32_t rc = launch_act_to_f16(ctx, ds, x, src, x16, rowscale, M, w->in);
     if (rc != RSTQ_OK) return rc;
     cudaError_t le;
 

@@ -1,13 +1,16 @@
 """The block quantizer's two arithmetics (f32 with a tie check, double).
 
 Codes, scales and sums are the oracle's bit for bit wherever the f32 arithmetic hands over to the double one: a
-maximum of zero, tiny, huge; elements on and next to every k + 0.5.
+maximum of zero, tiny, huge; elements on and next to every k + 0.5.  The GEMM's pre-pass quantizes by the same rule:
+its result is, bit for bit, that of the float mode on code * scale from the quantizer kernel's arrays.
 """
 import numpy as np
 import pytest
+import torch
 
 from oracle import oracle as orc
 from raster_b200 import Context
+from raster_b200 import _lib as L
 
 pytestmark = pytest.mark.gpu
 
@@ -48,4 +51,37 @@ def test_codes_scales_sums_bit_for_bit(ctx):
     assert np.array_equal(s.download().view(np.uint32), os_.view(np.uint32))
     assert np.array_equal(z.download(), oz)
     for b in (bx, q, s, z):
+        b.free()
+
+
+@pytest.mark.parametrize("act", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("in_,M", [(32, 64), (288, 65), (4128, 100), (8192, 64), (8224, 70), (12288, 66)])
+def test_pre_pass_quantizes_like_the_quantizer(ctx, act, in_, M):
+    """Rows in one pass of registers (<= 8192) and longer, whole and partial warps of 8-element pieces."""
+    out = 136
+    rng = np.random.default_rng(in_ + M)
+    wq, ws = orc.quantize_weight(rng.standard_normal(out * in_).astype(np.float32), 4)
+    w = ctx.bind_weight(wq, ws, out, in_, L.FMT_Q4_0, L.LAYOUT_ROWMAJOR)
+    blocks = hard_blocks()
+    blocks = blocks[np.abs(blocks).max(1) <= 1e6]
+    x = torch.from_numpy(blocks[rng.integers(0, len(blocks), M * in_ // 32)].ravel()).to(act).cuda()
+    xf = x.to(torch.float32)
+    torch.cuda.synchronize()
+    n = M * in_
+    bx = ctx.wrap_buffer(x.data_ptr(), n, np.float32 if act == torch.float32 else np.uint16)
+    by = ctx.make_buffer(M * out, np.float32)
+    ctx.qmatmul(w, bx, by, M, L.F32 if act == torch.float32 else L.BF16, L.F32, L.MODE_A8)
+    ctx.sync()
+    got = by.download()
+    bxf, q, s = ctx.wrap_buffer(xf.data_ptr(), n, np.float32), ctx.make_buffer(n, np.int8), ctx.make_buffer(n // 32, np.float32)
+    z = ctx.make_buffer(n // 32, np.int32)
+    ctx.quant_act_i8(bxf, q, s, z, M, in_)
+    ctx.sync()
+    v = (q.download().reshape(-1, 32).astype(np.float32) * s.download()[:, None]).ravel()
+    bv = ctx.array_to_buffer(v)
+    ctx.qmatmul(w, bv, by, M, L.F32, L.F32, L.MODE_F)
+    ctx.sync()
+    assert np.isfinite(got).all()
+    assert np.array_equal(got.view(np.uint32), by.download().view(np.uint32))
+    for b in (bx, by, bxf, q, s, z, bv, w):
         b.free()
