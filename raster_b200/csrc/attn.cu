@@ -364,14 +364,16 @@ gqa_decode_fast_kernel(const AttnParams p) {
     const float4* kb = reinterpret_cast<const float4*>(p.k + (int64_t)hkv * hd) + sub;
     const float4* vb = reinterpret_cast<const float4*>(p.v + (int64_t)hkv * hd) + sub;
     // the rows of this lane group's first position are on their way while the query heads are staged (with the merge
-    // at the end in fewer trips: 32 q / 8 kv heads x 4096 14.5 -> 13.2 us, x 128 7.5 -> 6.6; 32 / 32 x 1024 9.6 -> 8.9)
+    // at the end in fewer trips, caches from HBM: 32 q / 8 kv heads x 4096 16.1 -> 14.1 us, x 512 8.9 -> 8.0;
+    // 32 / 32 x 1024 12.7 -> 11.6; 64 / 8 x 8192 of 64 elements 26.1 -> 24.4).  The loop takes them over at its top and
+    // requests the next ones there: moved to the bottom of the loop, the take-over cost the long caches 2.5 us.
     const int64_t jf = j0 + warp * 4 + grp;
-    float4 kk[VEC], vv[VEC];
+    float4 kn[VEC], vn[VEC];
     if (jf < j1) {
 #pragma unroll
-        for (int u = 0; u < VEC; ++u) kk[u] = __ldg(kb + jf * kv4 + 8 * u);
+        for (int u = 0; u < VEC; ++u) kn[u] = __ldg(kb + jf * kv4 + 8 * u);
 #pragma unroll
-        for (int u = 0; u < VEC; ++u) vv[u] = __ldg(vb + jf * kv4 + 8 * u);
+        for (int u = 0; u < VEC; ++u) vn[u] = __ldg(vb + jf * kv4 + 8 * u);
     }
     float4* s_q = reinterpret_cast<float4*>(s_part + kAttnWarps * gc * row);
     for (int i = threadIdx.x; i < gc * hd4; i += blockDim.x) {
@@ -393,8 +395,13 @@ gqa_decode_fast_kernel(const AttnParams p) {
     // a few positions per lane group, so an exposed load latency per step is most of the kernel
     // (not with one head per CTA, where four CTAs per SM hide the latency already: measured)
     constexpr bool PF = GC > 1;
-    float4 kn[VEC], vn[VEC];
     for (int64_t j = jf; j < j1; j += kAttnWarps * 4) {
+        float4 kk[VEC], vv[VEC];
+#pragma unroll
+        for (int u = 0; u < VEC; ++u) {
+            kk[u] = kn[u];
+            vv[u] = vn[u];
+        }
         const int64_t jn = j + kAttnWarps * 4;
         if (PF && jn < j1) {
 #pragma unroll
@@ -427,17 +434,11 @@ gqa_decode_fast_kernel(const AttnParams p) {
                 }
             }
         }
-        if (PF) {
+        if (!PF && jn < j1) {   // fetch the next position's rows now
 #pragma unroll
-            for (int u = 0; u < VEC; ++u) {
-                kk[u] = kn[u];
-                vv[u] = vn[u];
-            }
-        } else if (jn < j1) {   // fetch the next position's rows now
+            for (int u = 0; u < VEC; ++u) kn[u] = __ldg(kb + jn * kv4 + 8 * u);
 #pragma unroll
-            for (int u = 0; u < VEC; ++u) kk[u] = __ldg(kb + jn * kv4 + 8 * u);
-#pragma unroll
-            for (int u = 0; u < VEC; ++u) vv[u] = __ldg(vb + jn * kv4 + 8 * u);
+            for (int u = 0; u < VEC; ++u) vn[u] = __ldg(vb + jn * kv4 + 8 * u);
         }
     }
     // the four position groups of the warp -> one state (every lane ends with the merged values)
