@@ -118,7 +118,8 @@ typedef struct rstq_event rstq_event;
 #define RSTQ_TUNE_GEMM_WIDE 13    /* prefill GEMM above 128 tokens, 256-token tiles (one accumulator, one issuing
                                      thread) instead of 128-token ones: 0 (default) = where the grid then needs
                                      fewer cycles over its waves of thread blocks, 1 = never, 2 = always,
-                                     3 = as 0 but never two thread blocks per tile (each half of K) */
+                                     3 = as 0 but never several thread blocks per tile, 4 = as 0 but always equal
+                                     ranges of the K-steps of all tiles, on every SM */
 #define RSTQ_TUNE_TP_TAIL 15      /* fused decode + exchange (rstq_tp_qmatmul): how many thread blocks of the decode kernel
                                      stay for the exchange's tail (wait for the peers' results, write y); the others
                                      leave their SMs to the next launch, which fills its weight rings meanwhile.
@@ -159,7 +160,8 @@ RSTQ_API int32_t rstq_init(const int32_t* devices, rstq_ctx** ctx, int32_t ndev)
 RSTQ_API int32_t rstq_shutdown(rstq_ctx* ctx);
 /* How the prefill GEMM (M above the decode kernel's range) would tile a call on a device of sm_count SMs
  * at the default settings: plan2[0] = tokens per tile (32, 64, 128 or 256), plan2[1] = thread blocks per
- * tile (2 = each takes half of K; the second hands its sums to the first).  Pure host arithmetic: no
+ * tile (2 = each takes half of K; the second hands its sums to the first; 1 also where whole tiles would leave
+ * most SMs idle in the last wave and the thread blocks take equal ranges of all tiles' K instead).  Pure host arithmetic: no
  * device, no context.  No counterpart in the reference (its GEMM is one work-item per output). */
 RSTQ_API int32_t rstq_gemm_plan(int32_t* plan2, int64_t out, int64_t in, int64_t m, int32_t sm_count);
 /* What the FIRST decode launch of rstq_qmatmul (mode, bits 4 / 8, act_dtype) on an out x in weight with m tokens

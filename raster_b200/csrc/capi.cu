@@ -606,7 +606,8 @@ int32_t rstq_gemm_plan(int32_t* plan2, int64_t out, int64_t in, int64_t m, int32
                  "out = %lld, in = %lld, m = %lld, sm_count = %d", (long long)out, (long long)in, (long long)m, sm_count);
     int ntok = 0;
     bool split = false;
-    gemm_plan(out, in, m, sm_count, true, 0, &ntok, &split);
+    int ranges = 0;
+    gemm_plan(out, in, m, sm_count, true, 0, &ntok, &split, &ranges);
     plan2[0] = ntok;
     plan2[1] = split ? 2 : 1;
     return RSTQ_OK;
@@ -693,7 +694,7 @@ int32_t rstq_tune(rstq_ctx* ctx, int32_t key, int64_t value) {
             ctx->tune_q6k_units = value != 0;
             return RSTQ_OK;
         case RSTQ_TUNE_GEMM_WIDE:
-            RSTQ_REQUIRE(value >= 0 && value <= 3, RSTQ_E_INVALID, "256-token tile selector 0..3");
+            RSTQ_REQUIRE(value >= 0 && value <= 4, RSTQ_E_INVALID, "256-token tile selector 0..4");
             ctx->tune_gemm_wide = value;
             return RSTQ_OK;
         case RSTQ_TUNE_ACT_IMAGE:

@@ -28,6 +28,8 @@
 // Every mbarrier wait is time-bounded; on expiry the CTA reports through the
 // status word, drains and still frees its tensor memory.
 
+#include <type_traits>
+
 #include "internal.h"
 #include "mma_helpers.cuh"
 #include "quant_helpers.cuh"
@@ -176,12 +178,14 @@ struct GemmParams {
     int* status;
     int64_t out;            // output features
     int nb, ngroups;        // K blocks per row, 32-row groups stored
-    int M, ksteps, ttiles;
-    int tiles, ksplit;      // feature x token tiles; K is cut into ksplit ranges of ksteps steps (last may be shorter)
-    int ksteps_total;
-    float* part;            // ksplit > 1 (gemm_tmem_kernel): the K range 1 CTA of a tile leaves its f32 accumulator
-                            // here ([tile][warp][column][lane]), the K range 0 CTA adds it to its own and stores y
-    int* pair_flags;        // one word per tile, zero between launches: set when `part` of the tile is complete
+    int M, ksteps, ttiles;  // ksteps: K-steps of a tile
+    // gemm_tmem_kernel: the K-steps of all tiles, tile after tile, are one sequence and CTA c runs the range
+    // [range_start(c), range_start(c + 1)) of it
+    int64_t uq, ur;         // uq steps each, the first ur CTAs one more
+    int half;               // > 0 instead: two CTAs per tile, the first runs the tile's first `half` steps
+    float* part;            // a range that begins inside a tile leaves that tile's f32 sums here ([CTA][warp][column]
+                            // [lane]); the CTA that holds the tile's first step adds them to its own and stores y
+    int* part_flags;        // one word per CTA, zero between launches: set when its `part` is complete
     float wmul, wdiv;       // 2^ew applied to the block scales, 2^-ew applied to the result
     int out_dtype;
     unsigned long long* dbg;  // optional timeline of CTA 0 (see RSTQ_TUNE_TIMELINE), or null
@@ -477,8 +481,8 @@ gemm_tc_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tmap) {
 // from shared memory, which halves the shared-memory traffic of the K loop.
 // Warp roles: 0 = TMA (activations) and the L2 requests for the weights, 1 and 18 = MMA (even / odd
 // K-steps), 2..17 = dequant, then epilogue: warp & 3 = 32-row group (= its tensor-memory
-// sub-partition); t = (warp - 2) >> 2 picks, on whole K-steps, the set (t & 1: even / odd K-steps) and
-// the pair of blocks (2 (t >> 1), + 1) of a K-step, otherwise the one block t of every K-step.
+// sub-partition); t = (warp - 2) >> 2 picks the set (t & 1: even / odd K-steps) and the pair of
+// blocks (2 (t >> 1), + 1) of a K-step.
 constexpr int kGemmThreadsT = (3 + kDqWarps) * 32;  // TMA warp, MMA warp (even K-steps), 16 dequant / epilogue warps, MMA warp (odd K-steps)
 // pipeline stages (B in shared memory, A in tensor memory): what is left of the 512 columns after two
 // accumulators, at most 4: with exactly four the dequant warps run their two-set schedule, which
@@ -557,7 +561,16 @@ struct RawT<8> {
     float4 s;
 };
 
-template <int BITS, int NTOK>
+static __device__ __align__(16) uint8_t g_zero_unit[kUnitBytesQ8];   // never written
+__device__ __forceinline__ int64_t gemm_range_start(const GemmParams& p, int64_t c) {
+    if (p.half > 0) return (c >> 1) * p.ksteps + (c & 1) * p.half;
+    return c * p.uq + (c < p.ur ? c : p.ur);
+}
+
+// SEGS: ranges that touch several tiles, and rows whose last K-step is a partial one.  A kernel of its own: with the
+// loop over segments and the second K loop around it a single tile ran 3 % slower (4096 x 4096, M = 512: 21.3 ->
+// 22.0 us).
+template <int BITS, int NTOK, bool SEGS>
 __global__ void __launch_bounds__(kGemmThreadsT, 1)
 gemm_tmem_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tmap) {
     constexpr int UNIT = BITS == 4 ? kUnitBytesQ4 : kUnitBytesQ8;
@@ -573,43 +586,56 @@ gemm_tmem_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tmap) {
     if (p.dbg && blockIdx.x == 0 && threadIdx.x == 64) { p.dbg[300] = (unsigned long long)clock64(); p.dbg[304] = gtime_ns(); }
     __shared__ int s_abort;
     __shared__ uint32_t s_tmem;
-    __shared__ __align__(8) uint64_t s_bar[2 * 6 + 1];
+    __shared__ __align__(8) uint64_t s_bar[2 * 6 + 2];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     const uint32_t sbase = smem_u32(smem);
     const uint32_t bar0 = smem_u32(s_bar);
-    // full[s]: 16 dequant warps have stored A of the stage and the TMA bytes of B have landed;
-    // empty[s]: the MMAs that read the stage have completed (tcgen05.commit)
-    const uint32_t full = bar0, empty = bar0 + 8 * kNSTT, acc_full = bar0 + 16 * kNSTT;
-    const int kz = blockIdx.x / p.tiles, tile = blockIdx.x - kz * p.tiles;  // K range, output tile
-    const int ft = tile / p.ttiles, tt = tile - ft * p.ttiles;
-    const int ks_begin = kz * p.ksteps;
-    const int tok0 = tt * NTOK;
+    // full[s]: the eight dequant warps of the step's set have stored A of the stage and the TMA bytes of B have
+    // landed; empty[s]: the MMAs that read the stage have completed (tcgen05.commit); acc_full: a segment's sums are
+    // complete; acc_free: the epilogue has read them (and is done with the activation stages it borrows)
+    const uint32_t full = bar0, empty = bar0 + 8 * kNSTT, acc_full = bar0 + 16 * kNSTT, acc_free = acc_full + 8;
     volatile int* abort_flag = &s_abort;
-    const int ksteps = min(p.ksteps, p.ksteps_total - ks_begin);
+    // This CTA's range of the step sequence.  It is worked off in segments, one per tile it touches; step q of the
+    // range (counted over all segments) uses ring stage q mod kNSTT.  Where tiles are shared the ranges are dealt out
+    // from the back: a CTA then waits only for CTAs launched before it.
+    const int KS = p.ksteps, cta = SEGS || p.half > 0 ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x;
+    int tile_first, k_first, steps_own;   // first tile, first step in it, number of steps
+    if (p.half > 0) {
+        tile_first = cta >> 1;
+        k_first = (cta & 1) * p.half;
+        steps_own = (cta & 1) ? KS - p.half : p.half;
+    } else if (!SEGS || (p.uq == KS && p.ur == 0)) {
+        tile_first = cta;
+        k_first = 0;
+        steps_own = KS;
+    } else {
+        const uint32_t r0 = (uint32_t)gemm_range_start(p, cta);
+        tile_first = (int)(r0 / (uint32_t)KS);
+        k_first = (int)(r0 - (uint32_t)tile_first * KS);
+        steps_own = (int)((uint32_t)gemm_range_start(p, cta + 1) - r0);
+    }
 
-    // four-stage ring and whole K-steps: the dequant warps work as two sets of eight on alternate
-    // K-steps (see there), so a stage collects eight arrivals instead of sixteen
-    const bool paired = (p.nb & 3) == 0;
     if (tid == 0) asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmap)) : "memory");
-    if (paired && warp >= 2 && warp < 2 + kDqWarps) {
+    if (warp >= 2 && warp < 2 + kDqWarps) {
         // the first weights this warp will load: ask for them now, so that the HBM round trip
         // runs while the CTA sets itself up (barriers, tensor memory, the CTA-wide sync)
         const int t = (warp - 2) >> 2, pset = t & 1, blk0 = 2 * (t >> 1);
-        int64_t g = (int64_t)ft * 4 + (warp & 3);
+        int64_t g = (int64_t)(tile_first / p.ttiles) * 4 + (warp & 3);
         g = g < p.ngroups ? g : (int64_t)p.ngroups - 1;
-        const uint8_t* q = p.w + (g * p.nb + 4 * (ks_begin + pset) + blk0) * UNIT + lane * 128;
-        if (lane * 128 < 2 * UNIT) {
 #pragma unroll
-            for (int d = 0; d < 2; ++d)
-                if (pset + 2 * d < ksteps) asm volatile("prefetch.global.L2 [%0];" ::"l"(q + (size_t)d * 8 * UNIT));
+        for (int d = 0; d < 2; ++d) {
+            const int b = 4 * (k_first + pset + 2 * d) + blk0;
+            if (b + 1 < p.nb && lane * 128 < 2 * UNIT)
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(p.w + (g * p.nb + b) * UNIT + lane * 128));
         }
     }
     if (tid < kNSTT) {
-        mbar_init(full + 8 * tid, (paired ? kDqWarps / 2 : kDqWarps) + 1);
+        mbar_init(full + 8 * tid, kDqWarps / 2 + 1);
         mbar_init(empty + 8 * tid, 1);
     } else if (tid == kNSTT) {
-        mbar_init(acc_full, (ISS == 2 && ksteps >= 2) ? 2 : 1);  // one arrival per MMA issuer that has steps
+        mbar_init(acc_full, ISS);   // one arrival per MMA issuer and segment
+        mbar_init(acc_free, kDqWarps);
         s_abort = 0;
     }
     if (tid <= kNSTT) asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -633,40 +659,52 @@ gemm_tmem_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tmap) {
             // weights to be brought into L2 kPfSteps K-steps ahead of those loads, four K-steps (16
             // units, one contiguous run per row group) per request.
             constexpr int kPfSteps = kWeightPfSteps;
-            const int nb_end = min(p.nb, 4 * (ks_begin + ksteps));
-            auto request = [&](int ks) {  // K-steps ks .. ks + 3 of this CTA's range
-                const int b0 = 4 * (ks_begin + ks);
-                const int nblk = min(16, nb_end - b0);
-                if (nblk <= 0) return;
-#pragma unroll
-                for (int g = 0; g < 4; ++g) {
-                    const int64_t gg = (int64_t)ft * 4 + g;
-                    if (gg < p.ngroups) {
-                        const uint8_t* q = p.w + (gg * p.nb + b0) * UNIT;
-                        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(q), "r"((uint32_t)(nblk * UNIT))
-                                     : "memory");
-                    }
-                }
-            };
-            asm volatile("griddepcontrol.wait;" ::: "memory");  // activations come from the pre-pass
-            int s = 0, issued = 0;
+            int s = 0, issued = 0, seg = 0, left = steps_own;
             uint32_t ph = 0;
             bool ok = true;
-            for (int ks = 0; ks < ksteps; ++ks) {
-                // weight requests: none before the wait above (they would compete for HBM with the
-                // pre-pass this kernel waits for) nor before the first activation tiles are on their
-                // way; the dequant warps load K-steps 0 .. 3 themselves
-                if (kPfSteps > 0 && ks == kNSTT)
-                    for (int k2 = 4; k2 < 8 + kPfSteps; k2 += 4) request(k2);
-                if (kPfSteps > 0 && (ks & 3) == 0 && ks >= 4) request(ks + 4 + kPfSteps);
-                ok = mbar_block(empty + 8 * s, ph ^ 1u, abort_flag);
-                if (!ok) break;
-                const uint32_t dst = sbase + s * BSTAGE;
-                mbar_expect_tx(full + 8 * s, BSTAGE);
-                tma_load_2d(dst, &tmap, (ks_begin + ks) * kKStep, tok0, full + 8 * s);
-                tma_load_2d(dst + NTOK * 128, &tmap, (ks_begin + ks) * kKStep + 64, tok0, full + 8 * s);
-                ++issued;
-                if (++s == kNSTT) { s = 0; ph ^= 1u; }
+            for (int tile = tile_first, k0 = k_first; ok; ++tile, k0 = 0) {
+                const int n = min(KS - k0, left);
+                const int ft = tile / p.ttiles, tok0 = (tile - ft * p.ttiles) * NTOK;
+                const int nb_end = min(p.nb, 4 * (k0 + n));
+                auto request = [&](int ks) {  // K-steps ks .. ks + 3 of this segment
+                    const int b0 = 4 * (k0 + ks);
+                    const int nblk = min(16, nb_end - b0);
+                    if (nblk <= 0) return;
+#pragma unroll
+                    for (int g = 0; g < 4; ++g) {
+                        const int64_t gg = (int64_t)ft * 4 + g;
+                        if (gg < p.ngroups) {
+                            const uint8_t* q = p.w + (gg * p.nb + b0) * UNIT;
+                            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(q), "r"((uint32_t)(nblk * UNIT))
+                                         : "memory");
+                        }
+                    }
+                };
+                if (seg == 0) {
+                    asm volatile("griddepcontrol.wait;" ::: "memory");  // activations come from the pre-pass
+                } else {
+                    // a further tile: its first weights on their way while the epilogue of the one before runs
+                    for (int k2 = 0; k2 < 8 + kPfSteps; k2 += 4) request(k2);
+                    ok = mbar_block(acc_free, (uint32_t)(seg - 1) & 1u, abort_flag);
+                }
+                for (int ks = 0; ks < n && ok; ++ks) {
+                    // weight requests: none before the wait above (they would compete for HBM with the
+                    // pre-pass this kernel waits for) nor before the first activation tiles are on their
+                    // way; the dequant warps load K-steps 0 .. 3 themselves
+                    if (seg == 0 && ks == kNSTT)
+                        for (int k2 = 4; k2 < 8 + kPfSteps; k2 += 4) request(k2);
+                    if ((ks & 3) == 0 && ks >= 4) request(ks + 4 + kPfSteps);
+                    ok = mbar_block(empty + 8 * s, ph ^ 1u, abort_flag);
+                    if (!ok) break;
+                    const uint32_t dst = sbase + s * BSTAGE;
+                    mbar_expect_tx(full + 8 * s, BSTAGE);
+                    tma_load_2d(dst, &tmap, (k0 + ks) * kKStep, tok0, full + 8 * s);
+                    tma_load_2d(dst + NTOK * 128, &tmap, (k0 + ks) * kKStep + 64, tok0, full + 8 * s);
+                    ++issued;
+                    if (++s == kNSTT) { s = 0; ph ^= 1u; }
+                }
+                if (!SEGS || (left -= n) == 0) break;
+                ++seg;
             }
             if (!ok) {  // let the copies already issued land before this CTA's shared memory goes away
                 for (int k = issued > kNSTT ? issued - kNSTT : 0; k < issued; ++k) {
@@ -694,63 +732,47 @@ gemm_tmem_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tmap) {
         const uint32_t d_lo = (uint32_t)d0, d_hi = (uint32_t)(d0 >> 32);
         const uint32_t dcol = tmem + (uint32_t)(m * NTOK);
         static_assert(kKStep == 128, "eight MMAs per step");
-        if (m < ksteps) {
-            int s = m;
-            uint32_t ph = 0;
-            bool any = false;
-            bool ok = mbar_spin(full + 8 * s, 0, abort_flag);
-            if (dbg && lane == 0) dbg[306 + 2 * m] = (unsigned long long)clock64();
-            for (int ks = m; ks < ksteps && ok; ks += ISS) {
+        bool any = false, ok = true;
+        int q0 = 0, seg = 0, left = steps_own;
+        for (int k0 = k_first; ok; k0 = 0) {
+            const int n = min(KS - k0, left);
+            const int first = ISS == 2 ? (m + q0) & 1 : 0;   // this issuer's first step of the segment: q0 + first = m (mod 2)
+            int s = (q0 + first) % kNSTT;
+            uint32_t ph = (uint32_t)((q0 + first) / kNSTT) & 1u;
+            if (seg > 0) ok = mbar_spin(acc_free, (uint32_t)(seg - 1) & 1u, abort_flag);
+            if (ok && first < n) ok = mbar_spin(full + 8 * s, ph, abort_flag);
+            if (dbg && lane == 0 && seg == 0) dbg[306 + 2 * m] = (unsigned long long)clock64();
+            for (int ks = first; ks < n && ok; ks += ISS) {
                 int s2 = s + ISS;
                 uint32_t ph2 = ph;
                 if (s2 >= kNSTT) { s2 -= kNSTT; ph2 ^= 1u; }
                 const uint32_t a0 = tmem + A_COL0 + s * kAColsPerStage, b_lo = d_lo + (uint32_t)s * (BSTAGE >> 4);
-                // the block also tests the barrier of this issuer's next step (ks + 2) early
-                const uint32_t n2 = umma_f16_ts_step<NTOK * 8>(dcol, a0, b_lo, d_hi, idesc, ks != m, leader, empty, 0u,
+                // the block also tests the barrier of this issuer's next step (ks + ISS) early
+                const uint32_t n2 = umma_f16_ts_step<NTOK * 8>(dcol, a0, b_lo, d_hi, idesc, ks != first, leader, empty, 0u,
                                                                full + 8 * s2, ph2);
                 umma_commit_if(empty + 8 * s, leader);  // the stage is free once these MMAs have read it
                 any = true;
-                if (ks + ISS < ksteps && !n2) ok = mbar_spin(full + 8 * s2, ph2, abort_flag);
-                    s = s2;
+                if (ks + ISS < n && !n2) ok = mbar_spin(full + 8 * s2, ph2, abort_flag);
+                s = s2;
                 ph = ph2;
             }
             if (dbg && lane == 0) dbg[307 + 2 * m] = (unsigned long long)clock64();
-            if (any) {
-                umma_commit_if(acc_full, leader);
-                if (!ok) {  // gave up: the tensor core must be idle before tensor memory is freed
-                    const unsigned long long t0 = gtime_ns();
-                    while (!mbar_try(acc_full, 0) && gtime_ns() - t0 < kWaitLimitNs) {
-                    }
+            if (ok || any) umma_commit_if(acc_full, leader);   // (arrives at once where this issuer had no step)
+            if (!ok && any) {  // gave up: the tensor core must be idle before tensor memory is freed
+                const unsigned long long t0 = gtime_ns();
+                while (!mbar_try(acc_full, (uint32_t)seg & 1u) && gtime_ns() - t0 < kWaitLimitNs) {
                 }
             }
+            if (!SEGS || (left -= n) == 0) break;
+            ++seg;
+            q0 += n;
         }
     } else if (warp == 2 + kDqWarps) {
         // the second issuer warp of the two-accumulator tiles: nothing to do on a 256-token tile
     } else {
         // ---------------- dequant warps ----------------
-        const int dq = warp - 2, grp = warp & 3, sub = dq >> 2;
+        const int dq = warp - 2, grp = warp & 3;
         const int gid = lane >> 2;
-        const int64_t g_glob = (int64_t)ft * 4 + grp;
-        const bool g_valid = g_glob < p.ngroups;
-        const uint8_t* wptr = p.w + (g_glob * p.nb + sub + 4 * ks_begin) * UNIT + lane * 16;
-        const uint8_t* sptr = p.w + (g_glob * p.nb + sub + 4 * ks_begin) * UNIT + CODES + gid * 16;
-        int bk_next = sub + 4 * ks_begin;
-        auto load = [&](RawT<BITS>& r) {
-            if (g_valid && bk_next < p.nb) {
-                if constexpr (BITS == 4) {
-                    r.c = __ldg(reinterpret_cast<const uint4*>(wptr));
-                } else {
-                    r.c0 = __ldg(reinterpret_cast<const uint4*>(wptr));
-                    r.c1 = __ldg(reinterpret_cast<const uint4*>(wptr + 512));
-                }
-                r.s = __ldg(reinterpret_cast<const float4*>(sptr));
-            } else {
-                r = RawT<BITS>{};  // zero scale: rows / blocks beyond the matrix contribute 0
-            }
-            wptr += 4 * UNIT;
-            sptr += 4 * UNIT;
-            bk_next += 4;
-        };
         const float wmul = p.wmul;
         // this warp's rows are tensor-memory lanes 32*grp .. 32*grp + 31; its block is 16 columns wide
         const uint32_t t_lane = (uint32_t)(grp * 32) << 16;
@@ -794,96 +816,82 @@ gemm_tmem_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tmap) {
                 }
             }
         };
-        // one K-step of this warp: wait for the stage, convert, store, hand over
-        auto step = [&](const RawT<BITS>& r, int st, uint32_t parity) -> bool {
-            if (!__all_sync(0xffffffffu, mbar_block(empty + 8 * st, parity, abort_flag))) return false;
-            tc_fence_after();
-            convert_store(r, tmem + A_COL0 + st * kAColsPerStage, sub);
-            tmem_st_wait();
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(full + 8 * st);
-            return true;
-        };
-
+        // Two sets of eight warps take alternate K-steps, a warp converting two adjacent
+        // blocks of its row group per step: while one set converts, the other waits for its
+        // stage or stores, so the issue slots do not idle between bursts, and the fixed cost
+        // of a step (barrier test, store wait, arrival) is paid once per two units.
+        // Blocks past the end of a row (nb no multiple of 4) are read from a unit of zeros.
+        const int t = dq >> 2, pset = t & 1, blk0 = 2 * (t >> 1);
+        const uint32_t s_delta = (uint32_t)(CODES + gid * 16 - lane * 16);
         bool ok = true;
-        if (paired) {
-            // Two sets of eight warps take alternate K-steps, a warp converting two adjacent
-            // blocks of its row group per step: while one set converts, the other waits for its
-            // stage or stores, so the issue slots do not idle between bursts, and the fixed cost
-            // of a step (barrier test, store wait, arrival) is paid once per two units.
-            // Own step i of set `pset` is K-step pset + 2i, stage pset + 2 (i & 1), ring pass i / 2.
-            const int t = dq >> 2, pset = t & 1, blk0 = 2 * (t >> 1);
-            const int n_own = (ksteps - pset + 1) >> 1;
-            const int64_t g_ld = g_valid ? g_glob : (int64_t)p.ngroups - 1;
-            const uint8_t* wl = p.w + (g_ld * p.nb + 4 * (ks_begin + pset) + blk0) * UNIT + lane * 16;
-            const uint32_t s_delta = (uint32_t)(CODES + gid * 16 - lane * 16);
-            auto fetch2 = [&](RawT<BITS> (&r)[2], int own_off) {
+        int q0 = 0, seg = 0, left = steps_own;
+        for (int tile = tile_first, k0 = k_first;; ++tile, k0 = 0) {   // (also when a wait ran out: the warps meet at a barrier)
+        const int n = min(KS - k0, left);
+        const int ft = tile / p.ttiles, tok0 = (tile - ft * p.ttiles) * NTOK;
+        {
+            const int first = (pset + q0) & 1;            // own steps: q0 + first + 2 i
+            const int n_own = (n - first + 1) >> 1;
+            int64_t g_ld = (int64_t)ft * 4 + grp;         // (groups beyond the matrix: any valid rows, never stored)
+            g_ld = g_ld < p.ngroups ? g_ld : (int64_t)p.ngroups - 1;
+            int b_own = 4 * (k0 + first) + blk0;          // first block of own step i
+            const uint8_t* wl = p.w + (g_ld * p.nb + b_own) * UNIT + lane * 16;
+            auto fetch2 = [&](auto partial, RawT<BITS> (&r)[2], int own_off) {
                 const uint8_t* q = wl + (size_t)own_off * (8 * UNIT);
 #pragma unroll
                 for (int u = 0; u < 2; ++u, q += UNIT) {
+                    const uint8_t* a = q;
+                    if (decltype(partial)::value && b_own + own_off * 8 + u >= p.nb) a = g_zero_unit + lane * 16;
                     if constexpr (BITS == 4) {
-                        r[u].c = __ldg(reinterpret_cast<const uint4*>(q));
+                        r[u].c = __ldg(reinterpret_cast<const uint4*>(a));
                     } else {
-                        r[u].c0 = __ldg(reinterpret_cast<const uint4*>(q));
-                        r[u].c1 = __ldg(reinterpret_cast<const uint4*>(q + 512));
+                        r[u].c0 = __ldg(reinterpret_cast<const uint4*>(a));
+                        r[u].c1 = __ldg(reinterpret_cast<const uint4*>(a + 512));
                     }
-                    r[u].s = __ldg(reinterpret_cast<const float4*>(q + s_delta));
+                    r[u].s = __ldg(reinterpret_cast<const float4*>(a + s_delta));
                 }
             };
-            auto step2 = [&](const RawT<BITS> (&r)[2], int st, uint32_t parity) -> bool {
+            auto step2 = [&](const RawT<BITS> (&r)[2], int q) -> bool {
+                // ring position q % stages, pass q / stages (the first pass finds every stage free: parity 1)
+                const int st = q % kNSTT;
+                const uint32_t parity = (uint32_t)(((q / kNSTT) & 1) ^ 1);
                 if (!__all_sync(0xffffffffu, mbar_block(empty + 8 * st, parity, abort_flag))) return false;
                 tc_fence_after();
-                    const uint32_t a_stage = tmem + A_COL0 + st * kAColsPerStage;
+                const uint32_t a_stage = tmem + A_COL0 + st * kAColsPerStage;
                 convert_store(r[0], a_stage, blk0);
                 convert_store(r[1], a_stage, blk0 + 1);
-                    tmem_st_wait();
-                    tc_fence_before();
+                tmem_st_wait();
+                tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(full + 8 * st);
-                    return true;
+                return true;
             };
-            RawT<BITS> raw[2][2];
+            auto k_loop = [&](auto partial) {
+                RawT<BITS> raw[2][2];
 #pragma unroll
-            for (int d = 0; d < 2; ++d) {
-                raw[d][0] = RawT<BITS>{};
-                raw[d][1] = RawT<BITS>{};
-                if (d < n_own) fetch2(raw[d], d);
-            }
-            // stage and "stage free" parity of K-step ks: ring position ks % stages, pass ks / stages
-            // (the first pass finds every stage free: parity 1)
-            auto stage_of = [&](int ks) { return ks % kNSTT; };
-            auto parity_of = [&](int ks) { return (uint32_t)(((ks / kNSTT) & 1) ^ 1); };
-            int i = 0;
-            for (; i + 2 <= n_own && ok; i += 2) {
-                const int ks = pset + 2 * i;
-                ok = step2(raw[0], stage_of(ks), parity_of(ks));
-                if (i + 2 < n_own) fetch2(raw[0], 2);
-                if (ok) {
-                    ok = step2(raw[1], stage_of(ks + 2), parity_of(ks + 2));
-                    if (i + 3 < n_own) fetch2(raw[1], 3);
+                for (int d = 0; d < 2; ++d) {
+                    raw[d][0] = RawT<BITS>{};
+                    raw[d][1] = RawT<BITS>{};
+                    if (d < n_own) fetch2(partial, raw[d], d);
                 }
-                wl += (size_t)16 * UNIT;
-            }
-            if (ok && i < n_own) ok = step2(raw[0], stage_of(pset + 2 * i), parity_of(pset + 2 * i));
-        } else {
-            RawT<BITS> raw[kPrefetch];
-#pragma unroll
-            for (int j = 0; j < kPrefetch; ++j) load(raw[j]);
-            int s = 0;
-            uint32_t ph = 0;
-            for (int ks0 = 0; ks0 < ksteps && ok; ks0 += kPrefetch) {
-#pragma unroll
-                for (int j = 0; j < kPrefetch; ++j) {
-                    const int ks = ks0 + j;
-                    if (ks < ksteps && ok) {
-                        ok = step(raw[j], s, ph ^ 1u);
-                        if (ok) {
-                            load(raw[j]);
-                            if (++s == kNSTT) { s = 0; ph ^= 1u; }
-                        }
+                int i = 0;
+                for (; i + 2 <= n_own && ok; i += 2) {
+                    const int q = q0 + first + 2 * i;
+                    ok = step2(raw[0], q);
+                    if (i + 2 < n_own) fetch2(partial, raw[0], 2);
+                    if (ok) {
+                        ok = step2(raw[1], q + 2);
+                        if (i + 3 < n_own) fetch2(partial, raw[1], 3);
                     }
+                    wl += (size_t)16 * UNIT;
+                    if (decltype(partial)::value) b_own += 16;
                 }
+                if (ok && i < n_own) ok = step2(raw[0], q0 + first + 2 * i);
+            };
+            if constexpr (SEGS) {
+                if (4 * (k0 + n) > p.nb) k_loop(std::true_type{});   // the row's last K-step is a partial one
+                else k_loop(std::false_type{});
+            } else {
+                k_loop(std::false_type{});
             }
         }
 
@@ -907,29 +915,36 @@ gemm_tmem_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tmap) {
             }
         }
         if (ok) {
-            const bool got = mbar_block(acc_full, 0, abort_flag);
+            const bool got = mbar_block(acc_full, (uint32_t)seg & 1u, abort_flag);
             ok = __all_sync(0xffffffffu, got);
         }
         if (dbg && tid == 64) dbg[302] = (unsigned long long)clock64();
-        // Two CTAs on one tile (each half of K): the K range 1 CTA hands its accumulator over through
-        // L2, the K range 0 CTA adds it to its own (always a + b in this order) and writes y.
-        const bool pair = p.ksplit > 1;
-        const bool giver = pair && kz == 1, taker = pair && kz == 0;
-        float* part = pair ? p.part + ((size_t)tile * kDqWarps + dq) * (CPW * 32) : nullptr;
-        if (ok && taker) {
+        // A tile cut between CTAs: those holding its later steps (as the first segment of their ranges, so early)
+        // hand their sums over through L2; the CTA holding its first step (its last segment) adds them to its own,
+        // always in CTA order, and writes y.  A giver waits for nobody, and all CTAs are resident together.
+        const bool giver = (SEGS || p.half > 0) && k0 > 0;
+        int takes = 0;   // CTAs behind this one with steps of this tile
+        if (!SEGS) takes = p.half > 0 && !giver;
+        else if (!giver && n < KS)
+            while (cta + 1 + takes < (int)gridDim.x && gemm_range_start(p, cta + 1 + takes) < (int64_t)(tile + 1) * KS) ++takes;
+        constexpr size_t kPart = (size_t)kDqWarps * CPW * 32;   // floats per CTA
+        float* part = p.part + cta * kPart + (size_t)dq * (CPW * 32);
+        if (ok && takes > 0) {
             int got = 1;
             if (lane == 0) {
                 const unsigned long long t0 = gtime_ns();
-                for (;;) {
-                    int v;
-                    asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p.pair_flags + tile) : "memory");
-                    if (v != 0) break;
-                    if (*abort_flag || gtime_ns() - t0 > kWaitLimitNs) {
-                        *abort_flag = 1;
-                        got = 0;
-                        break;
+                for (int k = 1; k <= takes && got; ++k) {
+                    for (;;) {
+                        int v;
+                        asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p.part_flags + cta + k) : "memory");
+                        if (v != 0) break;
+                        if (*abort_flag || gtime_ns() - t0 > kWaitLimitNs) {
+                            *abort_flag = 1;
+                            got = 0;
+                            break;
+                        }
+                        __nanosleep(64);
                     }
-                    __nanosleep(64);
                 }
             }
             ok = __shfl_sync(0xffffffffu, got, 0) != 0;
@@ -946,11 +961,13 @@ gemm_tmem_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tmap) {
                 // all loads of the chunk first, one wait, then the stores with the output type decided
                 // once (a lane owns one feature: consecutive lanes write consecutive elements of a row)
                 uint32_t v[CH];
-                const uint32_t t0 = tmem + ((uint32_t)(sp * 32) << 16) + (uint32_t)(cq * CPW + h * CH);
+                // (a segment of one step has its sums in that step's accumulator alone)
+                const uint32_t t0 = tmem + ((uint32_t)(sp * 32) << 16) + (uint32_t)(cq * CPW + h * CH) +
+                                    (ISS == 2 && n == 1 ? (uint32_t)(q0 & 1) * NTOK : 0u);
 #pragma unroll
                 for (int c0 = 0; c0 < CH; c0 += 8) tmem_ld8(t0 + c0, *reinterpret_cast<uint32_t(*)[8]>(&v[c0]));
                 tmem_ld_wait();
-                if (ISS == 2 && ksteps >= 2) {  // the odd K-steps went into the second accumulator
+                if (ISS == 2 && n >= 2) {  // the odd K-steps went into the second accumulator
                     uint32_t v2[CH];
 #pragma unroll
                     for (int c0 = 0; c0 < CH; c0 += 8) tmem_ld8(t0 + NTOK + c0, *reinterpret_cast<uint32_t(*)[8]>(&v2[c0]));
@@ -964,10 +981,10 @@ gemm_tmem_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tmap) {
                     for (int j = 0; j < CH; ++j) part[(h * CH + j) * 32 + lane] = __uint_as_float(v[j]);
                     continue;
                 }
-                if (taker) {
+                for (int k = 1; k <= (SEGS ? takes : (takes > 0 ? 1 : 0)); ++k) {
+                    const float* from = part + k * kPart + (h * CH) * 32 + lane;
 #pragma unroll
-                    for (int j = 0; j < CH; ++j)
-                        v[j] = __float_as_uint(__uint_as_float(v[j]) + __ldcg(part + (h * CH + j) * 32 + lane));
+                    for (int j = 0; j < CH; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) + __ldcg(from + j * 32));
                 }
                 if ((p.out & 7) == 0) {
                     // Fast path: transpose the warp's 32-feature x CH-token tile through shared memory
@@ -1014,16 +1031,27 @@ gemm_tmem_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tmap) {
                 }
             }
         }
-        if (pair) {
-            // giver: every warp's part is out before the flag goes up; taker: every warp has read its
-            // part before the flag goes down again (the next launch's giver writes only after this
+        if (giver || takes > 0) {
+            // giver: every warp's part is out before the flag goes up; taker: every warp has read the
+            // parts before the flags go down again (the next launch's givers write only after this
             // grid has completed).  All sixteen warps meet here whether or not a wait ran out.
             if (giver && ok) __threadfence();
             asm volatile("bar.sync 6, %0;" ::"r"(kDqWarps * 32) : "memory");
             if (dq == 0 && lane == 0) {
-                if (taker) p.pair_flags[tile] = 0;
-                else if (ok) asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(p.pair_flags + tile), "r"(1) : "memory");
+                if (!giver)
+                    for (int k = 1; k <= takes; ++k) p.part_flags[cta + k] = 0;
+                else if (ok) asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(p.part_flags + cta), "r"(1) : "memory");
             }
+        }
+        if (!SEGS || (left -= n) == 0) break;
+        q0 += n;
+        ++seg;
+        if (ok) {   // the accumulators and the activation stages are free for the next segment
+            fence_async_smem();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(acc_free);
+        }
         }
     }
     if (dbg && tid == 64) { dbg[303] = (unsigned long long)clock64(); dbg[305] = gtime_ns(); }
@@ -1039,7 +1067,9 @@ static int32_t gemm_attr() {
     if constexpr (NTOK <= 128)
         RSTQ_CUDA(cudaFuncSetAttribute(gemm_tc_kernel<BITS, NTOK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        kNST * (kAStage + NTOK * kKStep * 2) + 1024));
-    RSTQ_CUDA(cudaFuncSetAttribute(gemm_tmem_kernel<BITS, NTOK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    RSTQ_CUDA(cudaFuncSetAttribute(gemm_tmem_kernel<BITS, NTOK, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   gemm_stages(NTOK) * (NTOK * kKStep * 2) + 1024));
+    RSTQ_CUDA(cudaFuncSetAttribute(gemm_tmem_kernel<BITS, NTOK, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    gemm_stages(NTOK) * (NTOK * kKStep * 2) + 1024));
     return RSTQ_OK;
 }
@@ -1081,13 +1111,19 @@ static int32_t launch_act_to_f16(rstq_ctx* ctx, DeviceState& ds, const void* x, 
 // (measured: a 128-wide K-step 690 cycles; a 256-wide one 1140 with 64 CTAs running, 1240 with 96,
 // 1400 with all 148 -- their activation tiles are twice as large and all come from L2; set-up, first
 // loads and epilogue of a CTA about 8000 resp. 9000 cycles; the hand-over of a pair about 1500)
+// (kRangeCycles: what the second segment of a range costs, in cycles over the plain model.  Measured, int4 / int8,
+// whole tiles or pairs -> ranges, us: 11008 x 4096 at M = 512 60.2 -> 55.8, 28672 x 8192 at M = 32 62.1 -> 55.8,
+// at M = 256 108.7 -> 102.3, 8192 x 28672 at M = 256 105.5 -> 104.4; but 4096 x 4096 at M = 768 32.3 -> 34.1, 8192 x 8192
+// at M = 512 53.8 -> 59.3, 12288 x 4096 at M = 300 43.8 -> 45.7: the break-even lies at 9000 - 14000.)
+constexpr int64_t kRangeCycles = 13000;
 void gemm_plan(int64_t out, int64_t in, int64_t M, int sm_count, bool tmem_kernel, int wide, int* ntok_out,
-               bool* split_out) {
+               bool* split_out, int* ranges_out) {
     const int64_t ftiles = (out + 127) / 128, sm = sm_count > 0 ? sm_count : 1;
     const int64_t ksteps_total = (in / 32 + 3) / 4;
     auto cycles = [&](int nt, bool* split) {
         const int64_t tiles = ftiles * ((M + nt - 1) / nt);
-        *split = tmem_kernel && tiles * 2 <= sm && tiles <= kPairTiles && ksteps_total >= 16 && wide != 3;
+        *split = tmem_kernel && tiles * 2 <= sm && tiles * 2 <= kGemmSharers &&
+                 tiles * 2 * 128 * nt * 4 <= kPairScratchBytes && ksteps_total >= 16 && wide != 3;
         const int64_t ctas = *split ? tiles * 2 : tiles, active = ctas < sm ? ctas : sm;
         const int64_t c = nt == 256 ? 1140 + (active > 64 ? (active - 64) * 31 / 10 : 0) : 690;
         const int64_t fixed = nt == 256 ? 9000 : 8000;
@@ -1102,6 +1138,23 @@ void gemm_plan(int64_t out, int64_t in, int64_t M, int sm_count, bool tmem_kerne
         if (wide == 2 || c_wide < c_narrow) {
             ntok = 256;
             split = split_w;
+        }
+    }
+    // Equal ranges of the step sequence on all SMs instead of whole tiles (or pairs) per thread block: no SM waits
+    // for the last wave, at the price of a second segment per thread block (an epilogue, a refill of the pipeline,
+    // a hand-over).
+    *ranges_out = 0;
+    if (tmem_kernel && wide != 3) {
+        const int64_t tiles = ftiles * ((M + ntok - 1) / ntok), steps = tiles * ksteps_total;
+        const int64_t fit = kPairScratchBytes / (128 * 4 * ntok), cap = fit < kGemmSharers ? fit : kGemmSharers;
+        int64_t G = sm < cap ? sm : cap;
+        G = G < steps ? G : steps;
+        const int64_t per = (steps + G - 1) / G;
+        const int64_t c = ntok == 256 ? 1140 + (G > 64 ? (G - 64) * 31 / 10 : 0) : 690, fixed = ntok == 256 ? 9000 : 8000;
+        bool s2 = false;
+        if (steps < (1ll << 31) && (wide == 4 || (per >= 8 && per * c + fixed + kRangeCycles < cycles(ntok, &s2)))) {
+            *ranges_out = (int)G;
+            split = false;
         }
     }
     *ntok_out = ntok;
@@ -1131,7 +1184,8 @@ int32_t launch_gemm(rstq_ctx* ctx, DeviceState& ds, const rstq_weight* w, const 
     const int64_t ftiles = (w->out + 127) / 128;
     int ntok = 128;
     bool split = false;
-    gemm_plan(w->out, w->in, M, ds.sm_count, a_in_tmem && acc32 != nullptr, (int)ctx->tune_gemm_wide, &ntok, &split);
+    int ranges = 0;
+    gemm_plan(w->out, w->in, M, ds.sm_count, a_in_tmem && acc32 != nullptr, (int)ctx->tune_gemm_wide, &ntok, &split, &ranges);
     // pre-pass: activations -> fp16 with one exponent per token row.  kind::f16 wants A and B of
     // one type (fp16 weights against bf16 activations raise "illegal instruction"), and fp16 on
     // both sides keeps three more mantissa bits of the weights than bf16 would.
@@ -1158,7 +1212,7 @@ int32_t launch_gemm(rstq_ctx* ctx, DeviceState& ds, const rstq_weight* w, const 
     p.nb = (int)w->nb;
     p.ngroups = (int)(w->outp / 32);
     p.M = (int)M;
-    p.ksteps_total = (int)((w->nb + 3) / 4);
+    p.ksteps = (int)((w->nb + 3) / 4);
     p.ttiles = (int)((M + ntok - 1) / ntok);
     // gemm_tmem_kernel converts codes as fp16 subnormals (code * 2^-24): its block scales carry
     // 2^kSubnormalShift more and the result the remaining 2^(24 - kSubnormalShift)
@@ -1167,28 +1221,37 @@ int32_t launch_gemm(rstq_ctx* ctx, DeviceState& ds, const rstq_weight* w, const 
     p.out_dtype = out_dtype;
     p.dbg = ds.dbg;
     RSTQ_REQUIRE(ftiles * p.ttiles < (1ll << 30), RSTQ_E_LIMIT, "grid too large");
-    p.tiles = (int)(ftiles * p.ttiles);
-    p.ksplit = split ? 2 : 1;
-    p.ksteps = (p.ksteps_total + p.ksplit - 1) / p.ksplit;
-    p.part = split ? acc32 : nullptr;   // [tile][16 warps][columns per warp][32 lanes] f32: tiles * 128 * ntok floats
-    p.pair_flags = ds.counters + ds.counters_len - kPairTiles;
-    const dim3 grid((unsigned)(p.tiles * p.ksplit));
+    const int64_t tiles = ftiles * p.ttiles;
+    const int64_t ctas = ranges > 0 ? ranges : (split ? tiles * 2 : tiles);
+    p.half = split ? (p.ksteps + 1) / 2 : 0;
+    p.uq = ranges > 0 ? tiles * p.ksteps / ranges : p.ksteps;
+    p.ur = ranges > 0 ? tiles * p.ksteps % ranges : 0;
+    p.part = acc32;   // [CTA][16 warps][columns per warp][32 lanes] f32: 128 * ntok floats each
+    p.part_flags = ds.counters + ds.counters_len - kGemmSharers;
+    const bool general = ranges > 0 || (w->nb & 3) != 0;
+    const dim3 grid((unsigned)ctas);
     const size_t smem = a_in_tmem ? gemm_stages(ntok) * ((size_t)ntok * kKStep * 2) + 1024
                                   : kNST * (kAStage + (size_t)ntok * kKStep * 2) + 1024;
-#define GL(B, N)                                                                                     \
-    le = a_in_tmem ? launch_pdl(gemm_tmem_kernel<B, N>, grid, dim3(kGemmThreadsT), smem, ds, p, tmap) \
-                   : launch_pdl(gemm_tc_kernel<B, N>, grid, dim3(kGemmThreads), smem, ds, p, tmap)
+#define GT(B, N)                                                                                          \
+    le = general ? launch_pdl(gemm_tmem_kernel<B, N, true>, grid, dim3(kGemmThreadsT), smem, ds, p, tmap)  \
+                 : launch_pdl(gemm_tmem_kernel<B, N, false>, grid, dim3(kGemmThreadsT), smem, ds, p, tmap)
+#define GL(B, N)                 \
+    do {                         \
+        if (a_in_tmem) GT(B, N); \
+        else le = launch_pdl(gemm_tc_kernel<B, N>, grid, dim3(kGemmThreads), smem, ds, p, tmap); \
+    } while (0)
     if (w->bits == 4) {
         if (ntok == 32) GL(4, 32);
         else if (ntok == 64) GL(4, 64);
         else if (ntok == 128) GL(4, 128);
-        else le = launch_pdl(gemm_tmem_kernel<4, 256>, grid, dim3(kGemmThreadsT), smem, ds, p, tmap);
+        else GT(4, 256);
     } else {
         if (ntok == 32) GL(8, 32);
         else if (ntok == 64) GL(8, 64);
         else if (ntok == 128) GL(8, 128);
-        else le = launch_pdl(gemm_tmem_kernel<8, 256>, grid, dim3(kGemmThreadsT), smem, ds, p, tmap);
+        else GT(8, 256);
     }
+#undef GT
 #undef GL
     ctx->launches++;
     RSTQ_CUDA(le);

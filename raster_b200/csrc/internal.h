@@ -52,10 +52,10 @@ int32_t cuda_fail(cudaError_t e, const char* what, const char* file, int line);
 // One 16-byte load per lane thus feeds two 16-row tensor-core tiles with no
 // data movement between lanes.
 constexpr int kUnitBytesQ4 = 640;
-// prefill GEMM, two CTAs per tile: at most this many tiles (their flags are the last words of
+// prefill GEMM, tiles shared by several CTAs: at most this many CTAs (their flags are the last words of
 // DeviceState::counters, their partial tiles of up to 128 x 256 floats live in the GEMM scratch)
-constexpr int kPairTiles = 128;
-constexpr int64_t kPairScratchBytes = (int64_t)kPairTiles * 128 * 256 * 4;
+constexpr int kGemmSharers = 256;
+constexpr int64_t kPairScratchBytes = 160ll * 128 * 256 * 4;
 constexpr int kUnitBytesQ6K = 1280;  // 1024 bytes of 8-bit codes as in the 8-bit unit, then 64 scales (one per row and 16 elements)
 constexpr int kUnitBytesQ4K = 768;  // a 4-bit unit with the 32 Q4_K minima (db * bq, added as they are) behind the 32 scales
 constexpr int kUnitBytesQ8 = 1152;
@@ -329,7 +329,7 @@ int32_t gemv_configure(DeviceState& ds);  // shared-memory attributes, once per 
 // gemm_tc.cu
 // gemm_tc.cu: token-tile width (32 / 64 / 128 / 256) and whether two CTAs share a tile, for a device of sm_count SMs
 void gemm_plan(int64_t out, int64_t in, int64_t M, int sm_count, bool tmem_kernel, int wide, int* ntok_out,
-               bool* split_out);
+               bool* split_out, int* ranges_out);
 int32_t launch_gemm(rstq_ctx* ctx, DeviceState& ds, const rstq_weight* w, const void* x, int src, void* y,
                     int out_dtype, int64_t M, void* x16, float* rowscale, float* acc32);
 int32_t gemm_configure(DeviceState& ds);

@@ -1,0 +1,44 @@
+"""Prefill GEMM over equal ranges of K-steps: tiles cut between thread blocks at any step.
+
+A range that begins inside a tile hands its f32 sums to the thread block with the tile's first step.  Forced here
+(selector 4) at sizes where that can go wrong: one step per range, tiles cut many times, rows whose last K-step is
+partial, one and two accumulators, a ragged number of tokens.  The result is the whole-tile one up to the order of
+f32 additions: at most 260 partial sums of a row, each rounded to 2^-23 of a running value that stays below
+about 4 max|y|, as a random walk sqrt(260) * 4 * 2^-23 = 8e-6 of max|y|; the bound against f64 is the GEMM's own.
+"""
+import numpy as np
+import pytest
+
+from oracle import oracle as orc
+from raster_b200 import _lib as L
+from raster_b200 import synth
+
+pytestmark = pytest.mark.gpu
+TUNE_GEMM_WIDE = 13
+
+
+@pytest.mark.parametrize("bits", [4, 8])
+@pytest.mark.parametrize("out,in_,M", [(200, 160, 33), (300, 4128, 100), (2500, 1056, 60), (19000, 1056, 20),
+                                       (3000, 2080, 300), (1032, 8192, 515)])
+def test_ranges_against_whole_tiles(ctx, bits, out, in_, M):
+    w = synth.normal(out + in_ + bits, out * in_, 0.02)
+    wq, ws = orc.quantize_weight(w, bits)
+    x = synth.normal(out + in_ + M, M * in_)
+    bw = ctx.bind_weight(wq, ws, out, in_, L.FMT_Q4_0 if bits == 4 else L.FMT_Q8_0, L.LAYOUT_ROWMAJOR)
+    y = {}
+    try:
+        for how in (3, 4):
+            ctx.tune(TUNE_GEMM_WIDE, how)
+            y[how] = ctx.qmatmul_host(bw, x, M, L.F32, L.MODE_F).reshape(M, out).astype(np.float64)
+        again = ctx.qmatmul_host(bw, x, M, L.F32, L.MODE_F).reshape(M, out)
+    finally:
+        ctx.tune(TUNE_GEMM_WIDE, 0)
+    assert np.array_equal(again.astype(np.float64), y[4])          # sums in a fixed order
+    top = np.abs(y[3]).max()
+    assert np.abs(y[4] - y[3]).max() <= 4 * 8e-6 * top
+    rows = np.unique(np.concatenate([np.arange(0, out, max(1, out // 64)), [out - 1]]))
+    c = np.ascontiguousarray(wq.reshape(out, -1)[rows]).ravel()
+    s = np.ascontiguousarray(ws.reshape(out, -1)[rows]).ravel()
+    ref = orc.matmul_dq_f64(c, s, 0 if bits == 4 else 1, x, M, in_, rows.size).reshape(M, rows.size)
+    assert np.abs(y[4][:, rows] - ref).max() <= 1e-3 * np.abs(ref).max()
+    bw.free()
