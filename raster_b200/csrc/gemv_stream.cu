@@ -310,6 +310,12 @@ __device__ __forceinline__ int quant_exact(float x, double id) {
     const int q = (int)f + ((v - f) >= 0.5 ? 1 : 0);
     return max(-127, min(127, q));
 }
+// the larger of the two; a NaN if one of them is
+__device__ __forceinline__ float max_nan(float a, float b) {
+    float m;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(m) : "f"(a), "f"(b));
+    return m;
+}
 // PARAM: x lies in the parameter block.  Its lanes read different words, which the constant path would serve one
 // address at a time; through the generic address they are ordinary cached loads.
 __device__ __forceinline__ uint4 ldgen_u4(const void* p) {
@@ -354,9 +360,9 @@ __device__ __forceinline__ void stage_a8_quant(const StreamParams& p, const void
         const float f[8] = {__uint_as_float(raw[it][0].x), __uint_as_float(raw[it][0].y), __uint_as_float(raw[it][0].z),
                             __uint_as_float(raw[it][0].w), __uint_as_float(raw[it][1].x), __uint_as_float(raw[it][1].y),
                             __uint_as_float(raw[it][1].z), __uint_as_float(raw[it][1].w)};
-        float mx = 0.f;
+        float mx = fabsf(f[0]);   // (elements that are no number do not count unless all are)
 #pragma unroll
-        for (int k = 0; k < 8; ++k) mx = fmaxf(mx, fabsf(f[k]));
+        for (int k = 1; k < 8; ++k) mx = fmaxf(mx, fabsf(f[k]));
         mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
         mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
         if (UK != 0) {
@@ -381,10 +387,10 @@ __device__ __forceinline__ void stage_a8_quant(const StreamParams& p, const void
             for (int k = 0; k < 8; ++k) {
                 const float u = fmaf(f[k], idf, kMagicFlt);
                 const float frac = fmaf(f[k], idf, kMagicFlt - u);   // x * idf - n, n = u - magic exactly
-                amb = fmaxf(amb, fabsf(frac));
+                amb = max_nan(amb, fabsf(frac));                     // a NaN takes the double path as well
                 ub[k] = __float_as_uint(u);
             }
-            exact = amb > 0.5f - 2e-4f;
+            exact = !(amb <= 0.5f - 2e-4f);
             wa = __byte_perm(__byte_perm(ub[0], ub[1], 0x0040), __byte_perm(ub[2], ub[3], 0x0040), 0x5410);
             wb = __byte_perm(__byte_perm(ub[4], ub[5], 0x0040), __byte_perm(ub[6], ub[7], 0x0040), 0x5410);
         }

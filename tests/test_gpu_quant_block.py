@@ -11,6 +11,7 @@ import torch
 from oracle import oracle as orc
 from raster_b200 import Context
 from raster_b200 import _lib as L
+from raster_b200.quant import cpu_quant as cq
 
 pytestmark = pytest.mark.gpu
 
@@ -84,4 +85,39 @@ def test_pre_pass_quantizes_like_the_quantizer(ctx, act, in_, M):
     assert np.isfinite(got).all()
     assert np.array_equal(got.view(np.uint32), by.download().view(np.uint32))
     for b in (bx, by, bxf, q, s, z, bv, w):
+        b.free()
+
+
+@pytest.mark.parametrize("fmt", ["q4_0", "q8_0", "q4k", "q6k"])
+@pytest.mark.parametrize("nan", [slice(5, 6), slice(64, 96), slice(256, 512), slice(300, 1000, 3)])   # an element, a block, a super-block, every third
+def test_elements_that_are_no_number_get_the_same_code_on_every_route(ctx, fmt, nan):
+    """One token: the quantizer inside the decode kernel (x from a buffer, x among the launch's parameters) and the
+    quantizer kernel in front of it give the same results, bit for bit, and as many of them are NaN."""
+    out, in_ = 2048, 2048
+    rng = np.random.default_rng(3)
+    W = (rng.standard_normal(out * in_) * 0.02).astype(np.float32)
+    if fmt == "q4k":
+        w = ctx.bind_weight_q4k(cq.quantize_weight_q4k(W), out, in_)
+    elif fmt == "q6k":
+        w = ctx.bind_weight_q6k(cq.quantize_weight_q6k(W), out, in_)
+    else:
+        q = cq.quantize_weight(W, cq.q4_0 if fmt == "q4_0" else cq.q8_0)
+        w = ctx.bind_weight(q["wq"], q["ws"], out, in_, L.FMT_Q4_0 if fmt == "q4_0" else L.FMT_Q8_0, L.LAYOUT_ROWMAJOR)
+    x = rng.standard_normal(in_).astype(np.float32)
+    x[nan] = np.nan
+    bx, by, got = ctx.array_to_buffer(x), ctx.make_buffer(out, np.float32), {}
+    try:
+        for fused in (0, 1):
+            ctx.tune(L.TUNE_FUSE_QUANT, fused)
+            ctx.qmatmul(w, bx, by, 1)
+            ctx.sync()
+            got[fused] = by.download()
+    finally:
+        ctx.tune(L.TUNE_FUSE_QUANT, 1)
+    # a scale is a NaN, and with it every result, only where all elements under it are
+    whole = (nan.stop - nan.start) // (nan.step or 1) >= (256 if fmt in ("q4k", "q6k") else 32) and not nan.step
+    assert np.isnan(got[0]).all() if whole else np.isfinite(got[0]).all()
+    assert np.array_equal(got[0], got[1], equal_nan=True)
+    assert np.array_equal(got[0], ctx.qmatmul_host(w, x)[0], equal_nan=True)
+    for b in (bx, by, w):
         b.free()
