@@ -49,14 +49,14 @@ struct DxPrep {
     const float* dy;
     const float* scales;
     __half *yh, *yl;        // [m][opad]
-    float* rowscale;        // [m]: 2^e, the row holds dy * 2^-e with max|.| in [2^13, 2^14)
+    int* rowexp;            // [m]: e, the row holds dy * 2^-e with max|.| in [2^13, 2^14)
     float* colmax;          // [kDxParts][nb]: max|scale| of a part's rows
     int64_t m, out, nb, opad;
 };
 
-// 2^-e (as two factors: a subnormal maximum needs more than one f32 holds) and 2^e that bring a finite maximum
-// into [2^(top-1), 2^top)
-__device__ __forceinline__ void dx_exponent(float mx, int top, float* down, float* down2, float* up) {
+// The exponent e that brings a finite maximum into [2^(top-1), 2^top) as max * 2^-e, and 2^-e as two factors (a
+// subnormal maximum needs more than one f32 holds).
+__device__ __forceinline__ int dx_exponent(float mx, int top, float* down, float* down2) {
     int e = 0;
     if (mx > 0.f && mx < __int_as_float(0x7F800000)) {
         int ex;
@@ -67,7 +67,14 @@ __device__ __forceinline__ void dx_exponent(float mx, int top, float* down, floa
     const int e1 = e < -100 ? -100 : e;
     *down = ldexpf(1.0f, -e1);
     *down2 = ldexpf(1.0f, e1 - e);
-    *up = ldexpf(1.0f, e);
+    return e;
+}
+// v * 2^e.  In two halves, whose powers f32 holds and between which nothing leaves its range that the result does
+// not leave; below 2^-252 every v here (< 2^60) ends as zero.  (ldexpf does the same 3 us slower over 512 x 4096 results.)
+__device__ __forceinline__ float dx_scale(float v, int e) {
+    e = e < -252 ? -252 : e;
+    const int h = e >> 1;
+    return v * __int_as_float((h + 127) << 23) * __int_as_float((e - h + 127) << 23);
 }
 __device__ __forceinline__ float dx_block_max(float mx, float* red) {   // 256 threads
 #pragma unroll
@@ -176,8 +183,8 @@ dx_prep_kernel(const DxPrep p) {
             for (int j = 0; j < 16; ++j) mx = fmaxf(mx, fabsf(held[0][j]));
         }
     }
-    float down, down2, up;
-    dx_exponent(dx_block_max(mx, s_red), 14, &down, &down2, &up);
+    float down, down2;
+    const int e = dx_exponent(dx_block_max(mx, s_red), 14, &down, &down2);
     auto store16 = [&](int64_t o, const float (&v)[16]) {
         uint32_t h[8], l[8];
 #pragma unroll
@@ -202,13 +209,13 @@ dx_prep_kernel(const DxPrep p) {
             store16(o, held[0]);
         }
     }
-    if (threadIdx.x == 0) p.rowscale[m] = up;
+    if (threadIdx.x == 0) p.rowexp[m] = e;
 }
 
 // ---- the GEMM -----------------------------------------------------------------------------------
 struct DxParams {
     const float* scales;
-    const float* rowscale;
+    const int* rowexp;
     const float* colmax;
     float* dx;
     int* status;
@@ -300,6 +307,7 @@ dx_tmem_kernel(const DxParams p, const __grid_constant__ CUtensorMap map_w, cons
     extern __shared__ uint8_t smem_raw[];
     __shared__ int s_abort;
     __shared__ uint32_t s_tmem;
+    __shared__ int s_colexp[4];
     __shared__ __align__(8) uint64_t s_bar[2 * kDxStages + 2 * kDxRaw + 1];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -427,8 +435,9 @@ dx_tmem_kernel(const DxParams p, const __grid_constant__ CUtensorMap map_w, cons
             for (int i = lane; i < kDxParts; i += 32) mx = fmaxf(mx, __ldg(p.colmax + i * nb + b));
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        float down, down2, cs;   // the block's scales are used times 2^-e, the largest in [2^6, 2^7)
-        dx_exponent(mx, 7, &down, &down2, &cs);
+        float down, down2;   // the block's scales are used times 2^-ce, the largest in [2^6, 2^7)
+        const int ce = dx_exponent(mx, 7, &down, &down2);
+        if (lane == 0) s_colexp[blk] = ce;   // (the four warps of a block of columns agree)
         int s = set, rs = set;
         uint32_t ph = 0, rph = 0;
         for (int k = k0 + set; k < k1; k += 2) {
@@ -524,8 +533,9 @@ dx_tmem_kernel(const DxParams p, const __grid_constant__ CUtensorMap map_w, cons
             for (int j = 0; j < CH; ++j) {
                 const float v = __uint_as_float(a[j]) + __uint_as_float(b[j]);
                 const int tok = tok0 + col + j;
-                if (p.split > 1) s_out[(col + j) * 128 + blk * 32 + 4 * (lane & 7) + (lane >> 3)] = v * cs;
-                else if (tok < p.m && i_ok) p.dx[(int64_t)tok * p.in + i] = v * cs * __ldg(p.rowscale + tok);
+                // (both exponents at once: one of them alone can take a finite result through infinity or zero)
+                if (p.split > 1) s_out[(col + j) * 128 + blk * 32 + 4 * (lane & 7) + (lane >> 3)] = v;
+                else if (tok < p.m && i_ok) p.dx[(int64_t)tok * p.in + i] = dx_scale(v, ce + __ldg(p.rowexp + tok));
             }
         }
     }
@@ -549,7 +559,7 @@ dx_tmem_kernel(const DxParams p, const __grid_constant__ CUtensorMap map_w, cons
                 }
                 const int64_t i = (int64_t)ft * 128 + c;
                 if (tok < p.m && i < p.in)
-                    p.dx[(int64_t)tok * p.in + i] = v * __ldg(p.rowscale + tok);
+                    p.dx[(int64_t)tok * p.in + i] = dx_scale(v, s_colexp[c >> 5] + __ldg(p.rowexp + tok));
             }
         }
         __syncwarp();
@@ -624,7 +634,7 @@ int32_t launch_qlinear_q8_dx(rstq_ctx* ctx, DeviceState& ds, const float* dy, co
     int32_t rc = dev_reserve_any_time(ds, &ds.dx_scratch, &ds.dx_scratch_bytes, 2 * yb + rb + cb);
     if (rc != RSTQ_OK) return rc;
     char* base = (char*)ds.dx_scratch;
-    DxPrep q{dy, scales, (__half*)base, (__half*)(base + yb), (float*)(base + 2 * yb), (float*)(base + 2 * yb + rb),
+    DxPrep q{dy, scales, (__half*)base, (__half*)(base + yb), (int*)(base + 2 * yb), (float*)(base + 2 * yb + rb),
              m, out, nb, opad};
     CUtensorMap mw, mh, ml, ms;
     const bool tma_scales = nb % 4 == 0;   // rows of whole 16 bytes
@@ -637,7 +647,7 @@ int32_t launch_qlinear_q8_dx(rstq_ctx* ctx, DeviceState& ds, const float* dy, co
     if (!tma_scales) ms = mw;   // not used then
     RSTQ_CUDA(launch_pdl(dx_prep_kernel, dim3((unsigned)(m + kDxParts)), dim3(256), 0, ds, q));
     ctx->launches++;
-    DxParams p{scales, q.rowscale, q.colmax, dx, ds.status, in, out, tma_scales, (int)m, (int)steps, (int)ttiles, split};
+    DxParams p{scales, q.rowexp, q.colmax, dx, ds.status, in, out, tma_scales, (int)m, (int)steps, (int)ttiles, split};
     RSTQ_CUDA(nt == 32   ? dx_launch<32>(ds, p, (int)tiles, mw, mh, ml, ms)
               : nt == 64 ? dx_launch<64>(ds, p, (int)tiles, mw, mh, ml, ms)
                          : dx_launch<128>(ds, p, (int)tiles, mw, mh, ml, ms));

@@ -49,10 +49,11 @@ def test_dx_at_the_edges(ctx, m, in_, out):
           (rng.standard_normal(out * in_ // 32) * 0.01).astype(np.float32))
 
 
-@pytest.mark.parametrize("row,col", [(1e-41, 1.0), (1e30, 1e-30), (1e-20, 1e15), (1e34, 1e-36)])
-def test_dx_keeps_rows_and_column_blocks_of_any_magnitude(ctx, row, col):
-    """A token row and a column block far below the rest keep their own relative precision."""
-    m, in_, out = 40, 256, 320
+@pytest.mark.parametrize("m,in_,out", [(40, 256, 320), (20, 256, 2048)])   # whole tiles, tiles shared by a cluster
+@pytest.mark.parametrize("row,col", [(1e-41, 1.0), (1e30, 1e-30), (1e-20, 1e15), (1e34, 1e-36), (1e-36, 1e34), (1e-30, 1e30),
+                                     (1e-41, 1e34), (1e34, 1e-41)])
+def test_dx_keeps_rows_and_column_blocks_of_any_magnitude(ctx, row, col, m, in_, out):
+    """A token row and a column block far above or below the rest keep their own relative precision."""
     rng = np.random.default_rng(5)
     dy = (rng.uniform(0.5, 1, (m, out)) * rng.choice([-1, 1], (m, out))).astype(np.float32)
     dy[7] *= np.float32(row)
