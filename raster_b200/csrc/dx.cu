@@ -3,24 +3,21 @@
 // the dequant-transpose GEMM dX = dY . dequant(W), W = [out, in] signed 8-bit codes in the
 // reference's row-major layout with one f32 scale per 32 columns.
 //
-// Two launches.  dx_prep_kernel rewrites the f32 factors as pairs of fp16 (value = hi + lo, 22 significant
-// bits; a power of two per token row / per 32-column block keeps both in range), dx_tmem_kernel is a
-// tcgen05 GEMM over them with the weights dequantized on the way into tensor memory:
+// Two launches.  dx_prep_kernel writes dy as three bf16 terms, dx_tmem_kernel is a tcgen05 GEMM over them with the
+// weights dequantized, in f32, and split the same way on their way into tensor memory:
 //
-//   D[128 columns i, NT tokens] += W'[i, o] * dy[m, o],  W' = Wh + Wl, dy = Yh + Yl
-//                                = Wh Yh + Wh Yl + Wl Yh      (Wl Yl is below 2^-22 of the product)
+//   D[128 columns i, NT tokens] += W'[i, o] * dy[m, o],  W' = W1 + W2 + W3, dy = Y1 + Y2 + Y3
+//                                = W1 Y1 + (W1 Y2 + W2 Y1) + (W1 Y3 + W2 Y2 + W3 Y1)
 //
-// which is an f32-grade product (measured <= 4e-7 of max|dx| against the f64 oracle) at three fp16 MMAs.
-// The f32 scale times an integer code needs no wider arithmetic: with s = sh + sl in fp16,
-// Wh = rn(c sh), the residual c sh - Wh is exact in an fp16 fma, Wl = rn(c sl + residual).
+// Three terms hold all 24 bits of an f32 (each is rounded to nearest, so the rest takes the sign bit with it), and what
+// is left out is below 2^-24 of the product: the f32 product of the f32 values, whatever the spread inside a row or
+// a column block, at six bf16 MMAs.  A power of two per token row and per 32-column block keeps elements down to
+// 2^-130 of the largest beside them out of bf16's subnormals.
+// (Pairs of fp16 terms need three MMAs, but hold 22 bits, and those only of elements above 2^-17 of their row's
+// largest, scales above 2^-9: a scale 2^-20 of its block's largest kept 11 bits.)
 //
-// What bounds it: the tensor core, nominally 192 cycles per 16 rows o of a 128 x 128 tile.  Yh and Yl lie one
-// above the other in shared memory, so Wh times both is ONE instruction of twice the width: two MMAs per 16 rows
-// (128 + 64 cycles) instead of three of 64, because a tcgen05 instruction costs its issuer 50 - 60 cycles.
-// Measured, us per call back to back (before: bf16 mma.sync with three terms, 263 / 898):
-//   4096 x 4096, m = 512: 56.5 (0.91 PFLOP/s of fp16 MMAs; the loop 49, at 1200 cycles per 64 rows and 1.68 GHz:
-//   with neither copies nor conversions 1028 -- 1.6 PFLOP/s for the chip, cuBLAS's own rate on it, so what is left
-//   is power), m = 2048: 213, m = 64: 23.5
+#include <type_traits>
+
 #include "internal.h"
 #include "mma_helpers.cuh"
 #include "tcgen05_helpers.cuh"
@@ -28,15 +25,19 @@
 namespace rstq {
 
 constexpr int kDxStep = 64;                    // rows o per pipeline stage
-constexpr int kDxStages = 4;                   // dy in shared memory and W' in tensor memory
-constexpr int kDxRaw = 8;                      // codes and scales in shared memory
+constexpr int kDxDy = 3;                       // stages of dy in shared memory
+constexpr int kDxRaw = 8;                      // stages of codes and scales in shared memory
 constexpr int kDxSet = 8;                      // dequant warps of a stage: 4 blocks of 32 columns x 2 halves of its rows
 constexpr int kDxDq = 2 * kDxSet;              // two sets on alternate stages
 constexpr int kDxThreads = (kDxDq + 3) * 32;   // + two copy warps and the MMA warp
 constexpr int kDxCodes = kDxStep * 128;        // bytes of codes per stage
 constexpr int kDxScales = 1024;                // bytes of scales per stage: 64 rows x 4 blocks
 constexpr int kDxRawBytes = kDxCodes + kDxScales;
-__host__ __device__ constexpr int dx_ring_bytes(int nt) { return kDxStages * 2 * nt * 128 + kDxRaw * kDxRawBytes; }
+__host__ __device__ constexpr int dx_ring_bytes(int nt) { return kDxDy * 3 * nt * 128 + kDxRaw * kDxRawBytes; }
+// Tensor memory: the accumulators (nt columns each), then the ring of W' (32 columns per term and stage).
+constexpr int kDxWCols = 96;
+__host__ __device__ constexpr int dx_accs(int nt) { return nt > 64 ? 2 : 3; }
+__host__ __device__ constexpr int dx_wstages(int nt) { return (512 - dx_accs(nt) * nt) / kDxWCols; }   // 2, 3 or 4
 
 // Position p of an element inside its group of 16 rows o: the order in which a lane of the dequant warps holds
 // them (rows 2t, 2t + 1, 2t + 8, 2t + 9 for t = p / 4).  Any order serves, as long as dy has the same one; this
@@ -48,8 +49,8 @@ constexpr int kDxParts = 64;                   // thread blocks that look at the
 struct DxPrep {
     const float* dy;
     const float* scales;
-    __half *yh, *yl;        // [m][opad]
-    int* rowexp;            // [m]: e, the row holds dy * 2^-e with max|.| in [2^13, 2^14)
+    uint16_t* y;            // [3][m][opad]: bf16 terms of dy * 2^-e
+    int* rowexp;            // [m]: e, which brings max|dy| of the row into [2^19, 2^20)
     float* colmax;          // [kDxParts][nb]: max|scale| of a part's rows
     int64_t m, out, nb, opad;
 };
@@ -63,14 +64,13 @@ __device__ __forceinline__ int dx_exponent(float mx, int top, float* down, float
         frexpf(mx, &ex);
         e = ex - top;
     }
-    e = e < -149 ? -149 : e;   // 2^-149 is the smallest f32
     const int e1 = e < -100 ? -100 : e;
     *down = ldexpf(1.0f, -e1);
     *down2 = ldexpf(1.0f, e1 - e);
     return e;
 }
 // v * 2^e.  In two halves, whose powers f32 holds and between which nothing leaves its range that the result does
-// not leave; below 2^-252 every v here (< 2^60) ends as zero.  (ldexpf does the same 3 us slower over 512 x 4096 results.)
+// not leave; below 2^-252 every v here (< 2^71) ends as zero.  (ldexpf does the same 3 us slower over 512 x 4096 results.)
 __device__ __forceinline__ float dx_scale(float v, int e) {
     e = e < -252 ? -252 : e;
     const int h = e >> 1;
@@ -87,17 +87,28 @@ __device__ __forceinline__ float dx_block_max(float mx, float* red) {   // 256 t
     __syncthreads();
     return mx;
 }
-__device__ __forceinline__ void dx_split(float a, float b, uint32_t* hi, uint32_t* lo) {
-    const __half2 h = __floats2half2_rn(a, b);
-    const float2 f = __half22float2(h);
-    // (an infinity has no remainder)
-    const __half2 l = __floats2half2_rn(fabsf(f.x) < 7e4f ? a - f.x : 0.f, fabsf(f.y) < 7e4f ? b - f.y : 0.f);
-    *hi = *reinterpret_cast<const uint32_t*>(&h);
-    *lo = *reinterpret_cast<const uint32_t*>(&l);
+// b (upper half) and a (lower half) as three bf16 terms each.  INF: an infinity goes into the last term, which meets the
+// first term of the other factor alone -- next to the zeros among the other terms it would come out as a NaN.
+template <bool INF>
+__device__ __forceinline__ void dx_terms(float b, float a, uint32_t* t1, uint32_t* t2, uint32_t* t3) {
+    uint32_t keep = 0xFFFFFFFFu;
+    if (INF) {
+        if (isinf(a)) keep &= 0xFFFF0000u;
+        if (isinf(b)) keep &= 0x0000FFFFu;
+    }
+    const uint32_t p1 = pack_bf16x2(b, a) & keep;
+    a -= __uint_as_float(p1 << 16);
+    b -= __uint_as_float(p1 & 0xFFFF0000u);
+    const uint32_t p2 = pack_bf16x2(b, a) & keep;
+    a -= __uint_as_float(p2 << 16);
+    b -= __uint_as_float(p2 & 0xFFFF0000u);
+    *t1 = p1;
+    *t2 = p2;
+    *t3 = pack_bf16x2(b, a);
 }
 
 // Latency-bound: every element is read once into registers (rows up to 8192), found the maximum of, and written
-// as two halves; the blocks that look at the scales read theirs as one run and leave a maximum per column block
+// as three terms; the blocks that look at the scales read theirs as one run and leave a maximum per column block
 // (a strip of column blocks per thread block instead took 45 us at 4096 x 4096: 16 bytes of every row).
 constexpr int kDxMaxCols = 4096;
 __global__ void __launch_bounds__(256)
@@ -184,18 +195,18 @@ dx_prep_kernel(const DxPrep p) {
         }
     }
     float down, down2;
-    const int e = dx_exponent(dx_block_max(mx, s_red), 14, &down, &down2);
+    const int e = dx_exponent(dx_block_max(mx, s_red), 20, &down, &down2);
     auto store16 = [&](int64_t o, const float (&v)[16]) {
-        uint32_t h[8], l[8];
+        uint32_t t[3][8];
 #pragma unroll
-        for (int q = 0; q < 8; ++q)   // half2 q: positions 2q, 2q + 1
-            dx_split(v[dx_row_of(2 * q)] * down * down2, v[dx_row_of(2 * q + 1)] * down * down2, &h[q], &l[q]);
-        uint4* dh = reinterpret_cast<uint4*>(p.yh + m * p.opad + o);
-        uint4* dl = reinterpret_cast<uint4*>(p.yl + m * p.opad + o);
-        dh[0] = make_uint4(h[0], h[1], h[2], h[3]);
-        dh[1] = make_uint4(h[4], h[5], h[6], h[7]);
-        dl[0] = make_uint4(l[0], l[1], l[2], l[3]);
-        dl[1] = make_uint4(l[4], l[5], l[6], l[7]);
+        for (int q = 0; q < 8; ++q)   // positions 2q, 2q + 1
+            dx_terms<true>(v[dx_row_of(2 * q + 1)] * down * down2, v[dx_row_of(2 * q)] * down * down2, &t[0][q], &t[1][q], &t[2][q]);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            uint4* d = reinterpret_cast<uint4*>(p.y + (k * p.m + m) * p.opad + o);
+            d[0] = make_uint4(t[k][0], t[k][1], t[k][2], t[k][3]);
+            d[1] = make_uint4(t[k][4], t[k][5], t[k][6], t[k][7]);
+        }
     };
     if (keep) {
 #pragma unroll
@@ -224,19 +235,9 @@ struct DxParams {
     int m, steps, ttiles, split;   // split: thread blocks (one cluster) that share a tile, each a range of o
 };
 
-__device__ __forceinline__ uint32_t hsub2_u32(uint32_t a, uint32_t b) {
-    uint32_t d;
-    asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-    return d;
-}
 __device__ __forceinline__ uint32_t lds_u32(uint32_t a) {
     uint32_t v;
     asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
-    return v;
-}
-__device__ __forceinline__ uint4 lds_u128(uint32_t a) {
-    uint4 v;
-    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
     return v;
 }
 // A copy thread that gave up: let the copies it has issued land before this block's shared memory goes away.
@@ -252,71 +253,76 @@ __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-// The MMAs of one stage (64 rows o) as one block of instructions: per 16 rows Wh against (Yh, Yl) and Wl against
-// Yh.  The barrier of the next stage is tested among them and the answer read at the end: tested after the last
-// MMA instead, the round trips of the tests left the tensor core idle for 400 of 1225 cycles per stage.
-__device__ __forceinline__ uint32_t dx_mma_step(uint32_t d, uint32_t w, uint32_t b_lo, uint32_t b_hi, uint32_t id_both, uint32_t id_hi,
-                                                uint32_t accumulate, uint32_t leader, uint32_t next_bar, uint32_t next_parity) {
-    uint32_t next_ready;
-    asm volatile(
-        "{\n"
-        ".reg .pred p, q, t, r;\n"
-        ".reg .b64 b0, b1, b2, b3;\n"
-        ".reg .b32 h1, h2, h3, l0, l1, l2, l3, b;\n"
-        "setp.ne.b32 p, %7, 0;\n"
-        "setp.ne.b32 q, %8, 0;\n"
-        "setp.eq.b32 t, 0, 0;\n"
-        "mov.b64 b0, {%3, %4};\n"
-        "add.u32 b, %3, 2; mov.b64 b1, {b, %4};\n"
-        "add.u32 b, %3, 4; mov.b64 b2, {b, %4};\n"
-        "add.u32 b, %3, 6; mov.b64 b3, {b, %4};\n"
-        "add.u32 h1, %2, 8;  add.u32 h2, %2, 16; add.u32 h3, %2, 24;\n"
-        "add.u32 l0, %2, 32; add.u32 l1, %2, 40; add.u32 l2, %2, 48; add.u32 l3, %2, 56;\n"
-        "tcgen05.fence::after_thread_sync;\n"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%1], [%2], b0, %5, p;\n"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%1], [l0], b0, %6, t;\n"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%1], [h1], b1, %5, t;\n"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%1], [l1], b1, %6, t;\n"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%1], [h2], b2, %5, t;\n"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%1], [l2], b2, %6, t;\n"
-        "mbarrier.test_wait.parity.shared::cta.b64 r, [%9], %10;\n"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%1], [h3], b3, %5, t;\n"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%1], [l3], b3, %6, t;\n"
-        "selp.u32 %0, 1, 0, r;\n"
-        "}"
-        : "=r"(next_ready)
-        : "r"(d), "r"(w), "r"(b_lo), "r"(b_hi), "r"(id_both), "r"(id_hi), "r"(accumulate), "r"(leader), "r"(next_bar), "r"(next_parity)
-        : "memory");
-    return next_ready;
+// The MMAs of 16 rows o.  The three terms of dy lie one above the other in shared memory, so a term of W' times several
+// of them is one instruction as far as the width allows (256): a tcgen05 instruction costs its issuer 50 - 60
+// cycles, and A is read from tensor memory once for both.  Up to 64 tokens the accumulators are the three sums in
+// the order of their size.  Above, W2 Y1 goes to the first product for the sake of that: 4096 x 4096, m = 512 102.6 ->
+// 91.9 us, 2-norm error against the f64 product 4.4e-6 -> 9.2e-6 (three bf16 terms of dy * s on mma.sync: 1.1e-5;
+// pairs of fp16: 9.7e-6 -- the f32 sums decide it, not the products).
+template <int NT>
+__device__ __forceinline__ void dx_mma16(uint32_t d, uint32_t w, uint32_t b_lo, uint32_t b_hi, uint32_t accumulate, uint32_t leader) {
+    constexpr uint32_t id1 = idesc_bf16(NT), id2 = idesc_bf16(2 * NT), id3 = idesc_bf16(NT <= 64 ? 3 * NT : NT);
+    if constexpr (NT <= 64) {
+        asm volatile(
+            "{\n"
+            ".reg .pred p, q, t;\n"
+            ".reg .b64 b0;\n"
+            "setp.ne.b32 p, %10, 0;\n"
+            "setp.ne.b32 q, %11, 0;\n"
+            "setp.eq.b32 t, 0, 0;\n"
+            "mov.b64 b0, {%6, %7};\n"
+            "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%3], b0, %12, p;\n"   // W1 (Y1, Y2, Y3)
+            "@q tcgen05.mma.cta_group::1.kind::f16 [%1], [%4], b0, %9, t;\n"    // W2 (Y1, Y2)
+            "@q tcgen05.mma.cta_group::1.kind::f16 [%2], [%5], b0, %8, t;\n"    // W3 Y1
+            "}" ::"r"(d), "r"(d + NT), "r"(d + 2 * NT), "r"(w), "r"(w + 32), "r"(w + 64), "r"(b_lo), "r"(b_hi), "r"(id1), "r"(id2),
+            "r"(accumulate), "r"(leader), "r"(id3)
+            : "memory");
+    } else {
+        asm volatile(
+            "{\n"
+            ".reg .pred p, q, t;\n"
+            ".reg .b64 b0, b2;\n"
+            "setp.ne.b32 p, %8, 0;\n"
+            "setp.ne.b32 q, %9, 0;\n"
+            "setp.eq.b32 t, 0, 0;\n"
+            "mov.b64 b0, {%5, %7};\n"
+            "mov.b64 b2, {%6, %7};\n"
+            "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%2], b0, %11, p;\n"   // W1 (Y1, Y2)
+            "@q tcgen05.mma.cta_group::1.kind::f16 [%1], [%2], b2, %10, t;\n"   // W1 Y3
+            "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%3], b0, %11, t;\n"   // W2 (Y1, Y2)
+            "@q tcgen05.mma.cta_group::1.kind::f16 [%1], [%4], b0, %10, t;\n"   // W3 Y1
+            "}" ::"r"(d), "r"(d + NT), "r"(w), "r"(w + 32), "r"(w + 64), "r"(b_lo), "r"(b_lo + 2 * NT * 8), "r"(b_hi), "r"(accumulate),
+            "r"(leader), "r"(id1), "r"(id2)
+            : "memory");
+    }
 }
 
 // Warps 0 .. 15 dequantize and store the tile (warp & 3 = 32-column block = its tensor-memory lanes, (warp >> 2) & 1 =
-// half of the stage's rows o, warp >> 3 = even / odd stages), warp 16 copies codes and scales, 17 issues the MMAs, 18 copies dy.  The codes have a
-// ring of their own, twice as deep: one ring for everything made a stage wait for copy, conversion and MMA in turn
-// (3000 cycles; with four stages 1250 per step against the 768 of the MMAs).  Tensor memory: columns 0 .. NT-1 hold
-// Wh Yh + Wl Yh, NT .. 2 NT-1 Wh Yl, 256 .. 511 the ring of W' (32 columns Wh, 32 Wl per stage).
+// half of the stage's rows o, warp >> 3 = even / odd stages), warp 16 copies codes and scales, 17 issues the MMAs, 18
+// copies dy.  Codes, dy and W' have rings of their own: with one ring a stage waited for copy, conversion and MMA in turn.
 // Tensor-memory lane gid + 8 r of a block is column 4 gid + r of it: a lane of the dequant warp reads the codes
 // of four neighbouring columns as one word per row, and the 16x256b store wants exactly these four lanes of it.
 // Every mbarrier wait is time-bounded; on expiry the block reports through the status word, lets its copies
 // land, still meets its barriers and frees its tensor memory.
 template <int NT>
 __global__ void __launch_bounds__(kDxThreads, 1)
-dx_tmem_kernel(const DxParams p, const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_h,
-               const __grid_constant__ CUtensorMap map_l, const __grid_constant__ CUtensorMap map_s) {
-    constexpr int YB = NT * 128;                 // bytes of Yh (or Yl) per stage
+dx_tmem_kernel(const DxParams p, const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_y,
+               const __grid_constant__ CUtensorMap map_s) {
+    constexpr int YB = 3 * NT * 128;             // bytes of dy per stage
+    constexpr int WS = dx_wstages(NT), ACC = dx_accs(NT) * NT;
     extern __shared__ uint8_t smem_raw[];
     __shared__ int s_abort;
     __shared__ uint32_t s_tmem;
     __shared__ int s_colexp[4];
-    __shared__ __align__(8) uint64_t s_bar[2 * kDxStages + 2 * kDxRaw + 1];
+    __shared__ __align__(8) uint64_t s_bar[2 * kDxDy + 2 * WS + 2 * kDxRaw + 1];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     const uint32_t sbase = smem_u32(smem), bar0 = smem_u32(s_bar);
-    // ready: the stage of dy has arrived and its W' is in tensor memory; empty: its MMAs are done;
+    // y_full: a stage of dy has arrived; w_full: a stage of W' is in tensor memory; y_free, w_free: their MMAs are done;
     // raw: codes and scales of a step have arrived; taken: they are in registers
-    const uint32_t ready = bar0, empty = bar0 + 8 * kDxStages;
-    const uint32_t raw = bar0 + 16 * kDxStages, taken = raw + 8 * kDxRaw, acc_full = taken + 8 * kDxRaw;
-    const uint32_t rbase = sbase + kDxStages * 2 * YB;
+    const uint32_t y_full = bar0, y_free = y_full + 8 * kDxDy, w_full = y_free + 8 * kDxDy, w_free = w_full + 8 * WS;
+    const uint32_t raw = w_free + 8 * WS, taken = raw + 8 * kDxRaw, acc_full = taken + 8 * kDxRaw;
+    const uint32_t rbase = sbase + kDxDy * YB;
     const int part = blockIdx.x % p.split, tile = blockIdx.x / p.split;
     const int ft = tile / p.ttiles, tok0 = (tile - ft * p.ttiles) * NT;
     const int k0 = (int)((int64_t)p.steps * part / p.split), k1 = (int)((int64_t)p.steps * (part + 1) / p.split);
@@ -324,12 +330,15 @@ dx_tmem_kernel(const DxParams p, const __grid_constant__ CUtensorMap map_w, cons
 
     if (tid == 0) {
         asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&map_w)) : "memory");
-        asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&map_h)) : "memory");
-        asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&map_l)) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&map_y)) : "memory");
     }
-    if (tid < kDxStages) {
-        mbar_init(ready + 8 * tid, kDxSet + 1);
-        mbar_init(empty + 8 * tid, 1);
+    if (tid < kDxDy) {
+        mbar_init(y_full + 8 * tid, 1);
+        mbar_init(y_free + 8 * tid, 1);
+    }
+    if (tid < WS) {
+        mbar_init(w_full + 8 * tid, kDxSet);
+        mbar_init(w_free + 8 * tid, 1);
     }
     if (tid < kDxRaw) {
         mbar_init(raw + 8 * tid, 1);
@@ -376,37 +385,40 @@ dx_tmem_kernel(const DxParams p, const __grid_constant__ CUtensorMap map_w, cons
             int s = 0, issued = 0;
             uint32_t ph = 0;
             for (int k = k0; k < k1; ++k) {
-                ok = mbar_block(empty + 8 * s, ph ^ 1u, abort_flag);
+                ok = mbar_block(y_free + 8 * s, ph ^ 1u, abort_flag);
                 if (!ok) break;
-                const uint32_t dst = sbase + s * 2 * YB, bar = ready + 8 * s;
-                mbar_expect_tx(bar, 2 * YB);
-                tma_load_2d(dst, &map_h, k * kDxStep, tok0, bar);
-                tma_load_2d(dst + YB, &map_l, k * kDxStep, tok0, bar);
+                mbar_expect_tx(y_full + 8 * s, YB);
+                tma_load_3d(sbase + s * YB, &map_y, k * kDxStep, tok0, 0, y_full + 8 * s);
                 ++issued;
-                if (++s == kDxStages) { s = 0; ph ^= 1u; }
+                if (++s == kDxDy) { s = 0; ph ^= 1u; }
             }
-            if (!ok) dx_drain(ready, issued, kDxStages);
+            if (!ok) dx_drain(y_full, issued, kDxDy);
         }
     } else if (warp == kDxDq + 1) {
         // ---------------- MMAs ----------------
-        constexpr uint32_t id_both = idesc_f16(2 * NT), id_hi = idesc_f16(NT);
         const uint32_t leader = lane == 0;
         const uint64_t d0 = smem_desc_sw128(sbase);
         const uint32_t d_lo = (uint32_t)d0, d_hi = (uint32_t)(d0 >> 32);
-        int s = 0;
-        uint32_t ph = 0;
-        bool any = false;
-        ok = mbar_spin(ready, 0, abort_flag);
-        for (int k = k0; k < k1 && ok; ++k) {
-            const int s2 = s + 1 == kDxStages ? 0 : s + 1;
-            const uint32_t ph2 = s2 ? ph : ph ^ 1u;
-            const uint32_t n2 = dx_mma_step(tmem, tmem + 256 + s * 64, d_lo + (uint32_t)s * (2 * YB >> 4), d_hi, id_both, id_hi, k != k0,
-                                            leader, ready + 8 * s2, ph2);
-            umma_commit_if(empty + 8 * s, leader);
+        int ys = 0, ws = 0;
+        uint32_t yph = 0, wph = 0;
+        bool any = false, ready = false;
+        for (int k = k0; k < k1; ++k) {
+            if (!ready) ok = mbar_spin(y_full + 8 * ys, yph, abort_flag) && mbar_spin(w_full + 8 * ws, wph, abort_flag);
+            if (!ok) break;
+            tc_fence_after();
+            const uint32_t w = tmem + ACC + ws * kDxWCols, b = d_lo + (uint32_t)ys * (YB >> 4);
+            const int ys2 = ys + 1 == kDxDy ? 0 : ys + 1, ws2 = ws + 1 == WS ? 0 : ws + 1;
+            const uint32_t yph2 = ys2 ? yph : yph ^ 1u, wph2 = ws2 ? wph : wph ^ 1u;
+            dx_mma16<NT>(tmem, w, b, d_hi, k != k0, leader);
+            dx_mma16<NT>(tmem, w + 8, b + 2, d_hi, 1u, leader);
+            dx_mma16<NT>(tmem, w + 16, b + 4, d_hi, 1u, leader);
+            // (the next stage's barriers are tested ahead of the last MMAs: their round trips run beside them)
+            ready = mbar_test(y_full + 8 * ys2, yph2) & mbar_test(w_full + 8 * ws2, wph2);
+            dx_mma16<NT>(tmem, w + 24, b + 6, d_hi, 1u, leader);
+            umma_commit_if(w_free + 8 * ws, leader);
+            umma_commit_if(y_free + 8 * ys, leader);
             any = true;
-            if (k + 1 < k1 && !n2) ok = mbar_spin(ready + 8 * s2, ph2, abort_flag);
-            s = s2;
-            ph = ph2;
+            ys = ys2; ws = ws2; yph = yph2; wph = wph2;
         }
         if (any) {
             umma_commit_if(acc_full, leader);
@@ -427,7 +439,7 @@ dx_tmem_kernel(const DxParams p, const __grid_constant__ CUtensorMap map_w, cons
         // holds as element gid & 3 (eight lanes hold the same eight rows)
         const int my_row = half * 32 + (gid >> 2) * 16 + 2 * t + (gid & 1) + (gid & 2) * 4;
         const uint32_t soff = kDxCodes + my_row * 16 + blk * 4;
-        const uint32_t tdst = tmem + 256 + ((uint32_t)(blk * 32) << 16) + half * 16;
+        const uint32_t tdst = tmem + ACC + ((uint32_t)(blk * 32) << 16) + half * 16;
         const int64_t nb = p.in >> 5, b = (int64_t)ft * 4 + blk;
         asm volatile("griddepcontrol.wait;" ::: "memory");
         float mx = 0.f;
@@ -435,11 +447,12 @@ dx_tmem_kernel(const DxParams p, const __grid_constant__ CUtensorMap map_w, cons
             for (int i = lane; i < kDxParts; i += 32) mx = fmaxf(mx, __ldg(p.colmax + i * nb + b));
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        float down, down2;   // the block's scales are used times 2^-ce, the largest in [2^6, 2^7)
-        const int ce = dx_exponent(mx, 7, &down, &down2);
+        float down, down2;   // the block's scales are used times 2^-ce, the largest in [2^12, 2^13)
+        const int ce = dx_exponent(mx, 13, &down, &down2);
         if (lane == 0) s_colexp[blk] = ce;   // (the four warps of a block of columns agree)
-        int s = set, rs = set;
-        uint32_t ph = 0, rph = 0;
+        const bool infinite = isinf(mx);   // a scale of this column block (of the whole matrix)
+        int ws = set % WS, rs = set;
+        uint32_t wph = 0, rph = 0;
         for (int k = k0 + set; k < k1; k += 2) {
             float sf = 0.f;
             if (!p.tma_scales) {
@@ -458,58 +471,55 @@ dx_tmem_kernel(const DxParams p, const __grid_constant__ CUtensorMap map_w, cons
                 w[g][3] = lds_u32(st + off1 + g * 2048 + 1024);
             }
             if (p.tma_scales) sf = __uint_as_float(lds_u32(st + soff));
-            // split it, and gather the eight the lane's rows need: (sh, sh), (sh, sh), (sl, sl), (sl, sl) per group
-            uint32_t mine;
-            {
-                const float v = sf * down * down2;
-                const __half h = __float2half_rn(v), l = __float2half_rn(v - __half2float(h));
-                mine = (uint32_t)__half_as_ushort(h) | ((uint32_t)__half_as_ushort(l) << 16);
-            }
-            uint4 sc[2];
+            // gather the eight scales the lane's rows need
+            sf *= down;
+            sf *= down2;
+            float sc[2][4];
 #pragma unroll
-            for (int g = 0; g < 2; ++g) {
-                uint32_t v[4];
+            for (int g = 0; g < 2; ++g)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) v[j] = __shfl_sync(0xffffffffu, mine, (g * 4 + j) * 4 + t);
-                sc[g] = make_uint4(__byte_perm(v[0], v[1], 0x5410), __byte_perm(v[2], v[3], 0x5410),
-                                   __byte_perm(v[0], v[1], 0x7632), __byte_perm(v[2], v[3], 0x7632));
-            }
+                for (int j = 0; j < 4; ++j) {
+                    sc[g][j] = __shfl_sync(0xffffffffu, sf, (g * 4 + j) * 4 + t);
+                    w[g][j] ^= 0x80808080u;   // code + 128
+                }
             __syncwarp();
             if (lane == 0) mbar_arrive(taken + 8 * rs);
             rs += 2;
             if (rs >= kDxRaw) { rs -= kDxRaw; rph ^= 1u; }
-            ok = __all_sync(0xffffffffu, mbar_block(empty + 8 * s, ph ^ 1u, abort_flag));
+            ok = __all_sync(0xffffffffu, mbar_block(w_free + 8 * ws, wph ^ 1u, abort_flag));
             if (!ok) break;
             tc_fence_after();
+            auto convert = [&](auto inf) {
 #pragma unroll
-            for (int q = 0; q < 2; ++q) {      // columns 4 gid + 2q, + 2q + 1
-                uint32_t vh[8], vl[8];
+                for (int q = 0; q < 2; ++q) {      // columns 4 gid + 2q, + 2q + 1
+                    uint32_t v1[8], v2[8], v3[8];
 #pragma unroll
-                for (int g = 0; g < 2; ++g)
+                    for (int g = 0; g < 2; ++g)
 #pragma unroll
-                    for (int c = 0; c < 2; ++c) {
-                        const uint32_t sel = (2 * q + c) | ((4 + 2 * q + c) << 8);   // this column's byte of the two rows; the odd bytes are masked away
+                        for (int c = 0; c < 2; ++c)
 #pragma unroll
-                        for (int h = 0; h < 2; ++h) {
-                            const uint32_t sh = h ? sc[g].y : sc[g].x, sl = h ? sc[g].w : sc[g].z;
-                            // (code ^ 0x80) under the exponent byte of 1024 is 1024 + 128 + code exactly
-                            const uint32_t e = __byte_perm(w[g][2 * h], w[g][2 * h + 1], sel);
-                            const uint32_t v = hsub2_u32((e & 0x00FF00FFu) ^ 0x64806480u, 0x64806480u);
-                            const uint32_t hi = hmul2_u32(v, sh);
-                            const uint32_t rest = hfma2_u32(v, sh, hi ^ 0x80008000u);
-                            vh[g * 4 + c * 2 + h] = hi;
-                            vl[g * 4 + c * 2 + h] = hfma2_u32(v, sl, rest);
-                        }
-                    }
-                tmem_st_16x256b_x2(tdst + s * 64 + ((uint32_t)(16 * q) << 16), vh);
-                tmem_st_16x256b_x2(tdst + s * 64 + 32 + ((uint32_t)(16 * q) << 16), vl);
-            }
+                            for (int h = 0; h < 2; ++h) {   // rows 2t + 8h, 2t + 8h + 1
+                                // under the upper half of 2^23 the byte is 2^23 + 128 + code exactly
+                                const uint32_t sel = 0x7440u | (uint32_t)(2 * q + c);
+                                const float a = __uint_as_float(__byte_perm(w[g][2 * h], 0x4B000000u, sel)) - 8388736.0f;
+                                const float b = __uint_as_float(__byte_perm(w[g][2 * h + 1], 0x4B000000u, sel)) - 8388736.0f;
+                                const int e = g * 4 + c * 2 + h;
+                                dx_terms<decltype(inf)::value>(b * sc[g][2 * h + 1], a * sc[g][2 * h], &v1[e], &v2[e], &v3[e]);
+                            }
+                    const uint32_t dst = tdst + ws * kDxWCols + ((uint32_t)(16 * q) << 16);
+                    tmem_st_16x256b_x2(dst, v1);
+                    tmem_st_16x256b_x2(dst + 32, v2);
+                    tmem_st_16x256b_x2(dst + 64, v3);
+                }
+            };
+            if (infinite) convert(std::true_type{});
+            else convert(std::false_type{});
             tmem_st_wait();
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(ready + 8 * s);
-            s += 2;
-            if (s >= kDxStages) { s -= kDxStages; ph ^= 1u; }
+            if (lane == 0) mbar_arrive(w_full + 8 * ws);
+            ws += 2;
+            if (ws >= WS) { ws -= WS; wph ^= 1u; }
         }
         if (ok) ok = __all_sync(0xffffffffu, mbar_block(acc_full, 0, abort_flag));
         tc_fence_after();
@@ -529,6 +539,14 @@ dx_tmem_kernel(const DxParams p, const __grid_constant__ CUtensorMap map_w, cons
                 tmem_ld8(ta + NT + j, *reinterpret_cast<uint32_t(*)[8]>(&b[j]));
             }
             tmem_ld_wait();
+            if constexpr (dx_accs(NT) == 3) {
+                uint32_t c[CH];
+#pragma unroll
+                for (int j = 0; j < CH; j += 8) tmem_ld8(ta + 2 * NT + j, *reinterpret_cast<uint32_t(*)[8]>(&c[j]));
+                tmem_ld_wait();
+#pragma unroll
+                for (int j = 0; j < CH; ++j) b[j] = __float_as_uint(__uint_as_float(b[j]) + __uint_as_float(c[j]));
+            }
 #pragma unroll
             for (int j = 0; j < CH; ++j) {
                 const float v = __uint_as_float(a[j]) + __uint_as_float(b[j]);
@@ -571,11 +589,11 @@ dx_tmem_kernel(const DxParams p, const __grid_constant__ CUtensorMap map_w, cons
     if (tid == 0 && s_abort) atomicExch(p.status, 2);
 }
 
-static bool dx_map(EncodeTiledFn enc, CUtensorMap* map, CUtensorMapDataType type, const void* base, int64_t x, int64_t y,
-                   int64_t stride, int box_x, int box_y, bool swizzle = true) {
-    const cuuint64_t dims[2] = {(cuuint64_t)x, (cuuint64_t)y}, strides[1] = {(cuuint64_t)stride};
-    const cuuint32_t box[2] = {(cuuint32_t)box_x, (cuuint32_t)box_y}, estr[2] = {1, 1};
-    return enc(map, type, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+// dims, box: innermost first; strides: bytes between rows and, of three dimensions, planes
+static bool dx_map(EncodeTiledFn enc, CUtensorMap* map, CUtensorMapDataType type, const void* base, int rank, const cuuint64_t (&dims)[3],
+                   const cuuint64_t (&strides)[2], const cuuint32_t (&box)[3], bool swizzle = true) {
+    const cuuint32_t estr[3] = {1, 1, 1};
+    return enc(map, type, rank, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                swizzle ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
@@ -589,8 +607,8 @@ int32_t dx_configure() {
 }
 
 template <int NT>
-static cudaError_t dx_launch(const DeviceState& ds, const DxParams& p, int tiles, const CUtensorMap& w, const CUtensorMap& h,
-                             const CUtensorMap& l, const CUtensorMap& s) {
+static cudaError_t dx_launch(const DeviceState& ds, const DxParams& p, int tiles, const CUtensorMap& w, const CUtensorMap& y,
+                             const CUtensorMap& s) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(tiles * p.split));
     cfg.blockDim = dim3(kDxThreads);
@@ -611,7 +629,7 @@ static cudaError_t dx_launch(const DeviceState& ds, const DxParams& p, int tiles
     }
     cfg.attrs = a;
     cfg.numAttrs = (unsigned)n;
-    return cudaLaunchKernelEx(&cfg, dx_tmem_kernel<NT>, p, w, h, l, s);
+    return cudaLaunchKernelEx(&cfg, dx_tmem_kernel<NT>, p, w, y, s);
 }
 
 int32_t launch_qlinear_q8_dx(rstq_ctx* ctx, DeviceState& ds, const float* dy, const int8_t* codes,
@@ -630,27 +648,28 @@ int32_t launch_qlinear_q8_dx(rstq_ctx* ctx, DeviceState& ds, const float* dy, co
     int split = 1;
     while (split < 8 && tiles * split * 2 <= ds.sm_count && steps >= 16 * split) split *= 2;
 
-    const int64_t yb = (m * opad * 2 + 255) & ~255ll, rb = (m * 4 + 255) & ~255ll, cb = kDxParts * nb * 4;
-    int32_t rc = dev_reserve_any_time(ds, &ds.dx_scratch, &ds.dx_scratch_bytes, 2 * yb + rb + cb);
+    const int64_t yb = (3 * m * opad * 2 + 255) & ~255ll, rb = (m * 4 + 255) & ~255ll, cb = kDxParts * nb * 4;
+    int32_t rc = dev_reserve_any_time(ds, &ds.dx_scratch, &ds.dx_scratch_bytes, yb + rb + cb);
     if (rc != RSTQ_OK) return rc;
     char* base = (char*)ds.dx_scratch;
-    DxPrep q{dy, scales, (__half*)base, (__half*)(base + yb), (int*)(base + 2 * yb), (float*)(base + 2 * yb + rb),
-             m, out, nb, opad};
-    CUtensorMap mw, mh, ml, ms;
+    DxPrep q{dy, scales, (uint16_t*)base, (int*)(base + yb), (float*)(base + yb + rb), m, out, nb, opad};
+    CUtensorMap mw, my, ms;
     const bool tma_scales = nb % 4 == 0;   // rows of whole 16 bytes
-    RSTQ_REQUIRE(dx_map(enc, &mw, CU_TENSOR_MAP_DATA_TYPE_UINT8, codes, in, out, in, 128, kDxStep) &&
-                     dx_map(enc, &mh, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, q.yh, opad, m, opad * 2, kDxStep, nt) &&
-                     dx_map(enc, &ml, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, q.yl, opad, m, opad * 2, kDxStep, nt) &&
-                     (!tma_scales || dx_map(enc, &ms, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, scales, nb, out, nb * 4, 4, kDxStep, false)),
+    const cuuint64_t i_ = (cuuint64_t)in, o_ = (cuuint64_t)out, m_ = (cuuint64_t)m, op_ = (cuuint64_t)opad, nb_ = (cuuint64_t)nb;
+    RSTQ_REQUIRE(dx_map(enc, &mw, CU_TENSOR_MAP_DATA_TYPE_UINT8, codes, 2, {i_, o_, 1}, {i_, 0}, {128, kDxStep, 1}) &&
+                     dx_map(enc, &my, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, q.y, 3, {op_, m_, 3}, {op_ * 2, op_ * m_ * 2},
+                            {kDxStep, (cuuint32_t)nt, 3}) &&
+                     (!tma_scales || dx_map(enc, &ms, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, scales, 2, {nb_, o_, 1}, {nb_ * 4, 0},
+                                            {4, kDxStep, 1}, false)),
                  RSTQ_E_CUDA, "cuTensorMapEncodeTiled failed (m = %lld, in = %lld, out = %lld)", (long long)m, (long long)in,
                  (long long)out);
     if (!tma_scales) ms = mw;   // not used then
     RSTQ_CUDA(launch_pdl(dx_prep_kernel, dim3((unsigned)(m + kDxParts)), dim3(256), 0, ds, q));
     ctx->launches++;
     DxParams p{scales, q.rowexp, q.colmax, dx, ds.status, in, out, tma_scales, (int)m, (int)steps, (int)ttiles, split};
-    RSTQ_CUDA(nt == 32   ? dx_launch<32>(ds, p, (int)tiles, mw, mh, ml, ms)
-              : nt == 64 ? dx_launch<64>(ds, p, (int)tiles, mw, mh, ml, ms)
-                         : dx_launch<128>(ds, p, (int)tiles, mw, mh, ml, ms));
+    RSTQ_CUDA(nt == 32   ? dx_launch<32>(ds, p, (int)tiles, mw, my, ms)
+              : nt == 64 ? dx_launch<64>(ds, p, (int)tiles, mw, my, ms)
+                         : dx_launch<128>(ds, p, (int)tiles, mw, my, ms));
     ctx->launches++;
     return RSTQ_OK;
 }

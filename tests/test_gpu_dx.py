@@ -29,10 +29,11 @@ def check(ctx, m, in_, out, dy, codes, scales):
     dx = run(ctx, m, in_, out, dy, codes, scales)
     w = codes.reshape(out, in_).astype(np.float64) * np.repeat(scales.reshape(out, in_ // 32).astype(np.float64), 32, axis=1)
     d = dy.reshape(m, out).astype(np.float64)
-    # Per product: two halves of 11 bits each hold a factor to 2^-22 of it, and the product of the two low
-    # halves (2^-22 at most) is left out.  Per sum: 16 products at a time are added to an f32, each addition
-    # off by at most 2^-23 of the sum of magnitudes; up to 8 partial sums and two scalings follow.
-    bound = (3 * 2.0 ** -22 + (out / 16 + 12) * 2.0 ** -23) * (np.abs(d) @ np.abs(w))
+    # Per product: code * scale is rounded to f32 (2^-24), both factors are then held whole, and what the six products of
+    # their terms leave out is at most 2 * 2^-8 * 2^-17 of it.  Per sum: 16 products at a time are added to an f32, twice
+    # (first and second terms), each addition off by at most 2^-23 of the sum of magnitudes; up to 8 partial sums and
+    # two scalings follow.
+    bound = (2 * 2.0 ** -24 + (out / 8 + 12) * 2.0 ** -23) * (np.abs(d) @ np.abs(w))
     assert np.all(np.abs(dx - d @ w) <= bound)
     assert np.abs(dx - d @ w).max() <= 2e-5 * np.abs(d @ w).max() + 1e-300
 
@@ -68,6 +69,48 @@ def test_dx_keeps_rows_and_column_blocks_of_any_magnitude(ctx, row, col, m, in_,
             a, b = dx[rows, cols], want[rows, cols]
             # 2e-5 as above, and half a step of the subnormal grid of the result
             assert np.abs(a - b).max() <= 2e-5 * np.abs(b).max() + 1.5e-45 * (1 if np.abs(b).max() < 1e-37 else 0)
+
+
+@pytest.mark.parametrize("m,in_,out", [(8, 96, 320), (40, 256, 320), (130, 128, 70)])
+@pytest.mark.parametrize("below", [12, 24, 40, 90])
+@pytest.mark.parametrize("what", ["dy", "scales"])
+def test_dx_holds_all_bits_of_small_elements(ctx, what, below, m, in_, out):
+    """Elements 2^-below of the largest of their row (scales: of their column block), which meets zeros: what
+    remains is the sum of the small ones, with the precision that f32 gives it."""
+    rng = np.random.default_rng(below)
+    dy = (rng.uniform(0.5, 1, (m, out)) * rng.choice([-1, 1], (m, out))).astype(np.float32)
+    scales = rng.uniform(0.5, 1, (out, in_ // 32)).astype(np.float32)
+    codes = rng.integers(-127, 128, (out, in_)).astype(np.int8)
+    if what == "dy":
+        dy[:, 1:] *= np.float32(2.0 ** -below)
+        codes[0] = 0
+    else:
+        scales[1:] *= np.float32(2.0 ** -below)
+        dy[:, 0] = 0
+    dx = run(ctx, m, in_, out, dy.ravel(), codes.ravel(), scales.ravel())
+    w = codes.astype(np.float64) * np.repeat(scales.astype(np.float64), 32, axis=1)
+    d = dy.astype(np.float64)
+    assert np.all(np.abs(dx - d @ w) <= (2 * 2.0 ** -24 + (out / 8 + 12) * 2.0 ** -23) * (np.abs(d) @ np.abs(w)))
+
+
+@pytest.mark.parametrize("m", [3, 40])
+def test_dx_of_infinities_and_nans(ctx, m):
+    """What f32 arithmetic makes of them: an infinity times a code of zero is a NaN, else an infinity of its sign; other
+    rows and other column blocks do not notice."""
+    in_, out = 128, 200
+    rng = np.random.default_rng(1)
+    dy = rng.standard_normal((m, out)).astype(np.float32)
+    dy[0, 7], dy[1, 9], dy[2, 70] = np.inf, np.nan, -np.inf
+    codes = rng.integers(-127, 128, (out, in_)).astype(np.int8)
+    codes[7, ::5] = 0
+    scales = rng.uniform(0.25, 0.5, (out, in_ // 32)).astype(np.float32)
+    scales[13, 2] = np.inf
+    with np.errstate(all="ignore"):
+        w = codes.astype(np.float32) * np.repeat(scales, 32, axis=1)
+        want = np.stack([(dy[i][:, None] * w).sum(0) for i in range(m)])
+    dx = run(ctx, m, in_, out, dy.ravel(), codes.ravel(), scales.ravel())
+    assert np.array_equal(np.isnan(dx), np.isnan(want))
+    assert np.array_equal(dx[np.isinf(want)], want[np.isinf(want)]) and np.isfinite(dx[np.isfinite(want)]).all()
 
 
 def test_dx_recorded_without_a_first_call(ctx):
