@@ -184,14 +184,16 @@ __device__ __forceinline__ void attn_finish(const AttnParams& p, float* s_part, 
     if (!*s_last_p) return;
     // The last CTA of this KV head merges the S slices.  What it reads -- maxima, sums, weighted V -- lies a trip to L2
     // away, and three such trips in a row were most of this tail: warp g takes the (max, sum) pairs of head g, up
-    // to kPairs per lane at once, while every thread requests its first kHold weighted values; then the slice weights
-    // exp(m_s - M) go round through shared memory (the per-warp states are dead by now; the host keeps
-    // S + 1 <= 8 * row).
+    // to kPairs per lane at once (128 slices: more than one per SM is rare), while every thread requests its first kHold
+    // weighted values; then the slice weights exp(m_s - M) go round through shared memory (the per-warp states are dead
+    // by now; the host keeps S + 1 <= 8 * row).  kHold: 148 SMs give 32 heads 18 slices, so 20 covers most calls; with
+    // one head per CTA four CTAs share an SM at 64 registers, where 20 (and 18, 14, 12) spill and 16 does not:
+    // 32 / 32 heads x 1024 10.65 -> 9.92 us, 16 / 16 x 2048 12.2 -> 10.8, four 7B layers 220.7 -> 218.3.
     const float* all = p.part + (((int64_t)hkv * gridDim.z + gz) * p.S * GS) * row;
     const int S = p.S;
     float* s_w = s_part;            // [gc][S] weights
     float* s_L = s_part + gc * S;   // [gc]
-    constexpr int kPairs = 4, kHold = 20;
+    constexpr int kPairs = 4, kHold = GS == 1 ? 16 : 20;
     float held[kHold];
     {
         const int i = threadIdx.x, g = i / hd, d = i - g * hd;
