@@ -569,7 +569,9 @@ __device__ __forceinline__ int64_t gemm_range_start(const GemmParams& p, int64_t
 
 // SEGS: ranges that touch several tiles, and rows whose last K-step is a partial one.  A kernel of its own: with the
 // loop over segments and the second K loop around it a single tile ran 3 % slower (4096 x 4096, M = 512: 21.3 ->
-// 22.0 us).
+// 22.0 us); with what is left of the bookkeeping (ring positions, segment lengths, a division per role) as constants
+// there, int8 4096 x 4096 takes 24.42 us at M = 512 (24.58 without, 24.38 before there were segments), 18.6 at
+// M = 256 (18.8).
 template <int BITS, int NTOK, bool SEGS>
 __global__ void __launch_bounds__(kGemmThreadsT, 1)
 gemm_tmem_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tmap) {
@@ -615,18 +617,19 @@ gemm_tmem_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tmap) {
         k_first = (int)(r0 - (uint32_t)tile_first * KS);
         steps_own = (int)((uint32_t)gemm_range_start(p, cta + 1) - r0);
     }
+    const int ft_first = tile_first / p.ttiles, tok_first = (tile_first - ft_first * p.ttiles) * NTOK;
 
     if (tid == 0) asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmap)) : "memory");
     if (warp >= 2 && warp < 2 + kDqWarps) {
         // the first weights this warp will load: ask for them now, so that the HBM round trip
         // runs while the CTA sets itself up (barriers, tensor memory, the CTA-wide sync)
         const int t = (warp - 2) >> 2, pset = t & 1, blk0 = 2 * (t >> 1);
-        int64_t g = (int64_t)(tile_first / p.ttiles) * 4 + (warp & 3);
+        int64_t g = (int64_t)ft_first * 4 + (warp & 3);
         g = g < p.ngroups ? g : (int64_t)p.ngroups - 1;
 #pragma unroll
         for (int d = 0; d < 2; ++d) {
             const int b = 4 * (k_first + pset + 2 * d) + blk0;
-            if (b + 1 < p.nb && lane * 128 < 2 * UNIT)
+            if ((SEGS ? b + 1 < p.nb : pset + 2 * d < steps_own) && lane * 128 < 2 * UNIT)
                 asm volatile("prefetch.global.L2 [%0];" ::"l"(p.w + (g * p.nb + b) * UNIT + lane * 128));
         }
     }
@@ -634,7 +637,7 @@ gemm_tmem_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tmap) {
         mbar_init(full + 8 * tid, kDqWarps / 2 + 1);
         mbar_init(empty + 8 * tid, 1);
     } else if (tid == kNSTT) {
-        mbar_init(acc_full, ISS);   // one arrival per MMA issuer and segment
+        mbar_init(acc_full, ISS == 2 && (SEGS || steps_own >= 2) ? 2 : 1);   // one arrival per MMA issuer (that has steps) and segment
         mbar_init(acc_free, kDqWarps);
         s_abort = 0;
     }
@@ -662,9 +665,8 @@ gemm_tmem_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tmap) {
             int s = 0, issued = 0, seg = 0, left = steps_own;
             uint32_t ph = 0;
             bool ok = true;
-            for (int tile = tile_first, k0 = k_first; ok; ++tile, k0 = 0) {
-                const int n = min(KS - k0, left);
-                const int ft = tile / p.ttiles, tok0 = (tile - ft * p.ttiles) * NTOK;
+            for (int tile = tile_first, k0 = k_first, ft = ft_first, tok0 = tok_first; ok; k0 = 0) {
+                const int n = SEGS ? min(KS - k0, left) : steps_own;
                 const int nb_end = min(p.nb, 4 * (k0 + n));
                 auto request = [&](int ks) {  // K-steps ks .. ks + 3 of this segment
                     const int b0 = 4 * (k0 + ks);
@@ -680,7 +682,7 @@ gemm_tmem_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tmap) {
                         }
                     }
                 };
-                if (seg == 0) {
+                if (!SEGS || seg == 0) {
                     asm volatile("griddepcontrol.wait;" ::: "memory");  // activations come from the pre-pass
                 } else {
                     // a further tile: its first weights on their way while the epilogue of the one before runs
@@ -691,7 +693,7 @@ gemm_tmem_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tmap) {
                     // weight requests: none before the wait above (they would compete for HBM with the
                     // pre-pass this kernel waits for) nor before the first activation tiles are on their
                     // way; the dequant warps load K-steps 0 .. 3 themselves
-                    if (seg == 0 && ks == kNSTT)
+                    if ((!SEGS || seg == 0) && ks == kNSTT)
                         for (int k2 = 4; k2 < 8 + kPfSteps; k2 += 4) request(k2);
                     if ((ks & 3) == 0 && ks >= 4) request(ks + 4 + kPfSteps);
                     ok = mbar_block(empty + 8 * s, ph ^ 1u, abort_flag);
@@ -705,6 +707,9 @@ gemm_tmem_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tmap) {
                 }
                 if (!SEGS || (left -= n) == 0) break;
                 ++seg;
+                ++tile;
+                ft = tile / p.ttiles;
+                tok0 = (tile - ft * p.ttiles) * NTOK;
             }
             if (!ok) {  // let the copies already issued land before this CTA's shared memory goes away
                 for (int k = issued > kNSTT ? issued - kNSTT : 0; k < issued; ++k) {
@@ -735,11 +740,11 @@ gemm_tmem_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tmap) {
         bool any = false, ok = true;
         int q0 = 0, seg = 0, left = steps_own;
         for (int k0 = k_first; ok; k0 = 0) {
-            const int n = min(KS - k0, left);
-            const int first = ISS == 2 ? (m + q0) & 1 : 0;   // this issuer's first step of the segment: q0 + first = m (mod 2)
-            int s = (q0 + first) % kNSTT;
-            uint32_t ph = (uint32_t)((q0 + first) / kNSTT) & 1u;
-            if (seg > 0) ok = mbar_spin(acc_free, (uint32_t)(seg - 1) & 1u, abort_flag);
+            const int n = SEGS ? min(KS - k0, left) : steps_own;
+            const int first = ISS == 2 ? (SEGS ? (m + q0) & 1 : m) : 0;   // this issuer's first step of the segment: q0 + first = m (mod 2)
+            int s = SEGS ? (q0 + first) % kNSTT : first;
+            uint32_t ph = SEGS ? (uint32_t)((q0 + first) / kNSTT) & 1u : 0u;
+            if (SEGS && seg > 0) ok = mbar_spin(acc_free, (uint32_t)(seg - 1) & 1u, abort_flag);
             if (ok && first < n) ok = mbar_spin(full + 8 * s, ph, abort_flag);
             if (dbg && lane == 0 && seg == 0) dbg[306 + 2 * m] = (unsigned long long)clock64();
             for (int ks = first; ks < n && ok; ks += ISS) {
@@ -757,7 +762,7 @@ gemm_tmem_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tmap) {
                 ph = ph2;
             }
             if (dbg && lane == 0) dbg[307 + 2 * m] = (unsigned long long)clock64();
-            if (ok || any) umma_commit_if(acc_full, leader);   // (arrives at once where this issuer had no step)
+            if (any || (SEGS && ok)) umma_commit_if(acc_full, leader);   // (arrives at once where this issuer had no step)
             if (!ok && any) {  // gave up: the tensor core must be idle before tensor memory is freed
                 const unsigned long long t0 = gtime_ns();
                 while (!mbar_try(acc_full, (uint32_t)seg & 1u) && gtime_ns() - t0 < kWaitLimitNs) {
@@ -825,11 +830,10 @@ gemm_tmem_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tmap) {
         const uint32_t s_delta = (uint32_t)(CODES + gid * 16 - lane * 16);
         bool ok = true;
         int q0 = 0, seg = 0, left = steps_own;
-        for (int tile = tile_first, k0 = k_first;; ++tile, k0 = 0) {   // (also when a wait ran out: the warps meet at a barrier)
-        const int n = min(KS - k0, left);
-        const int ft = tile / p.ttiles, tok0 = (tile - ft * p.ttiles) * NTOK;
+        for (int tile = tile_first, k0 = k_first, ft = ft_first, tok0 = tok_first;; k0 = 0) {   // (also when a wait ran out: the warps meet at a barrier)
+        const int n = SEGS ? min(KS - k0, left) : steps_own;
         {
-            const int first = (pset + q0) & 1;            // own steps: q0 + first + 2 i
+            const int first = SEGS ? (pset + q0) & 1 : pset;   // own steps: q0 + first + 2 i
             const int n_own = (n - first + 1) >> 1;
             int64_t g_ld = (int64_t)ft * 4 + grp;         // (groups beyond the matrix: any valid rows, never stored)
             g_ld = g_ld < p.ngroups ? g_ld : (int64_t)p.ngroups - 1;
@@ -933,7 +937,7 @@ gemm_tmem_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tmap) {
             int got = 1;
             if (lane == 0) {
                 const unsigned long long t0 = gtime_ns();
-                for (int k = 1; k <= takes && got; ++k) {
+                for (int k = 1; k <= (SEGS ? takes : 1) && got; ++k) {
                     for (;;) {
                         int v;
                         asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p.part_flags + cta + k) : "memory");
@@ -963,7 +967,7 @@ gemm_tmem_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tmap) {
                 uint32_t v[CH];
                 // (a segment of one step has its sums in that step's accumulator alone)
                 const uint32_t t0 = tmem + ((uint32_t)(sp * 32) << 16) + (uint32_t)(cq * CPW + h * CH) +
-                                    (ISS == 2 && n == 1 ? (uint32_t)(q0 & 1) * NTOK : 0u);
+                                    (SEGS && ISS == 2 && n == 1 ? (uint32_t)(q0 & 1) * NTOK : 0u);
 #pragma unroll
                 for (int c0 = 0; c0 < CH; c0 += 8) tmem_ld8(t0 + c0, *reinterpret_cast<uint32_t(*)[8]>(&v[c0]));
                 tmem_ld_wait();
@@ -1039,13 +1043,16 @@ gemm_tmem_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tmap) {
             asm volatile("bar.sync 6, %0;" ::"r"(kDqWarps * 32) : "memory");
             if (dq == 0 && lane == 0) {
                 if (!giver)
-                    for (int k = 1; k <= takes; ++k) p.part_flags[cta + k] = 0;
+                    for (int k = 1; k <= (SEGS ? takes : 1); ++k) p.part_flags[cta + k] = 0;
                 else if (ok) asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(p.part_flags + cta), "r"(1) : "memory");
             }
         }
         if (!SEGS || (left -= n) == 0) break;
         q0 += n;
         ++seg;
+        ++tile;
+        ft = tile / p.ttiles;
+        tok0 = (tile - ft * p.ttiles) * NTOK;
         if (ok) {   // the accumulators and the activation stages are free for the next segment
             fence_async_smem();
             tc_fence_before();
