@@ -161,9 +161,12 @@ RSTQ_API int32_t rstq_shutdown(rstq_ctx* ctx);
 /* How the prefill GEMM (M above the decode kernel's range) would tile a call on a device of sm_count SMs
  * at the default settings: plan2[0] = tokens per tile (32, 64, 128 or 256), plan2[1] = thread blocks per
  * tile (2 = each takes half of K; the second hands its sums to the first; 1 also where whole tiles would leave
- * most SMs idle in the last wave and the thread blocks take equal ranges of all tiles' K instead).  Pure host arithmetic: no
+ * most SMs idle in the last wave and the thread blocks take equal ranges of all tiles' K instead: rstq_gemm_ranges).  Pure host arithmetic: no
  * device, no context.  No counterpart in the reference (its GEMM is one work-item per output). */
 RSTQ_API int32_t rstq_gemm_plan(int32_t* plan2, int64_t out, int64_t in, int64_t m, int32_t sm_count);
+/* In how many equal ranges of all tiles' K-steps (thread blocks) that call would run; 0 = as whole tiles, or two thread
+ * blocks per tile (rstq_gemm_plan).  Pure host arithmetic as well. */
+RSTQ_API int32_t rstq_gemm_ranges(int32_t* ranges, int64_t out, int64_t in, int64_t m, int32_t sm_count);
 /* What the FIRST decode launch of rstq_qmatmul (mode, bits 4 / 8, act_dtype) on an out x in weight with m tokens
  * would be at the default settings on a device of sm_count SMs: plan6[0] = tokens it takes (up to 16; 0 = a
  * row of activations does not fit at all), [1] = ring stages, [2] = units per chunk, [3] = 1 when the

@@ -600,17 +600,27 @@ int32_t rstq_shutdown(rstq_ctx* ctx) {
     return RSTQ_OK;
 }
 
-int32_t rstq_gemm_plan(int32_t* plan2, int64_t out, int64_t in, int64_t m, int32_t sm_count) {
-    RSTQ_REQUIRE(plan2, RSTQ_E_INVALID, "null argument");
+static int32_t plan_of(int64_t out, int64_t in, int64_t m, int32_t sm_count, int* ntok, bool* split, int* ranges) {
     RSTQ_REQUIRE(out >= 1 && in >= 32 && in % 32 == 0 && m >= 1 && sm_count >= 1, RSTQ_E_SHAPE,
                  "out = %lld, in = %lld, m = %lld, sm_count = %d", (long long)out, (long long)in, (long long)m, sm_count);
-    int ntok = 0;
+    gemm_plan(out, in, m, sm_count, true, 0, ntok, split, ranges);
+    return RSTQ_OK;
+}
+int32_t rstq_gemm_plan(int32_t* plan2, int64_t out, int64_t in, int64_t m, int32_t sm_count) {
+    RSTQ_REQUIRE(plan2, RSTQ_E_INVALID, "null argument");
+    int ntok = 0, ranges = 0;
     bool split = false;
-    int ranges = 0;
-    gemm_plan(out, in, m, sm_count, true, 0, &ntok, &split, &ranges);
+    const int32_t rc = plan_of(out, in, m, sm_count, &ntok, &split, &ranges);
+    if (rc != RSTQ_OK) return rc;
     plan2[0] = ntok;
     plan2[1] = split ? 2 : 1;
     return RSTQ_OK;
+}
+int32_t rstq_gemm_ranges(int32_t* out_ranges, int64_t out, int64_t in, int64_t m, int32_t sm_count) {
+    RSTQ_REQUIRE(out_ranges, RSTQ_E_INVALID, "null argument");
+    int ntok = 0;
+    bool split = false;
+    return plan_of(out, in, m, sm_count, &ntok, &split, out_ranges);
 }
 
 int32_t rstq_decode_plan(int32_t* plan6, int32_t mode, int32_t bits, int64_t out, int64_t in, int64_t m, int32_t act_dtype,

@@ -29,6 +29,13 @@ def gemm_plan(out: int, in_: int, m: int, sm_count: int = 148) -> dict:
     return {"tile_tokens": plan[0], "blocks_per_tile": plan[1]}
 
 
+def gemm_ranges(out: int, in_: int, m: int, sm_count: int = 148) -> int:
+    """In how many equal ranges of all tiles' K-steps that call would run (rstq_gemm_ranges); 0 = as gemm_plan says."""
+    n = C.c_int32()
+    L.check(L.load().rstq_gemm_ranges(C.byref(n), out, in_, m, sm_count))
+    return n.value
+
+
 def decode_plan(mode: int, bits: int, out: int, in_: int, m: int, act_dtype: int = L.F32, sm_count: int = 148) -> dict:
     """What the first decode launch of a call would be (rstq_decode_plan: host arithmetic, no device): tokens it
     takes, ring stages, units per chunk, whether the activations ride the weight ring, dynamic shared memory,

@@ -89,6 +89,28 @@ def test_gemm_plan_is_host_arithmetic_and_follows_the_wave_model():
     assert lib.rstq_gemm_plan(None, 4096, 4096, 64, 148) == L.E_INVALID
 
 
+def test_gemm_ranges_where_whole_tiles_leave_sms_idle():
+    """rstq_gemm_ranges: one range per SM where whole tiles would leave SMs idle for much of the last wave, whole tiles
+    (or pairs) on the other side of the line.  Whatever is chosen, the parts of ranges fit the scratch they go to
+    (160 parts of 128 x 256 sums) and there are no more than 256 of them."""
+    from raster_b200 import runtime as R
+    for out, in_, m in [(28672, 8192, 32), (28672, 8192, 256), (11008, 4096, 512)]:
+        assert R.gemm_ranges(out, in_, m) == 148
+    for out, in_, m in [(8192, 8192, 512), (12288, 4096, 300), (4096, 4096, 768), (4096, 4096, 512), (4096, 4096, 64)]:
+        assert R.gemm_ranges(out, in_, m) == 0
+    for sm in (1, 20, 74, 132, 148, 160, 200, 296):
+        for out in (32, 1000, 4096, 11008, 28672, 131072):
+            for in_ in (32, 160, 1024, 4128, 28672):
+                for m in (17, 33, 64, 100, 129, 300, 512, 2048):
+                    n = R.gemm_ranges(out, in_, m, sm)
+                    p = R.gemm_plan(out, in_, m, sm)
+                    assert 0 <= n <= min(sm, 256) and n * p["tile_tokens"] <= 160 * 256
+                    assert n == 0 or p["blocks_per_tile"] == 1
+    with pytest.raises(Exception):
+        R.gemm_ranges(4096, 100, 64)
+    assert L.load().rstq_gemm_ranges(None, 4096, 4096, 64, 148) == L.E_INVALID
+
+
 def test_decode_plan_is_host_arithmetic_and_always_fits_shared_memory():
     """rstq_decode_plan needs no device: what the first decode launch of a call would be.  One token keeps its
     activations resident; several tokens of MODE_A8 ride the weight ring in one launch whatever K is (three
