@@ -96,7 +96,13 @@ def test_gemm_ranges_where_whole_tiles_leave_sms_idle():
     from raster_b200 import runtime as R
     for out, in_, m in [(28672, 8192, 32), (28672, 8192, 256), (11008, 4096, 512)]:
         assert R.gemm_ranges(out, in_, m) == 148
-    for out, in_, m in [(8192, 8192, 512), (12288, 4096, 300), (4096, 4096, 768), (4096, 4096, 512), (4096, 4096, 64)]:
+    for out, in_, m in [(20000, 2048, 200), (14336, 4096, 512), (5120, 5120, 1024), (22016, 4096, 32), (24576, 3072, 20),
+                        (24576, 3072, 64), (28672, 4096, 64)]:
+        assert R.gemm_ranges(out, in_, m) == 148
+    # one wave, too little saved, too many tiles per range, rows of one or two K-steps
+    for out, in_, m in [(8192, 8192, 512), (12288, 4096, 300), (4096, 4096, 768), (4096, 4096, 512), (4096, 4096, 64),
+                        (4096, 4096, 2048), (4096, 11008, 2048), (27648, 1024, 256), (6144, 8192, 1024), (9000, 6144, 900),
+                        (5120, 13824, 300), (26000, 2048, 32), (11008, 4096, 1024), (11008, 4096, 2048), (28672, 256, 2048), (28672, 128, 2048)]:
         assert R.gemm_ranges(out, in_, m) == 0
     for sm in (1, 20, 74, 132, 148, 160, 200, 296):
         for out in (32, 1000, 4096, 11008, 28672, 131072):
