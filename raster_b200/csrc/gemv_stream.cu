@@ -32,6 +32,8 @@
 //    instead of hanging.
 #include <string.h>
 
+#include <type_traits>
+
 #include "internal.h"
 #include "mma_helpers.cuh"
 #include "sync_helpers.cuh"
@@ -129,10 +131,13 @@ struct StreamParams {
 // 32 764 bytes) and every thread block quantizes them from there -- no copy, no second launch and no read over PCIe.
 template <int N>
 struct StreamParamsX : StreamParams {
-    float xv[N];
+    alignas(16) float xv[N];   // read 16 bytes at a time
 };
+template <typename P>
+constexpr bool kXInParams = !std::is_same_v<P, StreamParams>;
 constexpr int kParamXSmall = 4096, kParamXLarge = kParamXMax;
 static_assert(sizeof(StreamParamsX<kParamXLarge>) <= 32764, "kernel parameter limit");
+static_assert(alignof(StreamParamsX<kParamXSmall>) == 16 && alignof(StreamParamsX<kParamXLarge>) == 16, "16-byte loads of xv");
 
 __device__ __forceinline__ void consumer_bar() {
     asm volatile("bar.sync 1, %0;" ::"n"(kConsumers) : "memory");
@@ -1107,7 +1112,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) gemv_stream_kernel(const __
                                  : "memory");
         }
     };
-    if constexpr (sizeof(P) > sizeof(StreamParams)) {
+    if constexpr (kXInParams<P>) {
         stage_a8_quant<BITS, true>(p, p.xv, smem, tid);
     } else if (QF) {
         stage_a8_quant<BITS, false, UK>(p, p.x, smem, tid);
