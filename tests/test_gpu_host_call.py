@@ -32,8 +32,9 @@ def test_host_call(ctx, bits, out, in_):
         assert np.abs(fn(x, wqi, wsi, in_, out, ctx) - ref).max() <= 4e-6 * np.abs(ref).max()
 
 
-def test_results_that_are_the_waiting_pattern_end_the_call(ctx):
-    """A scale of infinity makes every result a NaN: the wait must end although results may never 'arrive'."""
+def test_nan_results_are_returned(ctx):
+    """A scale of infinity makes every result a NaN (another one than the pattern that is waited for to go: the wait for
+    that is tested in test_host_wait.py)."""
     out, in_ = 64, 256
     codes = np.full(out * in_, 200, np.uint8)
     scales = np.full(out * in_ // 32, np.float32(np.inf))
