@@ -132,15 +132,24 @@ class ClockSampler:
                 "reasons": sorted(reasons), "samples": len(sm)}
 
 
-def make_weights(rank=0):
-    """Quantized host weights of both shapes in the reference layouts."""
+def make_weights(rank=0, by_oracle=False):
+    """Quantized host weights of both shapes in the reference layouts.  by_oracle: through the oracle's quantizer and
+    layout (the same bytes), without this library in the process."""
     from raster_b200 import synth
-    from raster_b200.quant import cpu_quant as cq
+    if by_oracle:
+        from oracle import oracle as orc
+    else:
+        from raster_b200.quant import cpu_quant as cq
     ws = []
     for i, (name, out, in_) in enumerate(SHAPES):
         w = synth.normal(SEED_W + 10 * i + 1000 * rank, out * in_, SIGMA_W)
-        q = cq.quantize_weight(w, cq.q4_0)
-        r = cq.repack_stream(q["wq"], q["ws"], out, in_, cq.q4_0)
+        if by_oracle:
+            wq, s = orc.quantize_weight(w, 4)
+            wqi, wsi = orc.repack_stream(wq, s, out, in_, 4, 8)
+            q, r = {"wq": wq, "ws": s}, {"wqi": wqi, "wsi": wsi}
+        else:
+            q = cq.quantize_weight(w, cq.q4_0)
+            r = cq.repack_stream(q["wq"], q["ws"], out, in_, cq.q4_0)
         x = synth.normal(SEED_X + 10 * i, 8 * in_)
         ws.append({"name": name, "out": out, "in": in_, "wq": q["wq"], "ws": q["ws"],
                    "wqi": r["wqi"], "wsi": r["wsi"], "x": x})
@@ -979,7 +988,7 @@ def run_reference(args):
     the GPU arm: both shapes over R rotated weight copies per step."""
     if int(os.environ.get("RANK", "0")) != 0:
         return
-    weights = make_weights(0)
+    weights = make_weights(0, by_oracle=True)
     per_pass = sum(stream_bytes(w["out"], w["in"]) for w in weights)
     from oracle import oracle as orc
     try:
