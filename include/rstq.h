@@ -240,7 +240,8 @@ RSTQ_API int32_t rstq_weight_bind_q6k(rstq_ctx* ctx, rstq_weight** w, const void
 /* The host codecs these arrays come from, on the host's cores (no device, no context): quantize-weight
  * (src/raster/compiler/backend/cpu/quant.clj:42-70; format Q4_0 or Q8_0, codes n/2 or n bytes, scales n/32),
  * quantize-weight-q4k (:95-150) and quantize-weight-q6k (:222-262), n elements of f32.  Bit for bit the
- * reference's double arithmetic.  Returns 1, with the outputs undefined, when w holds an infinity or a NaN. */
+ * reference's double arithmetic.  Returns 1, with the outputs undefined, when w holds an infinity or a NaN;
+ * _q4k also for a super-block whose minimum is some 2^31 times a sub-block's step (its codes are beyond 32 bits). */
 RSTQ_API int32_t rstq_quantize_weight(const float* w, void* codes, float* scales, int64_t n, int32_t format);
 RSTQ_API int32_t rstq_quantize_weight_q4k(const float* w, void* wq, float* da, float* db, int8_t* aq, int8_t* bq,
                                           int64_t n);

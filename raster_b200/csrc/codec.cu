@@ -6,12 +6,13 @@
 // vectorizes, and then the read of the f32 matrix; blocks are independent, so the array is cut over the
 // host's cores.  Measured at 4096 x 4096 on 16 cores: 4 ms (q4_0, q8_0), 5 - 6 ms (q4_K, q6_K); 4 ns per element
 // and core.
-// Only finite inputs are taken: the callers keep the general path for the rest (return value 1).
+// Only finite inputs are taken, and of q4_K only minima that do not dwarf their block's spread: the callers keep the
+// general path for the rest (return value 1).
 //
-// Compiled for AVX2 without fused multiply-add, and for the base architecture: a contracted product would
-// round differently from the reference's two steps.
-// (comparisons may then be turned into masks; results do not change)
-#pragma GCC optimize("no-trapping-math")
+// Compiled for AVX2 (on x86) and for the base architecture, without contraction into fused multiply-adds: a contracted
+// product would round differently from the reference's two steps.
+// (no trapping math: comparisons may then be turned into masks; results do not change)
+#pragma GCC optimize("no-trapping-math", "fp-contract=off")
 #include <math.h>
 #include <string.h>
 
@@ -22,7 +23,13 @@
 
 namespace rstq {
 
+#if defined(__x86_64__) && !defined(RSTQ_NO_AVX2)
 #define RSTQ_AVX2 __attribute__((target("avx2")))
+#define RSTQ_HAS_AVX2() ((bool)__builtin_cpu_supports("avx2"))
+#else   // other hosts: the base architecture's form alone
+#define RSTQ_AVX2
+#define RSTQ_HAS_AVX2() false
+#endif
 #define RSTQ_INLINE static inline __attribute__((always_inline))
 
 // Math.round of v (nearest integer, ties upward) for |v| < 2^31: v - trunc(v) is exact, so the two
@@ -228,7 +235,7 @@ static int32_t run_codec(const Job& job, int64_t blocks, int64_t block_elems) {
         const Job* job;
         bool avx2;
         int bad[33];
-    } arg{&job, (bool)__builtin_cpu_supports("avx2"), {0}};
+    } arg{&job, RSTQ_HAS_AVX2(), {0}};
     host_parallel(blocks, 65536 / block_elems, [](void* p, int slot, int64_t b0, int64_t b1) {
         Arg& a = *(Arg*)p;
         const bool ok = a.avx2 ? a.job->avx2(b0, b1) : a.job->base(b0, b1);

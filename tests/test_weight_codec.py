@@ -1,8 +1,13 @@
 """The library's host codecs against the numpy form of the same arithmetic: every byte equal."""
+import ctypes as C
+import os
+import subprocess
+
 import numpy as np
 import pytest
 
 from raster_b200 import _lib as L
+from raster_b200 import build
 from raster_b200.quant import cpu_quant as cq
 
 CODECS = {"q4_0": lambda w: cq.quantize_weight(w, cq.q4_0), "q8_0": lambda w: cq.quantize_weight(w, cq.q8_0),
@@ -52,3 +57,28 @@ def test_codec_entry_points_check_their_arguments():
     assert lib.rstq_quantize_weight(p, p, p, 32, L.FMT_Q8_S) == L.E_INVALID
     assert lib.rstq_quantize_weight_q4k(p, p, p, p, p, p, 128) == L.E_SHAPE
     assert lib.rstq_quantize_weight_q6k(p, p, p, None, 256) == L.E_INVALID
+
+
+@pytest.fixture(scope="module")
+def base_form(tmp_path_factory):
+    """The codecs as a host without AVX2 (one that is no x86, for instance) compiles them."""
+    cuda = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(build._nvcc()))), "include")
+    d = tmp_path_factory.mktemp("codec")
+    (d / "c.cpp").write_text('#include "codec.cu"\nnamespace rstq { void set_error(const char*, ...) {} }\n')
+    subprocess.run(["g++", "-O3", "-std=c++17", "-shared", "-fPIC", "-pthread", "-DRSTQ_NO_AVX2", "-I", build.CSRC, "-I", cuda,
+                    "-I", os.path.join(build.HERE, "..", "include"), str(d / "c.cpp"), "-o", str(d / "c.so")], check=True)
+    lib = C.CDLL(str(d / "c.so"))
+    for n in ("rstq_quantize_weight", "rstq_quantize_weight_q4k", "rstq_quantize_weight_q6k"):
+        getattr(lib, n).argtypes = L.SIGNATURES[n]
+    return lib
+
+
+@pytest.mark.parametrize("fmt", sorted(CODECS))
+@pytest.mark.parametrize("kind", ["normal", "ties", "wide range", "far from zero"])
+def test_base_form_gives_the_same_bytes(monkeypatch, base_form, fmt, kind):
+    w = values(kind, 256 * 67)
+    want = CODECS[fmt](w)
+    monkeypatch.setattr(L, "load", lambda: base_form)
+    got = CODECS[fmt](w)
+    for k in want:
+        assert got[k].tobytes() == want[k].tobytes(), k
