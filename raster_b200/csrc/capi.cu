@@ -356,11 +356,17 @@ static cudaError_t put_products(rstq_ctx* ctx, DeviceState& ds, const ProductSca
     return cudaGetLastError();
 }
 static int64_t products_tmp_bytes(int64_t n, int per) { return ((n / per * 4 + 255) & ~255ll) + ((n + 255) & ~255ll); }
-static void trim_bind_stage(DeviceState& ds) {
-    if (ds.bind_stage_bytes <= kBindStageKeep) return;
+static void trim_bind_stage(DeviceState& ds, int64_t keep = kBindStageKeep) {
+    if (ds.bind_stage_bytes <= keep) return;
     cudaFree(ds.bind_stage);
     ds.bind_stage = nullptr;
     ds.bind_stage_bytes = 0;
+}
+// The staging block for `need` bytes.  An outgrown one is freed, not parked: no graph names it, and every bind has
+// waited for its copies.
+static int32_t reserve_bind_stage(DeviceState& ds, int64_t need) {
+    if (need > ds.bind_stage_bytes && !ds.capturing) trim_bind_stage(ds, 0);
+    return dev_reserve(ds, &ds.bind_stage, &ds.bind_stage_bytes, need);
 }
 
 // `products`: the block scales as products (whole matrix, row-major; `scales` is then not read); d == nullptr
@@ -440,7 +446,7 @@ static int32_t bind_impl(rstq_ctx* ctx, rstq_weight** wout, const void* codes,
     // it took as long as the copy of a 10 MB matrix.
     const int64_t scales_off = (codes_bytes + 255) & ~255ll, tmp_off = scales_off + ((scales_bytes + 255) & ~255ll);
     const int64_t tmp_bytes = products && products->d ? products_tmp_bytes(sh_out * nb_full, products->per) : 0;
-    if ((rc = dev_reserve(ds, &ds.bind_stage, &ds.bind_stage_bytes, tmp_off + tmp_bytes)) != RSTQ_OK) {
+    if ((rc = reserve_bind_stage(ds, tmp_off + tmp_bytes)) != RSTQ_OK) {
         delete w;
         return rc;
     }
@@ -897,7 +903,7 @@ int32_t rstq_weight_bind_q4k(rstq_ctx* ctx, rstq_weight** wout, const void* wq, 
     if (rc != RSTQ_OK) return rc;
     w->zp = 0;  // codes are 0 .. 15 as they stand; the offset is the min term
     DeviceState& ds = ctx->devs[dev];
-    if ((rc = dev_reserve(ds, &ds.bind_stage, &ds.bind_stage_bytes, products_tmp_bytes(n, 8))) != RSTQ_OK) {
+    if ((rc = reserve_bind_stage(ds, products_tmp_bytes(n, 8))) != RSTQ_OK) {
         rstq_weight_free(w);
         return rc;
     }
@@ -954,7 +960,7 @@ int32_t rstq_weight_bind_q6k(rstq_ctx* ctx, rstq_weight** wout, const void* wq, 
         if (rc != RSTQ_OK) return rc;
         DeviceState& ds = ctx->devs[dev];
         const int64_t d16_bytes = (n16 * 4 + 255) & ~255ll;
-        if ((rc = dev_reserve(ds, &ds.bind_stage, &ds.bind_stage_bytes, d16_bytes + products_tmp_bytes(n16, 16))) != RSTQ_OK) {
+        if ((rc = reserve_bind_stage(ds, d16_bytes + products_tmp_bytes(n16, 16))) != RSTQ_OK) {
             rstq_weight_free(w);
             return rc;
         }
