@@ -498,27 +498,21 @@ constexpr int kWeightPfSteps = 8;  // K-steps of packed weights requested into L
 // One 128-element K-step as a single block of instructions, so that nothing but a branch sits
 // between the last MMA of a step and the first of the next: eight MMAs (A columns a0 + 8 kk, B
 // descriptor b_lo + 2 (kk & 3) + BHALF (kk >> 2) in 16-byte units, BHALF = second 64-element half
-// of the stage), with the two barrier operations of the pipeline tucked in between them where the
-// issuing lane is waiting for the tensor core anyway: the commit that frees the PREVIOUS stage
-// (it then also covers the first MMAs of this one, so that stage is released a little later,
-// which the ring absorbs) and a non-blocking test of the NEXT stage's barrier, whose answer is
-// read at the end.  first = 0 makes MMA 0 overwrite the accumulator; lanes with leader = 0
-// issue no tensor-core instruction.
+// of the stage), with a non-blocking test of the NEXT stage's barrier tucked in between them, where the
+// issuing lane is waiting for the tensor core anyway; its answer is read at the end.  first = 0
+// makes MMA 0 overwrite the accumulator; lanes with leader = 0 issue no tensor-core instruction.
 template <int BHALF>
 __device__ __forceinline__ uint32_t umma_f16_ts_step(uint32_t d_tmem, uint32_t a0, uint32_t b_lo, uint32_t b_hi,
                                                      uint32_t idesc, uint32_t first, uint32_t leader,
-                                                     uint32_t prev_empty, uint32_t commit_prev,
                                                      uint32_t next_full, uint32_t next_parity) {
     uint32_t next_ready;
     asm volatile(
         "{\n"
-        ".reg .pred p, q, t, r, c;\n"
+        ".reg .pred p, q, t, r;\n"
         ".reg .b64 bd0, bd1, bd2, bd3, bd4, bd5, bd6, bd7;\n"
         ".reg .b32 a1, a2, a3, a4, a5, a6, a7, b;\n"
         "setp.ne.b32 p, %6, 0;\n"
         "setp.ne.b32 q, %7, 0;\n"
-        "setp.ne.b32 c, %13, 0;\n"
-        "and.pred c, c, q;\n"
         "setp.eq.b32 t, 0, 0;\n"
         "mov.b64 bd0, {%3, %4};\n"
         "add.u32 a1, %2, 8;  add.u32 b, %3, 2;   mov.b64 bd1, {b, %4};\n"
@@ -531,9 +525,8 @@ __device__ __forceinline__ uint32_t umma_f16_ts_step(uint32_t d_tmem, uint32_t a
         "tcgen05.fence::after_thread_sync;\n"
         "@q tcgen05.mma.cta_group::1.kind::f16 [%1], [%2], bd0, %5, p;\n"
         "@q tcgen05.mma.cta_group::1.kind::f16 [%1], [a1], bd1, %5, t;\n"
-        "mbarrier.test_wait.parity.shared::cta.b64 r, [%14], %15;\n"
+        "mbarrier.test_wait.parity.shared::cta.b64 r, [%12], %13;\n"
         "@q tcgen05.mma.cta_group::1.kind::f16 [%1], [a2], bd2, %5, t;\n"
-        "@c tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%12];\n"
         "@q tcgen05.mma.cta_group::1.kind::f16 [%1], [a3], bd3, %5, t;\n"
         "@q tcgen05.mma.cta_group::1.kind::f16 [%1], [a4], bd4, %5, t;\n"
         "@q tcgen05.mma.cta_group::1.kind::f16 [%1], [a5], bd5, %5, t;\n"
@@ -543,8 +536,7 @@ __device__ __forceinline__ uint32_t umma_f16_ts_step(uint32_t d_tmem, uint32_t a
         "}"
         : "=r"(next_ready)
         : "r"(d_tmem), "r"(a0), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(first), "r"(leader), "n"(BHALF),
-          "n"(BHALF + 2), "n"(BHALF + 4), "n"(BHALF + 6), "r"(prev_empty), "r"(commit_prev), "r"(next_full),
-          "r"(next_parity)
+          "n"(BHALF + 2), "n"(BHALF + 4), "n"(BHALF + 6), "r"(next_full), "r"(next_parity)
         : "memory");
     return next_ready;
 }
@@ -753,8 +745,8 @@ gemm_tmem_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tmap) {
                 if (s2 >= kNSTT) { s2 -= kNSTT; ph2 ^= 1u; }
                 const uint32_t a0 = tmem + A_COL0 + s * kAColsPerStage, b_lo = d_lo + (uint32_t)s * (BSTAGE >> 4);
                 // the block also tests the barrier of this issuer's next step (ks + ISS) early
-                const uint32_t n2 = umma_f16_ts_step<NTOK * 8>(dcol, a0, b_lo, d_hi, idesc, ks != first, leader, empty, 0u,
-                                                               full + 8 * s2, ph2);
+                const uint32_t n2 = umma_f16_ts_step<NTOK * 8>(dcol, a0, b_lo, d_hi, idesc, ks != first, leader, full + 8 * s2,
+                                                               ph2);
                 umma_commit_if(empty + 8 * s, leader);  // the stage is free once these MMAs have read it
                 any = true;
                 if (ks + ISS < n && !n2) ok = mbar_spin(full + 8 * s2, ph2, abort_flag);

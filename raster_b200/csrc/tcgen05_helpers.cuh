@@ -97,16 +97,7 @@ __device__ __forceinline__ void tmem_st_16x256b_x2(uint32_t taddr, const uint32_
 __device__ __forceinline__ void tmem_st_wait() {
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
-// D[tmem] (+)= A[tmem] * B[smem desc], issued by the lanes whose `leader` is non-zero (one lane).
-// The descriptor comes as two words so that stepping through a stage is one 32-bit add.
-__device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint32_t bdesc_lo, uint32_t bdesc_hi,
-                                            uint32_t idesc, uint32_t accumulate, uint32_t leader) {
-    asm volatile(
-        "{ .reg .pred p, q; .reg .b64 bd; setp.ne.b32 p, %5, 0; setp.ne.b32 q, %6, 0; mov.b64 bd, {%2, %3}; "
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], bd, %4, p; }" ::"r"(d_tmem),
-        "r"(a_tmem), "r"(bdesc_lo), "r"(bdesc_hi), "r"(idesc), "r"(accumulate), "r"(leader)
-        : "memory");
-}
+// umma_commit by the lanes whose `leader` is non-zero (one lane)
 __device__ __forceinline__ void umma_commit_if(uint32_t bar, uint32_t leader) {
     asm volatile(
         "{ .reg .pred q; setp.ne.b32 q, %1, 0; "
