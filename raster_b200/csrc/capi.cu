@@ -61,20 +61,37 @@ int32_t dev_reserve(DeviceState& ds, void** p, int64_t* have, int64_t need) {
     return RSTQ_OK;
 }
 
-// The same for an operator that callers may record without a first call outside the capture: the allocation
-// does not belong to the capture, and an outgrown block is parked like any that a graph may name.
-int32_t dev_reserve_any_time(DeviceState& ds, void** p, int64_t* have, int64_t need) {
-    if (need <= *have || !ds.capturing) return dev_reserve(ds, p, have, need);
-    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-    RSTQ_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
-    void* fresh = nullptr;
-    need = (need + 0xFFFFF) & ~0xFFFFFll;
-    const cudaError_t e = cudaMalloc(&fresh, (size_t)need);
-    RSTQ_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
-    RSTQ_CUDA(e);
-    if (*p) ds.retired.push_back(*p);
-    *p = fresh;
-    *have = need;
+// Scratch of the backward-data operator, which callers may record without a first call outside the capture: in a graph of
+// this library's, or in one of their own on a stream they lent (rstq_stream_set).  An allocation made meanwhile does
+// not belong to the capture.  A block that a graph of the caller's may name is never freed before the context: nothing
+// tells when that graph is gone.
+int32_t dx_reserve(DeviceState& ds, int64_t need) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (!ds.capturing && ds.stream != ds.own_stream) RSTQ_CUDA(cudaStreamIsCapturing(ds.stream, &st));
+    const bool foreign = st != cudaStreamCaptureStatusNone;
+    if (need > ds.dx_scratch_bytes) {
+        need = (need + 0xFFFFF) & ~0xFFFFFll;
+        if (ds.dx_scratch && ds.dx_named) {
+            ds.kept.push_back(ds.dx_scratch);
+        } else if (ds.dx_scratch) {
+            if (ds.capturing || foreign || ds.live_graphs > 0) ds.retired.push_back(ds.dx_scratch);
+            else {
+                RSTQ_CUDA(cudaStreamSynchronize(ds.stream));
+                RSTQ_CUDA(cudaFree(ds.dx_scratch));
+            }
+        }
+        ds.dx_scratch = nullptr;
+        ds.dx_scratch_bytes = 0;
+        ds.dx_named = false;
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        RSTQ_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+        const cudaError_t e = cudaMalloc(&ds.dx_scratch, (size_t)need);
+        if (e != cudaSuccess) ds.dx_scratch = nullptr;
+        RSTQ_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+        RSTQ_CUDA(e);
+        ds.dx_scratch_bytes = need;
+    }
+    ds.dx_named |= foreign;
     return RSTQ_OK;
 }
 
@@ -593,6 +610,7 @@ int32_t rstq_shutdown(rstq_ctx* ctx) {
         if (ds.f_image) cudaFree(ds.f_image);
         if (ds.bind_stage) cudaFree(ds.bind_stage);
         if (ds.dx_scratch) cudaFree(ds.dx_scratch);
+        for (void* k : ds.kept) cudaFree(k);
         if (ds.partials) cudaFree(ds.partials);
         if (ds.counters) cudaFree(ds.counters);
         if (ds.status) cudaFree(ds.status);

@@ -649,7 +649,7 @@ int32_t launch_qlinear_q8_dx(rstq_ctx* ctx, DeviceState& ds, const float* dy, co
     while (split < 8 && tiles * split * 2 <= ds.sm_count && steps >= 16 * split) split *= 2;
 
     const int64_t yb = (3 * m * opad * 2 + 255) & ~255ll, rb = (m * 4 + 255) & ~255ll, cb = kDxParts * nb * 4;
-    int32_t rc = dev_reserve_any_time(ds, &ds.dx_scratch, &ds.dx_scratch_bytes, yb + rb + cb);
+    int32_t rc = dx_reserve(ds, yb + rb + cb);
     if (rc != RSTQ_OK) return rc;
     char* base = (char*)ds.dx_scratch;
     DxPrep q{dy, scales, (uint16_t*)base, (int*)(base + yb), (float*)(base + yb + rb), m, out, nb, opad};

@@ -106,8 +106,10 @@ struct DeviceState {
     int64_t pinned_bytes = 0;
     void* io_dev = nullptr;        // device staging for the host-array entry points
     int64_t io_dev_bytes = 0;
-    void* dx_scratch = nullptr;    // backward-data: its f32 factors as fp16 pairs
+    void* dx_scratch = nullptr;    // backward-data: dy as bf16 terms
     int64_t dx_scratch_bytes = 0;
+    bool dx_named = false;         // a graph of the caller's may name that block
+    std::vector<void*> kept;       // outgrown blocks that such a graph may name: freed with the context
     void* bind_stage = nullptr;    // the host arrays of the weight being bound, before they are re-tiled (at most
     int64_t bind_stage_bytes = 0;  // kBindStageKeep bytes are kept between binds)
     int* status = nullptr;         // device status word: nonzero after a bounded wait ran out
@@ -344,7 +346,7 @@ int32_t matmul_device(rstq_ctx* ctx, rstq_weight* w, const void* x, void* y, int
 // capi.cu: grow-only device scratch (refuses to grow during graph capture; the outgrown block is
 // freed at once, or parked until the last live graph of the device is destroyed)
 int32_t dev_reserve(DeviceState& ds, void** p, int64_t* have, int64_t need);
-int32_t dev_reserve_any_time(DeviceState& ds, void** p, int64_t* have, int64_t need);
+int32_t dx_reserve(DeviceState& ds, int64_t need);   // ds.dx_scratch, during a capture as well
 int32_t dev_release_scratch(DeviceState& ds, void* p);
 constexpr int kParamXMax = 7936;            // longest row of f32 activations that fits a launch's parameters beside the rest
 constexpr int64_t kFusedQuantMaxIn = 12288; // longest row the decode kernel quantizes itself (3 passes of 512 threads x 8)

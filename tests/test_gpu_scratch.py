@@ -38,3 +38,45 @@ def test_binding_while_a_graph_is_alive_holds_no_outgrown_staging_blocks(ctx):
     for b in (small, bx, by):
         b.free()
     assert free[0] - free[-1] < 32 << 20, free
+
+
+def dx_case(ctx, seed, m, in_, out):
+    rng = np.random.default_rng(seed)
+    a = (rng.standard_normal(m * out).astype(np.float32), rng.integers(-127, 128, out * in_).astype(np.int8),
+         rng.uniform(0.01, 0.02, out * in_ // 32).astype(np.float32))
+    bufs = [ctx.array_to_buffer(x) for x in a] + [ctx.make_buffer(m * in_, np.float32)]
+    d = a[0].reshape(m, out).astype(np.float64)
+    return bufs, d @ (a[1].reshape(out, in_) * np.repeat(a[2].reshape(out, -1).astype(np.float64), 32, axis=1))
+
+
+def test_backward_recorded_in_a_graph_of_the_caller(ctx):
+    """On a lent stream, without a call before it, and replayed after the scratch has grown and its old place (were it
+    free) been scribbled on."""
+    m, in_, out = 100, 256, 640
+    bufs, want = dx_case(ctx, 1, m, in_, out)
+    big, _ = dx_case(ctx, 2, 700, in_, out)
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    ctx.set_stream(stream.cuda_stream)
+    try:
+        with torch.cuda.graph(graph, stream=stream):
+            ctx.qlinear_q8_dx_device(*bufs, m, in_, out)
+        ctx.qlinear_q8_dx_device(*big, 700, in_, out)
+        ctx.sync()
+        other = [ctx.make_buffer(1 << 20, np.uint8) for _ in range(4)]
+        for b in other:
+            b.fill_bytes(0x7F)
+        for _ in range(2):
+            bufs[3].fill_bytes(0xFF)
+            ctx.sync()
+            with torch.cuda.stream(stream):
+                graph.replay()
+            torch.cuda.synchronize()
+            got = bufs[3].download().reshape(m, in_)
+            assert np.abs(got - want).max() <= 1e-5 * np.abs(want).max()
+    finally:
+        torch.cuda.synchronize()
+        del graph
+        ctx.set_stream(None)
+    for b in bufs + big + other:
+        b.free()
