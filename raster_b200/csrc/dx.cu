@@ -11,8 +11,8 @@
 //
 // Three terms hold all 24 bits of an f32 (each is rounded to nearest, so the rest takes the sign bit with it), and what
 // is left out is below 2^-24 of the product: the f32 product of the f32 values, whatever the spread inside a row or
-// a column block, at six bf16 MMAs.  A power of two per token row and per 32-column block keeps elements down to
-// 2^-130 of the largest beside them out of bf16's subnormals.
+// a column block, at six bf16 MMAs.  A power of two per token row and per 32-column block keeps elements far
+// below the largest beside them (2^-90 is tested) out of bf16's subnormals.
 // (Pairs of fp16 terms need three MMAs, but hold 22 bits, and those only of elements above 2^-17 of their row's
 // largest, scales above 2^-9: a scale 2^-20 of its block's largest kept 11 bits.)
 //

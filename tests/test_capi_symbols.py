@@ -81,7 +81,7 @@ def test_gemm_plan_is_host_arithmetic_and_follows_the_wave_model():
     assert of(4096, 4096, 512) == (128, 1)
     assert of(4096, 4096, 768) == (256, 1)
     assert of(4096, 4096, 2048) == (256, 1)
-    assert of(28672, 8192, 256) == (256, 1)          # 224 wide tiles: two waves instead of four
+    assert of(28672, 8192, 256) == (256, 1)          # 224 wide tiles, run as ranges of their K-steps (below)
     assert of(28672, 8192, 16) == (32, 1)            # 224 tiles: more than half the SMs, no split
     assert of(4096, 256, 64) == (64, 1)              # K too short to cut
     assert of(4096, 4096, 512, sm=296) == (128, 2)   # a part twice as wide would split

@@ -772,13 +772,13 @@ def test_qlinear_q8_dx_operator(ctx, m, in_, out):
 
 
 def test_qlinear_q8_dx_on_device_buffers(ctx):
-    """The device-resident entry: both kernels (tensor cores for m >= 16 and out % 8 == 0, f32 otherwise)
-    against the oracle, and the two against each other on a shape both accept."""
+    """The device-resident entry at two token-tile widths (32 and 64) against the oracle, and the two against each
+    other on the rows both have."""
     in_, out = 384, 200
     q = train.q8_quantize(synth.normal(91, out * in_, 0.2), out, in_)
     bc, bs = ctx.array_to_buffer(q["codes"]), ctx.array_to_buffer(q["scales"])
     got = {}
-    for m in (15, 48):                                   # 15 tokens: f32 kernel; 48: tensor cores
+    for m in (15, 48):                                   # 15 tokens: tiles of 32; 48: of 64
         dy = synth.normal(92, m * out)
         bdy, bdx = ctx.array_to_buffer(dy), ctx.make_buffer(m * in_, np.float32)
         ctx.qlinear_q8_dx_device(bdy, bc, bs, bdx, m, in_, out)
@@ -786,7 +786,7 @@ def test_qlinear_q8_dx_on_device_buffers(ctx):
         got[m] = bdx.download()
         assert relerr(got[m], orc.qlinear_q8_dx(dy, q["codes"], q["scales"], m, in_, out)) <= TOL_F
         bdy.free(), bdx.free()
-    assert relerr(got[48][:15 * in_], got[15]) <= TOL_F   # same dy rows (same seed prefix), other kernel
+    assert relerr(got[48][:15 * in_], got[15]) <= TOL_F   # same dy rows (same seed prefix), other tiles
     bc.free(), bs.free()
 
 
