@@ -240,8 +240,10 @@ static int32_t gemm_scratch(DeviceState& ds, int64_t M, int64_t in, int64_t out,
 }
 
 // One token of a K-quant: the decode kernel quantizes the activations itself, as for the plain formats (7B-class
-// MLP, Q4_K + Q6_K: 22.5 us for its two calls with a quantizer launch each).  From 1 MB of weights up; smaller
-// matrices keep the quantizer and the decode kernel as two launches.
+// MLP, Q4_K + Q6_K: 22.5 us for its two calls with a quantizer launch each, 19.8 now).  From 1 MB of weights up.  The line is no
+// crossover: one launch is faster below it as well (from a graph, two -> one: Q4_K 8 x 256 2.98 -> 2.12 us, 1000 x 1024 3.50 -> 2.46,
+// 32 x 12288 6.69 -> 6.66; above, Q6_K 1000 x 1024 3.69 -> 2.45).  It keeps small matrices at the launch count that callers
+// were given for them (rstq_launch_count; two).
 static bool kquant_fuses(const DeviceState& ds, const rstq_weight* w, int64_t M) {
     return M == 1 && ds.fuse_quant && !ds.x_on_host && w->in <= kFusedQuantMaxIn && w->data_bytes >= (1ll << 20);
 }

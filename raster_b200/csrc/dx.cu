@@ -16,6 +16,9 @@
 // (Pairs of fp16 terms need three MMAs, but hold 22 bits, and those only of elements above 2^-17 of their row's
 // largest, scales above 2^-9: a scale 2^-20 of its block's largest kept 11 bits.)
 //
+// What bounds it: the tensor core at the power cap, nominally 1536 cycles per 64 rows of a 128 x 128 tile, 2440 measured.
+// us per call back to back (bf16 mma.sync with three terms of dy * s, before): 4096 x 4096, m = 512 91.9 (260), m = 64
+// 29.3 (172); 1024 x 1024, m = 16 16.5 (44.7), m = 2048 35.0 (69.3); 11008 x 2048, m = 300 136 (457).
 #include <type_traits>
 
 #include "internal.h"
