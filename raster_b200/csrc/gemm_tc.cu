@@ -1112,13 +1112,14 @@ static int32_t launch_act_to_f16(rstq_ctx* ctx, DeviceState& ds, const void* x, 
 // loads and epilogue of a CTA about 8000 resp. 9000 cycles; the hand-over of a pair about 1500)
 // (kRangeCycles: what the second segment of a range costs, in cycles over the plain model.  The model counts neither
 // further segments nor the power cap, under which idle SMs buy the others a higher clock: ranges are taken only over at
-// most four tiles each, and where it sees 15 % saved; up to 64 tokens, far from the cap, 6 %.  Measured over seconds, int4 /
+// most four tiles each, and where it sees 15 % saved; up to 64 tokens, far from the cap, 6 %; against pairs, which wait for no last wave, anything
+// (8192 x 28672 at M = 256, bf16: over seconds 124.9 / 126.2, but a first call of both matrices of the 70B-class MLP 228 -> 219).  Measured over seconds, int4 /
 // int8, whole tiles or pairs -> ranges, us.  Above the line: 24576 x 3072 at M = 64 29.5 -> 27.0, at M = 20 31.3 -> 26.4;
 // 28672 x 4096 at M = 64 43.1 -> 42.3; 28672 x 8192 at M = 32 62.1 -> 57.3, at M = 256 128.3 -> 124.9; 11008 x 4096 at M = 512
 // 65.2 -> 64.2 (in a burst 60.4 -> 55.9); 20000 x 2048 at M = 200 37.0 -> 34.2; 14336 x 4096 at M = 512 70.2 -> 69.9.
 // Below it, where the model alone would take them: 26000 x 2048 at M = 32 21.5 -> 22.2; 4096 x 4096 at M = 2048 79.6 -> 82.9, 4096 x 11008 at M = 2048
 // 189 -> 200, 9000 x 6144 at M = 900 107 -> 112, 27648 x 1024 at M = 256 29.0 -> 31.1, 6144 x 8192 at M = 1024 130 -> 134,
-// 5120 x 13824 at M = 300 65.9 -> 67.3, 8192 x 28672 at M = 256 124.8 -> 126.2.  More than four tiles per range:
+// 5120 x 13824 at M = 300 65.9 -> 67.3.  More than four tiles per range:
 // 11008 x 4096 at M = 1024 and 2048, as fast either way.)
 constexpr int64_t kRangeCycles = 13000;
 void gemm_plan(int64_t out, int64_t in, int64_t M, int sm_count, bool tmem_kernel, int wide, int* ntok_out,
@@ -1157,7 +1158,8 @@ void gemm_plan(int64_t out, int64_t in, int64_t M, int sm_count, bool tmem_kerne
         const int64_t per = (steps + G - 1) / G;
         const int64_t c = ntok == 256 ? 1140 + (G > 64 ? (G - 64) * 31 / 10 : 0) : 690, fixed = ntok == 256 ? 9000 : 8000;
         bool s2 = false;
-        const bool pays = per <= 3 * ksteps_total && (per * c + fixed + kRangeCycles) * 100 < cycles(ntok, &s2) * (ntok <= 64 ? 94 : 85);
+        const int64_t other = cycles(ntok, &s2);
+        const bool pays = per <= 3 * ksteps_total && (per * c + fixed + kRangeCycles) * 100 < other * (s2 ? 100 : (ntok <= 64 ? 94 : 85));
         if (steps < (1ll << 31) && (wide == 4 || pays)) {
             *ranges_out = (int)G;
             split = false;

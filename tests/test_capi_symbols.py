@@ -97,7 +97,7 @@ def test_gemm_ranges_where_whole_tiles_leave_sms_idle():
     for out, in_, m in [(28672, 8192, 32), (28672, 8192, 256), (11008, 4096, 512)]:
         assert R.gemm_ranges(out, in_, m) == 148
     for out, in_, m in [(20000, 2048, 200), (14336, 4096, 512), (5120, 5120, 1024), (22016, 4096, 32), (24576, 3072, 20),
-                        (24576, 3072, 64), (28672, 4096, 64)]:
+                        (24576, 3072, 64), (28672, 4096, 64), (8192, 28672, 256)]:
         assert R.gemm_ranges(out, in_, m) == 148
     # one wave, too little saved, too many tiles per range, rows of one or two K-steps
     for out, in_, m in [(8192, 8192, 512), (12288, 4096, 300), (4096, 4096, 768), (4096, 4096, 512), (4096, 4096, 64),
