@@ -8,6 +8,8 @@
 // and the fusion the chain invites: rms-norm whose output is quantized to int8 blocks in the same
 // kernel (the normalized row never goes to memory; codes, scales and block sums are exactly what
 // quant_act_i8_kernel would produce from rms_norm's f32 output).
+#include <initializer_list>
+
 #include "internal.h"
 #include "quant_helpers.cuh"
 
@@ -15,7 +17,7 @@ namespace rstq {
 
 constexpr int kRowThreads = 1024;
 
-// sum over the CTA; every thread gets the result
+// sum over the CTA; every thread gets the result (once per kernel: s_red is not written again)
 __device__ __forceinline__ float cta_sum(float v, float* s_red) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -24,7 +26,6 @@ __device__ __forceinline__ float cta_sum(float v, float* s_red) {
     float t = 0.f;
 #pragma unroll
     for (int i = 0; i < kRowThreads / 32; ++i) t += s_red[i];
-    __syncthreads();
     return t;
 }
 
@@ -37,7 +38,11 @@ __device__ __forceinline__ float cta_sum(float v, float* s_red) {
 // dependent chain -- loads, a block reduction, the double-precision quantizer -- and not its bytes.
 // With 256 threads and two passes over memory it took 15 us per launch on a 4096-feature row, a third
 // of a whole decoder layer.
+// A row goes to up to kRowParts CTAs (a power of two, gridDim.y): each adds up the whole row's squares, in the same order
+// and so to the same bits, and finishes only its own 1024-element pieces, so that a warp runs the quantizer's chain
+// once instead of once per piece: four 7B layers (eight such launches of 4096 features) 217.8 -> 213.2 us.
 constexpr int kRowKeep = 8;
+constexpr int kRowParts = 4;
 
 __device__ __forceinline__ void quant_block_store(float v, int lane, int64_t blk, int8_t* __restrict__ xq,
                                                   float* __restrict__ xs, int32_t* __restrict__ xsum) {
@@ -55,7 +60,7 @@ __device__ __forceinline__ void quant_block_store(float v, int lane, int64_t blk
 }
 
 template <bool QUANT, bool RES = false>
-__global__ void __launch_bounds__(kRowThreads)
+__global__ void __launch_bounds__(kRowThreads, 1)
 rms_norm_kernel(const float* __restrict__ x, const float* __restrict__ w, float* __restrict__ out,
                 int8_t* __restrict__ xq, float* __restrict__ xs, int32_t* __restrict__ xsum, int64_t features,
                 float eps, float gain_offset, const float* __restrict__ res = nullptr, float* sum = nullptr) {
@@ -63,6 +68,8 @@ rms_norm_kernel(const float* __restrict__ x, const float* __restrict__ w, float*
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const int64_t r = blockIdx.x;
+    const int part = (int)blockIdx.y, others = (int)gridDim.y - 1;
+    auto own = [&](int k) { return (k & others) == part; };          // pieces of 1024 elements
     const float* xr = RES ? sum + r * features : x + r * features;   // where the row is read back from
     float keep[kRowKeep], gain[kRowKeep];
     float ss = 0.f;
@@ -70,23 +77,17 @@ rms_norm_kernel(const float* __restrict__ x, const float* __restrict__ w, float*
     for (int k = 0; k < kRowKeep; ++k) {
         const int64_t i = threadIdx.x + (int64_t)k * kRowThreads;
         float v = 0.f;
-        if (i < features) {
-            if (RES) {
-                v = x[r * features + i] + res[r * features + i];
-                sum[r * features + i] = v;
-            } else {
-                v = xr[i];
-            }
-        }
+        if (i < features) v = RES ? x[r * features + i] + res[r * features + i] : xr[i];
+        if (RES && i < features && own(k)) sum[r * features + i] = v;
         keep[k] = v;
-        gain[k] = i < features ? gain_offset + w[i] : 0.f;   // fetched now: its latency hides under the reduction
+        gain[k] = i < features && own(k) ? gain_offset + w[i] : 0.f;   // fetched now: its latency hides under the reduction
         ss = fmaf(v, v, ss);
     }
     for (int64_t i = threadIdx.x + (int64_t)kRowKeep * kRowThreads; i < features; i += kRowThreads) {
         float v;
         if (RES) {
             v = x[r * features + i] + res[r * features + i];
-            sum[r * features + i] = v;   // read back below by this same thread
+            if (own((int)(i / kRowThreads))) sum[r * features + i] = v;   // read back below by this same thread
         } else {
             v = xr[i];
         }
@@ -101,13 +102,14 @@ rms_norm_kernel(const float* __restrict__ x, const float* __restrict__ w, float*
 #pragma unroll
     for (int k = 0; k < kRowKeep; ++k) {
         const int64_t i = threadIdx.x + (int64_t)k * kRowThreads;
-        if (i < features) {
+        if (i < features && own(k)) {
             const float v = keep[k] * inv * gain[k];
             if (QUANT) quant_block_store(v, lane, r * nb + (i >> 5), xq, xs, xsum);
             else out[r * features + i] = v;
         }
     }
     for (int64_t i = threadIdx.x + (int64_t)kRowKeep * kRowThreads; i < features; i += kRowThreads) {
+        if (!own((int)(i / kRowThreads))) continue;
         const float v = xr[i] * inv * (gain_offset + w[i]);
         if (QUANT) quant_block_store(v, lane, r * nb + (i >> 5), xq, xs, xsum);
         else out[r * features + i] = v;
@@ -172,6 +174,24 @@ static bool chain_buf(const rstq_buf* b, const rstq_ctx* ctx, int64_t bytes) {
     return b && b->magic == kBufMagic && b->ctx == ctx && b->bytes >= bytes;
 }
 
+// CTAs of an rms-norm launch: a row is shared while that leaves every CTA an SM of its own.  Not where an output lies over
+// an input (x normalized in place): a CTA would read what another has written.
+struct Span {
+    const void* p;
+    int64_t bytes;
+};
+static Span span_of(const rstq_buf* b, int64_t bytes) { return b ? Span{b->ptr, bytes} : Span{nullptr, 0}; }
+static dim3 row_grid(const DeviceState& ds, int64_t rows, int64_t features, std::initializer_list<Span> ins,
+                     std::initializer_list<Span> outs) {
+    for (const Span& i : ins)
+        for (const Span& o : outs)
+            if ((const char*)i.p < (const char*)o.p + o.bytes && (const char*)o.p < (const char*)i.p + i.bytes)
+                return dim3((unsigned)rows);
+    int parts = 1;
+    while (parts < kRowParts && features > (int64_t)parts * kRowThreads && rows * parts * 2 <= ds.sm_count) parts *= 2;
+    return dim3((unsigned)rows, (unsigned)parts);
+}
+
 extern "C" {
 
 int32_t rstq_rms_norm(rstq_ctx* ctx, rstq_buf* x, rstq_buf* weight, rstq_buf* out, int64_t rows, int64_t features,
@@ -186,7 +206,9 @@ int32_t rstq_rms_norm(rstq_ctx* ctx, rstq_buf* x, rstq_buf* weight, rstq_buf* ou
     DeviceState& ds = ctx->devs[x->dev];
     int32_t rc = use_dev(ctx, x->dev);
     if (rc != RSTQ_OK) return rc;
-    RSTQ_CUDA(launch_chain(rms_norm_kernel<false>, dim3((unsigned)rows), dim3(kRowThreads), ds, (const float*)x->ptr,
+    const dim3 grid = row_grid(ds, rows, features, {span_of(x, rows * features * 4), span_of(weight, features * 4)},
+                               {span_of(out, rows * features * 4)});
+    RSTQ_CUDA(launch_chain(rms_norm_kernel<false>, grid, dim3(kRowThreads), ds, (const float*)x->ptr,
                            (const float*)weight->ptr, (float*)out->ptr, (int8_t*)nullptr, (float*)nullptr,
                            (int32_t*)nullptr, features, (float)eps, (float)gain_offset, (const float*)nullptr,
                            (float*)nullptr));
@@ -210,7 +232,9 @@ int32_t rstq_rms_norm_quant_act(rstq_ctx* ctx, rstq_buf* x, rstq_buf* weight, rs
     DeviceState& ds = ctx->devs[x->dev];
     int32_t rc = use_dev(ctx, x->dev);
     if (rc != RSTQ_OK) return rc;
-    RSTQ_CUDA(launch_chain(rms_norm_kernel<true>, dim3((unsigned)rows), dim3(kRowThreads), ds, (const float*)x->ptr,
+    const dim3 grid = row_grid(ds, rows, features, {span_of(x, rows * features * 4), span_of(weight, features * 4)},
+                               {span_of(xq, rows * features), span_of(xs, rows * nb * 4), span_of(xsum, rows * nb * 4)});
+    RSTQ_CUDA(launch_chain(rms_norm_kernel<true>, grid, dim3(kRowThreads), ds, (const float*)x->ptr,
                            (const float*)weight->ptr, (float*)nullptr, (int8_t*)xq->ptr, (float*)xs->ptr,
                            xsum ? (int32_t*)xsum->ptr : (int32_t*)nullptr, features, (float)eps, (float)gain_offset,
                            (const float*)nullptr, (float*)nullptr));
@@ -271,7 +295,10 @@ int32_t rstq_residual_rms_norm_quant_act(rstq_ctx* ctx, rstq_buf* a, rstq_buf* b
     DeviceState& ds = ctx->devs[a->dev];
     int32_t rc = use_dev(ctx, a->dev);
     if (rc != RSTQ_OK) return rc;
-    RSTQ_CUDA(launch_chain(rms_norm_kernel<true, true>, dim3((unsigned)rows), dim3(kRowThreads), ds,
+    const dim3 grid = row_grid(ds, rows, features, {span_of(a, rows * features * 4), span_of(b, rows * features * 4), span_of(weight, features * 4)},
+                               {span_of(sum, rows * features * 4), span_of(xq, rows * features), span_of(xs, rows * nb * 4),
+                                span_of(xsum, rows * nb * 4)});
+    RSTQ_CUDA(launch_chain(rms_norm_kernel<true, true>, grid, dim3(kRowThreads), ds,
                            (const float*)a->ptr, (const float*)weight->ptr, (float*)nullptr, (int8_t*)xq->ptr,
                            (float*)xs->ptr, xsum ? (int32_t*)xsum->ptr : (int32_t*)nullptr, features, (float)eps,
                            (float)gain_offset, (const float*)b->ptr, (float*)sum->ptr));

@@ -156,3 +156,30 @@ def test_host_mirror_of_the_neighbours(ctx):
     assert relerr(nn.rms_norm_into(g, w, o3, 3, 100, 1e-6, 0.0, ctx), orc.rms_norm(g, w, 3, 100)) <= 2e-6
     with pytest.raises(ValueError):
         nn.silu_mul_into(g, u, out, 301, ctx)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows", [1, 37, 74, 75])
+@pytest.mark.parametrize("features", [1024, 1056, 4096, 8192, 8224, 13312])
+def test_rms_norm_shared_by_thread_blocks(ctx, rows, features):
+    """A row shared by several thread blocks (few rows) and a row per block (many): the same bits, also where a
+    row is normalized in place and so stays with one block."""
+    x, res = synth.normal(95, rows * features), synth.normal(96, rows * features)
+    w, nb = synth.normal(97, features, 0.1) + np.float32(1.0), features // 32
+    bx, br, bw = ctx.array_to_buffer(x), ctx.array_to_buffer(res), ctx.array_to_buffer(w)
+    b1, b2, bs = (ctx.make_buffer(rows * features, np.float32) for _ in range(3))
+    ctx.residual_add(bx, br, bs, rows * features)
+    ctx.rms_norm(bs, bw, b1, rows, features)
+    ctx.sync()
+    want, summed = b1.download(), bs.download()
+    assert relerr(want, orc.rms_norm(summed, w, rows, features)) <= 2e-6
+    q, s, z = (ctx.make_buffer(rows * features, np.int8), ctx.make_buffer(rows * nb, np.float32), ctx.make_buffer(rows * nb, np.int32))
+    ctx.residual_rms_norm_quant_act(bx, br, b2, bw, q, s, z, rows, features)
+    ctx.rms_norm(bs, bw, bs, rows, features)          # in place
+    ctx.sync()
+    assert np.array_equal(bs.download().view(np.uint32), want.view(np.uint32))
+    assert np.array_equal(b2.download().view(np.uint32), summed.view(np.uint32))
+    xq, xs, xsum = orc.quantize_act_i8(want, rows, features)
+    assert np.array_equal(q.download(), xq) and np.array_equal(s.download(), xs) and np.array_equal(z.download(), xsum)
+    for o in (bx, br, bw, b1, b2, bs, q, s, z):
+        o.free()
