@@ -82,3 +82,27 @@ def test_base_form_gives_the_same_bytes(monkeypatch, base_form, fmt, kind):
     got = CODECS[fmt](w)
     for k in want:
         assert got[k].tobytes() == want[k].tobytes(), k
+
+
+@pytest.mark.parametrize("fmt", ["q4_0", "q8_0"])
+def test_codec_next_to_its_ties(monkeypatch, fmt):
+    """Codes are taken in f32 except near a tie: quotients within a few f32 steps of k + 0.5, on either side of it and
+    of the line where the double path takes over, for scales over the normal range and beyond; and blocks whose
+    largest magnitude occurs with both signs, in either order."""
+    zp = 8 if fmt == "q4_0" else 128
+    rng = np.random.default_rng(11)
+    blocks = []
+    for e in (-130, -101, -100, -30, 0, 40, 99, 100, 110):
+        for _ in range(40):
+            s = np.float32(rng.uniform(1, 2) * 2.0 ** (e - 7))
+            k = rng.integers(-zp, zp, 32) + 0.5 + rng.choice([0, 1e-7, -1e-7, 1e-5, -1e-5, 9e-5, -9e-5, 1.1e-4, -1.1e-4], 32)
+            b = (k * np.float64(s)).astype(np.float32)
+            b[rng.permutation(32)[:2]] = np.float32(zp) * s * rng.choice([-1, 1], 2).astype(np.float32)
+            blocks.append(b)
+    w = np.concatenate(blocks)
+    assert np.isfinite(w).all()
+    got = CODECS[fmt](w)
+    monkeypatch.setattr(cq, "_native", lambda *a, **k: None)
+    want = CODECS[fmt](w)
+    for k in want:
+        assert got[k].tobytes() == want[k].tobytes(), k
