@@ -8,17 +8,17 @@
 // read inside the kernel (the reference's -buf variants), so a captured graph serves every token.
 //
 // Attention is one kernel where the reference has three phases: a CTA owns one KV head, a slice of
-// the cache positions and up to two query heads of the group (eight in the general kernel), which
-// it serves from the K / V rows it reads once; the group's other heads find the rows in L2 (the
-// reference reads them once per query head); warps walk the positions with an online
+// the cache positions and up to four (eight in the general kernel) query heads of the group, which it serves from the K / V rows
+// it reads once (the reference reads them once per query head); warps walk the positions with an online
 // softmax (running max, sum and weighted V in registers), the warps of a CTA are merged through
-// shared memory and the slices through a small scratch in device memory, where the last CTA to
-// arrive for a KV head writes out = sum_j p_j v_j.  The reference's score scratch `sc` is not used.
-// head_dim 64 and 128 take gqa_decode_fast_kernel (eight lanes per position, four positions per
+// shared memory and the slices through a small scratch in device memory, from which one CTA per
+// KV head writes out = sum_j p_j v_j.  The reference's score scratch `sc` is not used.
+// head_dim 64 and 128 take gqa_decode_stream_kernel (rows through shared memory, eight positions per
 // warp step); every other head_dim % 4 == 0 up to 256 takes the general gqa_decode_kernel (a
 // warp per position).
 #include "internal.h"
 #include "quant_helpers.cuh"
+#include "sync_helpers.cuh"
 
 namespace rstq {
 
@@ -27,6 +27,14 @@ constexpr int kAttnGroup = 8;     // query heads of one KV head served by a CTA
 constexpr int kAttnVec = 2;       // float4 per lane along head_dim: head_dim <= 256
 constexpr int kAttnCounters = 1024;
 constexpr float kNegInf = -1.0e38f;   // the reference's sentinel below any real score
+
+// A position or length in device memory, read from L2: a kernel that looks at it before its wait for the kernel
+// ahead, which may still write it, looks again afterwards.
+__device__ __forceinline__ int64_t ld_i64(const int64_t* p) {
+    int64_t v;
+    asm volatile("ld.volatile.global.s64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
 
 __global__ void __launch_bounds__(256)
 rope_pos_kernel(const float* __restrict__ x, float* __restrict__ out, int64_t heads, int64_t head_dim, double ln_theta,
@@ -102,6 +110,9 @@ struct AttnParams {
     int64_t cache_len;
     int n_q, group, n_kv, head_dim, S;
     float scale;
+    int gs;          // query heads per CTA as the scratch is laid out
+    int64_t maxpos;
+    int* status;
     // optional: the output quantized to int8 blocks of 32 as well (the o projection's input), by the
     // CTA that writes it; only with head_dim % 32 == 0 (a warp then owns whole blocks)
     int8_t* xq;
@@ -109,9 +120,6 @@ struct AttnParams {
     int32_t* xsum;
 };
 
-// Second half of both attention kernels: the per-warp states in shared memory ([warps][gc][row]:
-// weighted V, max, sum) are merged per CTA, then per KV head across the slices of the cache.
-// GS = query heads per CTA (the stride of the scratch).
 // one value of the output, and with it -- when asked for -- its 32-element quantizer block (the 32
 // lanes of the warp hold 32 consecutive elements of one head)
 __device__ __forceinline__ void attn_store(const AttnParams& p, int64_t e, float v, int lane) {
@@ -132,7 +140,8 @@ __device__ __forceinline__ void attn_store(const AttnParams& p, int64_t e, float
     }
 }
 
-template <int GS>
+// Second half of the general kernel: the per-warp states in shared memory ([warps][gc][row]: weighted V, max, sum) are
+// merged per CTA, then per KV head across the slices of the cache.
 __device__ __forceinline__ void attn_finish(const AttnParams& p, float* s_part, int* s_last_p, int gc, int g0, int hkv,
                                             int split, int gz, int hd, int row) {
     __shared__ float s_cw[kAttnGroup][kAttnWarps];   // weight of each warp's state in the CTA's state
@@ -157,7 +166,7 @@ __device__ __forceinline__ void attn_finish(const AttnParams& p, float* s_part, 
     }
     __syncthreads();
     // CTA state per (g, d): straight to out when there is one slice, else to the scratch
-    float* mine = p.part + ((((int64_t)hkv * gridDim.z + gz) * p.S + split) * GS) * row;
+    float* mine = p.part + ((((int64_t)hkv * gridDim.z + gz) * p.S + split) * kAttnGroup) * row;
     for (int i = threadIdx.x; i < gc * hd; i += blockDim.x) {
         const int g = i / hd, d = i - g * hd;
         const float* base = s_part + g * row + d;
@@ -186,20 +195,18 @@ __device__ __forceinline__ void attn_finish(const AttnParams& p, float* s_part, 
     // away, and three such trips in a row were most of this tail: warp g takes the (max, sum) pairs of head g, up
     // to kPairs per lane at once (128 slices: more than one per SM is rare), while every thread requests its first kHold
     // weighted values; then the slice weights exp(m_s - M) go round through shared memory (the per-warp states are dead
-    // by now; the host keeps S + 1 <= 8 * row).  kHold: 148 SMs give 32 heads 18 slices, so 20 covers most calls; with
-    // one head per CTA four CTAs share an SM at 64 registers, where 20 (and 18, 14, 12) spill and 16 does not:
-    // 32 / 32 heads x 1024 10.65 -> 9.92 us, 16 / 16 x 2048 12.2 -> 10.8, four 7B layers 220.7 -> 218.3.
-    const float* all = p.part + (((int64_t)hkv * gridDim.z + gz) * p.S * GS) * row;
+    // by now; the host keeps S + 1 <= 8 * row).
+    const float* all = p.part + (((int64_t)hkv * gridDim.z + gz) * p.S * kAttnGroup) * row;
     const int S = p.S;
     float* s_w = s_part;            // [gc][S] weights
     float* s_L = s_part + gc * S;   // [gc]
-    constexpr int kPairs = 4, kHold = GS == 1 ? 16 : 20;
+    constexpr int kPairs = 4, kHold = 20;
     float held[kHold];
     {
         const int i = threadIdx.x, g = i / hd, d = i - g * hd;
         const float* col = all + (int64_t)g * row + d;
 #pragma unroll
-        for (int k = 0; k < kHold; ++k) held[k] = i < gc * hd && k < S ? __ldcg(col + (int64_t)k * GS * row) : 0.f;
+        for (int k = 0; k < kHold; ++k) held[k] = i < gc * hd && k < S ? __ldcg(col + (int64_t)k * kAttnGroup * row) : 0.f;
     }
     if (warp < gc) {
         const float* st = all + (int64_t)warp * row + hd;
@@ -207,12 +214,12 @@ __device__ __forceinline__ void attn_finish(const AttnParams& p, float* s_part, 
 #pragma unroll
         for (int k = 0; k < kPairs; ++k) {
             const int sl = lane + 32 * k;
-            mv[k] = sl < S ? __ldcg(st + (int64_t)sl * GS * row) : kNegInf;
-            lv[k] = sl < S ? __ldcg(st + (int64_t)sl * GS * row + 1) : 0.f;
+            mv[k] = sl < S ? __ldcg(st + (int64_t)sl * kAttnGroup * row) : kNegInf;
+            lv[k] = sl < S ? __ldcg(st + (int64_t)sl * kAttnGroup * row + 1) : 0.f;
         }
 #pragma unroll
         for (int k = 0; k < kPairs; ++k) M = fmaxf(M, mv[k]);
-        for (int sl = lane + 32 * kPairs; sl < S; sl += 32) M = fmaxf(M, __ldcg(st + (int64_t)sl * GS * row));
+        for (int sl = lane + 32 * kPairs; sl < S; sl += 32) M = fmaxf(M, __ldcg(st + (int64_t)sl * kAttnGroup * row));
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
 #pragma unroll
@@ -225,8 +232,8 @@ __device__ __forceinline__ void attn_finish(const AttnParams& p, float* s_part, 
             }
         }
         for (int sl = lane + 32 * kPairs; sl < S; sl += 32) {
-            const float e = expf(__ldcg(st + (int64_t)sl * GS * row) - M);
-            Lsum = fmaf(__ldcg(st + (int64_t)sl * GS * row + 1), e, Lsum);
+            const float e = expf(__ldcg(st + (int64_t)sl * kAttnGroup * row) - M);
+            Lsum = fmaf(__ldcg(st + (int64_t)sl * kAttnGroup * row + 1), e, Lsum);
             s_w[warp * S + sl] = e;
         }
 #pragma unroll
@@ -246,7 +253,7 @@ __device__ __forceinline__ void attn_finish(const AttnParams& p, float* s_part, 
             sl = kHold;
         }
 #pragma unroll 8
-        for (; sl < S; ++sl) O = fmaf(__ldcg(col + (int64_t)sl * GS * row), s_w[g * S + sl], O);
+        for (; sl < S; ++sl) O = fmaf(__ldcg(col + (int64_t)sl * kAttnGroup * row), s_w[g * S + sl], O);
         attn_store(p, (int64_t)(hkv * p.group + g0 + g) * hd + d, O * (1.0f / s_L[g]), lane);
     }
 }
@@ -338,143 +345,403 @@ gqa_decode_kernel(const AttnParams p) {
             }
         }
     }
-    attn_finish<kAttnGroup>(p, s_part, &s_last, gc, g0, hkv, split, gz, hd, row);
+    attn_finish(p, s_part, &s_last, gc, g0, hkv, split, gz, hd, row);
 }
 
-// head_dim = 32 * VEC (64, 128): eight lanes share a cache position, so a warp works on four
-// positions at once and a dot needs three shuffles; a lane owns float4 columns sub, sub + 8, ... of
-// the head.  Query heads (pre-scaled) sit in shared memory; a CTA serves up to kFastGroup of them.
-// GC = query heads a CTA serves at most (1 or 2): the accumulators of unused heads would only cost
-// registers, and with one head per CTA four CTAs fit an SM instead of two.
-constexpr int kFastGroup = 2;
-template <int VEC, int GC>
-__global__ void __launch_bounds__(kAttnWarps * 32, GC == 1 ? 4 : 2)
-gqa_decode_fast_kernel(const AttnParams p) {
-    extern __shared__ __align__(16) float s_part[];   // [kAttnWarps][gc][hd + 4], then q [gc][hd]
-    __shared__ int s_last;
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    constexpr int hd = 32 * VEC, hd4 = hd / 4, row = hd + 4;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, grp = lane >> 3, sub = lane & 7;
+// ---- head_dim 64 and 128 ----------------------------------------------------------------------
+// Streams its slice of K and V through shared memory: one CTA per SM and KV head, serving up to four query heads from
+// rows that it reads once (larger groups find them in L2).  Each of 16 warps works alone on tiles of eight positions, with a ring of its own that
+// cp.async keeps full, so the bytes in flight (192 KB per SM) do not depend on registers:
+//   scores   eight lanes share a position; the sums of 8 positions x H heads over those lanes are reduced by halving
+//            (7 shuffles for 32 values), which leaves one (position, head) per lane: one exp per value
+//   softmax  online per tile (a maximum over eight positions, a rescale only where a maximum moved)
+//   output   a lane owns four dims of all heads, p comes back as one broadcast load per position
+// and the warps' states meet once, at the end.  The slices' states go through slots in device memory that hold kEmpty
+// between launches: the CTA of the last slice polls for the values themselves (no fence, counter or flag stands between
+// a store and its reader), merges and empties them.  It waits only for CTAs launched before it.
+// What bounds it: an SM takes in its 190 - 230 KB at about 65 B/ns, whether they come from HBM or L2; then a tail of about
+// 4 us (the last tile, the warps' merge, one trip through L2, the slices' merge) of which little is arithmetic.
+// us, back to back, against the kernel before it (two heads per CTA, rows through registers): 32 q / 8 kv heads x 4096
+// 13.8 -> 11.5, 64 / 8 x 2000 12.5 -> 11.1, 28 / 4 x 5000 14.4 -> 12.5, 32 / 16 x 2000 9.95 -> 9.72, 32 / 32 x 1000
+// 9.54 -> 9.45, 64 / 8 x 8000 of 64 elements 23.6 -> 15.7; four 7B layers at 1024 positions 213.2 -> 207.
+// Slower: one bulk copy per row instead of cp.async (20 cycles each, the first tile 2.3 us after the wait); a counter
+// that the last CTA to arrive reads instead of the polled slots (a tail of 4.4 us); slots read before the weights are
+// ready (most are empty then, and the second look costs a trip: 11.5 -> 12.4); eight heads per CTA in two passes
+// (28 / 4 x 5000 16.1); packed f32x2 arithmetic (11.8 -> 12.4).
+constexpr int kTilePos = 8;
+constexpr int kStreamWarps = 16;
+constexpr int kStreamThreads = kStreamWarps * 32;
+constexpr int kStreamHeads = 4;                       // query heads of one KV head per CTA
+constexpr int kRingBytes = 12288;                     // per warp
+constexpr int kHintPos = 256;                         // positions of a CTA requested into L2 ahead of time
+constexpr uint32_t kEmpty = 0xFFFFFFFFu;              // a NaN that no arithmetic produces
+__host__ __device__ constexpr int attn_unit_bytes(int hd) { return kTilePos * hd * 4; }      // a tile's rows of K, or of V
+__host__ __device__ constexpr int attn_units(int hd) { return kRingBytes / attn_unit_bytes(hd); }
+// shared memory: the warps' rings, the query heads, the warps' p
+__host__ __device__ constexpr int attn_q_off() { return kStreamWarps * kRingBytes; }
+__host__ __device__ constexpr int attn_p_off(int hd) { return attn_q_off() + kStreamHeads * hd * 4; }
+__host__ __device__ constexpr int attn_smem(int hd) { return attn_p_off(hd) + kStreamWarps * kTilePos * kStreamHeads * 4; }
+// ... and, once the rings are drained, in their place: the warps' states, then the merge of the slices
+constexpr int kMaxSlices = 160;                       // five (max, sum) pairs per lane of the merging warps
+__host__ __device__ constexpr int attn_w_off(int hd) { return kStreamWarps * kStreamHeads * (hd + 4) * 4; }       // slice weights
+__host__ __device__ constexpr int attn_o_off(int hd) { return attn_w_off(hd) + kStreamHeads * kMaxSlices * 4; }  // partial outputs
+static_assert(attn_o_off(128) + kStreamThreads * 16 <= attn_q_off(), "the merge fits where the rings were");
+
+// slots: a value is there once it is not kEmpty
+__device__ __forceinline__ float4 slot_read4(const float4* a) {
+    float4 v;
+    asm volatile("ld.volatile.global.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ float2 slot_read2(const float2* a) {
+    float2 v;
+    asm volatile("ld.volatile.global.v2.f32 {%0,%1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ bool slot_full(float v) { return __float_as_uint(v) != kEmpty; }
+__device__ __forceinline__ bool slot_full(const float4 v) { return slot_full(v.x) && slot_full(v.y) && slot_full(v.z) && slot_full(v.w); }
+__device__ __forceinline__ bool slot_full(const float2 v) { return slot_full(v.x) && slot_full(v.y); }
+__device__ __forceinline__ float slot_value(float v) { return slot_full(v) ? v : __uint_as_float(0x7FFFFFFFu); }
+__device__ __forceinline__ float4 slot_empty4() {
+    const float e = __uint_as_float(kEmpty);
+    return make_float4(e, e, e, e);
+}
+__device__ __forceinline__ float4 ld_shared_f4(uint32_t a) {
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a));
+    return v;
+}
+// H = query heads of the KV head that a CTA serves at most (1, 2 or 4).
+template <int HD, int H>
+__global__ void __launch_bounds__(kStreamThreads, 1)
+gqa_decode_stream_kernel(const AttnParams p) {
+    constexpr int VEC = HD / 32, ROW = HD + 4;      // VEC: float4 per lane of a position's eight lanes
+    constexpr uint32_t ROWB = HD * 4, UNITB = attn_unit_bytes(HD);
+    constexpr int NU = attn_units(HD);                              // units of the ring: K and V of a tile in turn
+    constexpr int LPP = HD / 4, PPS = 32 / LPP;                     // output: lanes per position, positions per step
+    extern __shared__ __align__(128) uint8_t s_raw[];
+    __shared__ int s_abort;
+    __shared__ float s_cw[kStreamHeads][kStreamWarps], s_cM[kStreamHeads], s_cL[kStreamHeads], s_L[kStreamHeads];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, grp = lane >> 3, sub = lane & 7;
     const int hkv = blockIdx.x, split = blockIdx.y, gz = blockIdx.z;
-    const int g0 = gz * GC;
-    const int gc = min(GC, p.group - g0);
-    const int64_t clen = p.clenbuf ? p.clenbuf[0] : p.cache_len;
-    const int64_t chunk = (clen + p.S - 1) / p.S;
-    const int64_t j0 = split * chunk, j1 = min(clen, j0 + chunk);
-    const int64_t kv4 = ((int64_t)p.n_kv * hd) >> 2;
-    const float4* kb = reinterpret_cast<const float4*>(p.k + (int64_t)hkv * hd) + sub;
-    const float4* vb = reinterpret_cast<const float4*>(p.v + (int64_t)hkv * hd) + sub;
-    // the rows of this lane group's first position are on their way while the query heads are staged (with the merge
-    // at the end in fewer trips, caches from HBM: 32 q / 8 kv heads x 4096 16.1 -> 14.1 us, x 512 8.9 -> 8.0;
-    // 32 / 32 x 1024 12.7 -> 11.6; 64 / 8 x 8192 of 64 elements 26.1 -> 24.4).  The loop takes them over at its top and
-    // requests the next ones there: moved to the bottom of the loop, the take-over cost the long caches 2.5 us.
-    const int64_t jf = j0 + warp * 4 + grp;
-    float4 kn[VEC], vn[VEC];
-    if (jf < j1) {
-#pragma unroll
-        for (int u = 0; u < VEC; ++u) kn[u] = __ldg(kb + jf * kv4 + 8 * u);
-#pragma unroll
-        for (int u = 0; u < VEC; ++u) vn[u] = __ldg(vb + jf * kv4 + 8 * u);
+    const int g0 = gz * kStreamHeads, gc = min(kStreamHeads, p.group - g0);
+    const int64_t kvrow = (int64_t)p.n_kv * HD;
+    const float* kb = p.k + (int64_t)hkv * HD;
+    const float* vb = p.v + (int64_t)hkv * HD;
+    const uint32_t base = smem_u32(s_raw), ring = base + warp * kRingBytes;
+    volatile int* abort_flag = &s_abort;
+
+    if (tid == 0) s_abort = 0;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    // (a length in device memory may still change: here it only says which rows of the cache to ask for)
+    auto range = [&](int64_t* j0, int64_t* j1) {
+        int64_t clen = p.clenbuf ? ld_i64(p.clenbuf) : p.cache_len;
+        clen = clen < 0 ? 0 : (clen > p.maxpos ? p.maxpos : clen);
+        const int64_t chunk = (clen + p.S - 1) / p.S;
+        *j0 = min(clen, split * chunk);
+        *j1 = min(clen, *j0 + chunk);
+    };
+    int64_t j0, j1;
+    range(&j0, &j1);
+    for (int i = tid; i < kHintPos * 2 * (HD / 32); i += kStreamThreads) {     // (128 bytes each)
+        const int r = i / (HD / 32), c = i % (HD / 32);
+        const int64_t j = j0 + (r >> 1);
+        if (j < j1) asm volatile("prefetch.global.L2 [%0];" ::"l"(((r & 1) ? vb : kb) + j * kvrow + c * 32));
     }
-    float4* s_q = reinterpret_cast<float4*>(s_part + kAttnWarps * gc * row);
-    for (int i = threadIdx.x; i < gc * hd4; i += blockDim.x) {
-        const float4 t = reinterpret_cast<const float4*>(p.q + (int64_t)(hkv * p.group + g0) * hd)[i];
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (p.clenbuf) range(&j0, &j1);
+
+    const int tiles = (int)((j1 - j0 + kTilePos - 1) / kTilePos);
+    const int mine = tiles > warp ? (tiles - warp + kStreamWarps - 1) / kStreamWarps : 0;   // tiles warp, warp + 16, ...
+    auto request = [&](int u) {    // unit u: K (even) or V (odd) of this warp's tile u / 2; an empty group beyond the last
+        if (u < 2 * mine) {
+            const int64_t j = j0 + (int64_t)(warp + (u >> 1) * kStreamWarps) * kTilePos;
+            const int np = (int)(j1 - j < kTilePos ? j1 - j : kTilePos);
+            const uint32_t dst = ring + (u % NU) * UNITB + lane * 16;
+            const float* src = ((u & 1) ? vb : kb) + (j + lane / LPP) * kvrow + (lane % LPP) * 4;
+#pragma unroll
+            for (int t = 0; t < kTilePos / PPS; ++t)
+                if (t * PPS + lane / LPP < np)
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + t * PPS * ROWB), "l"(src + t * PPS * kvrow) : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    auto arrived = [&]() {         // the oldest unit requested is in shared memory
+        asm volatile("cp.async.wait_group %0;" ::"n"(NU - 1) : "memory");
+        __syncwarp();
+    };
+#pragma unroll 1
+    for (int u = 0; u < NU; ++u) request(u);
+    float4* s_q = reinterpret_cast<float4*>(s_raw + attn_q_off());
+    for (int i = tid; i < H * (HD / 4); i += kStreamThreads) {
+        float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (i < gc * (HD / 4)) t = reinterpret_cast<const float4*>(p.q + (int64_t)(hkv * p.group + g0) * HD)[i];
         s_q[i] = make_float4(t.x * p.scale, t.y * p.scale, t.z * p.scale, t.w * p.scale);
     }
     __syncthreads();
-    const unsigned gmask = 0xFFu << (grp * 8);
-    float4 acc[GC][VEC];
-    float m[GC], l[GC];
+
+    const uint32_t qa = base + attn_q_off() + sub * 16;
+    float* s_p = reinterpret_cast<float*>(s_raw + attn_p_off(HD)) + warp * (kTilePos * H);
+    const uint32_t pa = smem_u32(s_p);
+    float4 acc[H];
+    float m = kNegInf, l = 0.f;     // of the head this lane holds scores of
 #pragma unroll
-    for (int g = 0; g < GC; ++g) {
-        m[g] = kNegInf;
-        l[g] = 0.f;
+    for (int h = 0; h < H; ++h) acc[h] = make_float4(0.f, 0.f, 0.f, 0.f);
+    // what the halving leaves in this lane: position 4 (sub & 1) + grp, head lane_h
+    const int lane_pos = 4 * (sub & 1) + grp;
+    const int lane_h = H == 4 ? ((sub >> 1) & 1) * 2 + (sub >> 2) : (H == 2 ? (sub >> 1) & 1 : 0);
+#pragma unroll 1
+    for (int i = 0; i < mine; ++i) {
+        const int64_t j = j0 + (int64_t)(warp + i * kStreamWarps) * kTilePos;
+        const int np = (int)(j1 - j < kTilePos ? j1 - j : kTilePos);
+        const uint32_t ka = ring + (2 * i % NU) * UNITB, va = ring + ((2 * i + 1) % NU) * UNITB;
+        arrived();
+        float4 kk[2][VEC];
 #pragma unroll
-        for (int u = 0; u < VEC; ++u) acc[g][u] = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-    // the rows of the next position are requested before the current one is worked on: a CTA has only
-    // a few positions per lane group, so an exposed load latency per step is most of the kernel
-    // (not with one head per CTA, where four CTAs per SM hide the latency already: measured)
-    constexpr bool PF = GC > 1;
-    for (int64_t j = jf; j < j1; j += kAttnWarps * 4) {
-        float4 kk[VEC], vv[VEC];
+        for (int t = 0; t < 2; ++t)
 #pragma unroll
-        for (int u = 0; u < VEC; ++u) {
-            kk[u] = kn[u];
-            vv[u] = vn[u];
+            for (int u = 0; u < VEC; ++u) kk[t][u] = ld_shared_f4(ka + (4 * t + grp) * ROWB + (sub + 8 * u) * 16);
+        __syncwarp();
+        request(2 * i + NU);
+        float v[2 * H];
+#pragma unroll
+        for (int h = 0; h < H; ++h) {
+            float s0 = 0.f, s1 = 0.f;
+#pragma unroll
+            for (int u = 0; u < VEC; ++u) {
+                const float4 qq = ld_shared_f4(qa + h * ROWB + u * 128);
+                s0 = fmaf(qq.x, kk[0][u].x, fmaf(qq.y, kk[0][u].y, fmaf(qq.z, kk[0][u].z, fmaf(qq.w, kk[0][u].w, s0))));
+                s1 = fmaf(qq.x, kk[1][u].x, fmaf(qq.y, kk[1][u].y, fmaf(qq.z, kk[1][u].z, fmaf(qq.w, kk[1][u].w, s1))));
+            }
+            v[h] = s0;
+            v[H + h] = s1;
         }
-        const int64_t jn = j + kAttnWarps * 4;
-        if (PF && jn < j1) {
 #pragma unroll
-            for (int u = 0; u < VEC; ++u) kn[u] = __ldg(kb + jn * kv4 + 8 * u);
+        for (int n = H, o = 1; o < 8; n >>= 1, o <<= 1) {
+            if (n >= 1) {        // 2 n values -> n: the lane keeps the half its bit names
+                const bool up = sub & o;
 #pragma unroll
-            for (int u = 0; u < VEC; ++u) vn[u] = __ldg(vb + jn * kv4 + 8 * u);
-        }
-#pragma unroll
-        for (int g = 0; g < GC; ++g) {
-            if (g < gc) {
-                float s = 0.f;
-#pragma unroll
-                for (int u = 0; u < VEC; ++u) {
-                    const float4 qq = s_q[g * hd4 + sub + 8 * u];
-                    s = fmaf(qq.x, kk[u].x, fmaf(qq.y, kk[u].y, fmaf(qq.z, kk[u].z, fmaf(qq.w, kk[u].w, s))));
+                for (int k = 0; k < n; ++k) {
+                    const float give = up ? v[k] : v[n + k], keep = up ? v[n + k] : v[k];
+                    v[k] = keep + __shfl_xor_sync(0xffffffffu, give, o);
                 }
-                s += __shfl_xor_sync(gmask, s, 1);   // the eight lanes of this position only: the other
-                s += __shfl_xor_sync(gmask, s, 2);   // groups of the warp may have left the loop already
-                s += __shfl_xor_sync(gmask, s, 4);
-                const float mn = fmaxf(m[g], s);
-                const float corr = expf(m[g] - mn), pj = expf(s - mn);
-                m[g] = mn;
-                l[g] = fmaf(l[g], corr, pj);
-#pragma unroll
-                for (int u = 0; u < VEC; ++u) {
-                    acc[g][u].x = fmaf(acc[g][u].x, corr, pj * vv[u].x);
-                    acc[g][u].y = fmaf(acc[g][u].y, corr, pj * vv[u].y);
-                    acc[g][u].z = fmaf(acc[g][u].z, corr, pj * vv[u].z);
-                    acc[g][u].w = fmaf(acc[g][u].w, corr, pj * vv[u].w);
-                }
+            } else {
+                v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
             }
         }
-        if (!PF && jn < j1) {   // fetch the next position's rows now
+        const bool valid = lane_pos < np;
+        float mx = valid ? v[0] : kNegInf;
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
+        const float mn = fmaxf(m, mx);
+        const float pj = valid ? expf(v[0] - mn) : 0.f;
+        if (__any_sync(0xffffffffu, mn != m)) {
+            const float corr = expf(m - mn);
+            l *= corr;
+            m = mn;
 #pragma unroll
-            for (int u = 0; u < VEC; ++u) kn[u] = __ldg(kb + jn * kv4 + 8 * u);
-#pragma unroll
-            for (int u = 0; u < VEC; ++u) vn[u] = __ldg(vb + jn * kv4 + 8 * u);
-        }
-    }
-    // the four position groups of the warp -> one state (every lane ends with the merged values)
-#pragma unroll
-    for (int g = 0; g < GC; ++g) {
-        if (g < gc) {
-#pragma unroll
-            for (int o = 8; o <= 16; o <<= 1) {
-                const float mo = __shfl_xor_sync(0xffffffffu, m[g], o);
-                const float lo = __shfl_xor_sync(0xffffffffu, l[g], o);
-                const float mn = fmaxf(m[g], mo);
-                const float es = expf(m[g] - mn), eo = expf(mo - mn);
-                m[g] = mn;
-                l[g] = fmaf(l[g], es, lo * eo);
-#pragma unroll
-                for (int u = 0; u < VEC; ++u) {
-                    acc[g][u].x = fmaf(acc[g][u].x, es, __shfl_xor_sync(0xffffffffu, acc[g][u].x, o) * eo);
-                    acc[g][u].y = fmaf(acc[g][u].y, es, __shfl_xor_sync(0xffffffffu, acc[g][u].y, o) * eo);
-                    acc[g][u].z = fmaf(acc[g][u].z, es, __shfl_xor_sync(0xffffffffu, acc[g][u].z, o) * eo);
-                    acc[g][u].w = fmaf(acc[g][u].w, es, __shfl_xor_sync(0xffffffffu, acc[g][u].w, o) * eo);
-                }
-            }
-            if (grp == 0) {
-                float* dst = s_part + (warp * gc + g) * row;
-#pragma unroll
-                for (int u = 0; u < VEC; ++u) reinterpret_cast<float4*>(dst)[sub + 8 * u] = acc[g][u];
-                if (sub == 0) {
-                    dst[hd] = m[g];
-                    dst[hd + 1] = l[g];
-                }
+            for (int h = 0; h < H; ++h) {
+                const float c = __shfl_sync(0xffffffffu, corr, H == 4 ? (h >> 1) * 2 + (h & 1) * 4 : 2 * h);
+                float4& a = acc[h];
+                a = make_float4(a.x * c, a.y * c, a.z * c, a.w * c);
             }
         }
+        l += pj;
+        s_p[lane_pos * H + lane_h] = pj;
+        arrived();         // V of the tile; and s_p is written
+        auto add = [&](int pos) {
+            const float4 vv = ld_shared_f4(va + pos * ROWB + (lane % LPP) * 16);
+            float pv[H];
+            if constexpr (H >= 4) {
+#pragma unroll
+                for (int h = 0; h < H; h += 4) *reinterpret_cast<float4*>(&pv[h]) = ld_shared_f4(pa + (pos * H + h) * 4);
+            } else {
+#pragma unroll
+                for (int h = 0; h < H; ++h) pv[h] = s_p[pos * H + h];
+            }
+#pragma unroll
+            for (int h = 0; h < H; ++h) {
+                acc[h].x = fmaf(pv[h], vv.x, acc[h].x);
+                acc[h].y = fmaf(pv[h], vv.y, acc[h].y);
+                acc[h].z = fmaf(pv[h], vv.z, acc[h].z);
+                acc[h].w = fmaf(pv[h], vv.w, acc[h].w);
+            }
+        };
+        if (np == kTilePos) {
+#pragma unroll
+            for (int t = 0; t < kTilePos; t += PPS) add(t + lane / LPP);
+        } else {      // (rows that were not copied are left out, not multiplied by zero)
+#pragma unroll 1
+            for (int pos = lane / LPP; pos < np; pos += PPS) add(pos);
+        }
+        __syncwarp();   // every lane is done with V and s_p
+        request(2 * i + 1 + NU);
     }
-    attn_finish<GC>(p, s_part, &s_last, gc, g0, hkv, split, gz, hd, row);
+
+    // ---- the warps' states -> the CTA's ----
+    l += __shfl_xor_sync(0xffffffffu, l, 1);
+    l += __shfl_xor_sync(0xffffffffu, l, 8);
+    l += __shfl_xor_sync(0xffffffffu, l, 16);
+    if (PPS == 2) {
+#pragma unroll
+        for (int h = 0; h < H; ++h) {
+            acc[h].x += __shfl_xor_sync(0xffffffffu, acc[h].x, 16);
+            acc[h].y += __shfl_xor_sync(0xffffffffu, acc[h].y, 16);
+            acc[h].z += __shfl_xor_sync(0xffffffffu, acc[h].z, 16);
+            acc[h].w += __shfl_xor_sync(0xffffffffu, acc[h].w, 16);
+        }
+    }
+    __syncthreads();    // the rings are drained: their place is free
+    float* s_part = reinterpret_cast<float*>(s_raw);     // [warp][gc][ROW]: weighted V, max, sum
+#pragma unroll
+    for (int h = 0; h < H; ++h)
+        if (h < gc && lane < LPP) reinterpret_cast<float4*>(s_part + (warp * gc + h) * ROW)[lane] = acc[h];
+    if (lane_h < gc && grp == 0) {       // (the lanes of a head agree)
+        s_part[(warp * gc + lane_h) * ROW + HD] = m;
+        s_part[(warp * gc + lane_h) * ROW + HD + 1] = l;
+    }
+    __syncthreads();
+    if (warp < gc && lane < kStreamWarps) {          // warp h merges the (max, sum) pairs of head h
+        const float* s = s_part + (lane * gc + warp) * ROW + HD;
+        const float mw = s[0], lw = s[1];
+        float M = mw;
+#pragma unroll
+        for (int o = kStreamWarps / 2; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xFFFFu, M, o));
+        const float e = expf(mw - M);
+        float L = lw * e;
+#pragma unroll
+        for (int o = kStreamWarps / 2; o > 0; o >>= 1) L += __shfl_xor_sync(0xFFFFu, L, o);
+        s_cw[warp][lane] = e;
+        if (lane == 0) {
+            s_cM[warp] = M;
+            s_cL[warp] = L;
+        }
+    }
+    __syncthreads();
+    const int cols = gc * LPP, S = p.S;              // float4 columns of the CTA's output (at most 128)
+    float4* s_o = reinterpret_cast<float4*>(s_raw + attn_o_off(HD));
+    float* all = p.part + ((int64_t)hkv * gridDim.z + gz) * S * (p.gs * ROW);
+    float* out_part = all + (int64_t)split * (p.gs * ROW);
+    if (tid < cols) {
+        const int h = tid / LPP, c = tid - h * LPP;
+        float4 O = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int w = 0; w < kStreamWarps; ++w) {
+            const float4 a = reinterpret_cast<const float4*>(s_part + (w * gc + h) * ROW)[c];
+            const float e = s_cw[h][w];
+            O.x = fmaf(a.x, e, O.x);
+            O.y = fmaf(a.y, e, O.y);
+            O.z = fmaf(a.z, e, O.z);
+            O.w = fmaf(a.w, e, O.w);
+        }
+        if (S == 1) s_o[tid] = O;      // (the one slice's state is the result's)
+        else reinterpret_cast<float4*>(out_part + h * ROW)[c] = make_float4(slot_value(O.x), slot_value(O.y), slot_value(O.z), slot_value(O.w));
+    }
+    int groups = 1;
+    if (S == 1) {
+        if (tid < gc) s_L[tid] = 1.0f / s_cL[tid];
+    } else {
+        if (tid < gc)
+            *reinterpret_cast<float2*>(out_part + tid * ROW + HD) = make_float2(slot_value(s_cM[tid]), slot_value(s_cL[tid]));
+        if (split != S - 1) return;
+        // ---- the slices' states -> out: the CTA of the last slice ----
+        // What it reads lies a trip to L2 away, so it is requested kHold float4 per thread at a time (slices g, g + groups,
+        // ...).  The code is run once and cold: short loops rather than unrolled ones.
+        constexpr int kHold = 10;
+        groups = kStreamThreads / cols;
+        const int g = tid / cols, c = tid - g * cols, ch = c / LPP, pitch = p.gs * ROW;
+        float* s_w = reinterpret_cast<float*>(s_raw + attn_w_off(HD));     // [gc][S]: maxima, then weights
+        float4* col = reinterpret_cast<float4*>(all + ch * ROW) + (c - ch * LPP);
+        float4 held[kHold];
+        auto hold = [&](int from) {       // (beyond the last slice that one again, without a branch: it is not looked at)
+#pragma unroll
+            for (int k = 0; k < kHold; ++k) held[k] = slot_read4(col + min(from + k * groups, S - 1) * (pitch / 4));
+        };
+        unsigned long long t0 = 0;
+        uint32_t polls = 0;
+        bool ok = true;
+        auto patience = [&]() {           // (the timer is slow to read: not while there is hope)
+            if ((++polls & 255u) != 0) return true;
+            const unsigned long long now = gtime_ns();
+            if (t0 == 0) t0 = now;
+            if (!*abort_flag && now - t0 <= kWaitLimitNs) return true;
+            *abort_flag = 1;
+            return ok = false;
+        };
+        if (warp < gc) {
+            float M = kNegInf, L = 0.f, ls[kMaxSlices / 32];
+#pragma unroll
+            for (int k = 0; k < kMaxSlices / 32; ++k) {
+                const int sl = lane + 32 * k;
+                ls[k] = 0.f;
+                if (sl < S) {
+                    float2* at = reinterpret_cast<float2*>(all + sl * pitch + warp * ROW + HD);
+                    float2 v;
+                    do v = slot_read2(at);
+                    while (!slot_full(v) && patience());
+                    *at = make_float2(__uint_as_float(kEmpty), __uint_as_float(kEmpty));
+                    s_w[warp * S + sl] = v.x;
+                    ls[k] = v.y;
+                    M = fmaxf(M, v.x);
+                }
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
+#pragma unroll
+            for (int k = 0; k < kMaxSlices / 32; ++k) {
+                const int sl = lane + 32 * k;
+                if (sl < S) {
+                    const float e = expf(s_w[warp * S + sl] - M);
+                    s_w[warp * S + sl] = e;
+                    L = fmaf(ls[k], e, L);
+                }
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) L += __shfl_xor_sync(0xffffffffu, L, o);
+            if (lane == 0) s_L[warp] = 1.0f / L;
+        }
+        __syncthreads();
+        if (g < groups) {
+            const float* w = s_w + ch * S;
+            float4 O = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 1
+            for (int from = g; from < S; from += kHold * groups) {
+                hold(from);
+                for (;;) {
+                    bool full = true;
+#pragma unroll
+                    for (int k = 0; k < kHold; ++k) full &= from + k * groups >= S || slot_full(held[k]);
+                    if (full || !patience()) break;
+                    hold(from);
+                }
+#pragma unroll
+                for (int k = 0; k < kHold; ++k) {
+                    const int sl = from + k * groups;
+                    if (sl < S) {
+                        col[sl * (pitch / 4)] = slot_empty4();
+                        const float e = w[sl];
+                        O.x = fmaf(held[k].x, e, O.x);
+                        O.y = fmaf(held[k].y, e, O.y);
+                        O.z = fmaf(held[k].z, e, O.z);
+                        O.w = fmaf(held[k].w, e, O.w);
+                    }
+                }
+            }
+            s_o[tid] = O;     // [group][column]
+        }
+        if (!ok) atomicExch(p.status, 2);
+    }
+    __syncthreads();
+    // the groups' partial outputs, [group][gc * HD], added up
+    const float* o = reinterpret_cast<const float*>(s_o);
+#pragma unroll 1
+    for (int i = tid; i < gc * HD; i += kStreamThreads) {
+        float v = o[i];
+#pragma unroll 1
+        for (int g = 1; g < groups; ++g) v += o[g * gc * HD + i];
+        attn_store(p, (int64_t)(hkv * p.group + g0) * HD + i, v * s_L[i / HD], lane);
+    }
 }
 
 template <typename K, typename... Args>
@@ -490,6 +757,18 @@ static cudaError_t launch_attn(K kernel, dim3 grid, dim3 block, size_t smem, con
     cfg.attrs = attr;
     cfg.numAttrs = ds.pdl ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+template <int HD>
+static int32_t attn_attr() {
+    RSTQ_CUDA(cudaFuncSetAttribute(gqa_decode_stream_kernel<HD, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, attn_smem(HD)));
+    RSTQ_CUDA(cudaFuncSetAttribute(gqa_decode_stream_kernel<HD, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, attn_smem(HD)));
+    RSTQ_CUDA(cudaFuncSetAttribute(gqa_decode_stream_kernel<HD, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, attn_smem(HD)));
+    return RSTQ_OK;
+}
+int32_t attn_configure() {
+    const int32_t rc = attn_attr<64>();
+    return rc != RSTQ_OK ? rc : attn_attr<128>();
 }
 
 }  // namespace rstq
@@ -593,22 +872,20 @@ static int32_t attention_impl(rstq_ctx* ctx, rstq_buf* q, rstq_buf* k, rstq_buf*
     int32_t rc = use_dev(ctx, q->dev);
     if (rc != RSTQ_OK) return rc;
     const bool fast = head_dim == 64 || head_dim == 128;
-    // heads per CTA of the fast kernel: two (one when the group is one).  Four leave no registers for the
-    // rows fetched ahead at head_dim 128 (23.2 against 16.2 us at 32 q / 8 kv x 4096, although K / V then pass
-    // through L2 twice) and lose at head_dim 64 too (14.8 against 13.3 us).
-    const int64_t fg = group >= 2 ? 2 : 1;
-    const int64_t gs = fast ? fg : kAttnGroup;                         // query heads per CTA
-    const int64_t gz = (group + gs - 1) / gs;
-    RSTQ_REQUIRE(n_kv * gz <= kAttnCounters, RSTQ_E_LIMIT, "n_kv x ceil(group / %d) = %lld exceeds %d", (int)gs,
-                 (long long)(n_kv * gz), kAttnCounters);
-    // slices of the cache: enough CTAs for three per SM, at least 64 positions each; sized from the
+    // query heads per CTA of the stream kernel: four (eight, in two passes over a tile, were slower)
+    const int64_t gmax = fast ? kStreamHeads : kAttnGroup;
+    const int64_t gs = group < gmax ? group : gmax, gz = (group + gs - 1) / gs;
+    const int64_t per = !fast ? kAttnGroup : (group >= 2 ? 2 : 1);      // (the limit of the entry point, not of the grid)
+    RSTQ_REQUIRE(n_kv * ((group + per - 1) / per) <= kAttnCounters, RSTQ_E_LIMIT, "n_kv x ceil(group / %d) = %lld exceeds %d", (int)per,
+                 (long long)(n_kv * ((group + per - 1) / per)), kAttnCounters);
+    // slices of the cache: one wave of CTAs, at least 64 positions each; sized from the
     // capacity when the length lives on the device, so that one captured launch serves every length
     const int64_t span = clenbuf ? maxpos : cache_len;
-    const int64_t resident = fast && fg == 1 ? 4 : 2;   // CTAs an SM holds (registers): aim at one wave
-    int64_t S = resident * (int64_t)ds.sm_count / (n_kv * gz);
+    int64_t S = (fast ? 1 : 2) * (int64_t)ds.sm_count / (n_kv * gz);
     if (S > (span + 63) / 64) S = (span + 63) / 64;
     const int64_t row = head_dim + 4;
-    if (S > 8 * row - 1) S = 8 * row - 1;   // the final merge keeps S weights + 1 sum per head in shared memory
+    if (!fast && S > 8 * row - 1) S = 8 * row - 1;   // the general kernel's merge keeps S weights + 1 sum per head in the states' place
+    if (fast && S > kMaxSlices) S = kMaxSlices;
     if (S > 512) S = 512;
     if (S < 1) S = 1;
     if (xq) {
@@ -619,18 +896,25 @@ static int32_t attention_impl(rstq_ctx* ctx, rstq_buf* q, rstq_buf* k, rstq_buf*
         RSTQ_REQUIRE(xq->dev == q->dev && xs->dev == q->dev && (!xsum || xsum->dev == q->dev), RSTQ_E_DEVICE,
                      "buffers live on different devices");
     }
-    const int64_t part_bytes = n_kv * gz * S * gs * row * 4;
-    const bool fresh = ds.attn_scratch_bytes < kAttnCounters * 4 + part_bytes;
-    rc = dev_reserve(ds, &ds.attn_scratch, &ds.attn_scratch_bytes, kAttnCounters * 4 + part_bytes);
-    if (rc != RSTQ_OK) return rc;
-    if (fresh) RSTQ_CUDA(cudaMemsetAsync(ds.attn_scratch, 0, kAttnCounters * 4, ds.stream));
+    const int64_t part_bytes = n_kv * gz * S * (fast ? gs : kAttnGroup) * row * 4;
+    if (fast && S > 1) {      // slots, empty between launches
+        const bool fresh = ds.attn_slots_bytes < part_bytes;
+        rc = dev_reserve(ds, &ds.attn_slots, &ds.attn_slots_bytes, part_bytes);
+        if (rc != RSTQ_OK) return rc;
+        if (fresh) RSTQ_CUDA(cudaMemsetAsync(ds.attn_slots, 0xFF, (size_t)ds.attn_slots_bytes, ds.stream));
+    } else if (!fast) {
+        const bool fresh = ds.attn_scratch_bytes < kAttnCounters * 4 + part_bytes;
+        rc = dev_reserve(ds, &ds.attn_scratch, &ds.attn_scratch_bytes, kAttnCounters * 4 + part_bytes);
+        if (rc != RSTQ_OK) return rc;
+        if (fresh) RSTQ_CUDA(cudaMemsetAsync(ds.attn_scratch, 0, kAttnCounters * 4, ds.stream));
+    }
     AttnParams p;
     p.q = (const float*)q->ptr;
     p.k = (const float*)k->ptr;
     p.v = (const float*)v->ptr;
     p.out = (float*)out->ptr;
-    p.counters = (int*)ds.attn_scratch;
-    p.part = (float*)((char*)ds.attn_scratch + kAttnCounters * 4);
+    p.counters = fast ? nullptr : (int*)ds.attn_scratch;
+    p.part = fast ? (float*)ds.attn_slots : (float*)((char*)ds.attn_scratch + kAttnCounters * 4);
     p.clenbuf = clenbuf ? (const int64_t*)clenbuf->ptr : nullptr;
     p.cache_len = cache_len;
     p.n_q = (int)n_q;
@@ -639,23 +923,23 @@ static int32_t attention_impl(rstq_ctx* ctx, rstq_buf* q, rstq_buf* k, rstq_buf*
     p.head_dim = (int)head_dim;
     p.S = (int)S;
     p.scale = (float)scale;
+    p.gs = (int)gs;
+    p.maxpos = maxpos;
+    p.status = ds.status;
     p.xq = xq ? (int8_t*)xq->ptr : nullptr;
     p.xs = xq ? (float*)xs->ptr : nullptr;
     p.xsum = xq && xsum ? (int32_t*)xsum->ptr : nullptr;
-    const int64_t gc = group < gs ? group : gs;
-    const dim3 grid((unsigned)n_kv, (unsigned)S, (unsigned)gz), block(kAttnWarps * 32);
+    const dim3 grid((unsigned)n_kv, (unsigned)S, (unsigned)gz), block((unsigned)(fast ? kStreamThreads : kAttnWarps * 32));
     if (fast) {
-        const size_t smem = (size_t)((kAttnWarps * gc * row + gc * head_dim) * 4);   // <= 17.5 KB
-        cudaError_t e;
-        if (head_dim == 64)
-            e = fg == 1 ? launch_attn(gqa_decode_fast_kernel<2, 1>, grid, block, smem, ds, p)
-                        : launch_attn(gqa_decode_fast_kernel<2, 2>, grid, block, smem, ds, p);
-        else
-            e = fg == 1 ? launch_attn(gqa_decode_fast_kernel<4, 1>, grid, block, smem, ds, p)
-                        : launch_attn(gqa_decode_fast_kernel<4, 2>, grid, block, smem, ds, p);
-        RSTQ_CUDA(e);
+        const size_t smem = (size_t)attn_smem((int)head_dim);
+#define RSTQ_ATTN(HD)                                                                                      \
+    (gs == 1 ? launch_attn(gqa_decode_stream_kernel<HD, 1>, grid, block, smem, ds, p)                      \
+     : gs == 2 ? launch_attn(gqa_decode_stream_kernel<HD, 2>, grid, block, smem, ds, p)                    \
+               : launch_attn(gqa_decode_stream_kernel<HD, 4>, grid, block, smem, ds, p))
+        RSTQ_CUDA(head_dim == 64 ? RSTQ_ATTN(64) : RSTQ_ATTN(128));
+#undef RSTQ_ATTN
     } else {
-        const size_t smem = (size_t)(kAttnWarps * gc * row * 4);
+        const size_t smem = (size_t)(kAttnWarps * gs * row * 4);
         if (smem > 48 * 1024)
             RSTQ_CUDA(cudaFuncSetAttribute(gqa_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         RSTQ_CUDA(launch_attn(gqa_decode_kernel, grid, block, smem, ds, p));

@@ -569,6 +569,7 @@ int32_t rstq_init(const int32_t* devices, rstq_ctx** ctxp, int32_t ndev) {
             if (r != RSTQ_OK) return r;
             if ((r = gemm_configure(ds)) != RSTQ_OK) return r;
             if ((r = dx_configure()) != RSTQ_OK) return r;
+            if ((r = attn_configure()) != RSTQ_OK) return r;
             RSTQ_CUDA(cudaStreamSynchronize(ds.stream));
             return RSTQ_OK;
         };
@@ -608,6 +609,7 @@ int32_t rstq_shutdown(rstq_ctx* ctx) {
         if (ds.act_scratch) cudaFree(ds.act_scratch);
         if (ds.gemm_scratch) cudaFree(ds.gemm_scratch);
         if (ds.attn_scratch) cudaFree(ds.attn_scratch);
+        if (ds.attn_slots) cudaFree(ds.attn_slots);
         if (ds.kq_scratch) cudaFree(ds.kq_scratch);
         if (ds.f_image) cudaFree(ds.f_image);
         if (ds.bind_stage) cudaFree(ds.bind_stage);
@@ -676,6 +678,7 @@ int32_t rstq_sync(rstq_ctx* ctx, int32_t dev) {
         RSTQ_CUDA(cudaMemsetAsync(ds.status, 0, 4, ds.stream));
         // a launch that gave up may have left hand-over flags set: the next launch must not take them
         RSTQ_CUDA(cudaMemsetAsync(ds.counters, 0, (size_t)ds.counters_len * 4, ds.stream));
+        if (ds.attn_slots) RSTQ_CUDA(cudaMemsetAsync(ds.attn_slots, 0xFF, (size_t)ds.attn_slots_bytes, ds.stream));
         RSTQ_CUDA(cudaStreamSynchronize(ds.stream));
         set_error("a time-bounded wait inside a kernel ran out (status %d); results since the "
                   "last rstq_sync are invalid", st);

@@ -102,6 +102,8 @@ struct DeviceState {
     int64_t f_image_bytes = 0;
     void* attn_scratch = nullptr;  // decode attention: arrival counters + per-slice softmax states
     int64_t attn_scratch_bytes = 0;
+    void* attn_slots = nullptr;    // ... of head_dim 64 and 128: slots of the slices' states, every word 0xFFFFFFFF between launches
+    int64_t attn_slots_bytes = 0;
     void* pinned = nullptr;        // host staging for the host-array entry points
     int64_t pinned_bytes = 0;
     void* io_dev = nullptr;        // device staging for the host-array entry points
@@ -335,6 +337,8 @@ void gemm_plan(int64_t out, int64_t in, int64_t M, int sm_count, bool tmem_kerne
 int32_t launch_gemm(rstq_ctx* ctx, DeviceState& ds, const rstq_weight* w, const void* x, int src, void* y,
                     int out_dtype, int64_t M, void* x16, float* rowscale, float* acc32);
 int32_t gemm_configure(DeviceState& ds);
+// attn.cu
+int32_t attn_configure();  // shared-memory attributes, once per device
 // dx.cu
 int32_t dx_configure();  // shared-memory attributes, once per device
 int32_t launch_qlinear_q8_dx(rstq_ctx* ctx, DeviceState& ds, const float* dy, const int8_t* codes,

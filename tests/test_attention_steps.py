@@ -233,3 +233,55 @@ def test_attention_with_quantized_output_equals_attention_then_quantizer(ctx, n_
     assert e.value.code == L.E_SHAPE                  # head_dim 32: no fused quantizer
     for o in (bq, bk, bv, bo, q1, s1, z1, q2, s2, z2):
         o.free()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("group,n_kv", [(1, 5), (2, 3), (3, 2), (4, 1), (5, 2), (7, 4), (8, 1), (9, 2), (17, 1)])
+def test_attention_at_the_edges_of_its_tiles(ctx, group, n_kv, hd):
+    """One, two, four and eight heads per pass and what is left over; lengths around a tile of 8 positions, a slice's 64
+    and a round of the warps.  Rows beyond the length hold NaN: they must not count.  1e-5 as above."""
+    n_q, maxpos, scale = group * n_kv, 2100, 1.0 / math.sqrt(hd)
+    q = synth.normal(71 + group, n_q * hd)
+    k0, v0 = synth.normal(72, maxpos * n_kv * hd), synth.normal(73, maxpos * n_kv * hd)
+    bq, bo = ctx.array_to_buffer(q), ctx.make_buffer(n_q * hd, np.float32)
+    bk, bv = ctx.make_buffer(k0.size, np.float32), ctx.make_buffer(v0.size, np.float32)
+    bl = ctx.make_buffer(1, np.int64)
+    for clen in (1, 7, 8, 9, 63, 64, 65, 200, 513, 2099):
+        k, v = k0.copy(), v0.copy()
+        k[clen * n_kv * hd:] = np.nan
+        v[clen * n_kv * hd:] = np.nan
+        bk.upload(k), bv.upload(v), bl.upload(np.array([clen], np.int64))
+        ref = orc.gqa_decode_attention(q, k0, v0, clen, n_q, group, n_kv, hd, scale)
+        ctx.gqa_decode_attention(bq, bk, bv, bo, clen, n_q, group, n_kv, hd, maxpos, scale)
+        ctx.sync()
+        assert relerr(bo.download(), ref) <= 1e-5, clen
+        ctx.gqa_decode_attention(bq, bk, bv, bo, 0, n_q, group, n_kv, hd, maxpos, scale, clenbuf=bl)
+        ctx.sync()
+        assert relerr(bo.download(), ref) <= 1e-5, clen
+    for o in (bq, bo, bk, bv, bl):
+        o.free()
+
+
+@pytest.mark.gpu
+def test_attention_of_special_values(ctx):
+    """Every bit pattern of a NaN comes through the slices' merge as a NaN, an infinite V as an infinity, and calls of other
+    shapes in between find the scratch as they need it."""
+    n_q, n_kv, hd, clen = 8, 2, 64, 700
+    group, scale = n_q // n_kv, 0.125
+    q, k, v = synth.normal(81, n_q * hd), synth.normal(82, clen * n_kv * hd), synth.normal(83, clen * n_kv * hd)
+    ref = orc.gqa_decode_attention(q, k, v, clen, n_q, group, n_kv, hd, scale).reshape(n_q, hd)
+    vv = v.reshape(clen, n_kv, hd)
+    vv.view(np.uint32)[650, 0, 5] = 0xFFFFFFFF
+    vv[20, 1, 7] = np.inf
+    bq, bk, bv, bo = ctx.array_to_buffer(q), ctx.array_to_buffer(k), ctx.array_to_buffer(v), ctx.make_buffer(n_q * hd, np.float32)
+    for n, h in ((clen, group), (64, group), (300, 1), (clen, group)):
+        heads = h * n_kv
+        ctx.gqa_decode_attention(bq, bk, bv, bo, n, heads, h, n_kv, hd, clen, scale)
+        ctx.sync()
+    out = bo.download().reshape(n_q, hd)
+    assert np.isnan(out[:group, 5]).all() and np.isposinf(out[group:, 7]).all()
+    out[:group, 5], out[group:, 7] = ref[:group, 5], ref[group:, 7]
+    assert relerr(out, ref) <= 1e-5
+    for o in (bq, bk, bv, bo):
+        o.free()
