@@ -667,8 +667,35 @@ __device__ __forceinline__ uint64_t mul_f32x2(uint64_t a, uint64_t b) {
     return r;
 }
 
+// Where a lane finds the activations of a block above one token: its fragment of token tile nt at b[nt] (mode F: the
+// second half of the block at + half), the records of its pair of tokens at z[nt], counted from the block's own.  Worked
+// out once per launch, not from the token count per unit.  With two units of two token tiles loaded ahead, us for the two
+// matrices of an MLP, MODE_A8: int4 70B at M = 16 95.1 -> 91.1, int8 7B at M = 12 35.8 -> 34.9, int4 7B at M = 8 23.1 ->
+// 22.9.  (Mode F: no difference; two units ahead there 108.6 -> 112.4 at M = 16, bf16.)
+// (columns beyond M are never stored, so any valid address will do for them)
+template <int NT>
+struct ActLanes {
+    uint32_t b[NT], z[NT], half;
+};
+template <int MODE, int NT>
+__device__ __forceinline__ ActLanes<NT> act_lanes(const StreamParams& p, int gid, int tig) {
+    ActLanes<NT> a;
+    const int C = MODE == MODE_A8 ? p.M : p.M * p.T, Mh = (p.M + 1) >> 1;
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt) {
+        int col = nt * 8 + gid, pr = nt * 4 + tig;
+        col = col < C ? col : C - 1;
+        pr = pr < Mh ? pr : 0;
+        a.b[nt] = (uint32_t)(col * 4 + tig) * 8;
+        a.z[nt] = (uint32_t)pr * 32;
+    }
+    a.half = (uint32_t)C * 32;
+    return a;
+}
+
+// xB, xZ: the block's fragments and records (plain units), else those of block 0 of the staged arrays
 template <int BITS, int NT, int UK = 0>
-__device__ __forceinline__ void unit_a8(const SUnit<BITS>& u, uint32_t actB, uint32_t actZ,
+__device__ __forceinline__ void unit_a8(const SUnit<BITS>& u, uint32_t actB, uint32_t actZ, const ActLanes<NT>& at,
                                         const StreamParams& p, int b, int gid, int tig,
                                         float (&acc)[NT][4][2]) {
     constexpr bool KQ = UK == 1;
@@ -713,19 +740,12 @@ __device__ __forceinline__ void unit_a8(const SUnit<BITS>& u, uint32_t actB, uin
         // (put_act_record); the fold of a row's two values is two packed f32 operations and two fmas:
         // t = (float(d) - bias) * xs for both tokens at once, acc += s * t each.
         const float sc[4] = {u.sc.x, u.sc.y, u.sc.z, u.sc.w};
-        const int M = p.M, Mh = (M + 1) >> 1;
-        const uint32_t xB = actB + b * M * 32, rec = actZ + b * Mh * 32;
         const uint64_t nbias = pack_f32x2(-kMagicFlt, -kMagicFlt);
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt) {
-            // columns beyond M are never stored, so any valid address will do for them
-            int col = nt * 8 + gid;
-            col = col < M ? col : M - 1;
-            const uint2 bb = lds64(xB + (col * 4 + tig) * 8);
-            int pr = nt * 4 + tig;
-            pr = pr < Mh ? pr : 0;
-            const ulonglong2 xv = lds128q(rec + pr * 32);         // {xs_a, xs_b}, {xs_a h, xs_b h}
-            const uint4 cv = lds128(rec + pr * 32 + 16);          // ca_a, ca_b, cb_a, cb_b
+            const uint2 bb = lds64(actB + at.b[nt]);
+            const ulonglong2 xv = lds128q(actZ + at.z[nt]);       // {xs_a, xs_b}, {xs_a h, xs_b h}
+            const uint4 cv = lds128(actZ + at.z[nt] + 16);        // ca_a, ca_b, cb_a, cb_b
 #pragma unroll
             for (int q = 0; q < 2; ++q) {
                 int d[4];
@@ -801,10 +821,16 @@ __device__ __forceinline__ uint32_t dq4_bf16x2(uint32_t w, uint32_t m4, uint32_t
     return d;
 }
 
+// D = A * B: the accumulator input is the zero register (as a variable it takes four moves)
+__device__ __forceinline__ void hmma_bf16_zero(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
+}
+
 template <int BITS, int NT>
-__device__ __forceinline__ void unit_f(const SUnit<BITS>& u, uint32_t actB,
-                                       const StreamParams& p, int b, int gid, int tig,
-                                       float (&acc)[NT][4][2]) {
+__device__ __forceinline__ void unit_f(const SUnit<BITS>& u, uint32_t xb, const ActLanes<NT>& at, float (&acc)[NT][4][2]) {
     // fr[h][i][j]: half h, row gid + 8i, j = 0 -> elements (+0, +2), j = 1 -> (+1, +3)
     uint32_t fr[2][4][2];
     const uint32_t c0[4] = {u.c0.x, u.c0.y, u.c0.z, u.c0.w};
@@ -840,21 +866,17 @@ __device__ __forceinline__ void unit_f(const SUnit<BITS>& u, uint32_t actB,
             }
     }
     const float sc[4] = {u.sc.x, u.sc.y, u.sc.z, u.sc.w};
-    const int C = p.M * p.T;
-    const uint32_t xb = actB + b * C * 64;
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) {
-        int col = nt * 8 + gid;
-        col = col < C ? col : C - 1;
-        const uint2 bx0 = lds64(xb + (col * 4 + tig) * 8);
-        const uint2 bx1 = lds64(xb + ((C + col) * 4 + tig) * 8);
+        const uint2 bx0 = lds64(xb + at.b[nt]);
+        const uint2 bx1 = lds64(xb + at.half + at.b[nt]);
 #pragma unroll
         for (int mt = 0; mt < 2; ++mt) {
             const int r0 = 2 * mt, r1 = 2 * mt + 1;
-            float c[4] = {0.f, 0.f, 0.f, 0.f};
+            float c[4];
             const uint32_t a_lo[4] = {fr[0][r0][0], fr[0][r1][0], fr[0][r0][1], fr[0][r1][1]};
             const uint32_t a_hi[4] = {fr[1][r0][0], fr[1][r1][0], fr[1][r0][1], fr[1][r1][1]};
-            hmma_bf16(c, a_lo, bx0.x, bx0.y);
+            hmma_bf16_zero(c, a_lo, bx0.x, bx0.y);
             hmma_bf16(c, a_hi, bx1.x, bx1.y);
             acc[nt][r0][0] = fmaf(sc[r0], c[0], acc[nt][r0][0]);
             acc[nt][r0][1] = fmaf(sc[r0], c[1], acc[nt][r0][1]);
@@ -1420,6 +1442,8 @@ __global__ void __launch_bounds__(kStreamThreads, 1) gemv_stream_kernel(const __
         const bool ring = p.ring;
         uint32_t actB = smem_u32(smem) + p.act_off;
         uint32_t actZ = smem_u32(smem) + p.act2_off;
+        const ActLanes<NT> at = act_lanes<MODE, NT>(p, gid, tig);
+        const uint32_t strideB = MODE == MODE_F ? 2 * at.half : at.half, strideZ = (uint32_t)((p.M + 1) >> 1) * 32;   // bytes of a block
         zero_acc();
         if (dbg) {  // timestamp of the first weights; the loop's own wait then passes at once
             if (!mbar_try(full0, 0)) alive = mbar_wait(full0, 0, abort_flag);
@@ -1432,29 +1456,39 @@ __global__ void __launch_bounds__(kStreamThreads, 1) gemv_stream_kernel(const __
                 alive = mbar_wait(full0 + 8 * s, ph, abort_flag);
             if (alive && !PROBE(2)) {
                 const int b0 = ring ? warp : b + warp;   // block index of this warp's first unit
-                if (n == kChunkUnits && NT == 1) {
-                    // a full chunk: this warp's units are all loaded before the first tile, so that
-                    // the shared-memory round trips of one unit run under the arithmetic of another
-                    SUnit<BITS> un[kUPW];
+                const uint32_t xB = actB + (uint32_t)b0 * strideB, xZ = actZ + (uint32_t)b0 * strideZ;
+                auto fold = [&](const SUnit<BITS>& un, int j) {
+                    const uint32_t uB = xB + (uint32_t)j * (kCW * strideB), uZ = xZ + (uint32_t)j * (kCW * strideZ);
+                    if (MODE == MODE_F) unit_f<BITS, NT>(un, uB, at, acc);
+                    else if (UK == 0) unit_a8<BITS, NT, UK>(un, uB, uZ, at, p, 0, gid, tig, acc);
+                    else unit_a8<BITS, NT, UK>(un, actB, actZ, at, p, b0 + j * kCW, gid, tig, acc);
+                };
+                // units of this warp, all loaded before the first tile, so that the shared-memory round trips of one run
+                // under the arithmetic of another
+                auto whole = [&](auto units) {
+                    constexpr int N = decltype(units)::value;
+                    SUnit<BITS> un[N];
 #pragma unroll
-                    for (int j = 0; j < kUPW; ++j) lds_unit<BITS, UK>(un[j], unit0 + j * kCW * UNIT, lane);
+                    for (int j = 0; j < N; ++j) lds_unit<BITS, UK>(un[j], unit0 + j * kCW * UNIT, lane);
 #pragma unroll
-                    for (int j = 0; j < kUPW; ++j) {
-                        if (MODE == MODE_A8) unit_a8<BITS, NT, UK>(un[j], actB, actZ, p, b0 + j * kCW, gid, tig, acc);
-                        else unit_f<BITS, NT>(un[j], actB, p, b0 + j * kCW, gid, tig, acc);
+                    for (int j = 0; j < N; ++j) fold(un[j], j);
+                };
+                if (n == kChunkUnits && (NT == 1 || (kUPW == 2 && MODE == MODE_A8))) {
+                    whole(std::integral_constant<int, kUPW>{});
+                } else if (kUPW == 4 && MODE == MODE_A8 && (n == kChunkUnits / 2 || (NT == 2 && n == kChunkUnits))) {
+                    whole(std::integral_constant<int, 2>{});   // (two token tiles: two units at a time are what the registers hold)
+                    if (NT == 2 && n == kChunkUnits) {
+                        SUnit<BITS> un[2];
+#pragma unroll
+                        for (int j = 0; j < 2; ++j) lds_unit<BITS, UK>(un[j], unit0 + (2 + j) * kCW * UNIT, lane);
+#pragma unroll
+                        for (int j = 0; j < 2; ++j) fold(un[j], 2 + j);
                     }
-                } else if (kUPW == 4 && n == kChunkUnits / 2 && NT == 1 && MODE == MODE_A8) {
-                    SUnit<BITS> un[2];   // a full chunk of the half-size ring
-#pragma unroll
-                    for (int j = 0; j < 2; ++j) lds_unit<BITS, UK>(un[j], unit0 + j * kCW * UNIT, lane);
-#pragma unroll
-                    for (int j = 0; j < 2; ++j) unit_a8<BITS, NT, UK>(un[j], actB, actZ, p, b0 + j * kCW, gid, tig, acc);
                 } else {
                     for (int j = 0; warp + j * kCW < n; ++j) {
                         SUnit<BITS> un;
                         lds_unit<BITS, UK>(un, unit0 + j * kCW * UNIT, lane);
-                        if (MODE == MODE_A8) unit_a8<BITS, NT, UK>(un, actB, actZ, p, b0 + j * kCW, gid, tig, acc);
-                        else unit_f<BITS, NT>(un, actB, p, b0 + j * kCW, gid, tig, acc);
+                        fold(un, j);
                     }
                 }
             }
