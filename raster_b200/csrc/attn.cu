@@ -384,6 +384,8 @@ __host__ __device__ constexpr int attn_q_off() { return kStreamWarps * kRingByte
 __host__ __device__ constexpr int attn_p_off(int hd) { return attn_q_off() + kStreamHeads * hd * 4; }
 __host__ __device__ constexpr int attn_smem(int hd) { return attn_p_off(hd) + kStreamWarps * kTilePos * kStreamHeads * 4; }
 // ... and, once the rings are drained, in their place: the warps' states, then the merge of the slices
+constexpr int kClusterMax = 8;                        // slices of a KV head that may be one cluster
+constexpr int64_t kClusterExtra = 65000;              // bytes of K and V that a slice may grow by for it
 constexpr int kMaxSlices = 160;                       // five (max, sum) pairs per lane of the merging warps
 __host__ __device__ constexpr int attn_w_off(int hd) { return kStreamWarps * kStreamHeads * (hd + 4) * 4; }       // slice weights
 __host__ __device__ constexpr int attn_o_off(int hd) { return attn_w_off(hd) + kStreamHeads * kMaxSlices * 4; }  // partial outputs
@@ -413,8 +415,21 @@ __device__ __forceinline__ float4 ld_shared_f4(uint32_t a) {
     asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a));
     return v;
 }
-// H = query heads of the KV head that a CTA serves at most (1, 2 or 4).
-template <int HD, int H>
+__device__ __forceinline__ void attn_cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// a value at the same place of a cluster's CTA `rank`
+__device__ __forceinline__ float ld_cluster(uint32_t at, int rank) {
+    uint32_t a;
+    float v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(at), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+    return v;
+}
+
+// H = query heads of the KV head that a CTA serves at most (1, 2 or 4).  CL: the slices of a KV head are one cluster.
+template <int HD, int H, bool CL>
 __global__ void __launch_bounds__(kStreamThreads, 1)
 gqa_decode_stream_kernel(const AttnParams p) {
     constexpr int VEC = HD / 32, ROW = HD + 4;      // VEC: float4 per lane of a position's eight lanes
@@ -637,8 +652,37 @@ gqa_decode_stream_kernel(const AttnParams p) {
             O.z = fmaf(a.z, e, O.z);
             O.w = fmaf(a.w, e, O.w);
         }
-        if (S == 1) s_o[tid] = O;      // (the one slice's state is the result's)
+        if (CL || S == 1) s_o[tid] = O;      // (without a cluster, the one slice's state is the result's)
         else reinterpret_cast<float4*>(out_part + h * ROW)[c] = make_float4(slot_value(O.x), slot_value(O.y), slot_value(O.z), slot_value(O.w));
+    }
+    if constexpr (CL) {
+        // The slices' states -> out, through distributed shared memory: a warp takes 32 neighbouring values of a head.
+        attn_cluster_sync();
+        const uint32_t o = smem_u32(s_o), m_at = smem_u32(s_cM), l_at = smem_u32(s_cL);
+        for (int b = split + S * warp; b < gc * (HD / 32); b += S * kStreamWarps) {
+            const int e = b * 32 + lane, h = b / (HD / 32);
+            float Os[kClusterMax], Ms[kClusterMax], Ls[kClusterMax], M = kNegInf, L = 0.f, O = 0.f;
+#pragma unroll
+            for (int k = 0; k < kClusterMax; ++k)
+                if (k < S) {
+                    Ms[k] = ld_cluster(m_at + h * 4, k);
+                    Ls[k] = ld_cluster(l_at + h * 4, k);
+                    Os[k] = ld_cluster(o + e * 4, k);
+                }
+#pragma unroll
+            for (int k = 0; k < kClusterMax; ++k)
+                if (k < S) M = fmaxf(M, Ms[k]);
+#pragma unroll
+            for (int k = 0; k < kClusterMax; ++k)
+                if (k < S) {
+                    const float w = expf(Ms[k] - M);
+                    L = fmaf(Ls[k], w, L);
+                    O = fmaf(Os[k], w, O);
+                }
+            attn_store(p, (int64_t)(hkv * p.group + g0) * HD + e, O * (1.0f / L), lane);
+        }
+        attn_cluster_sync();   // nobody leaves while its shared memory is read
+        return;
     }
     int groups = 1;
     if (S == 1) {
@@ -746,31 +790,62 @@ gqa_decode_stream_kernel(const AttnParams p) {
     }
 }
 
+// cluster: thread blocks along y that are one
 template <typename K, typename... Args>
-static cudaError_t launch_attn(K kernel, dim3 grid, dim3 block, size_t smem, const DeviceState& ds, Args... args) {
+static cudaError_t launch_attn_cluster(K kernel, dim3 grid, dim3 block, size_t smem, const DeviceState& ds, unsigned cluster, Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = ds.stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute attr[2];
+    int n = 0;
+    if (ds.pdl) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster > 1) {
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = attr[n].val.clusterDim.z = 1;
+        attr[n++].val.clusterDim.y = cluster;
+    }
     cfg.attrs = attr;
-    cfg.numAttrs = ds.pdl ? 1 : 0;
+    cfg.numAttrs = (unsigned)n;
     return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+template <typename K, typename... Args>
+static cudaError_t launch_attn(K kernel, dim3 grid, dim3 block, size_t smem, const DeviceState& ds, Args... args) {
+    return launch_attn_cluster(kernel, grid, block, smem, ds, 1u, args...);
 }
 
 template <int HD>
 static int32_t attn_attr() {
-    RSTQ_CUDA(cudaFuncSetAttribute(gqa_decode_stream_kernel<HD, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, attn_smem(HD)));
-    RSTQ_CUDA(cudaFuncSetAttribute(gqa_decode_stream_kernel<HD, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, attn_smem(HD)));
-    RSTQ_CUDA(cudaFuncSetAttribute(gqa_decode_stream_kernel<HD, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, attn_smem(HD)));
+    RSTQ_CUDA(cudaFuncSetAttribute(gqa_decode_stream_kernel<HD, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, attn_smem(HD)));
+    RSTQ_CUDA(cudaFuncSetAttribute(gqa_decode_stream_kernel<HD, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, attn_smem(HD)));
+    RSTQ_CUDA(cudaFuncSetAttribute(gqa_decode_stream_kernel<HD, 2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, attn_smem(HD)));
+    RSTQ_CUDA(cudaFuncSetAttribute(gqa_decode_stream_kernel<HD, 2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, attn_smem(HD)));
+    RSTQ_CUDA(cudaFuncSetAttribute(gqa_decode_stream_kernel<HD, 4, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, attn_smem(HD)));
+    RSTQ_CUDA(cudaFuncSetAttribute(gqa_decode_stream_kernel<HD, 4, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, attn_smem(HD)));
     return RSTQ_OK;
 }
-int32_t attn_configure() {
-    const int32_t rc = attn_attr<64>();
-    return rc != RSTQ_OK ? rc : attn_attr<128>();
+int32_t attn_configure(DeviceState& ds) {
+    int32_t rc = attn_attr<64>();
+    if (rc == RSTQ_OK) rc = attn_attr<128>();
+    // how many clusters of each size the device holds at once (148 SMs: 74, 45, 33, 26, 22, 15, 15)
+    for (int c = 2; c <= kClusterMax && rc == RSTQ_OK; ++c) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(1, (unsigned)c);
+        cfg.blockDim = dim3(kStreamThreads);
+        cfg.dynamicSmemBytes = attn_smem(128);
+        cudaLaunchAttribute a[1];
+        a[0].id = cudaLaunchAttributeClusterDimension;
+        a[0].val.clusterDim.x = a[0].val.clusterDim.z = 1;
+        a[0].val.clusterDim.y = (unsigned)c;
+        cfg.attrs = a;
+        cfg.numAttrs = 1;
+        RSTQ_CUDA(cudaOccupancyMaxActiveClusters(&ds.attn_clusters[c], gqa_decode_stream_kernel<128, 4, true>, &cfg));
+    }
+    return rc;
 }
 
 }  // namespace rstq
@@ -890,6 +965,18 @@ static int32_t attention_impl(rstq_ctx* ctx, rstq_buf* q, rstq_buf* k, rstq_buf*
     if (fast && S > kMaxSlices) S = kMaxSlices;
     if (S > 512) S = 512;
     if (S < 1) S = 1;
+    // Up to eight slices may be one cluster and meet in distributed shared memory, which saves 1 - 1.5 us of the tail (32 /
+    // 32 heads x 1000 9.65 -> 8.24 us, 32 / 8 x 200 6.68 -> 5.19, four 7B layers 206.5 -> 196.8), as long as all clusters
+    // are resident together: 16 of eight took two waves, 32 / 16 x 2000 16.1 us against 10.4.  Fewer, longer slices are taken
+    // for it where each grows by less than about 1 us of its stream (32 / 16 x 500, nine -> six: 6.89 -> 5.38; x 2000:
+    // 9.81 -> 10.55, so not there).
+    bool clustered = false;
+    for (int64_t c = fast ? (S < kClusterMax ? S : kClusterMax) : 0; c > 1 && !clustered; --c) {
+        if (n_kv * gz > ds.attn_clusters[c]) continue;
+        if ((span / c - span / S) * head_dim * 8 > kClusterExtra) break;
+        S = c;
+        clustered = true;
+    }
     if (xq) {
         RSTQ_REQUIRE(fast, RSTQ_E_SHAPE, "the quantized output needs head_dim 64 or 128, got %lld", (long long)head_dim);
         const int64_t n = n_q * head_dim;
@@ -899,7 +986,7 @@ static int32_t attention_impl(rstq_ctx* ctx, rstq_buf* q, rstq_buf* k, rstq_buf*
                      "buffers live on different devices");
     }
     const int64_t part_bytes = n_kv * gz * S * (fast ? gs : kAttnGroup) * row * 4;
-    if (fast && S > 1) {      // slots, empty between launches
+    if (fast && !clustered && S > 1) {      // slots, empty between launches
         const bool fresh = ds.attn_slots_bytes < part_bytes;
         rc = dev_reserve(ds, &ds.attn_slots, &ds.attn_slots_bytes, part_bytes);
         if (rc != RSTQ_OK) return rc;
@@ -934,11 +1021,12 @@ static int32_t attention_impl(rstq_ctx* ctx, rstq_buf* q, rstq_buf* k, rstq_buf*
     const dim3 grid((unsigned)n_kv, (unsigned)S, (unsigned)gz), block((unsigned)(fast ? kStreamThreads : kAttnWarps * 32));
     if (fast) {
         const size_t smem = (size_t)attn_smem((int)head_dim);
-#define RSTQ_ATTN(HD)                                                                                      \
-    (gs == 1 ? launch_attn(gqa_decode_stream_kernel<HD, 1>, grid, block, smem, ds, p)                      \
-     : gs == 2 ? launch_attn(gqa_decode_stream_kernel<HD, 2>, grid, block, smem, ds, p)                    \
-               : launch_attn(gqa_decode_stream_kernel<HD, 4>, grid, block, smem, ds, p))
-        RSTQ_CUDA(head_dim == 64 ? RSTQ_ATTN(64) : RSTQ_ATTN(128));
+#define RSTQ_ATTN(HD, CL)                                                                                            \
+    (gs == 1 ? launch_attn_cluster(gqa_decode_stream_kernel<HD, 1, CL>, grid, block, smem, ds, CL ? (unsigned)S : 1u, p)   \
+     : gs == 2 ? launch_attn_cluster(gqa_decode_stream_kernel<HD, 2, CL>, grid, block, smem, ds, CL ? (unsigned)S : 1u, p) \
+               : launch_attn_cluster(gqa_decode_stream_kernel<HD, 4, CL>, grid, block, smem, ds, CL ? (unsigned)S : 1u, p))
+        if (clustered) RSTQ_CUDA(head_dim == 64 ? RSTQ_ATTN(64, true) : RSTQ_ATTN(128, true));
+        else RSTQ_CUDA(head_dim == 64 ? RSTQ_ATTN(64, false) : RSTQ_ATTN(128, false));
 #undef RSTQ_ATTN
     } else {
         const size_t smem = (size_t)(kAttnWarps * gs * row * 4);

@@ -569,7 +569,7 @@ int32_t rstq_init(const int32_t* devices, rstq_ctx** ctxp, int32_t ndev) {
             if (r != RSTQ_OK) return r;
             if ((r = gemm_configure(ds)) != RSTQ_OK) return r;
             if ((r = dx_configure()) != RSTQ_OK) return r;
-            if ((r = attn_configure()) != RSTQ_OK) return r;
+            if ((r = attn_configure(ds)) != RSTQ_OK) return r;
             RSTQ_CUDA(cudaStreamSynchronize(ds.stream));
             return RSTQ_OK;
         };
