@@ -667,35 +667,60 @@ __device__ __forceinline__ uint64_t mul_f32x2(uint64_t a, uint64_t b) {
     return r;
 }
 
-// Where a lane finds the activations of a block above one token: its fragment of token tile nt at b[nt] (mode F: the
-// second half of the block at + half), the records of its pair of tokens at z[nt], counted from the block's own.  Worked
-// out once per launch, not from the token count per unit.  With two units of two token tiles loaded ahead, us for the two
-// matrices of an MLP, MODE_A8: int4 70B at M = 16 95.1 -> 91.1, int8 7B at M = 12 35.8 -> 34.9, int4 7B at M = 8 23.1 ->
-// 22.9.  (Mode F: no difference; two units ahead there 108.6 -> 112.4 at M = 16, bf16.)
-// (columns beyond M are never stored, so any valid address will do for them)
-template <int NT>
-struct ActLanes {
-    uint32_t b[NT], z[NT], half;
-};
-template <int MODE, int NT>
-__device__ __forceinline__ ActLanes<NT> act_lanes(const StreamParams& p, int gid, int tig) {
-    ActLanes<NT> a;
-    const int C = MODE == MODE_A8 ? p.M : p.M * p.T, Mh = (p.M + 1) >> 1;
+// Plain units: everything that depends on the (block, token) alone comes ready-made in the pair record (put_act_record);
+// the fold of a row's two values is two packed f32 operations and two fmas: t = (float(d) - bias) * xs for both
+// tokens at once, acc += s * t each.  bb: the token's fragment; xv, cv: {xs_a, xs_b}, {xs_a h, xs_b h}; ca_a, ca_b, cb_a, cb_b.
+__device__ __forceinline__ void fold_plain(const uint32_t (&a)[2][4], const float (&sc)[4], uint2 bb, ulonglong2 xv, uint4 cv,
+                                           float (&acc)[4][2]) {
+    const uint64_t nbias = pack_f32x2(-kMagicFlt, -kMagicFlt);
 #pragma unroll
-    for (int nt = 0; nt < NT; ++nt) {
-        int col = nt * 8 + gid, pr = nt * 4 + tig;
-        col = col < C ? col : C - 1;
-        pr = pr < Mh ? pr : 0;
-        a.b[nt] = (uint32_t)(col * 4 + tig) * 8;
-        a.z[nt] = (uint32_t)pr * 32;
+    for (int q = 0; q < 2; ++q) {
+        int d[4];
+        imma_acc(d, a[q], bb.x, bb.y, (int)cv.x, (int)cv.y, (int)cv.z, (int)cv.w);
+        const uint64_t tl = mul_f32x2(add_f32x2(pack_b32x2((uint32_t)d[0], (uint32_t)d[1]), nbias), xv.x);
+        const uint64_t th = mul_f32x2(add_f32x2(pack_b32x2((uint32_t)d[2], (uint32_t)d[3]), nbias), xv.y);
+        const float s0 = sc[2 * q], s1 = sc[2 * q + 1];
+        acc[2 * q][0] = fmaf(s0, lo_f32x2(tl), acc[2 * q][0]);
+        acc[2 * q][1] = fmaf(s0, hi_f32x2(tl), acc[2 * q][1]);
+        acc[2 * q + 1][0] = fmaf(s1, lo_f32x2(th), acc[2 * q + 1][0]);
+        acc[2 * q + 1][1] = fmaf(s1, hi_f32x2(th), acc[2 * q + 1][1]);
     }
-    a.half = (uint32_t)C * 32;
-    return a;
 }
 
-// xB, xZ: the block's fragments and records (plain units), else those of block 0 of the staged arrays
+// MODE_A8, plain units, two token tiles (9 .. 16 tokens): where a lane finds its fragment of tile nt and the records of its
+// pair of tokens, counted from the block's own, is worked out once per launch, and a warp loads two units before the
+// first tile.  us for the two matrices of an MLP: int4 70B at 16 tokens 95.1 -> 91.1; 6000 x 5120 and 4000 x 7168 at 9 / 12 /
+// 16 tokens int4 25.0 / 25.5 / 25.7 -> 24.1 / 24.8 / 24.4, int8 28.2 / 28.7 / 29.3 -> 26.7 / 27.4 / 27.5.  (The same for one tile, for
+// K-quant units and in mode F: between nothing and 2.6 % slower.)
+struct TwoTiles {
+    uint32_t b[2], z[2], block_b, block_z;   // block_b, block_z: bytes of a block's fragments and records
+};
+__device__ __forceinline__ TwoTiles two_tiles(const StreamParams& p, int gid, int tig) {
+    TwoTiles a;
+    const int M = p.M, Mh = (M + 1) >> 1;
+#pragma unroll
+    for (int nt = 0; nt < 2; ++nt) {
+        // columns beyond M are never stored, so any valid address will do for them
+        const int col = nt * 8 + gid, pr = nt * 4 + tig;
+        a.b[nt] = (uint32_t)((col < M ? col : M - 1) * 4 + tig) * 8;
+        a.z[nt] = (uint32_t)(pr < Mh ? pr : 0) * 32;
+    }
+    a.block_b = (uint32_t)M * 32;
+    a.block_z = (uint32_t)Mh * 32;
+    return a;
+}
+template <int BITS>
+__device__ __forceinline__ void unit_two(const SUnit<BITS>& u, uint32_t xB, uint32_t rec, const TwoTiles& at, float (&acc)[2][4][2]) {
+    uint32_t a[2][4];
+    a_frags<BITS>(u, a);
+    const float sc[4] = {u.sc.x, u.sc.y, u.sc.z, u.sc.w};
+#pragma unroll
+    for (int nt = 0; nt < 2; ++nt)
+        fold_plain(a, sc, lds64(xB + at.b[nt]), lds128q(rec + at.z[nt]), lds128(rec + at.z[nt] + 16), acc[nt]);
+}
+
 template <int BITS, int NT, int UK = 0>
-__device__ __forceinline__ void unit_a8(const SUnit<BITS>& u, uint32_t actB, uint32_t actZ, const ActLanes<NT>& at,
+__device__ __forceinline__ void unit_a8(const SUnit<BITS>& u, uint32_t actB, uint32_t actZ,
                                         const StreamParams& p, int b, int gid, int tig,
                                         float (&acc)[NT][4][2]) {
     constexpr bool KQ = UK == 1;
@@ -736,28 +761,19 @@ __device__ __forceinline__ void unit_a8(const SUnit<BITS>& u, uint32_t actB, uin
         return;
     }
     if (UK == 0) {
-        // Plain units: everything that depends on the (block, token) alone comes ready-made in the pair record
-        // (put_act_record); the fold of a row's two values is two packed f32 operations and two fmas:
-        // t = (float(d) - bias) * xs for both tokens at once, acc += s * t each.
         const float sc[4] = {u.sc.x, u.sc.y, u.sc.z, u.sc.w};
-        const uint64_t nbias = pack_f32x2(-kMagicFlt, -kMagicFlt);
+        const int M = p.M, Mh = (M + 1) >> 1;
+        const uint32_t xB = actB + b * M * 32, rec = actZ + b * Mh * 32;
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt) {
-            const uint2 bb = lds64(actB + at.b[nt]);
-            const ulonglong2 xv = lds128q(actZ + at.z[nt]);       // {xs_a, xs_b}, {xs_a h, xs_b h}
-            const uint4 cv = lds128(actZ + at.z[nt] + 16);        // ca_a, ca_b, cb_a, cb_b
-#pragma unroll
-            for (int q = 0; q < 2; ++q) {
-                int d[4];
-                imma_acc(d, a[q], bb.x, bb.y, (int)cv.x, (int)cv.y, (int)cv.z, (int)cv.w);
-                const uint64_t tl = mul_f32x2(add_f32x2(pack_b32x2((uint32_t)d[0], (uint32_t)d[1]), nbias), xv.x);
-                const uint64_t th = mul_f32x2(add_f32x2(pack_b32x2((uint32_t)d[2], (uint32_t)d[3]), nbias), xv.y);
-                const float s0 = sc[2 * q], s1 = sc[2 * q + 1];
-                acc[nt][2 * q][0] = fmaf(s0, lo_f32x2(tl), acc[nt][2 * q][0]);
-                acc[nt][2 * q][1] = fmaf(s0, hi_f32x2(tl), acc[nt][2 * q][1]);
-                acc[nt][2 * q + 1][0] = fmaf(s1, lo_f32x2(th), acc[nt][2 * q + 1][0]);
-                acc[nt][2 * q + 1][1] = fmaf(s1, hi_f32x2(th), acc[nt][2 * q + 1][1]);
-            }
+            // columns beyond M are never stored, so any valid address will do for them
+            int col = nt * 8 + gid;
+            col = col < M ? col : M - 1;
+            int pr = nt * 4 + tig;
+            pr = pr < Mh ? pr : 0;
+            const uint2 bb = lds64(xB + (col * 4 + tig) * 8);
+            const ulonglong2 xv = lds128q(rec + pr * 32);
+            fold_plain(a, sc, bb, xv, lds128(rec + pr * 32 + 16), acc[nt]);
         }
         return;
     }
@@ -821,16 +837,10 @@ __device__ __forceinline__ uint32_t dq4_bf16x2(uint32_t w, uint32_t m4, uint32_t
     return d;
 }
 
-// D = A * B: the accumulator input is the zero register (as a variable it takes four moves)
-__device__ __forceinline__ void hmma_bf16_zero(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm volatile(
-        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
-        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
-        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
-}
-
 template <int BITS, int NT>
-__device__ __forceinline__ void unit_f(const SUnit<BITS>& u, uint32_t xb, const ActLanes<NT>& at, float (&acc)[NT][4][2]) {
+__device__ __forceinline__ void unit_f(const SUnit<BITS>& u, uint32_t actB,
+                                       const StreamParams& p, int b, int gid, int tig,
+                                       float (&acc)[NT][4][2]) {
     // fr[h][i][j]: half h, row gid + 8i, j = 0 -> elements (+0, +2), j = 1 -> (+1, +3)
     uint32_t fr[2][4][2];
     const uint32_t c0[4] = {u.c0.x, u.c0.y, u.c0.z, u.c0.w};
@@ -866,17 +876,21 @@ __device__ __forceinline__ void unit_f(const SUnit<BITS>& u, uint32_t xb, const 
             }
     }
     const float sc[4] = {u.sc.x, u.sc.y, u.sc.z, u.sc.w};
+    const int C = p.M * p.T;
+    const uint32_t xb = actB + b * C * 64;
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) {
-        const uint2 bx0 = lds64(xb + at.b[nt]);
-        const uint2 bx1 = lds64(xb + at.half + at.b[nt]);
+        int col = nt * 8 + gid;
+        col = col < C ? col : C - 1;
+        const uint2 bx0 = lds64(xb + (col * 4 + tig) * 8);
+        const uint2 bx1 = lds64(xb + ((C + col) * 4 + tig) * 8);
 #pragma unroll
         for (int mt = 0; mt < 2; ++mt) {
             const int r0 = 2 * mt, r1 = 2 * mt + 1;
-            float c[4];
+            float c[4] = {0.f, 0.f, 0.f, 0.f};
             const uint32_t a_lo[4] = {fr[0][r0][0], fr[0][r1][0], fr[0][r0][1], fr[0][r1][1]};
             const uint32_t a_hi[4] = {fr[1][r0][0], fr[1][r1][0], fr[1][r0][1], fr[1][r1][1]};
-            hmma_bf16_zero(c, a_lo, bx0.x, bx0.y);
+            hmma_bf16(c, a_lo, bx0.x, bx0.y);
             hmma_bf16(c, a_hi, bx1.x, bx1.y);
             acc[nt][r0][0] = fmaf(sc[r0], c[0], acc[nt][r0][0]);
             acc[nt][r0][1] = fmaf(sc[r0], c[1], acc[nt][r0][1]);
@@ -1442,8 +1456,9 @@ __global__ void __launch_bounds__(kStreamThreads, 1) gemv_stream_kernel(const __
         const bool ring = p.ring;
         uint32_t actB = smem_u32(smem) + p.act_off;
         uint32_t actZ = smem_u32(smem) + p.act2_off;
-        const ActLanes<NT> at = act_lanes<MODE, NT>(p, gid, tig);
-        const uint32_t strideB = MODE == MODE_F ? 2 * at.half : at.half, strideZ = (uint32_t)((p.M + 1) >> 1) * 32;   // bytes of a block
+        constexpr bool kTwo = NT == 2 && MODE == MODE_A8 && UK == 0;
+        TwoTiles at{};
+        if constexpr (kTwo) at = two_tiles(p, gid, tig);
         zero_acc();
         if (dbg) {  // timestamp of the first weights; the loop's own wait then passes at once
             if (!mbar_try(full0, 0)) alive = mbar_wait(full0, 0, abort_flag);
@@ -1456,39 +1471,45 @@ __global__ void __launch_bounds__(kStreamThreads, 1) gemv_stream_kernel(const __
                 alive = mbar_wait(full0 + 8 * s, ph, abort_flag);
             if (alive && !PROBE(2)) {
                 const int b0 = ring ? warp : b + warp;   // block index of this warp's first unit
-                const uint32_t xB = actB + (uint32_t)b0 * strideB, xZ = actZ + (uint32_t)b0 * strideZ;
-                auto fold = [&](const SUnit<BITS>& un, int j) {
-                    const uint32_t uB = xB + (uint32_t)j * (kCW * strideB), uZ = xZ + (uint32_t)j * (kCW * strideZ);
-                    if (MODE == MODE_F) unit_f<BITS, NT>(un, uB, at, acc);
-                    else if (UK == 0) unit_a8<BITS, NT, UK>(un, uB, uZ, at, p, 0, gid, tig, acc);
-                    else unit_a8<BITS, NT, UK>(un, actB, actZ, at, p, b0 + j * kCW, gid, tig, acc);
-                };
-                // units of this warp, all loaded before the first tile, so that the shared-memory round trips of one run
-                // under the arithmetic of another
-                auto whole = [&](auto units) {
-                    constexpr int N = decltype(units)::value;
-                    SUnit<BITS> un[N];
-#pragma unroll
-                    for (int j = 0; j < N; ++j) lds_unit<BITS, UK>(un[j], unit0 + j * kCW * UNIT, lane);
-#pragma unroll
-                    for (int j = 0; j < N; ++j) fold(un[j], j);
-                };
-                if (n == kChunkUnits && (NT == 1 || (kUPW == 2 && MODE == MODE_A8))) {
-                    whole(std::integral_constant<int, kUPW>{});
-                } else if (kUPW == 4 && MODE == MODE_A8 && (n == kChunkUnits / 2 || (NT == 2 && n == kChunkUnits))) {
-                    whole(std::integral_constant<int, 2>{});   // (two token tiles: two units at a time are what the registers hold)
-                    if (NT == 2 && n == kChunkUnits) {
+                if constexpr (kTwo) {
+                    const uint32_t xB = actB + (uint32_t)b0 * at.block_b, xZ = actZ + (uint32_t)b0 * at.block_z;
+                    int j = 0;
+                    for (; warp + (j + 1) * kCW < n; j += 2) {
                         SUnit<BITS> un[2];
 #pragma unroll
-                        for (int j = 0; j < 2; ++j) lds_unit<BITS, UK>(un[j], unit0 + (2 + j) * kCW * UNIT, lane);
+                        for (int i = 0; i < 2; ++i) lds_unit<BITS, UK>(un[i], unit0 + (j + i) * kCW * UNIT, lane);
 #pragma unroll
-                        for (int j = 0; j < 2; ++j) fold(un[j], 2 + j);
+                        for (int i = 0; i < 2; ++i)
+                            unit_two<BITS>(un[i], xB + (j + i) * (kCW * at.block_b), xZ + (j + i) * (kCW * at.block_z), at, acc);
                     }
+                    if (warp + j * kCW < n) {
+                        SUnit<BITS> un;
+                        lds_unit<BITS, UK>(un, unit0 + j * kCW * UNIT, lane);
+                        unit_two<BITS>(un, xB + j * (kCW * at.block_b), xZ + j * (kCW * at.block_z), at, acc);
+                    }
+                } else if (n == kChunkUnits && NT == 1) {
+                    // a full chunk: this warp's units are all loaded before the first tile, so that
+                    // the shared-memory round trips of one unit run under the arithmetic of another
+                    SUnit<BITS> un[kUPW];
+#pragma unroll
+                    for (int j = 0; j < kUPW; ++j) lds_unit<BITS, UK>(un[j], unit0 + j * kCW * UNIT, lane);
+#pragma unroll
+                    for (int j = 0; j < kUPW; ++j) {
+                        if (MODE == MODE_A8) unit_a8<BITS, NT, UK>(un[j], actB, actZ, p, b0 + j * kCW, gid, tig, acc);
+                        else unit_f<BITS, NT>(un[j], actB, p, b0 + j * kCW, gid, tig, acc);
+                    }
+                } else if (kUPW == 4 && n == kChunkUnits / 2 && NT == 1 && MODE == MODE_A8) {
+                    SUnit<BITS> un[2];   // a full chunk of the half-size ring
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) lds_unit<BITS, UK>(un[j], unit0 + j * kCW * UNIT, lane);
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) unit_a8<BITS, NT, UK>(un[j], actB, actZ, p, b0 + j * kCW, gid, tig, acc);
                 } else {
                     for (int j = 0; warp + j * kCW < n; ++j) {
                         SUnit<BITS> un;
                         lds_unit<BITS, UK>(un, unit0 + j * kCW * UNIT, lane);
-                        fold(un, j);
+                        if (MODE == MODE_A8) unit_a8<BITS, NT, UK>(un, actB, actZ, p, b0 + j * kCW, gid, tig, acc);
+                        else unit_f<BITS, NT>(un, actB, p, b0 + j * kCW, gid, tig, acc);
                     }
                 }
             }
