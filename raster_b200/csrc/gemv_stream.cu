@@ -689,9 +689,9 @@ __device__ __forceinline__ void fold_plain(const uint32_t (&a)[2][4], const floa
 
 // MODE_A8, plain units, two token tiles (9 .. 16 tokens): where a lane finds its fragment of tile nt and the records of its
 // pair of tokens, counted from the block's own, is worked out once per launch, and a warp loads two units before the
-// first tile.  us for the two matrices of an MLP: int4 70B at 16 tokens 95.1 -> 91.1; 6000 x 5120 and 4000 x 7168 at 9 / 12 /
-// 16 tokens int4 25.0 / 25.5 / 25.7 -> 24.1 / 24.8 / 24.4, int8 28.2 / 28.7 / 29.3 -> 26.7 / 27.4 / 27.5.  (The same for one tile, for
-// K-quant units and in mode F: between nothing and 2.6 % slower.)
+// first tile.  us for 6000 x 5120 and 4000 x 7168 at 9 / 12 / 16 tokens: int8 28.3 / 28.7 / 29.3 -> 27.0 / 27.5 / 27.6, int4
+// between nothing and 2 % of 25.1 / 25.5 / 25.7.  (The same for one tile, for K-quant units and in mode F: between nothing and
+// 2.6 % slower.)
 struct TwoTiles {
     uint32_t b[2], z[2], block_b, block_z;   // block_b, block_z: bytes of a block's fragments and records
 };
@@ -1473,19 +1473,25 @@ __global__ void __launch_bounds__(kStreamThreads, 1) gemv_stream_kernel(const __
                 const int b0 = ring ? warp : b + warp;   // block index of this warp's first unit
                 if constexpr (kTwo) {
                     const uint32_t xB = actB + (uint32_t)b0 * at.block_b, xZ = actZ + (uint32_t)b0 * at.block_z;
-                    int j = 0;
-                    for (; warp + (j + 1) * kCW < n; j += 2) {
+                    auto pair = [&](int j) {
                         SUnit<BITS> un[2];
 #pragma unroll
                         for (int i = 0; i < 2; ++i) lds_unit<BITS, UK>(un[i], unit0 + (j + i) * kCW * UNIT, lane);
 #pragma unroll
                         for (int i = 0; i < 2; ++i)
                             unit_two<BITS>(un[i], xB + (j + i) * (kCW * at.block_b), xZ + (j + i) * (kCW * at.block_z), at, acc);
-                    }
-                    if (warp + j * kCW < n) {
-                        SUnit<BITS> un;
-                        lds_unit<BITS, UK>(un, unit0 + j * kCW * UNIT, lane);
-                        unit_two<BITS>(un, xB + j * (kCW * at.block_b), xZ + j * (kCW * at.block_z), at, acc);
+                    };
+                    if (BITS == 8 && n == kChunkUnits) {
+                        pair(0);
+                    } else {      // (4 bits: unrolled over a whole chunk this gains nothing)
+                        int j = 0;
+                        if (BITS == 4)
+                            for (; warp + (j + 1) * kCW < n; j += 2) pair(j);
+                        for (; warp + j * kCW < n; ++j) {
+                            SUnit<BITS> un;
+                            lds_unit<BITS, UK>(un, unit0 + j * kCW * UNIT, lane);
+                            unit_two<BITS>(un, xB + j * (kCW * at.block_b), xZ + j * (kCW * at.block_z), at, acc);
+                        }
                     }
                 } else if (n == kChunkUnits && NT == 1) {
                     // a full chunk: this warp's units are all loaded before the first tile, so that
