@@ -828,8 +828,22 @@ static int32_t attn_attr() {
     RSTQ_CUDA(cudaFuncSetAttribute(gqa_decode_stream_kernel<HD, 4, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, attn_smem(HD)));
     return RSTQ_OK;
 }
+// Scratch of both kernels, the most that a call can need (0.3 and 2.5 MB): a call under capture needs no call before it,
+// and a recorded launch and rstq_sync's reset always mean the same blocks.  With more than one slice per KV head
+// (attention_impl's S) there are at most as many slices in all as the device has SMs, of the general kernel twice as many.
+static int32_t attn_reserve(DeviceState& ds) {
+    const int64_t slots = (int64_t)ds.sm_count * kStreamHeads * (128 + 4) * 4;
+    RSTQ_CUDA(cudaMalloc(&ds.attn_slots, (size_t)slots));
+    ds.attn_slots_bytes = slots;
+    RSTQ_CUDA(cudaMemsetAsync(ds.attn_slots, 0xFF, (size_t)slots, ds.stream));
+    const int64_t states = 2ll * ds.sm_count * kAttnGroup * (128 * kAttnVec + 4) * 4;
+    RSTQ_CUDA(cudaMalloc(&ds.attn_scratch, (size_t)(kAttnCounters * 4 + states)));
+    RSTQ_CUDA(cudaMemsetAsync(ds.attn_scratch, 0, kAttnCounters * 4, ds.stream));
+    return RSTQ_OK;
+}
 int32_t attn_configure(DeviceState& ds) {
-    int32_t rc = attn_attr<64>();
+    int32_t rc = attn_reserve(ds);
+    if (rc == RSTQ_OK) rc = attn_attr<64>();
     if (rc == RSTQ_OK) rc = attn_attr<128>();
     // how many clusters of each size the device holds at once (148 SMs: 74, 45, 33, 26, 22, 15, 15)
     for (int c = 2; c <= kClusterMax && rc == RSTQ_OK; ++c) {
@@ -984,18 +998,6 @@ static int32_t attention_impl(rstq_ctx* ctx, rstq_buf* q, rstq_buf* k, rstq_buf*
                      RSTQ_E_INVALID, "invalid, unaligned or too small quantizer buffer");
         RSTQ_REQUIRE(xq->dev == q->dev && xs->dev == q->dev && (!xsum || xsum->dev == q->dev), RSTQ_E_DEVICE,
                      "buffers live on different devices");
-    }
-    const int64_t part_bytes = n_kv * gz * S * (fast ? gs : kAttnGroup) * row * 4;
-    if (fast && !clustered && S > 1) {      // slots, empty between launches
-        const bool fresh = ds.attn_slots_bytes < part_bytes;
-        rc = dev_reserve(ds, &ds.attn_slots, &ds.attn_slots_bytes, part_bytes);
-        if (rc != RSTQ_OK) return rc;
-        if (fresh) RSTQ_CUDA(cudaMemsetAsync(ds.attn_slots, 0xFF, (size_t)ds.attn_slots_bytes, ds.stream));
-    } else if (!fast) {
-        const bool fresh = ds.attn_scratch_bytes < kAttnCounters * 4 + part_bytes;
-        rc = dev_reserve(ds, &ds.attn_scratch, &ds.attn_scratch_bytes, kAttnCounters * 4 + part_bytes);
-        if (rc != RSTQ_OK) return rc;
-        if (fresh) RSTQ_CUDA(cudaMemsetAsync(ds.attn_scratch, 0, kAttnCounters * 4, ds.stream));
     }
     AttnParams p;
     p.q = (const float*)q->ptr;

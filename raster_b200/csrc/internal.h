@@ -101,7 +101,6 @@ struct DeviceState {
     void* f_image = nullptr;       // mode F: the staged activations of a decode launch that ride the weight ring
     int64_t f_image_bytes = 0;
     void* attn_scratch = nullptr;  // decode attention: arrival counters + per-slice softmax states
-    int64_t attn_scratch_bytes = 0;
     void* attn_slots = nullptr;    // ... of head_dim 64 and 128: slots of the slices' states, every word 0xFFFFFFFF between launches
     int64_t attn_slots_bytes = 0;
     int attn_clusters[9] = {};     // ... and how many clusters of 2 .. 8 of its thread blocks the device holds at once
@@ -339,7 +338,7 @@ int32_t launch_gemm(rstq_ctx* ctx, DeviceState& ds, const rstq_weight* w, const 
                     int out_dtype, int64_t M, void* x16, float* rowscale, float* acc32);
 int32_t gemm_configure(DeviceState& ds);
 // attn.cu
-int32_t attn_configure(DeviceState& ds);  // shared-memory attributes and cluster counts, once per device
+int32_t attn_configure(DeviceState& ds);  // scratch, shared-memory attributes and cluster counts, once per device
 // dx.cu
 int32_t dx_configure();  // shared-memory attributes, once per device
 int32_t launch_qlinear_q8_dx(rstq_ctx* ctx, DeviceState& ds, const float* dy, const int8_t* codes,

@@ -10,6 +10,7 @@ import numpy as np
 import pytest
 
 from oracle import oracle as orc
+from raster_b200 import Context
 from raster_b200 import _lib as L
 from raster_b200 import synth
 
@@ -285,3 +286,56 @@ def test_attention_of_special_values(ctx):
     assert relerr(out, ref) <= 1e-5
     for o in (bq, bk, bv, bo):
         o.free()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("first,hd", [(128, 128), (128, 64), (128, 96), (96, 128)])
+def test_attention_recorded_at_a_length_not_seen_before(first, hd):
+    """A program that warms up on a short cache (of head_dim `first`) and then records a long one, in a graph of the
+    library's and in one of its own on a lent stream: nothing has to be allocated.  A larger call between the replays
+    leaves the recorded ones what they need.  1e-5 as above."""
+    torch = pytest.importorskip("torch")
+    n_q, n_kv, clen, scale = 8, 2, 3000, 0.1
+    ctx = Context(("cuda:0",))
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    bufs = []
+
+    def case(n_q, n_kv, hd, clen, seed):
+        a = synth.normal(seed, n_q * hd), synth.normal(seed + 1, clen * n_kv * hd), synth.normal(seed + 2, clen * n_kv * hd)
+        b = [ctx.array_to_buffer(x) for x in a] + [ctx.make_buffer(n_q * hd, np.float32)]
+        bufs.extend(b)
+        want = orc.gqa_decode_attention(*a, clen, n_q, n_q // n_kv, n_kv, hd, scale)
+        return b[3], want, lambda: ctx.gqa_decode_attention(*b, clen, n_q, n_q // n_kv, n_kv, hd, clen, scale)
+
+    try:
+        case(n_q, n_kv, first, 20, 111)[2]()
+        out, want, call = case(n_q, n_kv, hd, clen, 121)
+        ctx.graph_begin()
+        call()
+        g = ctx.graph_end()
+        other_out, other_want, other = case(64, 16, hd, 2500, 131)
+        for _ in range(2):
+            out.fill_bytes(0)
+            g.replay()
+            other()
+            g.replay()
+            ctx.sync()
+            assert relerr(out.download(), want) <= 1e-5 and relerr(other_out.download(), other_want) <= 1e-5
+        g.destroy()
+        torch.cuda.synchronize()
+        ctx.set_stream(stream.cuda_stream)
+        with torch.cuda.graph(graph, stream=stream):
+            call()
+        out.fill_bytes(0)
+        ctx.sync()
+        with torch.cuda.stream(stream):
+            graph.replay()
+        torch.cuda.synchronize()
+        assert relerr(out.download(), want) <= 1e-5
+    finally:
+        torch.cuda.synchronize()
+        del graph
+        ctx.set_stream(None)
+        for b in bufs:
+            b.free()
+        ctx.close()
