@@ -391,21 +391,30 @@ __host__ __device__ constexpr int attn_w_off(int hd) { return kStreamWarps * kSt
 __host__ __device__ constexpr int attn_o_off(int hd) { return attn_w_off(hd) + kStreamHeads * kMaxSlices * 4; }  // partial outputs
 static_assert(attn_o_off(128) + kStreamThreads * 16 <= attn_q_off(), "the merge fits where the rings were");
 
-// slots: a value is there once it is not kEmpty
+// slots: a value is there once it is not kEmpty.  Written and polled with strong (relaxed) accesses, for the value is the
+// hand-over; each word says for itself that it is there, so no order between them is needed.
 __device__ __forceinline__ float4 slot_read4(const float4* a) {
     float4 v;
-    asm volatile("ld.volatile.global.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(a) : "memory");
+    asm volatile("ld.relaxed.gpu.global.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(a) : "memory");
     return v;
 }
 __device__ __forceinline__ float2 slot_read2(const float2* a) {
     float2 v;
-    asm volatile("ld.volatile.global.v2.f32 {%0,%1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(a) : "memory");
+    asm volatile("ld.relaxed.gpu.global.v2.f32 {%0,%1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(a) : "memory");
     return v;
 }
 __device__ __forceinline__ bool slot_full(float v) { return __float_as_uint(v) != kEmpty; }
 __device__ __forceinline__ bool slot_full(const float4 v) { return slot_full(v.x) && slot_full(v.y) && slot_full(v.z) && slot_full(v.w); }
 __device__ __forceinline__ bool slot_full(const float2 v) { return slot_full(v.x) && slot_full(v.y); }
 __device__ __forceinline__ float slot_value(float v) { return slot_full(v) ? v : __uint_as_float(0x7FFFFFFFu); }
+__device__ __forceinline__ void slot_write(float4* a, float4 v) {
+    asm volatile("st.relaxed.gpu.global.v4.f32 [%0], {%1,%2,%3,%4};" ::"l"(a), "f"(slot_value(v.x)), "f"(slot_value(v.y)),
+                 "f"(slot_value(v.z)), "f"(slot_value(v.w))
+                 : "memory");
+}
+__device__ __forceinline__ void slot_write(float2* a, float2 v) {
+    asm volatile("st.relaxed.gpu.global.v2.f32 [%0], {%1,%2};" ::"l"(a), "f"(slot_value(v.x)), "f"(slot_value(v.y)) : "memory");
+}
 __device__ __forceinline__ float4 slot_empty4() {
     const float e = __uint_as_float(kEmpty);
     return make_float4(e, e, e, e);
@@ -653,7 +662,7 @@ gqa_decode_stream_kernel(const AttnParams p) {
             O.w = fmaf(a.w, e, O.w);
         }
         if (CL || S == 1) s_o[tid] = O;      // (without a cluster, the one slice's state is the result's)
-        else reinterpret_cast<float4*>(out_part + h * ROW)[c] = make_float4(slot_value(O.x), slot_value(O.y), slot_value(O.z), slot_value(O.w));
+        else slot_write(reinterpret_cast<float4*>(out_part + h * ROW) + c, O);
     }
     if constexpr (CL) {
         // The slices' states -> out, through distributed shared memory: a warp takes 32 neighbouring values of a head.
@@ -688,8 +697,7 @@ gqa_decode_stream_kernel(const AttnParams p) {
     if (S == 1) {
         if (tid < gc) s_L[tid] = 1.0f / s_cL[tid];
     } else {
-        if (tid < gc)
-            *reinterpret_cast<float2*>(out_part + tid * ROW + HD) = make_float2(slot_value(s_cM[tid]), slot_value(s_cL[tid]));
+        if (tid < gc) slot_write(reinterpret_cast<float2*>(out_part + tid * ROW + HD), make_float2(s_cM[tid], s_cL[tid]));
         if (split != S - 1) return;
         // ---- the slices' states -> out: the CTA of the last slice ----
         // What it reads lies a trip to L2 away, so it is requested kHold float4 per thread at a time (slices g, g + groups,

@@ -288,6 +288,47 @@ def test_attention_of_special_values(ctx):
         o.free()
 
 
+# shapes whose slices meet through slots: n_q, n_kv, head_dim, positions (slices: 18, 74, 40, 9)
+SLOT_SHAPES = [(32, 8, 128, 4000), (8, 2, 64, 6000), (7, 1, 128, 2500), (64, 16, 64, 4000)]
+
+
+@pytest.mark.gpu
+def test_attention_calls_in_a_row_through_slots(ctx):
+    """Calls of other slices, groups and head sizes one after another in one graph, replayed without a wait in between: each
+    launch finds the slots emptied by the one before it, which may still run when it starts.  One of them with the
+    quantized output, equal in bits to attention and then the quantizer.  1e-5 as above."""
+    calls, frees = [], []
+    for i, (n_q, n_kv, hd, clen) in enumerate(SLOT_SHAPES):
+        a = synth.normal(141 + i, n_q * hd), synth.normal(151 + i, clen * n_kv * hd), synth.normal(161 + i, clen * n_kv * hd)
+        b = [ctx.array_to_buffer(x) for x in a] + [ctx.make_buffer(n_q * hd, np.float32)]
+        calls.append((b, clen, n_q, n_q // n_kv, n_kv, hd, clen, 0.1, orc.gqa_decode_attention(*a, clen, n_q, n_q // n_kv, n_kv, hd, 0.1)))
+        frees += b
+    n = SLOT_SHAPES[0][0] * SLOT_SHAPES[0][2]
+    quant = [[ctx.make_buffer(n, np.int8), ctx.make_buffer(n // 32, np.float32), ctx.make_buffer(n // 32, np.int32)] for _ in range(2)]
+    frees += quant[0] + quant[1]
+    ctx.graph_begin()
+    for _ in range(3):
+        for i, (b, *shape, _) in enumerate(calls):
+            if i == 0:
+                ctx.gqa_decode_attention_quant_act(*b, *quant[0], *shape)
+            else:
+                ctx.gqa_decode_attention(*b, *shape)
+    g = ctx.graph_end()
+    for b, *_ in calls:
+        b[3].fill_bytes(0)
+    for _ in range(20):
+        g.replay()
+    ctx.quant_act_i8(calls[0][0][3], *quant[1], 1, n)
+    ctx.sync()
+    for b, *_, want in calls:
+        assert relerr(b[3].download(), want) <= 1e-5
+    for x, y in zip(*quant):
+        assert np.array_equal(x.download(), y.download())
+    g.destroy()
+    for o in frees:
+        o.free()
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("first,hd", [(128, 128), (128, 64), (128, 96), (96, 128)])
 def test_attention_recorded_at_a_length_not_seen_before(first, hd):
