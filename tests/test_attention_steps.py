@@ -241,14 +241,16 @@ def test_attention_with_quantized_output_equals_attention_then_quantizer(ctx, n_
 @pytest.mark.parametrize("group,n_kv", [(1, 5), (2, 3), (3, 2), (4, 1), (5, 2), (7, 4), (8, 1), (9, 2), (17, 1)])
 def test_attention_at_the_edges_of_its_tiles(ctx, group, n_kv, hd):
     """One, two, four and eight heads per pass and what is left over; lengths around a tile of 8 positions, a slice's 64
-    and a round of the warps.  Rows beyond the length hold NaN: they must not count.  1e-5 as above."""
+    and a round of the warps.  As a host scalar a length above 64 is a cluster of up to eight slices (150 three, 380 six,
+    440 seven with few KV heads), 2099 and every length in device memory (slices by the capacity) go through slots.  Rows
+    beyond the length hold NaN: they must not count.  1e-5 as above."""
     n_q, maxpos, scale = group * n_kv, 2100, 1.0 / math.sqrt(hd)
     q = synth.normal(71 + group, n_q * hd)
     k0, v0 = synth.normal(72, maxpos * n_kv * hd), synth.normal(73, maxpos * n_kv * hd)
     bq, bo = ctx.array_to_buffer(q), ctx.make_buffer(n_q * hd, np.float32)
     bk, bv = ctx.make_buffer(k0.size, np.float32), ctx.make_buffer(v0.size, np.float32)
     bl = ctx.make_buffer(1, np.int64)
-    for clen in (1, 7, 8, 9, 63, 64, 65, 200, 513, 2099):
+    for clen in (1, 7, 8, 9, 63, 64, 65, 150, 200, 380, 440, 513, 2099):
         k, v = k0.copy(), v0.copy()
         k[clen * n_kv * hd:] = np.nan
         v[clen * n_kv * hd:] = np.nan
@@ -265,15 +267,17 @@ def test_attention_at_the_edges_of_its_tiles(ctx, group, n_kv, hd):
 
 
 @pytest.mark.gpu
-def test_attention_of_special_values(ctx):
+@pytest.mark.parametrize("clen,at", [(700, 650), (3000, 1500), (3000, 2990)])
+def test_attention_of_special_values(ctx, clen, at):
     """Every bit pattern of a NaN comes through the slices' merge as a NaN, an infinite V as an infinity, and calls of other
-    shapes in between find the scratch as they need it."""
-    n_q, n_kv, hd, clen = 8, 2, 64, 700
+    shapes in between find the scratch as they need it.  700 positions are a cluster of eight slices; 3000 are 47 slices
+    that meet through slots (a cluster's would be longer by 160 KB each), the NaN in a middle one or in the merging one."""
+    n_q, n_kv, hd = 8, 2, 64
     group, scale = n_q // n_kv, 0.125
     q, k, v = synth.normal(81, n_q * hd), synth.normal(82, clen * n_kv * hd), synth.normal(83, clen * n_kv * hd)
     ref = orc.gqa_decode_attention(q, k, v, clen, n_q, group, n_kv, hd, scale).reshape(n_q, hd)
     vv = v.reshape(clen, n_kv, hd)
-    vv.view(np.uint32)[650, 0, 5] = 0xFFFFFFFF
+    vv.view(np.uint32)[at, 0, 5] = 0xFFFFFFFF
     vv[20, 1, 7] = np.inf
     bq, bk, bv, bo = ctx.array_to_buffer(q), ctx.array_to_buffer(k), ctx.array_to_buffer(v), ctx.make_buffer(n_q * hd, np.float32)
     for n, h in ((clen, group), (64, group), (300, 1), (clen, group)):
