@@ -122,6 +122,12 @@ struct AttnParams {
     int32_t* xsum;
 };
 
+// (a length in device memory never reaches beyond the caches)
+__device__ __forceinline__ int64_t attn_len(const AttnParams& p) {
+    const int64_t n = p.clenbuf ? ld_i64(p.clenbuf) : p.cache_len;
+    return n < 0 ? 0 : (n > p.maxpos ? p.maxpos : n);
+}
+
 // one value of the output, and with it -- when asked for -- its 32-element quantizer block (the 32
 // lanes of the warp hold 32 consecutive elements of one head)
 __device__ __forceinline__ void attn_store(const AttnParams& p, int64_t e, float v, int lane) {
@@ -271,7 +277,7 @@ gqa_decode_kernel(const AttnParams p) {
     const int hd = p.head_dim, hd4 = hd >> 2, row = hd + 4;   // row: weighted V, max, sum, 2 pad (16-byte rows)
     const int g0 = gz * kAttnGroup;
     const int gc = min(kAttnGroup, p.group - g0);            // query heads this CTA serves
-    const int64_t clen = p.clenbuf ? p.clenbuf[0] : p.cache_len;
+    const int64_t clen = attn_len(p);
     const int64_t chunk = (clen + p.S - 1) / p.S;
     const int64_t j0 = split * chunk, j1 = min(clen, j0 + chunk);
     const int64_t kvstride = (int64_t)p.n_kv * hd;
@@ -461,8 +467,7 @@ gqa_decode_stream_kernel(const AttnParams p) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     // (a length in device memory may still change: here it only says which rows of the cache to ask for)
     auto range = [&](int64_t* j0, int64_t* j1) {
-        int64_t clen = p.clenbuf ? ld_i64(p.clenbuf) : p.cache_len;
-        clen = clen < 0 ? 0 : (clen > p.maxpos ? p.maxpos : clen);
+        const int64_t clen = attn_len(p);
         const int64_t chunk = (clen + p.S - 1) / p.S;
         *j0 = min(clen, split * chunk);
         *j1 = min(clen, *j0 + chunk);

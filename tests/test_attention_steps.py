@@ -292,6 +292,25 @@ def test_attention_of_special_values(ctx, clen, at):
         o.free()
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("hd", [32, 64, 96, 128, 256])
+def test_attention_with_a_device_length_beyond_the_cache(ctx, hd):
+    """A length above the capacity counts as the capacity, for every kernel: the same bits."""
+    n_q, n_kv, maxpos = 4, 2, 333
+    a = synth.normal(171, n_q * hd), synth.normal(172, maxpos * n_kv * hd), synth.normal(173, maxpos * n_kv * hd)
+    b = [ctx.array_to_buffer(x) for x in a] + [ctx.make_buffer(n_q * hd, np.float32)]
+    bl, got = ctx.make_buffer(1, np.int64), []
+    for n in (maxpos, maxpos + 1, 10 ** 6):
+        bl.upload(np.array([n], np.int64))
+        ctx.gqa_decode_attention(*b, 0, n_q, n_q // n_kv, n_kv, hd, maxpos, 0.1, clenbuf=bl)
+        ctx.sync()
+        got.append(b[3].download())
+    assert relerr(got[0], orc.gqa_decode_attention(*a, maxpos, n_q, n_q // n_kv, n_kv, hd, 0.1)) <= 1e-5
+    assert all(np.array_equal(g.view(np.uint32), got[0].view(np.uint32)) for g in got[1:])
+    for o in (*b, bl):
+        o.free()
+
+
 # shapes whose slices meet through slots: n_q, n_kv, head_dim, positions (slices: 18, 74, 40, 9)
 SLOT_SHAPES = [(32, 8, 128, 4000), (8, 2, 64, 6000), (7, 1, 128, 2500), (64, 16, 64, 4000)]
 
