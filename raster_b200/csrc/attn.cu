@@ -16,6 +16,8 @@
 // head_dim 64 and 128 take gqa_decode_stream_kernel (rows through shared memory, eight positions per
 // warp step); every other head_dim % 4 == 0 up to 256 takes the general gqa_decode_kernel (a
 // warp per position).
+#include <algorithm>
+
 #include "internal.h"
 #include "quant_helpers.cuh"
 #include "sync_helpers.cuh"
@@ -377,25 +379,28 @@ gqa_decode_kernel(const AttnParams p) {
 // ready (most are empty then, and the second look costs a trip: 11.5 -> 12.4); eight heads per CTA in two passes
 // (28 / 4 x 5000 16.1); packed f32x2 arithmetic (11.8 -> 12.4).
 constexpr int kTilePos = 8;
-constexpr int kStreamWarps = 16;
-constexpr int kStreamThreads = kStreamWarps * 32;
+constexpr int kStreamWarps = 16;                      // one such CTA per SM ...
+constexpr int kNarrowWarps = 4;                       // ... or, with many KV heads, four of these
 constexpr int kStreamHeads = 4;                       // query heads of one KV head per CTA
 constexpr int kRingBytes = 12288;                     // per warp
-constexpr int kHintPos = 256;                         // positions of a CTA requested into L2 ahead of time
+constexpr int kHintPos = 16;                          // positions per warp of a CTA requested into L2 ahead of time
 constexpr uint32_t kEmpty = 0xFFFFFFFFu;              // a NaN that no arithmetic produces
 __host__ __device__ constexpr int attn_unit_bytes(int hd) { return kTilePos * hd * 4; }      // a tile's rows of K, or of V
 __host__ __device__ constexpr int attn_units(int hd) { return kRingBytes / attn_unit_bytes(hd); }
 // shared memory: the warps' rings, the query heads, the warps' p
-__host__ __device__ constexpr int attn_q_off() { return kStreamWarps * kRingBytes; }
-__host__ __device__ constexpr int attn_p_off(int hd) { return attn_q_off() + kStreamHeads * hd * 4; }
-__host__ __device__ constexpr int attn_smem(int hd) { return attn_p_off(hd) + kStreamWarps * kTilePos * kStreamHeads * 4; }
+__host__ __device__ constexpr int attn_q_off(int warps) { return warps * kRingBytes; }
+__host__ __device__ constexpr int attn_p_off(int hd, int warps) { return attn_q_off(warps) + kStreamHeads * hd * 4; }
+__host__ __device__ constexpr int attn_smem(int hd, int warps) { return attn_p_off(hd, warps) + warps * kTilePos * kStreamHeads * 4; }
 // ... and, once the rings are drained, in their place: the warps' states, then the merge of the slices
 constexpr int kClusterMax = 8;                        // slices of a KV head that may be one cluster
 constexpr int64_t kClusterExtra = 65000;              // bytes of K and V that a slice may grow by for it
 constexpr int kMaxSlices = 160;                       // five (max, sum) pairs per lane of the merging warps
-__host__ __device__ constexpr int attn_w_off(int hd) { return kStreamWarps * kStreamHeads * (hd + 4) * 4; }       // slice weights
-__host__ __device__ constexpr int attn_o_off(int hd) { return attn_w_off(hd) + kStreamHeads * kMaxSlices * 4; }  // partial outputs
-static_assert(attn_o_off(128) + kStreamThreads * 16 <= attn_q_off(), "the merge fits where the rings were");
+__host__ __device__ constexpr int attn_w_off(int hd, int warps) { return warps * kStreamHeads * (hd + 4) * 4; }       // slice weights
+__host__ __device__ constexpr int attn_o_off(int hd, int warps) { return attn_w_off(hd, warps) + kStreamHeads * kMaxSlices * 4; }  // partial outputs
+static_assert(attn_o_off(128, kStreamWarps) + kStreamWarps * 32 * 16 <= attn_q_off(kStreamWarps) &&
+                  attn_o_off(128, kNarrowWarps) + kNarrowWarps * 32 * 16 <= attn_q_off(kNarrowWarps),
+              "the merge fits where the rings were");
+static_assert(kNarrowWarps >= kStreamHeads && kNarrowWarps * 32 >= kStreamHeads * 128 / 4, "a warp per head, a thread per four dims in the merge");
 
 // slots: a value is there once it is not kEmpty.  Written and polled with strong (relaxed) accesses, for the value is the
 // hand-over; each word says for itself that it is there, so no order between them is needed.
@@ -444,16 +449,18 @@ __device__ __forceinline__ float ld_cluster(uint32_t at, int rank) {
 }
 
 // H = query heads of the KV head that a CTA serves at most (1, 2 or 4).  CL: the slices of a KV head are one cluster.
-template <int HD, int H, bool CL>
-__global__ void __launch_bounds__(kStreamThreads, 1)
+// WARPS: of the CTA; an SM holds kStreamWarps in all.
+template <int HD, int H, bool CL, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32, kStreamWarps / WARPS)
 gqa_decode_stream_kernel(const AttnParams p) {
+    constexpr int THREADS = WARPS * 32;
     constexpr int VEC = HD / 32, ROW = HD + 4;      // VEC: float4 per lane of a position's eight lanes
     constexpr uint32_t ROWB = HD * 4, UNITB = attn_unit_bytes(HD);
     constexpr int NU = attn_units(HD);                              // units of the ring: K and V of a tile in turn
     constexpr int LPP = HD / 4, PPS = 32 / LPP;                     // output: lanes per position, positions per step
     extern __shared__ __align__(128) uint8_t s_raw[];
     __shared__ int s_abort;
-    __shared__ float s_cw[kStreamHeads][kStreamWarps], s_cM[kStreamHeads], s_cL[kStreamHeads], s_L[kStreamHeads];
+    __shared__ float s_cw[kStreamHeads][WARPS], s_cM[kStreamHeads], s_cL[kStreamHeads], s_L[kStreamHeads];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, grp = lane >> 3, sub = lane & 7;
     const int hkv = blockIdx.x, split = blockIdx.y, gz = blockIdx.z;
     const int g0 = gz * kStreamHeads, gc = min(kStreamHeads, p.group - g0);
@@ -474,7 +481,7 @@ gqa_decode_stream_kernel(const AttnParams p) {
     };
     int64_t j0, j1;
     range(&j0, &j1);
-    for (int i = tid; i < kHintPos * 2 * (HD / 32); i += kStreamThreads) {     // (128 bytes each)
+    for (int i = tid; i < kHintPos * WARPS * 2 * (HD / 32); i += THREADS) {     // (128 bytes each)
         const int r = i / (HD / 32), c = i % (HD / 32);
         const int64_t j = j0 + (r >> 1);
         if (j < j1) asm volatile("prefetch.global.L2 [%0];" ::"l"(((r & 1) ? vb : kb) + j * kvrow + c * 32));
@@ -483,10 +490,10 @@ gqa_decode_stream_kernel(const AttnParams p) {
     if (p.clenbuf) range(&j0, &j1);
 
     const int tiles = (int)((j1 - j0 + kTilePos - 1) / kTilePos);
-    const int mine = tiles > warp ? (tiles - warp + kStreamWarps - 1) / kStreamWarps : 0;   // tiles warp, warp + 16, ...
+    const int mine = tiles > warp ? (tiles - warp + WARPS - 1) / WARPS : 0;   // tiles warp, warp + WARPS, ...
     auto request = [&](int u) {    // unit u: K (even) or V (odd) of this warp's tile u / 2; an empty group beyond the last
         if (u < 2 * mine) {
-            const int64_t j = j0 + (int64_t)(warp + (u >> 1) * kStreamWarps) * kTilePos;
+            const int64_t j = j0 + (int64_t)(warp + (u >> 1) * WARPS) * kTilePos;
             const int np = (int)(j1 - j < kTilePos ? j1 - j : kTilePos);
             const uint32_t dst = ring + (u % NU) * UNITB + lane * 16;
             const float* src = ((u & 1) ? vb : kb) + (j + lane / LPP) * kvrow + (lane % LPP) * 4;
@@ -503,16 +510,16 @@ gqa_decode_stream_kernel(const AttnParams p) {
     };
 #pragma unroll 1
     for (int u = 0; u < NU; ++u) request(u);
-    float4* s_q = reinterpret_cast<float4*>(s_raw + attn_q_off());
-    for (int i = tid; i < H * (HD / 4); i += kStreamThreads) {
+    float4* s_q = reinterpret_cast<float4*>(s_raw + attn_q_off(WARPS));
+    for (int i = tid; i < H * (HD / 4); i += THREADS) {
         float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
         if (i < gc * (HD / 4)) t = reinterpret_cast<const float4*>(p.q + (int64_t)(hkv * p.group + g0) * HD)[i];
         s_q[i] = make_float4(t.x * p.scale, t.y * p.scale, t.z * p.scale, t.w * p.scale);
     }
     __syncthreads();
 
-    const uint32_t qa = base + attn_q_off() + sub * 16;
-    float* s_p = reinterpret_cast<float*>(s_raw + attn_p_off(HD)) + warp * (kTilePos * H);
+    const uint32_t qa = base + attn_q_off(WARPS) + sub * 16;
+    float* s_p = reinterpret_cast<float*>(s_raw + attn_p_off(HD, WARPS)) + warp * (kTilePos * H);
     const uint32_t pa = smem_u32(s_p);
     float4 acc[H];
     float m = kNegInf, l = 0.f;     // of the head this lane holds scores of
@@ -523,7 +530,7 @@ gqa_decode_stream_kernel(const AttnParams p) {
     const int lane_h = H == 4 ? ((sub >> 1) & 1) * 2 + (sub >> 2) : (H == 2 ? (sub >> 1) & 1 : 0);
 #pragma unroll 1
     for (int i = 0; i < mine; ++i) {
-        const int64_t j = j0 + (int64_t)(warp + i * kStreamWarps) * kTilePos;
+        const int64_t j = j0 + (int64_t)(warp + i * WARPS) * kTilePos;
         const int np = (int)(j1 - j < kTilePos ? j1 - j : kTilePos);
         const uint32_t ka = ring + (2 * i % NU) * UNITB, va = ring + ((2 * i + 1) % NU) * UNITB;
         arrived();
@@ -633,16 +640,16 @@ gqa_decode_stream_kernel(const AttnParams p) {
         s_part[(warp * gc + lane_h) * ROW + HD + 1] = l;
     }
     __syncthreads();
-    if (warp < gc && lane < kStreamWarps) {          // warp h merges the (max, sum) pairs of head h
+    if (warp < gc && lane < WARPS) {          // warp h merges the (max, sum) pairs of head h
         const float* s = s_part + (lane * gc + warp) * ROW + HD;
         const float mw = s[0], lw = s[1];
         float M = mw;
 #pragma unroll
-        for (int o = kStreamWarps / 2; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xFFFFu, M, o));
+        for (int o = WARPS / 2; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync((1u << WARPS) - 1u, M, o));
         const float e = expf(mw - M);
         float L = lw * e;
 #pragma unroll
-        for (int o = kStreamWarps / 2; o > 0; o >>= 1) L += __shfl_xor_sync(0xFFFFu, L, o);
+        for (int o = WARPS / 2; o > 0; o >>= 1) L += __shfl_xor_sync((1u << WARPS) - 1u, L, o);
         s_cw[warp][lane] = e;
         if (lane == 0) {
             s_cM[warp] = M;
@@ -651,14 +658,14 @@ gqa_decode_stream_kernel(const AttnParams p) {
     }
     __syncthreads();
     const int cols = gc * LPP, S = p.S;              // float4 columns of the CTA's output (at most 128)
-    float4* s_o = reinterpret_cast<float4*>(s_raw + attn_o_off(HD));
+    float4* s_o = reinterpret_cast<float4*>(s_raw + attn_o_off(HD, WARPS));
     float* all = p.part + ((int64_t)hkv * gridDim.z + gz) * S * (p.gs * ROW);
     float* out_part = all + (int64_t)split * (p.gs * ROW);
     if (tid < cols) {
         const int h = tid / LPP, c = tid - h * LPP;
         float4 O = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-        for (int w = 0; w < kStreamWarps; ++w) {
+        for (int w = 0; w < WARPS; ++w) {
             const float4 a = reinterpret_cast<const float4*>(s_part + (w * gc + h) * ROW)[c];
             const float e = s_cw[h][w];
             O.x = fmaf(a.x, e, O.x);
@@ -673,7 +680,7 @@ gqa_decode_stream_kernel(const AttnParams p) {
         // The slices' states -> out, through distributed shared memory: a warp takes 32 neighbouring values of a head.
         attn_cluster_sync();
         const uint32_t o = smem_u32(s_o), m_at = smem_u32(s_cM), l_at = smem_u32(s_cL);
-        for (int b = split + S * warp; b < gc * (HD / 32); b += S * kStreamWarps) {
+        for (int b = split + S * warp; b < gc * (HD / 32); b += S * WARPS) {
             const int e = b * 32 + lane, h = b / (HD / 32);
             float Os[kClusterMax], Ms[kClusterMax], Ls[kClusterMax], M = kNegInf, L = 0.f, O = 0.f;
 #pragma unroll
@@ -708,9 +715,9 @@ gqa_decode_stream_kernel(const AttnParams p) {
         // What it reads lies a trip to L2 away, so it is requested kHold float4 per thread at a time (slices g, g + groups,
         // ...).  The code is run once and cold: short loops rather than unrolled ones.
         constexpr int kHold = 10;
-        groups = kStreamThreads / cols;
+        groups = THREADS / cols;
         const int g = tid / cols, c = tid - g * cols, ch = c / LPP, pitch = p.gs * ROW;
-        float* s_w = reinterpret_cast<float*>(s_raw + attn_w_off(HD));     // [gc][S]: maxima, then weights
+        float* s_w = reinterpret_cast<float*>(s_raw + attn_w_off(HD, WARPS));     // [gc][S]: maxima, then weights
         float4* col = reinterpret_cast<float4*>(all + ch * ROW) + (c - ch * LPP);
         float4 held[kHold];
         auto hold = [&](int from) {       // (beyond the last slice that one again, without a branch: it is not looked at)
@@ -795,7 +802,7 @@ gqa_decode_stream_kernel(const AttnParams p) {
     // the groups' partial outputs, [group][gc * HD], added up
     const float* o = reinterpret_cast<const float*>(s_o);
 #pragma unroll 1
-    for (int i = tid; i < gc * HD; i += kStreamThreads) {
+    for (int i = tid; i < gc * HD; i += THREADS) {
         float v = o[i];
 #pragma unroll 1
         for (int g = 1; g < groups; ++g) v += o[g * gc * HD + i];
@@ -831,14 +838,30 @@ static cudaError_t launch_attn(K kernel, dim3 grid, dim3 block, size_t smem, con
     return launch_attn_cluster(kernel, grid, block, smem, ds, 1u, args...);
 }
 
-template <int HD>
-static int32_t attn_attr() {
-    RSTQ_CUDA(cudaFuncSetAttribute(gqa_decode_stream_kernel<HD, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, attn_smem(HD)));
-    RSTQ_CUDA(cudaFuncSetAttribute(gqa_decode_stream_kernel<HD, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, attn_smem(HD)));
-    RSTQ_CUDA(cudaFuncSetAttribute(gqa_decode_stream_kernel<HD, 2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, attn_smem(HD)));
-    RSTQ_CUDA(cudaFuncSetAttribute(gqa_decode_stream_kernel<HD, 2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, attn_smem(HD)));
-    RSTQ_CUDA(cudaFuncSetAttribute(gqa_decode_stream_kernel<HD, 4, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, attn_smem(HD)));
-    RSTQ_CUDA(cudaFuncSetAttribute(gqa_decode_stream_kernel<HD, 4, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, attn_smem(HD)));
+template <int HD, int H>
+static int32_t attn_attrs() {
+    constexpr auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    RSTQ_CUDA(cudaFuncSetAttribute((gqa_decode_stream_kernel<HD, H, false, kStreamWarps>), attr, attn_smem(HD, kStreamWarps)));
+    RSTQ_CUDA(cudaFuncSetAttribute((gqa_decode_stream_kernel<HD, H, true, kStreamWarps>), attr, attn_smem(HD, kStreamWarps)));
+    RSTQ_CUDA(cudaFuncSetAttribute((gqa_decode_stream_kernel<HD, H, true, kNarrowWarps>), attr, attn_smem(HD, kNarrowWarps)));
+    return RSTQ_OK;
+}
+// how many clusters of each size the device holds at once (148 SMs, 16 warps: 74, 45, 33, 26, 22, 15, 15)
+template <int WARPS>
+static int32_t attn_count_clusters(int (&count)[kClusterMax + 1]) {
+    for (int c = 2; c <= kClusterMax; ++c) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(1, (unsigned)c);
+        cfg.blockDim = dim3(WARPS * 32);
+        cfg.dynamicSmemBytes = attn_smem(128, WARPS);
+        cudaLaunchAttribute a[1];
+        a[0].id = cudaLaunchAttributeClusterDimension;
+        a[0].val.clusterDim.x = a[0].val.clusterDim.z = 1;
+        a[0].val.clusterDim.y = (unsigned)c;
+        cfg.attrs = a;
+        cfg.numAttrs = 1;
+        RSTQ_CUDA(cudaOccupancyMaxActiveClusters(&count[c], (gqa_decode_stream_kernel<128, 4, true, WARPS>), &cfg));
+    }
     return RSTQ_OK;
 }
 // Scratch of both kernels, the most that a call can need (0.3 and 2.5 MB): a call under capture needs no call before it,
@@ -856,22 +879,14 @@ static int32_t attn_reserve(DeviceState& ds) {
 }
 int32_t attn_configure(DeviceState& ds) {
     int32_t rc = attn_reserve(ds);
-    if (rc == RSTQ_OK) rc = attn_attr<64>();
-    if (rc == RSTQ_OK) rc = attn_attr<128>();
-    // how many clusters of each size the device holds at once (148 SMs: 74, 45, 33, 26, 22, 15, 15)
-    for (int c = 2; c <= kClusterMax && rc == RSTQ_OK; ++c) {
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(1, (unsigned)c);
-        cfg.blockDim = dim3(kStreamThreads);
-        cfg.dynamicSmemBytes = attn_smem(128);
-        cudaLaunchAttribute a[1];
-        a[0].id = cudaLaunchAttributeClusterDimension;
-        a[0].val.clusterDim.x = a[0].val.clusterDim.z = 1;
-        a[0].val.clusterDim.y = (unsigned)c;
-        cfg.attrs = a;
-        cfg.numAttrs = 1;
-        RSTQ_CUDA(cudaOccupancyMaxActiveClusters(&ds.attn_clusters[c], gqa_decode_stream_kernel<128, 4, true>, &cfg));
-    }
+    if (rc == RSTQ_OK) rc = attn_attrs<64, 1>();
+    if (rc == RSTQ_OK) rc = attn_attrs<64, 2>();
+    if (rc == RSTQ_OK) rc = attn_attrs<64, 4>();
+    if (rc == RSTQ_OK) rc = attn_attrs<128, 1>();
+    if (rc == RSTQ_OK) rc = attn_attrs<128, 2>();
+    if (rc == RSTQ_OK) rc = attn_attrs<128, 4>();
+    if (rc == RSTQ_OK) rc = attn_count_clusters<kStreamWarps>(ds.attn_clusters);
+    if (rc == RSTQ_OK) rc = attn_count_clusters<kNarrowWarps>(ds.attn_narrow_clusters);
     return rc;
 }
 
@@ -997,7 +1012,21 @@ static int32_t attention_impl(rstq_ctx* ctx, rstq_buf* q, rstq_buf* k, rstq_buf*
     // are resident together: 16 of eight took two waves, 32 / 16 x 2000 16.1 us against 10.4.  Fewer, longer slices are taken
     // for it where each grows by less than about 1 us of its stream (32 / 16 x 500, nine -> six: 6.89 -> 5.38; x 2000:
     // 9.81 -> 10.55, so not there).
-    bool clustered = false;
+    // With more KV heads than half the SMs there is one block of 16 warps for each, and where these leave a third of the SMs
+    // without one, or two fifths in several rounds, blocks of four warps share the work more evenly: four per SM, as many
+    // slices (a cluster) as all fit at once, with a little to spare (112 clusters of five, of 112 that fit, took two rounds).
+    // Their merge takes longer, so a short cache of one round stays with 16 warps, and one of 64 positions for four query
+    // heads; else in several rounds a short cache is mostly the start and end of each, which four blocks per SM overlap.
+    // us, 16 warps -> four: 80 / 80 heads x 250 8.3 / 8.9, x 500 11.4 -> 9.7, x 2000 34.5 -> 28.5, 96 x 2000 35.1 -> 33.2 (112: 38.9 /
+    // 39.6), 160 x 100 9.4 -> 7.6, x 2000 62.5 -> 53.7, 256 x 500 24.8 -> 23.2 (x 2000: 78.5 / 84.5), 640 / 160 x 64 8.8 / 10.5.
+    const int64_t heads = n_kv * gz, rounds = (heads + ds.sm_count - 1) / ds.sm_count;
+    const bool narrow = fast && (rounds == 1 ? 2 * heads > ds.sm_count && 3 * heads <= 2 * ds.sm_count && span >= 384
+                                             : (gs < kStreamHeads || span > 64) && (5 * heads < 3 * rounds * ds.sm_count || span < 768));
+    bool clustered = narrow;
+    if (narrow) {
+        S = std::max<int64_t>(1, std::min({4 * ds.sm_count / heads, (span + 63) / 64, (int64_t)kClusterMax}));
+        while (S > 1 && 32 * heads > 31 * ds.attn_narrow_clusters[S]) --S;
+    }
     for (int64_t c = fast ? (S < kClusterMax ? S : kClusterMax) : 0; c > 1 && !clustered; --c) {
         if (n_kv * gz > ds.attn_clusters[c]) continue;
         if ((span / c - span / S) * head_dim * 8 > kClusterExtra) break;
@@ -1033,21 +1062,25 @@ static int32_t attention_impl(rstq_ctx* ctx, rstq_buf* q, rstq_buf* k, rstq_buf*
     p.xq = xq ? (int8_t*)xq->ptr : nullptr;
     p.xs = xq ? (float*)xs->ptr : nullptr;
     p.xsum = xq && xsum ? (int32_t*)xsum->ptr : nullptr;
-    const dim3 grid((unsigned)n_kv, (unsigned)S, (unsigned)gz), block((unsigned)(fast ? kStreamThreads : kAttnWarps * 32));
+    const dim3 grid((unsigned)n_kv, (unsigned)S, (unsigned)gz);
     if (fast) {
-        const size_t smem = (size_t)attn_smem((int)head_dim);
-#define RSTQ_ATTN(HD, CL)                                                                                            \
-    (gs == 1 ? launch_attn_cluster(gqa_decode_stream_kernel<HD, 1, CL>, grid, block, smem, ds, CL ? (unsigned)S : 1u, p)   \
-     : gs == 2 ? launch_attn_cluster(gqa_decode_stream_kernel<HD, 2, CL>, grid, block, smem, ds, CL ? (unsigned)S : 1u, p) \
-               : launch_attn_cluster(gqa_decode_stream_kernel<HD, 4, CL>, grid, block, smem, ds, CL ? (unsigned)S : 1u, p))
-        if (clustered) RSTQ_CUDA(head_dim == 64 ? RSTQ_ATTN(64, true) : RSTQ_ATTN(128, true));
-        else RSTQ_CUDA(head_dim == 64 ? RSTQ_ATTN(64, false) : RSTQ_ATTN(128, false));
+        auto launch = [&](auto kernel, int warps) {
+            return launch_attn_cluster(kernel, grid, dim3((unsigned)warps * 32), (size_t)attn_smem((int)head_dim, warps), ds,
+                                       clustered ? (unsigned)S : 1u, p);
+        };
+#define RSTQ_ATTN(HD, CL, WARPS)                                                  \
+    (gs == 1   ? launch(gqa_decode_stream_kernel<HD, 1, CL, WARPS>, WARPS)       \
+     : gs == 2 ? launch(gqa_decode_stream_kernel<HD, 2, CL, WARPS>, WARPS)       \
+               : launch(gqa_decode_stream_kernel<HD, 4, CL, WARPS>, WARPS))
+        if (narrow) RSTQ_CUDA(head_dim == 64 ? RSTQ_ATTN(64, true, kNarrowWarps) : RSTQ_ATTN(128, true, kNarrowWarps));
+        else if (clustered) RSTQ_CUDA(head_dim == 64 ? RSTQ_ATTN(64, true, kStreamWarps) : RSTQ_ATTN(128, true, kStreamWarps));
+        else RSTQ_CUDA(head_dim == 64 ? RSTQ_ATTN(64, false, kStreamWarps) : RSTQ_ATTN(128, false, kStreamWarps));
 #undef RSTQ_ATTN
     } else {
         const size_t smem = (size_t)(kAttnWarps * gs * row * 4);
         if (smem > 48 * 1024)
             RSTQ_CUDA(cudaFuncSetAttribute(gqa_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        RSTQ_CUDA(launch_attn(gqa_decode_kernel, grid, block, smem, ds, p));
+        RSTQ_CUDA(launch_attn(gqa_decode_kernel, grid, dim3(kAttnWarps * 32), smem, ds, p));
     }
     ctx->launches++;
     return RSTQ_OK;

@@ -103,7 +103,8 @@ struct DeviceState {
     void* attn_scratch = nullptr;  // decode attention: arrival counters + per-slice softmax states
     void* attn_slots = nullptr;    // ... of head_dim 64 and 128: slots of the slices' states, every word 0xFFFFFFFF between launches
     int64_t attn_slots_bytes = 0;
-    int attn_clusters[9] = {};     // ... and how many clusters of 2 .. 8 of its thread blocks the device holds at once
+    int attn_clusters[9] = {};     // ... and how many clusters of 2 .. 8 of its thread blocks the device holds at once,
+    int attn_narrow_clusters[9] = {};   // or of its blocks of a quarter of the warps
     void* pinned = nullptr;        // host staging for the host-array entry points
     int64_t pinned_bytes = 0;
     void* io_dev = nullptr;        // device staging for the host-array entry points

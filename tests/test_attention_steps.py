@@ -293,6 +293,40 @@ def test_attention_of_special_values(ctx, clen, at):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("group,n_kv", [(1, 74), (1, 75), (2, 80), (5, 40), (4, 96), (3, 100), (1, 148), (1, 149), (3, 250), (1, 600)])
+def test_attention_of_many_kv_heads(ctx, group, n_kv, hd):
+    """More than half as many KV heads (times passes over a group) as the device has SMs: thread blocks of 16 warps or of four,
+    by the heads and the length, the latter in clusters of six down to one.  Lengths around a tile, a round of the warps, a
+    slice and the line between the two; rows beyond them hold NaN.  With the quantized output too, equal in bits to
+    attention and then the quantizer.  1e-5 as above."""
+    n_q, maxpos, scale, n = group * n_kv, 460, 1.0 / math.sqrt(hd), group * n_kv * hd
+    q = synth.normal(181 + group, n)
+    k0, v0 = synth.normal(182, maxpos * n_kv * hd), synth.normal(183, maxpos * n_kv * hd)
+    bq, bo = ctx.array_to_buffer(q), ctx.make_buffer(n, np.float32)
+    bk, bv = ctx.make_buffer(k0.size, np.float32), ctx.make_buffer(v0.size, np.float32)
+    bl = ctx.make_buffer(1, np.int64)
+    quant = [[ctx.make_buffer(n, np.int8), ctx.make_buffer(n // 32, np.float32), ctx.make_buffer(n // 32, np.int32)] for _ in range(2)]
+    for clen in (1, 8, 31, 33, 65, 130, 383, 384, 460):
+        k, v = k0.copy(), v0.copy()
+        k[clen * n_kv * hd:] = np.nan
+        v[clen * n_kv * hd:] = np.nan
+        bk.upload(k), bv.upload(v), bl.upload(np.array([clen], np.int64))
+        ref = orc.gqa_decode_attention(q, k0, v0, clen, n_q, group, n_kv, hd, scale)
+        ctx.gqa_decode_attention(bq, bk, bv, bo, clen, n_q, group, n_kv, hd, maxpos, scale)
+        ctx.sync()
+        assert relerr(bo.download(), ref) <= 1e-5, clen
+        ctx.gqa_decode_attention_quant_act(bq, bk, bv, bo, *quant[0], 0, n_q, group, n_kv, hd, maxpos, scale, clenbuf=bl)
+        ctx.quant_act_i8(bo, *quant[1], 1, n)
+        ctx.sync()
+        assert relerr(bo.download(), ref) <= 1e-5, clen
+        for x, y in zip(*quant):
+            assert np.array_equal(x.download(), y.download())
+    for o in (bq, bo, bk, bv, bl, *quant[0], *quant[1]):
+        o.free()
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("hd", [32, 64, 96, 128, 256])
 def test_attention_with_a_device_length_beyond_the_cache(ctx, hd):
     """A length above the capacity counts as the capacity, for every kernel: the same bits."""
