@@ -390,8 +390,12 @@ RSTQ_API int32_t rstq_residual_add(rstq_ctx* ctx, rstq_buf* a, rstq_buf* b, rstq
  *                      softmax(scale * q.K^T) V over cache positions [0, cache_len), K / V caches
  *                      [maxpos][n_kv][head_dim], n_q = group * n_kv, head_dim % 4 == 0 and <= 256.
  * posbuf / clenbuf: NULL, or a device buffer holding one int64 that the kernel reads (the -buf
- * variants: a captured graph then serves every token; call once before capturing).  The
- * reference's score scratch `sc` has no counterpart (scores stay in registers).  All f32. */
+ * variants: a captured graph then serves every token; a length above maxpos counts as maxpos).  No
+ * call before the capture is needed: their scratch is allocated with the context.  The
+ * reference's score scratch `sc` has no counterpart (scores stay in registers).  All f32.
+ * With head_dim 64 or 128 and a long cache one thread block per KV head waits, for at most 2 s, for the
+ * others' partial results: should that run out, rstq_sync returns RSTQ_E_WAIT, and until it has been
+ * called the results of this and of later attention calls (replays too) are invalid. */
 RSTQ_API int32_t rstq_rope_pos(rstq_ctx* ctx, rstq_buf* x, rstq_buf* out, rstq_buf* posbuf, int64_t heads,
                                int64_t head_dim, double theta, int64_t pos);
 RSTQ_API int32_t rstq_kv_append(rstq_ctx* ctx, rstq_buf* src, rstq_buf* cache, rstq_buf* posbuf, int64_t kvrow,
