@@ -34,7 +34,7 @@ import sys
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 OUT = os.path.join(HERE, "_ref")
-REFERENCE = os.environ.get("RASTER_REFERENCE", "/root/reference")
+REFERENCE = os.environ.get("RASTER_REFERENCE", os.path.join(HERE, os.pardir, os.pardir, "reference"))   # beside this repository
 KERNELS_CLJ = "src/raster/quant/kernels.clj"
 
 HELPERS = ("wi8-dot-q4", "wi8-dot-q4-x8", "wi8-dot-q8-x8")

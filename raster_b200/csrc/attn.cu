@@ -11,8 +11,8 @@
 // the cache positions and up to four (eight in the general kernel) query heads of the group, which it serves from the K / V rows
 // it reads once (the reference reads them once per query head); warps walk the positions with an online
 // softmax (running max, sum and weighted V in registers), the warps of a CTA are merged through
-// shared memory and the slices through a small scratch in device memory, from which one CTA per
-// KV head writes out = sum_j p_j v_j.  The reference's score scratch `sc` is not used.
+// shared memory, and the slices of a KV head through distributed shared memory where they are a cluster, else through
+// a small scratch in device memory, from which one CTA writes out = sum_j p_j v_j.  The reference's score scratch `sc` is not used.
 // head_dim 64 and 128 take gqa_decode_stream_kernel (rows through shared memory, eight positions per
 // warp step); every other head_dim % 4 == 0 up to 256 takes the general gqa_decode_kernel (a
 // warp per position).
@@ -359,21 +359,26 @@ gqa_decode_kernel(const AttnParams p) {
 }
 
 // ---- head_dim 64 and 128 ----------------------------------------------------------------------
-// Streams its slice of K and V through shared memory: one CTA per SM and KV head, serving up to four query heads from
-// rows that it reads once (larger groups find them in L2).  Each of 16 warps works alone on tiles of eight positions, with a ring of its own that
-// cp.async keeps full, so the bytes in flight (192 KB per SM) do not depend on registers:
+// Streams its slice of K and V through shared memory: a CTA of 16 warps per SM (with many KV heads four CTAs of four), serving
+// up to four query heads of a KV head from rows that it reads once (larger groups find them in L2).  Each warp works alone on
+// tiles of eight positions, with a ring of its own that cp.async keeps full, so the bytes in flight (192 KB per SM) do not
+// depend on registers:
 //   scores   eight lanes share a position; the sums of 8 positions x H heads over those lanes are reduced by halving
 //            (7 shuffles for 32 values), which leaves one (position, head) per lane: one exp per value
 //   softmax  online per tile (a maximum over eight positions, a rescale only where a maximum moved)
 //   output   a lane owns four dims of all heads, p comes back as one broadcast load per position
-// and the warps' states meet once, at the end.  The slices' states go through slots in device memory that hold kEmpty
-// between launches: the CTA of the last slice polls for the values themselves (no fence, counter or flag stands between
-// a store and its reader), merges and empties them.  It waits only for CTAs launched before it.
-// What bounds it: an SM takes in its 190 - 230 KB at about 65 B/ns, whether they come from HBM or L2; then a tail of about
-// 4 us (the last tile, the warps' merge, one trip through L2, the slices' merge) of which little is arithmetic.
-// us, back to back, against the kernel before it (two heads per CTA, rows through registers): 32 q / 8 kv heads x 4096
-// 13.8 -> 11.5, 64 / 8 x 2000 12.5 -> 11.1, 28 / 4 x 5000 14.4 -> 12.5, 32 / 16 x 2000 9.95 -> 9.72, 32 / 32 x 1000
-// 9.54 -> 9.45, 64 / 8 x 8000 of 64 elements 23.6 -> 15.7; four 7B layers at 1024 positions 213.2 -> 207.
+// and the warps' states meet once, at the end.  The slices of a KV head then meet in one of two ways (attention_impl says
+// which): as a cluster of up to eight, each CTA merging its share of the output from the others' shared memory; or
+// through slots in device memory that hold kEmpty between launches: the CTA of the last slice polls for the values
+// themselves (no fence, counter or flag stands between a store and its reader), merges and empties them.  It waits only
+// for CTAs launched before it.
+// What bounds it: an SM takes in its 190 - 230 KB at about 65 B/ns, whether they come from HBM or L2; then a tail (the last
+// tile, the warps' merge, the slices' merge) of about 4 us through slots and 2.5 as a cluster, of which little is arithmetic.
+// us, back to back over 0.3 GB of caches in turn, against the kernel before it (two heads per CTA, rows through registers):
+// through slots 32 q / 8 kv heads x 4096 13.9 -> 12.6, 64 / 8 x 2000 12.7 -> 11.4, 28 / 4 x 5000 14.4 -> 13.2, 32 / 16 x 2000
+// 11.8 -> 11.4, 64 / 8 x 8000 of 64 elements 23.6 -> 16.0; as clusters 32 / 32 x 1000 11.0 -> 9.7, 32 / 8 x 1000 8.9 -> 7.8, 32 / 16
+// x 500 8.6 -> 6.3; four 7B layers at 1024 positions 221.2 -> 195.6.  One or two query heads per KV head and more than
+// about 130 MB of K and V, all at the rate of HBM: slower by 1 - 6 % (32 / 32 x 16384 83.1 -> 84.1, 32 / 16 x 40000 100.0 -> 104.2).
 // Slower: one bulk copy per row instead of cp.async (20 cycles each, the first tile 2.3 us after the wait); a counter
 // that the last CTA to arrive reads instead of the polled slots (a tail of 4.4 us); slots read before the weights are
 // ready (most are empty then, and the second look costs a trip: 11.5 -> 12.4); eight heads per CTA in two passes
@@ -1007,18 +1012,18 @@ static int32_t attention_impl(rstq_ctx* ctx, rstq_buf* q, rstq_buf* k, rstq_buf*
     if (fast && S > kMaxSlices) S = kMaxSlices;
     if (S > 512) S = 512;
     if (S < 1) S = 1;
-    // Up to eight slices may be one cluster and meet in distributed shared memory, which saves 1 - 1.5 us of the tail (32 /
-    // 32 heads x 1000 9.65 -> 8.24 us, 32 / 8 x 200 6.68 -> 5.19, four 7B layers 206.5 -> 196.8), as long as all clusters
+    // Up to eight slices may be one cluster and meet in distributed shared memory, which saves 0.3 - 1.5 us of the tail (against
+    // slots: 32 / 32 heads x 1000 10.3 -> 9.7 us, 32 / 8 x 200 6.8 -> 5.3, four 7B layers 204.5 -> 195.6), as long as all clusters
     // are resident together: 16 of eight took two waves, 32 / 16 x 2000 16.1 us against 10.4.  Fewer, longer slices are taken
-    // for it where each grows by less than about 1 us of its stream (32 / 16 x 500, nine -> six: 6.89 -> 5.38; x 2000:
+    // for it where each grows by less than about 1 us of its stream (32 / 16 x 500, nine -> six: 7.6 -> 6.3; x 2000:
     // 9.81 -> 10.55, so not there).
     // With more KV heads than half the SMs there is one block of 16 warps for each, and where these leave a third of the SMs
     // without one, or two fifths in several rounds, blocks of four warps share the work more evenly: four per SM, as many
     // slices (a cluster) as all fit at once, with a little to spare (112 clusters of five, of 112 that fit, took two rounds).
     // Their merge takes longer, so a short cache of one round stays with 16 warps, and one of 64 positions for four query
     // heads; else in several rounds a short cache is mostly the start and end of each, which four blocks per SM overlap.
-    // us, 16 warps -> four: 80 / 80 heads x 250 8.3 / 8.9, x 500 11.4 -> 9.7, x 2000 34.5 -> 28.5, 96 x 2000 35.1 -> 33.2 (112: 38.9 /
-    // 39.6), 160 x 100 9.4 -> 7.6, x 2000 62.5 -> 53.7, 256 x 500 24.8 -> 23.2 (x 2000: 78.5 / 84.5), 640 / 160 x 64 8.8 / 10.5.
+    // us, 16 warps -> four: 80 / 80 heads x 250 7.7 / 8.9, x 500 10.5 -> 9.6, x 2000 34.4 -> 28.5, 96 x 2000 35.4 -> 33.5 (112: 38.9 /
+    // 39.6), 160 x 100 9.3 -> 8.1, x 2000 63.7 -> 54.0, 256 x 500 25.5 -> 23.2 (x 2000: 78.5 / 84.5), 640 / 160 x 64 8.8 / 10.5.
     const int64_t heads = n_kv * gz, rounds = (heads + ds.sm_count - 1) / ds.sm_count;
     const bool narrow = fast && (rounds == 1 ? 2 * heads > ds.sm_count && 3 * heads <= 2 * ds.sm_count && span >= 384
                                              : (gs < kStreamHeads || span > 64) && (5 * heads < 3 * rounds * ds.sm_count || span < 768));
