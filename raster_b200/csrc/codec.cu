@@ -87,7 +87,7 @@ RSTQ_INLINE bool block_plain(const float* w, uint8_t* codes, float* scale, int b
 // 128 * 2^-23 of the double product (a rounding of the reciprocal, one of the product), so a t further than 1e-4 from
 // every tie rounds the same way.  A block with one that is not, or whose scale leaves the normal f32 range, takes
 // block_plain.  (Left to the compiler, these loops come out scalar: 2.7 - 3.0 ns per element and core, 0.7 so;
-// 4096 x 4096 on 8 cores 8.6 -> 3.8 ms, the rest the read of the f32 matrix and the pages of the results.)
+// 4096 x 4096 on 8 cores of one host 8.6 -> 3.8 ms, the rest the read of the f32 matrix and the pages of the results.)
 template <int BITS>
 RSTQ_AVX2 static inline bool block_plain_avx2(const float* w, uint8_t* codes, float* scale) {
     const __m256 sign = _mm256_set1_ps(-0.0f);
