@@ -361,8 +361,7 @@ gqa_decode_kernel(const AttnParams p) {
 // ---- head_dim 64 and 128 ----------------------------------------------------------------------
 // Streams its slice of K and V through shared memory: a CTA of 16 warps per SM (with many KV heads four CTAs of four), serving
 // up to four query heads of a KV head from rows that it reads once (larger groups find them in L2).  Each warp works alone on
-// tiles of eight positions, with a ring of its own that cp.async keeps full, so the bytes in flight (192 KB per SM) do not
-// depend on registers:
+// tiles of eight positions, with a ring of its own that cp.async keeps full, so the bytes in flight do not depend on registers:
 //   scores   eight lanes share a position; the sums of 8 positions x H heads over those lanes are reduced by halving
 //            (7 shuffles for 32 values), which leaves one (position, head) per lane: one exp per value
 //   softmax  online per tile (a maximum over eight positions, a rescale only where a maximum moved)
@@ -387,13 +386,17 @@ constexpr int kTilePos = 8;
 constexpr int kStreamWarps = 16;                      // one such CTA per SM ...
 constexpr int kNarrowWarps = 4;                       // ... or, with many KV heads, four of these
 constexpr int kStreamHeads = 4;                       // query heads of one KV head per CTA
-constexpr int kRingBytes = 12288;                     // per warp
 constexpr int kHintPos = 16;                          // positions per warp of a CTA requested into L2 ahead of time
 constexpr uint32_t kEmpty = 0xFFFFFFFFu;              // a NaN that no arithmetic produces
 __host__ __device__ constexpr int attn_unit_bytes(int hd) { return kTilePos * hd * 4; }      // a tile's rows of K, or of V
-__host__ __device__ constexpr int attn_units(int hd) { return kRingBytes / attn_unit_bytes(hd); }
+// A warp's ring: two tiles' worth of K or V of 128 elements (128 KB in flight per SM).  Three (192 KB), as at first, were slower almost
+// everywhere, as if SMs got in each other's way: 32 q / 8 kv heads x 4096 12.6 -> 11.7 us, 32 / 32 x 1000 9.7 -> 9.1, x 16384 83.7 ->
+// 78.8, 32 / 16 x 40000 105.7 -> 101.5.  The CTAs of four warps stay with three, which also keeps them at four per SM: with two, a
+// fifth finds room and the slices no longer spread evenly (160 / 160 x 2000 of 64 elements 29.4 -> 34.9).
+__host__ __device__ constexpr int attn_ring(int warps) { return warps == kStreamWarps ? 8192 : 12288; }
+__host__ __device__ constexpr int attn_units(int hd, int warps) { return attn_ring(warps) / attn_unit_bytes(hd); }
 // shared memory: the warps' rings, the query heads, the warps' p
-__host__ __device__ constexpr int attn_q_off(int warps) { return warps * kRingBytes; }
+__host__ __device__ constexpr int attn_q_off(int warps) { return warps * attn_ring(warps); }
 __host__ __device__ constexpr int attn_p_off(int hd, int warps) { return attn_q_off(warps) + kStreamHeads * hd * 4; }
 __host__ __device__ constexpr int attn_smem(int hd, int warps) { return attn_p_off(hd, warps) + warps * kTilePos * kStreamHeads * 4; }
 // ... and, once the rings are drained, in their place: the warps' states, then the merge of the slices
@@ -461,7 +464,7 @@ gqa_decode_stream_kernel(const AttnParams p) {
     constexpr int THREADS = WARPS * 32;
     constexpr int VEC = HD / 32, ROW = HD + 4;      // VEC: float4 per lane of a position's eight lanes
     constexpr uint32_t ROWB = HD * 4, UNITB = attn_unit_bytes(HD);
-    constexpr int NU = attn_units(HD);                              // units of the ring: K and V of a tile in turn
+    constexpr int NU = attn_units(HD, WARPS);                              // units of the ring: K and V of a tile in turn
     constexpr int LPP = HD / 4, PPS = 32 / LPP;                     // output: lanes per position, positions per step
     extern __shared__ __align__(128) uint8_t s_raw[];
     __shared__ int s_abort;
@@ -472,7 +475,7 @@ gqa_decode_stream_kernel(const AttnParams p) {
     const int64_t kvrow = (int64_t)p.n_kv * HD;
     const float* kb = p.k + (int64_t)hkv * HD;
     const float* vb = p.v + (int64_t)hkv * HD;
-    const uint32_t base = smem_u32(s_raw), ring = base + warp * kRingBytes;
+    const uint32_t base = smem_u32(s_raw), ring = base + warp * attn_ring(WARPS);
     volatile int* abort_flag = &s_abort;
 
     if (tid == 0) s_abort = 0;
