@@ -374,10 +374,10 @@ gqa_decode_kernel(const AttnParams p) {
 // What bounds it: an SM takes in its 190 - 230 KB at about 65 B/ns, whether they come from HBM or L2; then a tail (the last
 // tile, the warps' merge, the slices' merge) of about 4 us through slots and 2.5 as a cluster, of which little is arithmetic.
 // us, back to back over 0.3 GB of caches in turn, against the kernel before it (two heads per CTA, rows through registers):
-// through slots 32 q / 8 kv heads x 4096 13.9 -> 12.6, 64 / 8 x 2000 12.7 -> 11.4, 28 / 4 x 5000 14.4 -> 13.2, 32 / 16 x 2000
-// 11.8 -> 11.4, 64 / 8 x 8000 of 64 elements 23.6 -> 16.0; as clusters 32 / 32 x 1000 11.0 -> 9.7, 32 / 8 x 1000 8.9 -> 7.8, 32 / 16
-// x 500 8.6 -> 6.3; four 7B layers at 1024 positions 221.2 -> 195.6.  One or two query heads per KV head and more than
-// about 130 MB of K and V, all at the rate of HBM: slower by 1 - 6 % (32 / 32 x 16384 83.1 -> 84.1, 32 / 16 x 40000 100.0 -> 104.2).
+// through slots 32 q / 8 kv heads x 4096 13.9 -> 11.7, 64 / 8 x 2000 12.8 -> 10.7, 28 / 4 x 5000 14.4 -> 12.2, 32 / 16 x 2000
+// 11.8 -> 10.2, x 40000 99.7 -> 100.2, 64 / 8 x 8000 of 64 elements 23.7 -> 14.8; as clusters 32 / 32 x 1000 11.1 -> 9.1, 32 / 8 x 1000
+// 8.9 -> 7.7, 32 / 16 x 500 8.6 -> 6.3; four 7B layers at 1024 positions 222.5 -> 195.4.  Slower: two KV heads of 64 elements at 2500
+// positions (7.3 -> 8.5), 15 / 5 x 1800 of 64 (8.3 -> 8.7).
 // Slower: one bulk copy per row instead of cp.async (20 cycles each, the first tile 2.3 us after the wait); a counter
 // that the last CTA to arrive reads instead of the polled slots (a tail of 4.4 us); slots read before the weights are
 // ready (most are empty then, and the second look costs a trip: 11.5 -> 12.4); eight heads per CTA in two passes
@@ -401,7 +401,9 @@ __host__ __device__ constexpr int attn_p_off(int hd, int warps) { return attn_q_
 __host__ __device__ constexpr int attn_smem(int hd, int warps) { return attn_p_off(hd, warps) + warps * kTilePos * kStreamHeads * 4; }
 // ... and, once the rings are drained, in their place: the warps' states, then the merge of the slices
 constexpr int kClusterMax = 8;                        // slices of a KV head that may be one cluster
-constexpr int64_t kClusterExtra = 65000;              // bytes of K and V that a slice may grow by for it
+// bytes of K and V that a slice may grow by for it: about 1 us of its stream at four query heads, half as much again at one or
+// two, whose positions cost less arithmetic
+constexpr int64_t attn_cluster_extra(int64_t heads) { return heads > 2 ? 65000 : 96000; }
 constexpr int kMaxSlices = 160;                       // five (max, sum) pairs per lane of the merging warps
 __host__ __device__ constexpr int attn_w_off(int hd, int warps) { return warps * kStreamHeads * (hd + 4) * 4; }       // slice weights
 __host__ __device__ constexpr int attn_o_off(int hd, int warps) { return attn_w_off(hd, warps) + kStreamHeads * kMaxSlices * 4; }  // partial outputs
@@ -722,8 +724,11 @@ gqa_decode_stream_kernel(const AttnParams p) {
         // ---- the slices' states -> out: the CTA of the last slice ----
         // What it reads lies a trip to L2 away, so it is requested kHold float4 per thread at a time (slices g, g + groups,
         // ...).  The code is run once and cold: short loops rather than unrolled ones.
-        constexpr int kHold = 10;
-        groups = THREADS / cols;
+        // At least kSlotsPerThread slices each: with one (and the rest of what it holds read for nothing) the addition of up to 32
+        // groups' partial outputs took longer than it saved (2 / 2 heads x 1600 of 64 elements 8.0 -> 7.4 us, 32 / 16 x 2000
+        // 10.5 -> 10.1).
+        constexpr int kHold = 10, kSlotsPerThread = 4;
+        groups = min(THREADS / cols, (S + kSlotsPerThread - 1) / kSlotsPerThread);
         const int g = tid / cols, c = tid - g * cols, ch = c / LPP, pitch = p.gs * ROW;
         float* s_w = reinterpret_cast<float*>(s_raw + attn_w_off(HD, WARPS));     // [gc][S]: maxima, then weights
         float4* col = reinterpret_cast<float4*>(all + ch * ROW) + (c - ch * LPP);
@@ -1018,8 +1023,8 @@ static int32_t attention_impl(rstq_ctx* ctx, rstq_buf* q, rstq_buf* k, rstq_buf*
     // Up to eight slices may be one cluster and meet in distributed shared memory, which saves 0.3 - 1.5 us of the tail (against
     // slots: 32 / 32 heads x 1000 10.3 -> 9.7 us, 32 / 8 x 200 6.8 -> 5.3, four 7B layers 204.5 -> 195.6), as long as all clusters
     // are resident together: 16 of eight took two waves, 32 / 16 x 2000 16.1 us against 10.4.  Fewer, longer slices are taken
-    // for it where each grows by less than about 1 us of its stream (32 / 16 x 500, nine -> six: 7.6 -> 6.3; x 2000:
-    // 9.81 -> 10.55, so not there).
+    // for it where each grows by less than attn_cluster_extra (slots -> cluster: 32 / 16 x 500, nine -> six, 7.6 -> 6.3; x 1200 9.8 -> 8.4, x
+    // 1700 9.7 / 10.1; 2 / 2 x 1600 of 64 elements 7.4 -> 6.1; 32 / 8 x 1150, four heads, 7.7 / 8.4, x 1250 8.2 / 8.5).
     // With more KV heads than half the SMs there is one block of 16 warps for each, and where these leave a third of the SMs
     // without one, or two fifths in several rounds, blocks of four warps share the work more evenly: four per SM, as many
     // slices (a cluster) as all fit at once, with a little to spare (112 clusters of five, of 112 that fit, took two rounds).
@@ -1037,7 +1042,7 @@ static int32_t attention_impl(rstq_ctx* ctx, rstq_buf* q, rstq_buf* k, rstq_buf*
     }
     for (int64_t c = fast ? (S < kClusterMax ? S : kClusterMax) : 0; c > 1 && !clustered; --c) {
         if (n_kv * gz > ds.attn_clusters[c]) continue;
-        if ((span / c - span / S) * head_dim * 8 > kClusterExtra) break;
+        if ((span / c - span / S) * head_dim * 8 > attn_cluster_extra(gs)) break;
         S = c;
         clustered = true;
     }
