@@ -376,9 +376,9 @@ gqa_decode_kernel(const AttnParams p) {
 // us, back to back over 0.3 GB of caches in turn, against the kernel before it (two heads per CTA, rows through registers):
 // through slots 32 q / 8 kv heads x 4096 13.9 -> 11.7, 64 / 8 x 2000 12.8 -> 10.7, 28 / 4 x 5000 14.4 -> 12.2, 32 / 16 x 2000
 // 11.8 -> 10.2, x 40000 99.7 -> 100.2, 64 / 8 x 8000 of 64 elements 23.7 -> 14.8; as clusters 32 / 32 x 1000 11.1 -> 9.1, 32 / 8 x 1000
-// 8.9 -> 7.7, 32 / 16 x 500 8.6 -> 6.3; four 7B layers at 1024 positions 222.5 -> 195.4.  Slower: two KV heads of 64 elements at 2500
+// 8.9 -> 7.7, 32 / 16 x 500 8.6 -> 6.3; four 7B layers at 1024 positions 222.5 -> 195.4.  Slower than that: two KV heads of 64 elements at 2500
 // positions (7.3 -> 8.5), 15 / 5 x 1800 of 64 (8.3 -> 8.7).
-// Slower: one bulk copy per row instead of cp.async (20 cycles each, the first tile 2.3 us after the wait); a counter
+// Tried and slower: one bulk copy per row instead of cp.async (20 cycles each, the first tile 2.3 us after the wait); a counter
 // that the last CTA to arrive reads instead of the polled slots (a tail of 4.4 us); slots read before the weights are
 // ready (most are empty then, and the second look costs a trip: 11.5 -> 12.4); eight heads per CTA in two passes
 // (28 / 4 x 5000 16.1); packed f32x2 arithmetic (11.8 -> 12.4).
@@ -389,9 +389,9 @@ constexpr int kStreamHeads = 4;                       // query heads of one KV h
 constexpr int kHintPos = 16;                          // positions per warp of a CTA requested into L2 ahead of time
 constexpr uint32_t kEmpty = 0xFFFFFFFFu;              // a NaN that no arithmetic produces
 __host__ __device__ constexpr int attn_unit_bytes(int hd) { return kTilePos * hd * 4; }      // a tile's rows of K, or of V
-// A warp's ring: two tiles' worth of K or V of 128 elements (128 KB in flight per SM).  Three (192 KB), as at first, were slower almost
+// A warp's ring: K and V of one tile of 128 elements, of two of 64 (128 KB in flight per SM).  192 KB, as at first, was slower almost
 // everywhere, as if SMs got in each other's way: 32 q / 8 kv heads x 4096 12.6 -> 11.7 us, 32 / 32 x 1000 9.7 -> 9.1, x 16384 83.7 ->
-// 78.8, 32 / 16 x 40000 105.7 -> 101.5.  The CTAs of four warps stay with three, which also keeps them at four per SM: with two, a
+// 78.8, 32 / 16 x 40000 105.7 -> 101.5.  The CTAs of four warps stay with that, which also keeps them at four per SM: with less, a
 // fifth finds room and the slices no longer spread evenly (160 / 160 x 2000 of 64 elements 29.4 -> 34.9).
 __host__ __device__ constexpr int attn_ring(int warps) { return warps == kStreamWarps ? 8192 : 12288; }
 __host__ __device__ constexpr int attn_units(int hd, int warps) { return attn_ring(warps) / attn_unit_bytes(hd); }
@@ -1030,8 +1030,8 @@ static int32_t attention_impl(rstq_ctx* ctx, rstq_buf* q, rstq_buf* k, rstq_buf*
     // slices (a cluster) as all fit at once, with a little to spare (112 clusters of five, of 112 that fit, took two rounds).
     // Their merge takes longer, so a short cache of one round stays with 16 warps, and one of 64 positions for four query
     // heads; else in several rounds a short cache is mostly the start and end of each, which four blocks per SM overlap.
-    // us, 16 warps -> four: 80 / 80 heads x 250 7.7 / 8.9, x 500 10.5 -> 9.6, x 2000 34.4 -> 28.5, 96 x 2000 35.4 -> 33.5 (112: 38.9 /
-    // 39.6), 160 x 100 9.3 -> 8.1, x 2000 63.7 -> 54.0, 256 x 500 25.5 -> 23.2 (x 2000: 78.5 / 84.5), 640 / 160 x 64 8.8 / 10.5.
+    // us, 16 warps -> four: 80 / 80 heads x 250 7.2 / 8.0, x 500 10.7 -> 9.6, x 2000 33.9 -> 28.4, 90 x 1000 19.3 -> 17.5 (112 x 2000: 38.9 /
+    // 39.6), 160 x 100 8.6 -> 8.1, x 2000 62.5 -> 52.9, 256 x 500 25.0 -> 23.2 (x 2000: 78.3 / 84.5), 640 / 160 x 64 8.8 / 10.5.
     const int64_t heads = n_kv * gz, rounds = (heads + ds.sm_count - 1) / ds.sm_count;
     const bool narrow = fast && (rounds == 1 ? 2 * heads > ds.sm_count && 3 * heads <= 2 * ds.sm_count && span >= 384
                                              : (gs < kStreamHeads || span > 64) && (5 * heads < 3 * rounds * ds.sm_count || span < 768));
