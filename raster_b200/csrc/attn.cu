@@ -878,8 +878,8 @@ static int32_t attn_count_clusters(int (&count)[kClusterMax + 1]) {
     return RSTQ_OK;
 }
 // Scratch of both kernels, the most that a call can need (0.3 and 2.5 MB): a call under capture needs no call before it,
-// and a recorded launch and rstq_sync's reset always mean the same blocks.  With more than one slice per KV head
-// (attention_impl's S) there are at most as many slices in all as the device has SMs, of the general kernel twice as many.
+// and a recorded launch and rstq_sync's reset always mean the same blocks.  Slices that meet through slots are at most as
+// many in all as the device has SMs (attention_impl's S; clusters need none), those of the general kernel twice as many.
 static int32_t attn_reserve(DeviceState& ds) {
     const int64_t slots = (int64_t)ds.sm_count * kStreamHeads * (128 + 4) * 4;
     RSTQ_CUDA(cudaMalloc(&ds.attn_slots, (size_t)slots));
