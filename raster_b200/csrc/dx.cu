@@ -3,22 +3,30 @@
 // the dequant-transpose GEMM dX = dY . dequant(W), W = [out, in] signed 8-bit codes in the
 // reference's row-major layout with one f32 scale per 32 columns.
 //
-// Two launches.  dx_prep_kernel writes dy as three bf16 terms, dx_tmem_kernel is a tcgen05 GEMM over them with the
+// Two launches.  dx_prep_kernel writes dy as terms of 16 bits, dx_tmem_kernel is a tcgen05 GEMM over them with the
 // weights dequantized, in f32, and split the same way on their way into tensor memory:
 //
-//   D[128 columns i, NT tokens] += W'[i, o] * dy[m, o],  W' = W1 + W2 + W3, dy = Y1 + Y2 + Y3
-//                                = W1 Y1 + (W1 Y2 + W2 Y1) + (W1 Y3 + W2 Y2 + W3 Y1)
+//   D[128 columns i, NT tokens] += W'[i, o] * dy[m, o]
 //
-// Three terms hold all 24 bits of an f32 (each is rounded to nearest, so the rest takes the sign bit with it), and what
-// is left out is below 2^-24 of the product: the f32 product of the f32 values, whatever the spread inside a row or
-// a column block, at six bf16 MMAs.  A power of two per token row and per 32-column block keeps elements far
-// below the largest beside them (2^-90 is tested) out of bf16's subnormals.
-// (Pairs of fp16 terms need three MMAs, but hold 22 bits, and those only of elements above 2^-17 of their row's
-// largest, scales above 2^-9: a scale 2^-20 of its block's largest kept 11 bits.)
+// in one of two forms, tile by tile:
 //
-// What bounds it: the tensor core at the power cap, nominally 1536 cycles per 64 rows of a 128 x 128 tile, 2440 measured.
-// us per call back to back (bf16 mma.sync with three terms of dy * s, before): 4096 x 4096, m = 512 91.9 (260), m = 64
-// 29.3 (172); 1024 x 1024, m = 16 16.5 (44.7), m = 2048 35.0 (69.3); 11008 x 2048, m = 300 136 (457).
+//   pairs of fp16     W' = H + 2^-11 L, dy = h + 2^-11 l:  H h + 2^-11 (H l + L h)                             3 MMAs
+//   triples of bf16   W' = W1 + W2 + W3, dy = Y1 + Y2 + Y3:  W1 Y1 + (W1 Y2 + W2 Y1) + (W1 Y3 + W2 Y2 + W3 Y1)  6 MMAs
+//
+// A pair holds 23 bits.  Its second term is kept 2^11 larger than it is, in a sum of its own, and a power of two per token
+// row and per 32-column block brings the largest of them close to fp16's, so an element down to 2^-27 of its row's largest
+// (a scale down to 2^-20 of its column block's) has all of them: the tiles whose rows and column blocks hold nothing
+// smaller but zeros, and no infinity, take pairs.  Triples hold all 24 bits at any spread (2^-90 is tested); a tile with
+// one such row or column block takes them.  dx_prep_kernel writes both forms of dy and says which rows are which.
+//
+// The sums on the tensor core decide the error, not the products.  2-norm against the f64 product, over that of the product,
+// triples / pairs: 4096 x 4096, m = 512 9.2e-6 / 4.9e-6 (pairs add half as often to the first sum), m = 64 9.7e-7 / 6.5e-7
+// (even and odd steps have sums of their own), 1024 x 1024, m = 16 4.5e-7 / 3.6e-7.
+//
+// What bounds it: the tensor core at the power cap, for pairs nominally 768 cycles per 64 rows of a 128 x 128 tile; with the
+// conversions taken out the same MMAs take 1050, with them 1160.  us per call back to back, all tiles triples (before) ->
+// pairs: 4096 x 4096, m = 512 91.9 -> 58.9, m = 64 29.4 -> 25.8; 1024 x 1024, m = 16 16.6 -> 15.1; 11008 x 2048, m = 300
+// 135 -> 82.7.  With a row of small elements per tile, so triples: 91.6, 30.0, 17.4 (dy waits for the tile's form), 126.
 #include <type_traits>
 
 #include "internal.h"
@@ -28,7 +36,6 @@
 namespace rstq {
 
 constexpr int kDxStep = 64;                    // rows o per pipeline stage
-constexpr int kDxDy = 3;                       // stages of dy in shared memory
 constexpr int kDxRaw = 8;                      // stages of codes and scales in shared memory
 constexpr int kDxSet = 8;                      // dequant warps of a stage: 4 blocks of 32 columns x 2 halves of its rows
 constexpr int kDxDq = 2 * kDxSet;              // two sets on alternate stages
@@ -36,25 +43,35 @@ constexpr int kDxThreads = (kDxDq + 3) * 32;   // + two copy warps and the MMA w
 constexpr int kDxCodes = kDxStep * 128;        // bytes of codes per stage
 constexpr int kDxScales = 1024;                // bytes of scales per stage: 64 rows x 4 blocks
 constexpr int kDxRawBytes = kDxCodes + kDxScales;
-__host__ __device__ constexpr int dx_ring_bytes(int nt) { return kDxDy * 3 * nt * 128 + kDxRaw * kDxRawBytes; }
-// Tensor memory: the accumulators (nt columns each), then the ring of W' (32 columns per term and stage).
-constexpr int kDxWCols = 96;
-__host__ __device__ constexpr int dx_accs(int nt) { return nt > 64 ? 2 : 3; }
-__host__ __device__ constexpr int dx_wstages(int nt) { return (512 - dx_accs(nt) * nt) / kDxWCols; }   // 2, 3 or 4
+// A form's rings.  dy, in shared memory: four stages of pairs or three of triples (nine planes of nt x 128 bytes hold
+// either).  W', in tensor memory behind the accumulators (nt columns each): 32 columns per term and stage.
+template <int NT, bool PAIRS>
+struct DxForm {
+    static constexpr int terms = PAIRS ? 2 : 3;
+    static constexpr int ybytes = terms * NT * 128;
+    static constexpr int ystages = PAIRS ? 4 : 3;
+    static constexpr int accs = PAIRS ? (NT > 64 ? 2 : 4) : (NT > 64 ? 2 : 3);
+    static constexpr int wcols = 32 * terms;
+    static constexpr int wstages = (512 - accs * NT) / wcols < 4 ? (512 - accs * NT) / wcols : 4;   // 4; triples 2, 3 or 4
+};
+constexpr int kDxMaxY = 4, kDxMaxW = 4;        // barriers of either ring
+__host__ __device__ constexpr int dx_yring_bytes(int nt) { return 9 * nt * 128; }
+__host__ __device__ constexpr int dx_ring_bytes(int nt) { return dx_yring_bytes(nt) + kDxRaw * kDxRawBytes; }
 
 // Position p of an element inside its group of 16 rows o: the order in which a lane of the dequant warps holds
 // them (rows 2t, 2t + 1, 2t + 8, 2t + 9 for t = p / 4).  Any order serves, as long as dy has the same one; this
 // one reads the 128-byte-swizzled code tile without bank conflicts.
 __host__ __device__ constexpr int dx_row_of(int p) { return 2 * (p >> 2) + (p & 1) + ((p & 2) ? 8 : 0); }
 
-// ---- what the GEMM needs beforehand: dy as fp16 pairs, the largest scale of every column block ------
+// ---- what the GEMM needs beforehand: dy in both forms, the largest and the smallest scale of every column block ------
 constexpr int kDxParts = 64;                   // thread blocks that look at the scales, each at its share of the rows o
 struct DxPrep {
     const float* dy;
     const float* scales;
     uint16_t* y;            // [3][m][opad]: bf16 terms of dy * 2^-e
-    int* rowexp;            // [m]: e, which brings max|dy| of the row into [2^19, 2^20)
-    float* colmax;          // [kDxParts][nb]: max|scale| of a part's rows
+    uint16_t* y16;          // [2][m][opad]: fp16 terms of dy * 2^-(e + 5)
+    int* rowexp;            // [m]: 2 e, which brings max|dy| of the row into [2^19, 2^20), + 1 if pairs do not hold the row
+    float* colmax;          // [2][kDxParts][nb]: max|scale| of a part's rows; min|scale| of those that are not zero
     int64_t m, out, nb, opad;
 };
 
@@ -79,16 +96,47 @@ __device__ __forceinline__ float dx_scale(float v, int e) {
     const int h = e >> 1;
     return v * __int_as_float((h + 127) << 23) * __int_as_float((e - h + 127) << 23);
 }
-__device__ __forceinline__ float dx_block_max(float mx, float* red) {   // 256 threads
+// What pairs hold whole: with the largest magnitude of dy in [2^19, 2^20), of the scales in [2^12, 2^13), no element
+// and no scale but zeros below 2^-8.  (As fp16 both carry 2^-5 less: |dy| and |code * scale| stay below fp16's largest, and
+// 2^-13 is where the second term, 2^11 larger than it is, still has its 11 bits.)
+constexpr int kDxPrepMax = 512;     // threads per block of the pre-pass, at most
+constexpr float kDxPairMin = 0.00390625f;
+constexpr int kDxPairExp = 5;
+constexpr float kDxLow = 2048.0f;   // what the second terms of pairs are larger by
+__device__ __forceinline__ float dx_nonzero(float v) { return v == 0.f ? __int_as_float(0x7F800000) : fabsf(v); }
+__device__ __forceinline__ void dx_block_range(float& mx, float& mn, float (*red)[kDxPrepMax / 32]) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
+    for (int o = 16; o > 0; o >>= 1) {
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+    }
+    if ((threadIdx.x & 31) == 0) {
+        red[0][threadIdx.x >> 5] = mx;
+        red[1][threadIdx.x >> 5] = mn;
+    }
     __syncthreads();
-    mx = red[0];
-#pragma unroll
-    for (int i = 1; i < 8; ++i) mx = fmaxf(mx, red[i]);
+    mx = red[0][0];
+    mn = red[1][0];
+    for (int i = 1; i < (int)blockDim.x / 32; ++i) {
+        mx = fmaxf(mx, red[0][i]);
+        mn = fminf(mn, red[1][i]);
+    }
     __syncthreads();
-    return mx;
+}
+__device__ __forceinline__ uint32_t pack_f16x2(float hi, float lo) {
+    uint32_t d;
+    asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi), "f"(lo));
+    return d;
+}
+__device__ __forceinline__ float2 unpack_f16x2(uint32_t h) {
+    const __half2 v = *reinterpret_cast<const __half2*>(&h);
+    return __half22float2(v);
+}
+// b (upper half) and a (lower half) as pairs of fp16 terms
+__device__ __forceinline__ void dx_pair(float b, float a, uint32_t* t1, uint32_t* t2) {
+    *t1 = pack_f16x2(b, a);
+    const float2 h = unpack_f16x2(*t1);
+    *t2 = pack_f16x2((b - h.y) * kDxLow, (a - h.x) * kDxLow);
 }
 // b (upper half) and a (lower half) as three bf16 terms each.  INF: an infinity goes into the last term, which meets the
 // first term of the other factor alone -- next to the zeros among the other terms it would come out as a NaN.
@@ -110,53 +158,63 @@ __device__ __forceinline__ void dx_terms(float b, float a, uint32_t* t1, uint32_
     *t3 = pack_bf16x2(b, a);
 }
 
-// Latency-bound: every element is read once into registers (rows up to 8192), found the maximum of, and written
-// as three terms; the blocks that look at the scales read theirs as one run and leave a maximum per column block
-// (a strip of column blocks per thread block instead took 45 us at 4096 x 4096: 16 bytes of every row).
+// Latency-bound: every element is read once into registers (rows up to 16384), found the range of, and written in
+// both forms; the blocks that look at the scales read theirs as one run and leave a range per column block
+// (a strip of column blocks per thread block instead took 45 us at 4096 x 4096: 16 bytes of every row).  Adds 6.2 us to the
+// GEMM behind it at 4096 x 4096, m = 512 (9.4 with a whole group of 16 rows per thread: half sectors), 2.2 of them for the triples.
 constexpr int kDxMaxCols = 4096;
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(kDxPrepMax, 2)
 dx_prep_kernel(const DxPrep p) {
-    __shared__ float s_red[8];
-    __shared__ uint32_t s_max[kDxMaxCols];
+    __shared__ float s_red[2][kDxPrepMax / 32];
+    __shared__ uint32_t s_max[kDxMaxCols], s_min[kDxMaxCols];
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int nt = (int)blockDim.x;
     if (blockIdx.x < kDxParts) {
         const int64_t o0 = p.out * blockIdx.x / kDxParts, o1 = p.out * (blockIdx.x + 1) / kDxParts;
         for (int64_t c0 = 0; c0 < p.nb; c0 += kDxMaxCols) {     // (one pass up to 131 072 columns i)
             const int nc = (int)(p.nb - c0 < kDxMaxCols ? p.nb - c0 : kDxMaxCols);
-            for (int c = threadIdx.x; c < nc; c += 256) s_max[c] = 0u;
+            for (int c = threadIdx.x; c < nc; c += nt) {
+                s_max[c] = 0u;
+                s_min[c] = 0x7F800000u;
+            }
             __syncthreads();
             // a thread keeps its columns (four where rows are whole 16 bytes) and steps over the rows
             const bool vec = (p.nb & 3) == 0;
-            const int cols = vec ? nc >> 2 : nc, groups = cols < 256 ? 256 / cols : 1;
+            const int cols = vec ? nc >> 2 : nc, groups = cols < nt ? nt / cols : 1;
             const int rg = (int)threadIdx.x / cols;
-            if (rg < groups || cols >= 256) {
-                for (int c = (int)threadIdx.x - rg * cols; c < cols; c += 256) {
-                    float4 mx = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (rg < groups || cols >= nt) {
+                for (int c = (int)threadIdx.x - rg * cols; c < cols; c += nt) {
+                    float mx[4] = {0.f, 0.f, 0.f, 0.f}, mn[4];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) mn[j] = __int_as_float(0x7F800000);
                     const float* q = p.scales + c0 + (vec ? 4 * c : c);
 #pragma unroll 8
-                    for (int64_t o = o0 + (cols < 256 ? rg : 0); o < o1; o += groups) {
-                        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-                        if (vec) v = __ldg(reinterpret_cast<const float4*>(q + o * p.nb));
-                        else v.x = __ldg(q + o * p.nb);
-                        mx.x = fmaxf(mx.x, fabsf(v.x));
-                        mx.y = fmaxf(mx.y, fabsf(v.y));
-                        mx.z = fmaxf(mx.z, fabsf(v.z));
-                        mx.w = fmaxf(mx.w, fabsf(v.w));
+                    for (int64_t o = o0 + (cols < nt ? rg : 0); o < o1; o += groups) {
+                        float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
+                        if (vec) f = __ldg(reinterpret_cast<const float4*>(q + o * p.nb));
+                        else f.x = __ldg(q + o * p.nb);
+                        const float v[4] = {f.x, f.y, f.z, f.w};
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            mx[j] = fmaxf(mx[j], fabsf(v[j]));
+                            mn[j] = fminf(mn[j], dx_nonzero(v[j]));
+                        }
                     }
                     // (the bits of magnitudes order like the magnitudes)
-                    if (vec) {
-                        atomicMax(&s_max[4 * c], __float_as_uint(mx.x));
-                        atomicMax(&s_max[4 * c + 1], __float_as_uint(mx.y));
-                        atomicMax(&s_max[4 * c + 2], __float_as_uint(mx.z));
-                        atomicMax(&s_max[4 * c + 3], __float_as_uint(mx.w));
-                    } else {
-                        atomicMax(&s_max[c], __float_as_uint(mx.x));
-                    }
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        if (vec || j == 0) {
+                            atomicMax(&s_max[vec ? 4 * c + j : c], __float_as_uint(mx[j]));
+                            atomicMin(&s_min[vec ? 4 * c + j : c], __float_as_uint(mn[j]));
+                        }
                 }
             }
             __syncthreads();
-            for (int c = threadIdx.x; c < nc; c += 256) p.colmax[(int64_t)blockIdx.x * p.nb + c0 + c] = __uint_as_float(s_max[c]);
+            for (int c = threadIdx.x; c < nc; c += nt) {
+                p.colmax[(int64_t)blockIdx.x * p.nb + c0 + c] = __uint_as_float(s_max[c]);
+                p.colmax[(int64_t)(kDxParts + blockIdx.x) * p.nb + c0 + c] = __uint_as_float(s_min[c]);
+            }
             __syncthreads();
         }
         return;
@@ -164,66 +222,79 @@ dx_prep_kernel(const DxPrep p) {
     const int64_t m = (int64_t)blockIdx.x - kDxParts;
     const float* src = p.dy + m * p.out;
     const bool vec = (p.out & 3) == 0;
-    auto load16 = [&](int64_t o, float (&v)[16]) {   // o a multiple of 16
-        if (vec && o + 16 <= p.out) {
+    // Half a group of 16 rows o per thread and step: rows 4h .. 4h + 3 and 8 + 4h .. are positions 8h .. 8h + 7, so that a
+    // warp reads and writes whole 32-byte sectors.
+    auto load8 = [&](int64_t at, float (&v)[8]) {   // at: position, a multiple of 8
+        const int64_t o = (at & ~15ll) + ((at & 8) >> 1);
+        if (vec && o + 12 <= p.out) {
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const float4 f = __ldg(reinterpret_cast<const float4*>(src + o) + j);
+            for (int j = 0; j < 2; ++j) {
+                const float4 f = __ldg(reinterpret_cast<const float4*>(src + o + 8 * j));
                 v[4 * j] = f.x; v[4 * j + 1] = f.y; v[4 * j + 2] = f.z; v[4 * j + 3] = f.w;
             }
         } else {
 #pragma unroll
-            for (int j = 0; j < 16; ++j) v[j] = o + j < p.out ? __ldg(src + o + j) : 0.f;
+            for (int j = 0; j < 8; ++j) v[j] = o + (j & 3) + 2 * (j & 4) < p.out ? __ldg(src + o + (j & 3) + 2 * (j & 4)) : 0.f;
         }
     };
-    constexpr int kKeep = 2;   // x 256 threads x 16 elements
-    const bool keep = p.opad <= kKeep * 256 * 16;
-    float held[kKeep][16];
-    float mx = 0.f;
+    float mx = 0.f, mn = __int_as_float(0x7F800000);
+    auto range8 = [&](const float (&v)[8]) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            mx = fmaxf(mx, fabsf(v[j]));
+            mn = fminf(mn, dx_nonzero(v[j]));
+        }
+    };
+    constexpr int kKeep = 4;   // x threads x 8 elements
+    const bool keep = p.opad <= (int64_t)kKeep * nt * 8;
+    float held[kKeep][8];
     if (keep) {
 #pragma unroll
         for (int i = 0; i < kKeep; ++i) {
-            const int64_t o = (int64_t)(i * 256 + threadIdx.x) * 16;
-            if (o < p.opad) {
-                load16(o, held[i]);
-#pragma unroll
-                for (int j = 0; j < 16; ++j) mx = fmaxf(mx, fabsf(held[i][j]));
-            }
+            const int64_t at = (int64_t)(i * nt + threadIdx.x) * 8;
+            if (at < p.opad) load8(at, held[i]);
         }
-    } else {
-        for (int64_t o = threadIdx.x * 16; o < p.opad; o += 256 * 16) {
-            load16(o, held[0]);
 #pragma unroll
-            for (int j = 0; j < 16; ++j) mx = fmaxf(mx, fabsf(held[0][j]));
+        for (int i = 0; i < kKeep; ++i)
+            if ((int64_t)(i * nt + threadIdx.x) * 8 < p.opad) range8(held[i]);
+    } else {
+        for (int64_t at = threadIdx.x * 8; at < p.opad; at += nt * 8) {
+            load8(at, held[0]);
+            range8(held[0]);
         }
     }
     float down, down2;
-    const int e = dx_exponent(dx_block_max(mx, s_red), 20, &down, &down2);
-    auto store16 = [&](int64_t o, const float (&v)[16]) {
-        uint32_t t[3][8];
+    dx_block_range(mx, mn, s_red);
+    const int e = dx_exponent(mx, 20, &down, &down2);
+    const bool wide = isinf(mx) || mn * down * down2 < kDxPairMin;
+    auto store8 = [&](int64_t at, const float (&v)[8]) {
+        constexpr float kPair = 1.0f / (1 << kDxPairExp);
+        uint32_t t[5][4];
 #pragma unroll
-        for (int q = 0; q < 8; ++q)   // positions 2q, 2q + 1
-            dx_terms<true>(v[dx_row_of(2 * q + 1)] * down * down2, v[dx_row_of(2 * q)] * down * down2, &t[0][q], &t[1][q], &t[2][q]);
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            uint4* d = reinterpret_cast<uint4*>(p.y + (k * p.m + m) * p.opad + o);
-            d[0] = make_uint4(t[k][0], t[k][1], t[k][2], t[k][3]);
-            d[1] = make_uint4(t[k][4], t[k][5], t[k][6], t[k][7]);
+        for (int q = 0; q < 4; ++q) {   // positions at + 2q, + 1
+            const int r = 2 * (q >> 1) + 4 * (q & 1);
+            const float a = v[r] * down * down2, b = v[r + 1] * down * down2;
+            dx_terms<true>(b, a, &t[0][q], &t[1][q], &t[2][q]);
+            dx_pair(b * kPair, a * kPair, &t[3][q], &t[4][q]);
         }
+#pragma unroll
+        for (int k = 0; k < 5; ++k)
+            *reinterpret_cast<uint4*>((k < 3 ? p.y + (k * p.m + m) * p.opad : p.y16 + ((k - 3) * p.m + m) * p.opad) + at) =
+                make_uint4(t[k][0], t[k][1], t[k][2], t[k][3]);
     };
     if (keep) {
 #pragma unroll
         for (int i = 0; i < kKeep; ++i) {
-            const int64_t o = (int64_t)(i * 256 + threadIdx.x) * 16;
-            if (o < p.opad) store16(o, held[i]);
+            const int64_t at = (int64_t)(i * nt + threadIdx.x) * 8;
+            if (at < p.opad) store8(at, held[i]);
         }
     } else {
-        for (int64_t o = threadIdx.x * 16; o < p.opad; o += 256 * 16) {
-            load16(o, held[0]);
-            store16(o, held[0]);
+        for (int64_t at = threadIdx.x * 8; at < p.opad; at += nt * 8) {
+            load8(at, held[0]);
+            store8(at, held[0]);
         }
     }
-    if (threadIdx.x == 0) p.rowexp[m] = e;
+    if (threadIdx.x == 0) p.rowexp[m] = 2 * e + (wide ? 1 : 0);
 }
 
 // ---- the GEMM -----------------------------------------------------------------------------------
@@ -256,12 +327,11 @@ __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-// The MMAs of 16 rows o.  The three terms of dy lie one above the other in shared memory, so a term of W' times several
+// The MMAs of 16 rows o, triples.  The three terms of dy lie one above the other in shared memory, so a term of W' times several
 // of them is one instruction as far as the width allows (256): a tcgen05 instruction costs its issuer 50 - 60
 // cycles, and A is read from tensor memory once for both.  Up to 64 tokens the accumulators are the three sums in
-// the order of their size.  Above, W2 Y1 goes to the first product for the sake of that: 4096 x 4096, m = 512 102.6 ->
-// 91.9 us, 2-norm error against the f64 product 4.4e-6 -> 9.2e-6 (three bf16 terms of dy * s on mma.sync: 1.1e-5;
-// pairs of fp16: 9.7e-6 -- the f32 sums decide it, not the products).
+// the order of their size.  Above, W2 Y1 goes to the first product for the sake of that (4096 x 4096, m = 512: 102.6 ->
+// 91.9 us).
 template <int NT>
 __device__ __forceinline__ void dx_mma16(uint32_t d, uint32_t w, uint32_t b_lo, uint32_t b_hi, uint32_t accumulate, uint32_t leader) {
     constexpr uint32_t id1 = idesc_bf16(NT), id2 = idesc_bf16(2 * NT), id3 = idesc_bf16(NT <= 64 ? 3 * NT : NT);
@@ -300,9 +370,27 @@ __device__ __forceinline__ void dx_mma16(uint32_t d, uint32_t w, uint32_t b_lo, 
     }
 }
 
+// The same of pairs: H (h, l) as one instruction over 2 NT columns, L h to the sum of the second terms.
+template <int NT>
+__device__ __forceinline__ void dx_mma16_pairs(uint32_t d, uint32_t w, uint32_t b_lo, uint32_t b_hi, uint32_t accumulate, uint32_t leader) {
+    constexpr uint32_t id1 = idesc_f16(NT), id2 = idesc_f16(2 * NT);
+    asm volatile(
+        "{\n"
+        ".reg .pred p, q, t;\n"
+        ".reg .b64 b0;\n"
+        "setp.ne.b32 p, %6, 0;\n"
+        "setp.ne.b32 q, %7, 0;\n"
+        "setp.eq.b32 t, 0, 0;\n"
+        "mov.b64 b0, {%4, %5};\n"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%2], b0, %9, p;\n"   // H (h, l)
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%1], [%3], b0, %8, t;\n"   // L h
+        "}" ::"r"(d), "r"(d + NT), "r"(w), "r"(w + 32), "r"(b_lo), "r"(b_hi), "r"(accumulate), "r"(leader), "r"(id1), "r"(id2)
+        : "memory");
+}
+
 // Warps 0 .. 15 dequantize and store the tile (warp & 3 = 32-column block = its tensor-memory lanes, (warp >> 2) & 1 =
 // half of the stage's rows o, warp >> 3 = even / odd stages), warp 16 copies codes and scales, 17 issues the MMAs, 18
-// copies dy.  Codes, dy and W' have rings of their own: with one ring a stage waited for copy, conversion and MMA in turn.
+// copies dy.  Warps 0 .. 15 also find out which form the tile takes.  Codes, dy and W' have rings of their own: with one ring a stage waited for copy, conversion and MMA in turn.
 // Tensor-memory lane gid + 8 r of a block is column 4 gid + r of it: a lane of the dequant warp reads the codes
 // of four neighbouring columns as one word per row, and the 16x256b store wants exactly these four lanes of it.
 // Every mbarrier wait is time-bounded; on expiry the block reports through the status word, lets its copies
@@ -310,22 +398,20 @@ __device__ __forceinline__ void dx_mma16(uint32_t d, uint32_t w, uint32_t b_lo, 
 template <int NT>
 __global__ void __launch_bounds__(kDxThreads, 1)
 dx_tmem_kernel(const DxParams p, const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_y,
-               const __grid_constant__ CUtensorMap map_s) {
-    constexpr int YB = 3 * NT * 128;             // bytes of dy per stage
-    constexpr int WS = dx_wstages(NT), ACC = dx_accs(NT) * NT;
+               const __grid_constant__ CUtensorMap map_y16, const __grid_constant__ CUtensorMap map_s) {
     extern __shared__ uint8_t smem_raw[];
-    __shared__ int s_abort;
+    __shared__ int s_abort, s_wide;
     __shared__ uint32_t s_tmem;
     __shared__ int s_colexp[4];
-    __shared__ __align__(8) uint64_t s_bar[2 * kDxDy + 2 * WS + 2 * kDxRaw + 1];
+    __shared__ __align__(8) uint64_t s_bar[2 * kDxMaxY + 2 * kDxMaxW + 2 * kDxRaw + 1];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     const uint32_t sbase = smem_u32(smem), bar0 = smem_u32(s_bar);
     // y_full: a stage of dy has arrived; w_full: a stage of W' is in tensor memory; y_free, w_free: their MMAs are done;
     // raw: codes and scales of a step have arrived; taken: they are in registers
-    const uint32_t y_full = bar0, y_free = y_full + 8 * kDxDy, w_full = y_free + 8 * kDxDy, w_free = w_full + 8 * WS;
-    const uint32_t raw = w_free + 8 * WS, taken = raw + 8 * kDxRaw, acc_full = taken + 8 * kDxRaw;
-    const uint32_t rbase = sbase + kDxDy * YB;
+    const uint32_t y_full = bar0, y_free = y_full + 8 * kDxMaxY, w_full = y_free + 8 * kDxMaxY, w_free = w_full + 8 * kDxMaxW;
+    const uint32_t raw = w_free + 8 * kDxMaxW, taken = raw + 8 * kDxRaw, acc_full = taken + 8 * kDxRaw;
+    const uint32_t rbase = sbase + dx_yring_bytes(NT);
     const int part = blockIdx.x % p.split, tile = blockIdx.x / p.split;
     const int ft = tile / p.ttiles, tok0 = (tile - ft * p.ttiles) * NT;
     const int k0 = (int)((int64_t)p.steps * part / p.split), k1 = (int)((int64_t)p.steps * (part + 1) / p.split);
@@ -333,13 +419,13 @@ dx_tmem_kernel(const DxParams p, const __grid_constant__ CUtensorMap map_w, cons
 
     if (tid == 0) {
         asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&map_w)) : "memory");
-        asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&map_y)) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&map_y16)) : "memory");
     }
-    if (tid < kDxDy) {
+    if (tid < kDxMaxY) {
         mbar_init(y_full + 8 * tid, 1);
         mbar_init(y_free + 8 * tid, 1);
     }
-    if (tid < WS) {
+    if (tid < kDxMaxW) {
         mbar_init(w_full + 8 * tid, kDxSet);
         mbar_init(w_free + 8 * tid, 1);
     }
@@ -349,6 +435,7 @@ dx_tmem_kernel(const DxParams p, const __grid_constant__ CUtensorMap map_w, cons
     } else if (tid == kDxRaw) {
         mbar_init(acc_full, 1);
         s_abort = 0;
+        s_wide = 0;
     }
     if (tid <= kDxRaw) asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     if (warp == kDxDq + 1) {
@@ -361,7 +448,10 @@ dx_tmem_kernel(const DxParams p, const __grid_constant__ CUtensorMap map_w, cons
     tc_fence_after();
     const uint32_t tmem = s_tmem;
 
-    bool ok = true;
+    bool ok = true, wide = false;
+    auto exp_of = [&](int tok) { return (__ldg(p.rowexp + tok) >> 1) + (wide ? 0 : 2 * kDxPairExp); };
+    // The dequant warps decide the tile's form; they, the MMA warp and the warp that copies dy meet here.
+    auto form_known = [] { asm volatile("bar.sync 1, %0;" ::"r"((kDxDq + 2) * 32) : "memory"); };
     if (warp == kDxDq) {
         // ---------------- codes and scales ----------------
         if (lane == 0) {
@@ -383,46 +473,66 @@ dx_tmem_kernel(const DxParams p, const __grid_constant__ CUtensorMap map_w, cons
         }
     } else if (warp == kDxDq + 2) {
         // ---------------- dy ----------------
-        if (lane == 0) {
-            asm volatile("griddepcontrol.wait;" ::: "memory");
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        form_known();
+        auto copy = [&](auto pairs, const CUtensorMap* map) {
+            using F = DxForm<NT, decltype(pairs)::value>;
             int s = 0, issued = 0;
             uint32_t ph = 0;
             for (int k = k0; k < k1; ++k) {
                 ok = mbar_block(y_free + 8 * s, ph ^ 1u, abort_flag);
                 if (!ok) break;
-                mbar_expect_tx(y_full + 8 * s, YB);
-                tma_load_3d(sbase + s * YB, &map_y, k * kDxStep, tok0, 0, y_full + 8 * s);
+                mbar_expect_tx(y_full + 8 * s, F::ybytes);
+                tma_load_3d(sbase + s * F::ybytes, map, k * kDxStep, tok0, 0, y_full + 8 * s);
                 ++issued;
-                if (++s == kDxDy) { s = 0; ph ^= 1u; }
+                if (++s == F::ystages) { s = 0; ph ^= 1u; }
             }
-            if (!ok) dx_drain(y_full, issued, kDxDy);
+            if (!ok) dx_drain(y_full, issued, F::ystages);
+        };
+        if (lane == 0) {
+            if (s_wide) copy(std::false_type{}, &map_y);
+            else copy(std::true_type{}, &map_y16);
         }
     } else if (warp == kDxDq + 1) {
         // ---------------- MMAs ----------------
         const uint32_t leader = lane == 0;
         const uint64_t d0 = smem_desc_sw128(sbase);
         const uint32_t d_lo = (uint32_t)d0, d_hi = (uint32_t)(d0 >> 32);
-        int ys = 0, ws = 0;
-        uint32_t yph = 0, wph = 0;
-        bool any = false, ready = false;
-        for (int k = k0; k < k1; ++k) {
-            if (!ready) ok = mbar_spin(y_full + 8 * ys, yph, abort_flag) && mbar_spin(w_full + 8 * ws, wph, abort_flag);
-            if (!ok) break;
-            tc_fence_after();
-            const uint32_t w = tmem + ACC + ws * kDxWCols, b = d_lo + (uint32_t)ys * (YB >> 4);
-            const int ys2 = ys + 1 == kDxDy ? 0 : ys + 1, ws2 = ws + 1 == WS ? 0 : ws + 1;
-            const uint32_t yph2 = ys2 ? yph : yph ^ 1u, wph2 = ws2 ? wph : wph ^ 1u;
-            dx_mma16<NT>(tmem, w, b, d_hi, k != k0, leader);
-            dx_mma16<NT>(tmem, w + 8, b + 2, d_hi, 1u, leader);
-            dx_mma16<NT>(tmem, w + 16, b + 4, d_hi, 1u, leader);
-            // (the next stage's barriers are tested ahead of the last MMAs: their round trips run beside them)
-            ready = mbar_test(y_full + 8 * ys2, yph2) & mbar_test(w_full + 8 * ws2, wph2);
-            dx_mma16<NT>(tmem, w + 24, b + 6, d_hi, 1u, leader);
-            umma_commit_if(w_free + 8 * ws, leader);
-            umma_commit_if(y_free + 8 * ys, leader);
-            any = true;
-            ys = ys2; ws = ws2; yph = yph2; wph = wph2;
-        }
+        bool any = false;
+        form_known();
+        auto issue = [&](auto pairs) {
+            constexpr bool P = decltype(pairs)::value;
+            using F = DxForm<NT, P>;
+            int ys = 0, ws = 0;
+            uint32_t yph = 0, wph = 0;
+            bool ready = false;
+            for (int k = k0; k < k1; ++k) {
+                if (!ready) ok = mbar_spin(y_full + 8 * ys, yph, abort_flag) && mbar_spin(w_full + 8 * ws, wph, abort_flag);
+                if (!ok) break;
+                tc_fence_after();
+                // pairs of up to 64 tokens: even and odd steps have sums of their own
+                const uint32_t set = P && NT <= 64 ? (uint32_t)(k - k0) & 1u : 0u, d = tmem + set * 2 * NT;
+                const uint32_t w = tmem + F::accs * NT + ws * F::wcols, b = d_lo + (uint32_t)ys * (F::ybytes >> 4);
+                const int ys2 = ys + 1 == F::ystages ? 0 : ys + 1, ws2 = ws + 1 == F::wstages ? 0 : ws + 1;
+                const uint32_t yph2 = ys2 ? yph : yph ^ 1u, wph2 = ws2 ? wph : wph ^ 1u;
+                auto mma16 = [&](int j, uint32_t accumulate) {
+                    if constexpr (P) dx_mma16_pairs<NT>(d, w + 8 * j, b + 2 * j, d_hi, accumulate, leader);
+                    else dx_mma16<NT>(d, w + 8 * j, b + 2 * j, d_hi, accumulate, leader);
+                };
+                mma16(0, (uint32_t)(k - k0) > set);
+                mma16(1, 1u);
+                mma16(2, 1u);
+                // (the next stage's barriers are tested ahead of the last MMAs: their round trips run beside them)
+                ready = mbar_test(y_full + 8 * ys2, yph2) & mbar_test(w_full + 8 * ws2, wph2);
+                mma16(3, 1u);
+                umma_commit_if(w_free + 8 * ws, leader);
+                umma_commit_if(y_free + 8 * ys, leader);
+                any = true;
+                ys = ys2; ws = ws2; yph = yph2; wph = wph2;
+            }
+        };
+        if (s_wide) issue(std::false_type{});
+        else issue(std::true_type{});
         if (any) {
             umma_commit_if(acc_full, leader);
             if (!ok) {  // gave up: the tensor core must be idle before tensor memory is freed
@@ -442,87 +552,151 @@ dx_tmem_kernel(const DxParams p, const __grid_constant__ CUtensorMap map_w, cons
         // holds as element gid & 3 (eight lanes hold the same eight rows)
         const int my_row = half * 32 + (gid >> 2) * 16 + 2 * t + (gid & 1) + (gid & 2) * 4;
         const uint32_t soff = kDxCodes + my_row * 16 + blk * 4;
-        const uint32_t tdst = tmem + ACC + ((uint32_t)(blk * 32) << 16) + half * 16;
         const int64_t nb = p.in >> 5, b = (int64_t)ft * 4 + blk;
         asm volatile("griddepcontrol.wait;" ::: "memory");
-        float mx = 0.f;
+        float mx = 0.f, mn = __int_as_float(0x7F800000);
         if (b < nb)
-            for (int i = lane; i < kDxParts; i += 32) mx = fmaxf(mx, __ldg(p.colmax + i * nb + b));
+            for (int i = lane; i < kDxParts; i += 32) {
+                mx = fmaxf(mx, __ldg(p.colmax + i * nb + b));
+                mn = fminf(mn, __ldg(p.colmax + (kDxParts + i) * nb + b));
+            }
+        // a quarter of the tile's rows per (half, set): do pairs hold them all?
+        const int tok = tok0 + (warp >> 2) * (NT / 4) + lane;
+        const int row_wide = lane < NT / 4 && tok < p.m ? __ldg(p.rowexp + tok) & 1 : 0;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        for (int o = 16; o > 0; o >>= 1) {
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+            mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+        }
         float down, down2;   // the block's scales are used times 2^-ce, the largest in [2^12, 2^13)
         const int ce = dx_exponent(mx, 13, &down, &down2);
-        if (lane == 0) s_colexp[blk] = ce;   // (the four warps of a block of columns agree)
         const bool infinite = isinf(mx);   // a scale of this column block (of the whole matrix)
-        int ws = set % WS, rs = set;
-        uint32_t wph = 0, rph = 0;
-        for (int k = k0 + set; k < k1; k += 2) {
-            float sf = 0.f;
-            if (!p.tma_scales) {
-                const int64_t o = (int64_t)k * kDxStep + my_row;
-                if (o < p.out && b < nb) sf = __ldg(p.scales + o * nb + b);
-            }
-            ok = __all_sync(0xffffffffu, mbar_block(raw + 8 * rs, rph, abort_flag));
-            if (!ok) break;
-            const uint32_t st = rbase + rs * kDxRawBytes;
-            uint32_t w[2][4];
-#pragma unroll
-            for (int g = 0; g < 2; ++g) {
-                w[g][0] = lds_u32(st + off0 + g * 2048);
-                w[g][1] = lds_u32(st + off1 + g * 2048);
-                w[g][2] = lds_u32(st + off0 + g * 2048 + 1024);
-                w[g][3] = lds_u32(st + off1 + g * 2048 + 1024);
-            }
-            if (p.tma_scales) sf = __uint_as_float(lds_u32(st + soff));
-            // gather the eight scales the lane's rows need
-            sf *= down;
-            sf *= down2;
-            float sc[2][4];
-#pragma unroll
-            for (int g = 0; g < 2; ++g)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    sc[g][j] = __shfl_sync(0xffffffffu, sf, (g * 4 + j) * 4 + t);
-                    w[g][j] ^= 0x80808080u;   // code + 128
+        const bool any_wide = __any_sync(0xffffffffu, row_wide) || infinite || mn * down * down2 < kDxPairMin;
+        if (lane == 0) {
+            s_colexp[blk] = ce;   // (the four warps of a block of columns agree)
+            if (any_wide) s_wide = 1;
+        }
+        form_known();
+        wide = s_wide != 0;
+        // one stage after the other: body(codes, scales, where the stage's W' of this warp goes)
+        auto stages = [&](auto pairs, auto body) {
+            using F = DxForm<NT, decltype(pairs)::value>;
+            const uint32_t tdst = tmem + F::accs * NT + ((uint32_t)(blk * 32) << 16) + half * 16;
+            int ws = set % F::wstages, rs = set;
+            uint32_t wph = 0, rph = 0;
+            for (int k = k0 + set; k < k1; k += 2) {
+                float sf = 0.f;
+                if (!p.tma_scales) {
+                    const int64_t o = (int64_t)k * kDxStep + my_row;
+                    if (o < p.out && b < nb) sf = __ldg(p.scales + o * nb + b);
                 }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(taken + 8 * rs);
-            rs += 2;
-            if (rs >= kDxRaw) { rs -= kDxRaw; rph ^= 1u; }
-            ok = __all_sync(0xffffffffu, mbar_block(w_free + 8 * ws, wph ^ 1u, abort_flag));
-            if (!ok) break;
-            tc_fence_after();
-            auto convert = [&](auto inf) {
+                ok = __all_sync(0xffffffffu, mbar_block(raw + 8 * rs, rph, abort_flag));
+                if (!ok) break;
+                const uint32_t st = rbase + rs * kDxRawBytes;
+                uint32_t w[2][4];
 #pragma unroll
-                for (int q = 0; q < 2; ++q) {      // columns 4 gid + 2q, + 2q + 1
-                    uint32_t v1[8], v2[8], v3[8];
+                for (int g = 0; g < 2; ++g) {
+                    w[g][0] = lds_u32(st + off0 + g * 2048);
+                    w[g][1] = lds_u32(st + off1 + g * 2048);
+                    w[g][2] = lds_u32(st + off0 + g * 2048 + 1024);
+                    w[g][3] = lds_u32(st + off1 + g * 2048 + 1024);
+                }
+                if (p.tma_scales) sf = __uint_as_float(lds_u32(st + soff));
+                // gather the eight scales the lane's rows need: as f32, or as pairs of fp16 (the first term below)
+                sf *= down;
+                sf *= down2;
+                uint32_t own = __float_as_uint(sf);
+                if constexpr (decltype(pairs)::value) {
+                    const float first = __half2float(__float2half_rn(sf));
+                    own = pack_f16x2((sf - first) * kDxLow, first);
+                }
+                uint32_t sc[2][4];
 #pragma unroll
-                    for (int g = 0; g < 2; ++g)
+                for (int g = 0; g < 2; ++g)
 #pragma unroll
-                        for (int c = 0; c < 2; ++c)
+                    for (int j = 0; j < 4; ++j) {
+                        sc[g][j] = __shfl_sync(0xffffffffu, own, (g * 4 + j) * 4 + t);
+                        w[g][j] ^= 0x80808080u;   // code + 128
+                    }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(taken + 8 * rs);
+                rs += 2;
+                if (rs >= kDxRaw) { rs -= kDxRaw; rph ^= 1u; }
+                ok = __all_sync(0xffffffffu, mbar_block(w_free + 8 * ws, wph ^ 1u, abort_flag));
+                if (!ok) break;
+                tc_fence_after();
+                body(w, sc, tdst + ws * F::wcols);
+                tmem_st_wait();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(w_full + 8 * ws);
+                ws += 2;
+                if (ws >= F::wstages) { ws -= F::wstages; wph ^= 1u; }
+            }
+        };
+        // the code of column 4 gid + j, row h of group g: under the upper half of 2^23 the byte is 2^23 + 128 + code exactly
+        auto code = [](const uint32_t (&w)[2][4], int g, int h, int j) {
+            return __uint_as_float(__byte_perm(w[g][h], 0x4B000000u, 0x7440u | (uint32_t)j)) - 8388736.0f;
+        };
+        auto triples = [&](auto inf, const uint32_t (&w)[2][4], const uint32_t (&sc)[2][4], uint32_t dst) {
 #pragma unroll
-                            for (int h = 0; h < 2; ++h) {   // rows 2t + 8h, 2t + 8h + 1
-                                // under the upper half of 2^23 the byte is 2^23 + 128 + code exactly
-                                const uint32_t sel = 0x7440u | (uint32_t)(2 * q + c);
-                                const float a = __uint_as_float(__byte_perm(w[g][2 * h], 0x4B000000u, sel)) - 8388736.0f;
-                                const float b = __uint_as_float(__byte_perm(w[g][2 * h + 1], 0x4B000000u, sel)) - 8388736.0f;
+            for (int q = 0; q < 2; ++q, dst += 16u << 16) {      // columns 4 gid + 2q, + 2q + 1
+                uint32_t v1[8], v2[8], v3[8];
+#pragma unroll
+                for (int g = 0; g < 2; ++g)
+#pragma unroll
+                    for (int c = 0; c < 2; ++c)
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {   // rows 2t + 8h, 2t + 8h + 1
+                            const int e = g * 4 + c * 2 + h;
+                            dx_terms<decltype(inf)::value>(code(w, g, 2 * h + 1, 2 * q + c) * __uint_as_float(sc[g][2 * h + 1]),
+                                                           code(w, g, 2 * h, 2 * q + c) * __uint_as_float(sc[g][2 * h]), &v1[e],
+                                                           &v2[e], &v3[e]);
+                        }
+                tmem_st_16x256b_x2(dst, v1);
+                tmem_st_16x256b_x2(dst + 32, v2);
+                tmem_st_16x256b_x2(dst + 64, v3);
+            }
+        };
+        if (wide) {
+            stages(std::false_type{}, [&](const uint32_t (&w)[2][4], const uint32_t (&sc)[2][4], uint32_t dst) {
+                if (infinite) triples(std::true_type{}, w, sc, dst);
+                else triples(std::false_type{}, w, sc, dst);
+            });
+        } else {
+            down *= 1.0f / (1 << kDxPairExp);      // (no scale of such a block comes near f32's limits on the way)
+            stages(std::true_type{}, [&](const uint32_t (&w)[2][4], const uint32_t (&sc)[2][4], uint32_t dst) {
+                // Two rows at a time in packed fp16, scale = s1 + 2^-11 s2: H = code * s1 rounded, what the rounding left
+                // is exact (a multiple of s1's last place, at most 2^6 of them), L = 2^11 times that + code * s2 rounded
+                // once.  Seven instructions per two weights; from f32 products it was 14.
+                uint32_t v1[2][8], v2[2][8];
+#pragma unroll
+                for (int g = 0; g < 2; ++g)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {       // rows 2t + 8h, 2t + 8h + 1
+                        const uint32_t s1 = __byte_perm(sc[g][2 * h], sc[g][2 * h + 1], 0x5410);
+                        const uint32_t s2 = __byte_perm(sc[g][2 * h], sc[g][2 * h + 1], 0x7632);
+#pragma unroll
+                        for (int q = 0; q < 2; ++q) {   // columns 4 gid + 2q, + 2q + 1
+                            const uint32_t both = __byte_perm(w[g][2 * h], w[g][2 * h + 1], q ? 0x7362 : 0x5140);
+#pragma unroll
+                            for (int c = 0; c < 2; ++c) {
+                                // under the upper byte of 1024 the code + 128 is 1152 + code
+                                const uint32_t n = hadd2_u32(__byte_perm(both, 0x64u, c ? 0x4342 : 0x4140), 0xE480E480u);
+                                const uint32_t hi = hmul2_u32(n, s1);
+                                const uint32_t left = hfma2_u32(n, s1, hi ^ 0x80008000u);
                                 const int e = g * 4 + c * 2 + h;
-                                dx_terms<decltype(inf)::value>(b * sc[g][2 * h + 1], a * sc[g][2 * h], &v1[e], &v2[e], &v3[e]);
+                                v1[q][e] = hi;
+                                v2[q][e] = hfma2_u32(n, s2, hmul2_u32(left, 0x68006800u));
                             }
-                    const uint32_t dst = tdst + ws * kDxWCols + ((uint32_t)(16 * q) << 16);
-                    tmem_st_16x256b_x2(dst, v1);
-                    tmem_st_16x256b_x2(dst + 32, v2);
-                    tmem_st_16x256b_x2(dst + 64, v3);
+                        }
+                    }
+#pragma unroll
+                for (int q = 0; q < 2; ++q, dst += 16u << 16) {
+                    tmem_st_16x256b_x2(dst, v1[q]);
+                    tmem_st_16x256b_x2(dst + 32, v2[q]);
                 }
-            };
-            if (infinite) convert(std::true_type{});
-            else convert(std::false_type{});
-            tmem_st_wait();
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(w_full + 8 * ws);
-            ws += 2;
-            if (ws >= WS) { ws -= WS; wph ^= 1u; }
+            });
         }
         if (ok) ok = __all_sync(0xffffffffu, mbar_block(acc_full, 0, abort_flag));
         tc_fence_after();
@@ -542,21 +716,32 @@ dx_tmem_kernel(const DxParams p, const __grid_constant__ CUtensorMap map_w, cons
                 tmem_ld8(ta + NT + j, *reinterpret_cast<uint32_t(*)[8]>(&b[j]));
             }
             tmem_ld_wait();
-            if constexpr (dx_accs(NT) == 3) {
-                uint32_t c[CH];
+            if constexpr (NT <= 64) {
+                if (wide || k1 - k0 > 1) {   // triples: the third sum; pairs: the sums of the odd steps, if there are any
+                    uint32_t c[CH];
 #pragma unroll
-                for (int j = 0; j < CH; j += 8) tmem_ld8(ta + 2 * NT + j, *reinterpret_cast<uint32_t(*)[8]>(&c[j]));
-                tmem_ld_wait();
+                    for (int j = 0; j < CH; j += 8) tmem_ld8(ta + 2 * NT + j, *reinterpret_cast<uint32_t(*)[8]>(&c[j]));
+                    tmem_ld_wait();
+                    uint32_t (&to)[CH] = wide ? b : a;
 #pragma unroll
-                for (int j = 0; j < CH; ++j) b[j] = __float_as_uint(__uint_as_float(b[j]) + __uint_as_float(c[j]));
+                    for (int j = 0; j < CH; ++j) to[j] = __float_as_uint(__uint_as_float(to[j]) + __uint_as_float(c[j]));
+                    if (!wide) {
+#pragma unroll
+                        for (int j = 0; j < CH; j += 8) tmem_ld8(ta + 3 * NT + j, *reinterpret_cast<uint32_t(*)[8]>(&c[j]));
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int j = 0; j < CH; ++j) b[j] = __float_as_uint(__uint_as_float(b[j]) + __uint_as_float(c[j]));
+                    }
+                }
             }
+            const float low = wide ? 1.0f : 1.0f / kDxLow;
 #pragma unroll
             for (int j = 0; j < CH; ++j) {
-                const float v = __uint_as_float(a[j]) + __uint_as_float(b[j]);
+                const float v = fmaf(__uint_as_float(b[j]), low, __uint_as_float(a[j]));
                 const int tok = tok0 + col + j;
                 // (both exponents at once: one of them alone can take a finite result through infinity or zero)
                 if (p.split > 1) s_out[(col + j) * 128 + blk * 32 + 4 * (lane & 7) + (lane >> 3)] = v;
-                else if (tok < p.m && i_ok) p.dx[(int64_t)tok * p.in + i] = dx_scale(v, ce + __ldg(p.rowexp + tok));
+                else if (tok < p.m && i_ok) p.dx[(int64_t)tok * p.in + i] = dx_scale(v, ce + exp_of(tok));
             }
         }
     }
@@ -580,7 +765,7 @@ dx_tmem_kernel(const DxParams p, const __grid_constant__ CUtensorMap map_w, cons
                 }
                 const int64_t i = (int64_t)ft * 128 + c;
                 if (tok < p.m && i < p.in)
-                    p.dx[(int64_t)tok * p.in + i] = dx_scale(v, s_colexp[c >> 5] + __ldg(p.rowexp + tok));
+                    p.dx[(int64_t)tok * p.in + i] = dx_scale(v, s_colexp[c >> 5] + exp_of(tok));
             }
         }
         __syncwarp();
@@ -611,7 +796,7 @@ int32_t dx_configure() {
 
 template <int NT>
 static cudaError_t dx_launch(const DeviceState& ds, const DxParams& p, int tiles, const CUtensorMap& w, const CUtensorMap& y,
-                             const CUtensorMap& s) {
+                             const CUtensorMap& y16, const CUtensorMap& s) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(tiles * p.split));
     cfg.blockDim = dim3(kDxThreads);
@@ -632,7 +817,7 @@ static cudaError_t dx_launch(const DeviceState& ds, const DxParams& p, int tiles
     }
     cfg.attrs = a;
     cfg.numAttrs = (unsigned)n;
-    return cudaLaunchKernelEx(&cfg, dx_tmem_kernel<NT>, p, w, y, s);
+    return cudaLaunchKernelEx(&cfg, dx_tmem_kernel<NT>, p, w, y, y16, s);
 }
 
 int32_t launch_qlinear_q8_dx(rstq_ctx* ctx, DeviceState& ds, const float* dy, const int8_t* codes,
@@ -651,28 +836,31 @@ int32_t launch_qlinear_q8_dx(rstq_ctx* ctx, DeviceState& ds, const float* dy, co
     int split = 1;
     while (split < 8 && tiles * split * 2 <= ds.sm_count && steps >= 16 * split) split *= 2;
 
-    const int64_t yb = (3 * m * opad * 2 + 255) & ~255ll, rb = (m * 4 + 255) & ~255ll, cb = kDxParts * nb * 4;
-    int32_t rc = dx_reserve(ds, yb + rb + cb);
+    const int64_t yb = (3 * m * opad * 2 + 255) & ~255ll, hb = (2 * m * opad * 2 + 255) & ~255ll, rb = (m * 4 + 255) & ~255ll;
+    const int64_t cb = 2 * kDxParts * nb * 4;
+    int32_t rc = dx_reserve(ds, yb + hb + rb + cb);
     if (rc != RSTQ_OK) return rc;
     char* base = (char*)ds.dx_scratch;
-    DxPrep q{dy, scales, (uint16_t*)base, (int*)(base + yb), (float*)(base + yb + rb), m, out, nb, opad};
-    CUtensorMap mw, my, ms;
+    DxPrep q{dy, scales, (uint16_t*)base, (uint16_t*)(base + yb), (int*)(base + yb + hb), (float*)(base + yb + hb + rb), m, out, nb, opad};
+    CUtensorMap mw, my, mh, ms;
     const bool tma_scales = nb % 4 == 0;   // rows of whole 16 bytes
     const cuuint64_t i_ = (cuuint64_t)in, o_ = (cuuint64_t)out, m_ = (cuuint64_t)m, op_ = (cuuint64_t)opad, nb_ = (cuuint64_t)nb;
     RSTQ_REQUIRE(dx_map(enc, &mw, CU_TENSOR_MAP_DATA_TYPE_UINT8, codes, 2, {i_, o_, 1}, {i_, 0}, {128, kDxStep, 1}) &&
                      dx_map(enc, &my, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, q.y, 3, {op_, m_, 3}, {op_ * 2, op_ * m_ * 2},
                             {kDxStep, (cuuint32_t)nt, 3}) &&
+                     dx_map(enc, &mh, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, q.y16, 3, {op_, m_, 2}, {op_ * 2, op_ * m_ * 2},
+                            {kDxStep, (cuuint32_t)nt, 2}) &&
                      (!tma_scales || dx_map(enc, &ms, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, scales, 2, {nb_, o_, 1}, {nb_ * 4, 0},
                                             {4, kDxStep, 1}, false)),
                  RSTQ_E_CUDA, "cuTensorMapEncodeTiled failed (m = %lld, in = %lld, out = %lld)", (long long)m, (long long)in,
                  (long long)out);
     if (!tma_scales) ms = mw;   // not used then
-    RSTQ_CUDA(launch_pdl(dx_prep_kernel, dim3((unsigned)(m + kDxParts)), dim3(256), 0, ds, q));
+    RSTQ_CUDA(launch_pdl(dx_prep_kernel, dim3((unsigned)(m + kDxParts)), dim3(opad > 4096 ? kDxPrepMax : 256), 0, ds, q));
     ctx->launches++;
     DxParams p{scales, q.rowexp, q.colmax, dx, ds.status, in, out, tma_scales, (int)m, (int)steps, (int)ttiles, split};
-    RSTQ_CUDA(nt == 32   ? dx_launch<32>(ds, p, (int)tiles, mw, my, ms)
-              : nt == 64 ? dx_launch<64>(ds, p, (int)tiles, mw, my, ms)
-                         : dx_launch<128>(ds, p, (int)tiles, mw, my, ms));
+    RSTQ_CUDA(nt == 32   ? dx_launch<32>(ds, p, (int)tiles, mw, my, mh, ms)
+              : nt == 64 ? dx_launch<64>(ds, p, (int)tiles, mw, my, mh, ms)
+                         : dx_launch<128>(ds, p, (int)tiles, mw, my, mh, ms));
     ctx->launches++;
     return RSTQ_OK;
 }

@@ -131,3 +131,26 @@ def test_dx_recorded_without_a_first_call(ctx):
     g.destroy()
     for b in bufs:
         b.free()
+
+
+@pytest.mark.parametrize("m,in_,out", [(5, 96, 64), (40, 160, 128), (64, 256, 200), (300, 256, 320)])   # one step, even and odd steps
+@pytest.mark.parametrize("what,below", [("dy", 26), ("dy", 27), ("dy", 28), ("scales", 19), ("scales", 20), ("scales", 21)])
+def test_dx_pairs_and_triples_on_both_sides_of_the_line(ctx, what, below, m, in_, out):
+    """Rows whose smallest element, blocks whose smallest scale lies about where pairs of fp16 stop holding it whole, in
+    one token tile beside tiles of plain rows; the small ones alone decide some of the results."""
+    rng = np.random.default_rng(below + m)
+    dy = (rng.uniform(0.5, 1, (m, out)) * rng.choice([-1, 1], (m, out))).astype(np.float32)
+    scales = rng.uniform(0.5, 1, (out, in_ // 32)).astype(np.float32)
+    codes = rng.integers(-128, 128, (out, in_)).astype(np.int8)
+    if what == "dy":
+        dy[m // 2, 1:] *= np.float32(2.0 ** -below)
+        codes[0, ::3] = 0
+    else:
+        scales[1:, -1] *= np.float32(2.0 ** -below)
+        dy[::4, 0] = 0
+    dx = run(ctx, m, in_, out, dy.ravel(), codes.ravel(), scales.ravel())
+    w = codes.astype(np.float64) * np.repeat(scales.astype(np.float64), 32, axis=1)
+    d = dy.astype(np.float64)
+    # A product of pairs: 6 * 2^-24 for the weight (second term up to 1.5 times the first's half step, its rounding and
+    # that of the second term of the scale), 2 * 2^-24 for dy, 6 * 2^-24 for the product of the second terms, left out.
+    assert np.all(np.abs(dx - d @ w) <= (14 * 2.0 ** -24 + (out / 8 + 12) * 2.0 ** -23) * (np.abs(d) @ np.abs(w)))
