@@ -119,7 +119,8 @@ typedef struct rstq_event rstq_event;
                                      thread) instead of 128-token ones: 0 (default) = where the grid then needs
                                      fewer cycles over its waves of thread blocks, 1 = never, 2 = always,
                                      3 = as 0 but never several thread blocks per tile, 4 = as 0 but always equal
-                                     ranges of the K-steps of all tiles, on every SM */
+                                     ranges of the K-steps of all tiles, on every SM; 5, 6 = as 2, 4 with 256-token
+                                     tiles always on pairs of SMs (0: where there is enough work for every SM) */
 #define RSTQ_TUNE_TP_TAIL 15      /* fused decode + exchange (rstq_tp_qmatmul): how many thread blocks of the decode kernel
                                      stay for the exchange's tail (wait for the peers' results, write y); the others
                                      leave their SMs to the next launch, which fills its weight rings meanwhile.

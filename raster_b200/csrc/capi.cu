@@ -734,7 +734,7 @@ int32_t rstq_tune(rstq_ctx* ctx, int32_t key, int64_t value) {
             ctx->tune_q6k_units = value != 0;
             return RSTQ_OK;
         case RSTQ_TUNE_GEMM_WIDE:
-            RSTQ_REQUIRE(value >= 0 && value <= 4, RSTQ_E_INVALID, "256-token tile selector 0..4");
+            RSTQ_REQUIRE(value >= 0 && value <= 6, RSTQ_E_INVALID, "256-token tile selector 0..6");
             ctx->tune_gemm_wide = value;
             return RSTQ_OK;
         case RSTQ_TUNE_ACT_IMAGE:

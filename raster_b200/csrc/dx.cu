@@ -322,10 +322,6 @@ __device__ __noinline__ void dx_drain(uint32_t bars, int issued, int ring) {
         }
     }
 }
-__device__ __forceinline__ void cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 
 // The MMAs of 16 rows o, triples.  The three terms of dy lie one above the other in shared memory, so a term of W' times several
 // of them is one instruction as far as the width allows (256): a tcgen05 instruction costs its issuer 50 - 60

@@ -28,6 +28,7 @@
 // Every mbarrier wait is time-bounded; on expiry the CTA reports through the
 // status word, drains and still frees its tensor memory.
 
+#include <algorithm>
 #include <type_traits>
 
 #include "internal.h"
@@ -488,11 +489,18 @@ constexpr int kGemmThreadsT = (3 + kDqWarps) * 32;  // TMA warp, MMA warp (even 
 // accumulators, at most 4: with exactly four the dequant warps run their two-set schedule, which
 // measured faster than six stages on the one-set schedule where six would fit (M <= 64: 76 -> 68 us
 // at M = 16 on 28672 x 8192)
-__host__ __device__ constexpr int gemm_stages(int ntok) { return ntok > 128 ? 3 : ((512 - 2 * ntok) / 64 > 4 ? 4 : (512 - 2 * ntok) / 64); }
+__host__ __device__ constexpr int gemm_stages(int ntok, bool duo) { return ntok > 128 && !duo ? 3 : 4; }
 // A 256-token tile has one accumulator (256 columns) and one issuing thread: an MMA then takes the
 // tensor core 128 cycles, more than its issue costs; its activation stage is 64 KB, so three stages.
 __host__ __device__ constexpr int gemm_issuers(int ntok) { return ntok > 128 ? 1 : 2; }
 constexpr int kAColsPerStage = kKStep / 2;
+constexpr int kEpiLd = 36;   // floats per token row of the epilogue's staging tiles (16-byte aligned rows)
+// bytes of activations per stage and CTA: a pair of CTAs shares a tile's tokens
+__host__ __device__ constexpr int gemm_bstage(int ntok, bool duo) { return ntok * kKStep * 2 / (duo ? 2 : 1); }
+__host__ __device__ constexpr int gemm_smem(int ntok, bool duo) {
+    const int ring = gemm_stages(ntok, duo) * gemm_bstage(ntok, duo), epi = kDqWarps * (ntok / 4 < 32 ? ntok / 4 : 32) * kEpiLd * 4;
+    return (ring > epi ? ring : epi) + 1024;
+}
 constexpr int kWeightPfSteps = 8;  // K-steps of packed weights requested into L2 ahead of the loads
 
 // One 128-element K-step as a single block of instructions, so that nothing but a branch sits
@@ -501,43 +509,78 @@ constexpr int kWeightPfSteps = 8;  // K-steps of packed weights requested into L
 // of the stage), with a non-blocking test of the NEXT stage's barrier tucked in between them, where the
 // issuing lane is waiting for the tensor core anyway; its answer is read at the end.  first = 0
 // makes MMA 0 overwrite the accumulator; lanes with leader = 0 issue no tensor-core instruction.
-template <int BHALF>
+template <int BHALF, bool DUO>
 __device__ __forceinline__ uint32_t umma_f16_ts_step(uint32_t d_tmem, uint32_t a0, uint32_t b_lo, uint32_t b_hi,
                                                      uint32_t idesc, uint32_t first, uint32_t leader,
                                                      uint32_t next_full, uint32_t next_parity) {
     uint32_t next_ready;
-    asm volatile(
-        "{\n"
-        ".reg .pred p, q, t, r;\n"
-        ".reg .b64 bd0, bd1, bd2, bd3, bd4, bd5, bd6, bd7;\n"
-        ".reg .b32 a1, a2, a3, a4, a5, a6, a7, b;\n"
-        "setp.ne.b32 p, %6, 0;\n"
-        "setp.ne.b32 q, %7, 0;\n"
-        "setp.eq.b32 t, 0, 0;\n"
-        "mov.b64 bd0, {%3, %4};\n"
-        "add.u32 a1, %2, 8;  add.u32 b, %3, 2;   mov.b64 bd1, {b, %4};\n"
-        "add.u32 a2, %2, 16; add.u32 b, %3, 4;   mov.b64 bd2, {b, %4};\n"
-        "add.u32 a3, %2, 24; add.u32 b, %3, 6;   mov.b64 bd3, {b, %4};\n"
-        "add.u32 a4, %2, 32; add.u32 b, %3, %8;  mov.b64 bd4, {b, %4};\n"
-        "add.u32 a5, %2, 40; add.u32 b, %3, %9;  mov.b64 bd5, {b, %4};\n"
-        "add.u32 a6, %2, 48; add.u32 b, %3, %10; mov.b64 bd6, {b, %4};\n"
-        "add.u32 a7, %2, 56; add.u32 b, %3, %11; mov.b64 bd7, {b, %4};\n"
-        "tcgen05.fence::after_thread_sync;\n"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%1], [%2], bd0, %5, p;\n"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%1], [a1], bd1, %5, t;\n"
-        "mbarrier.test_wait.parity.shared::cta.b64 r, [%12], %13;\n"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%1], [a2], bd2, %5, t;\n"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%1], [a3], bd3, %5, t;\n"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%1], [a4], bd4, %5, t;\n"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%1], [a5], bd5, %5, t;\n"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%1], [a6], bd6, %5, t;\n"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%1], [a7], bd7, %5, t;\n"
-        "selp.u32 %0, 1, 0, r;\n"
-        "}"
-        : "=r"(next_ready)
-        : "r"(d_tmem), "r"(a0), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(first), "r"(leader), "n"(BHALF),
-          "n"(BHALF + 2), "n"(BHALF + 4), "n"(BHALF + 6), "r"(next_full), "r"(next_parity)
-        : "memory");
+    if constexpr (DUO) {   // the pair's barrier, which the other CTA arrives on as well
+        asm volatile(
+            "{\n"
+            ".reg .pred p, q, t, r;\n"
+            ".reg .b64 bd0, bd1, bd2, bd3, bd4, bd5, bd6, bd7;\n"
+            ".reg .b32 a1, a2, a3, a4, a5, a6, a7, b;\n"
+            "setp.ne.b32 p, %6, 0;\n"
+            "setp.ne.b32 q, %7, 0;\n"
+            "setp.eq.b32 t, 0, 0;\n"
+            "mov.b64 bd0, {%3, %4};\n"
+            "add.u32 a1, %2, 8;  add.u32 b, %3, 2;   mov.b64 bd1, {b, %4};\n"
+            "add.u32 a2, %2, 16; add.u32 b, %3, 4;   mov.b64 bd2, {b, %4};\n"
+            "add.u32 a3, %2, 24; add.u32 b, %3, 6;   mov.b64 bd3, {b, %4};\n"
+            "add.u32 a4, %2, 32; add.u32 b, %3, %8;  mov.b64 bd4, {b, %4};\n"
+            "add.u32 a5, %2, 40; add.u32 b, %3, %9;  mov.b64 bd5, {b, %4};\n"
+            "add.u32 a6, %2, 48; add.u32 b, %3, %10; mov.b64 bd6, {b, %4};\n"
+            "add.u32 a7, %2, 56; add.u32 b, %3, %11; mov.b64 bd7, {b, %4};\n"
+            "tcgen05.fence::after_thread_sync;\n"
+            "@q tcgen05.mma.cta_group::2.kind::f16 [%1], [%2], bd0, %5, p;\n"
+            "@q tcgen05.mma.cta_group::2.kind::f16 [%1], [a1], bd1, %5, t;\n"
+            "mbarrier.test_wait.parity.shared::cta.b64 r, [%12], %13;\n"
+            "@q tcgen05.mma.cta_group::2.kind::f16 [%1], [a2], bd2, %5, t;\n"
+            "@q tcgen05.mma.cta_group::2.kind::f16 [%1], [a3], bd3, %5, t;\n"
+            "@q tcgen05.mma.cta_group::2.kind::f16 [%1], [a4], bd4, %5, t;\n"
+            "@q tcgen05.mma.cta_group::2.kind::f16 [%1], [a5], bd5, %5, t;\n"
+            "@q tcgen05.mma.cta_group::2.kind::f16 [%1], [a6], bd6, %5, t;\n"
+            "@q tcgen05.mma.cta_group::2.kind::f16 [%1], [a7], bd7, %5, t;\n"
+            "selp.u32 %0, 1, 0, r;\n"
+            "}"
+            : "=r"(next_ready)
+            : "r"(d_tmem), "r"(a0), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(first), "r"(leader), "n"(BHALF),
+              "n"(BHALF + 2), "n"(BHALF + 4), "n"(BHALF + 6), "r"(next_full), "r"(next_parity)
+            : "memory");
+    } else {
+        asm volatile(
+            "{\n"
+            ".reg .pred p, q, t, r;\n"
+            ".reg .b64 bd0, bd1, bd2, bd3, bd4, bd5, bd6, bd7;\n"
+            ".reg .b32 a1, a2, a3, a4, a5, a6, a7, b;\n"
+            "setp.ne.b32 p, %6, 0;\n"
+            "setp.ne.b32 q, %7, 0;\n"
+            "setp.eq.b32 t, 0, 0;\n"
+            "mov.b64 bd0, {%3, %4};\n"
+            "add.u32 a1, %2, 8;  add.u32 b, %3, 2;   mov.b64 bd1, {b, %4};\n"
+            "add.u32 a2, %2, 16; add.u32 b, %3, 4;   mov.b64 bd2, {b, %4};\n"
+            "add.u32 a3, %2, 24; add.u32 b, %3, 6;   mov.b64 bd3, {b, %4};\n"
+            "add.u32 a4, %2, 32; add.u32 b, %3, %8;  mov.b64 bd4, {b, %4};\n"
+            "add.u32 a5, %2, 40; add.u32 b, %3, %9;  mov.b64 bd5, {b, %4};\n"
+            "add.u32 a6, %2, 48; add.u32 b, %3, %10; mov.b64 bd6, {b, %4};\n"
+            "add.u32 a7, %2, 56; add.u32 b, %3, %11; mov.b64 bd7, {b, %4};\n"
+            "tcgen05.fence::after_thread_sync;\n"
+            "@q tcgen05.mma.cta_group::1.kind::f16 [%1], [%2], bd0, %5, p;\n"
+            "@q tcgen05.mma.cta_group::1.kind::f16 [%1], [a1], bd1, %5, t;\n"
+            "mbarrier.test_wait.parity.shared::cta.b64 r, [%12], %13;\n"
+            "@q tcgen05.mma.cta_group::1.kind::f16 [%1], [a2], bd2, %5, t;\n"
+            "@q tcgen05.mma.cta_group::1.kind::f16 [%1], [a3], bd3, %5, t;\n"
+            "@q tcgen05.mma.cta_group::1.kind::f16 [%1], [a4], bd4, %5, t;\n"
+            "@q tcgen05.mma.cta_group::1.kind::f16 [%1], [a5], bd5, %5, t;\n"
+            "@q tcgen05.mma.cta_group::1.kind::f16 [%1], [a6], bd6, %5, t;\n"
+            "@q tcgen05.mma.cta_group::1.kind::f16 [%1], [a7], bd7, %5, t;\n"
+            "selp.u32 %0, 1, 0, r;\n"
+            "}"
+            : "=r"(next_ready)
+            : "r"(d_tmem), "r"(a0), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(first), "r"(leader), "n"(BHALF),
+              "n"(BHALF + 2), "n"(BHALF + 4), "n"(BHALF + 6), "r"(next_full), "r"(next_parity)
+            : "memory");
+    }
     return next_ready;
 }
 template <int BITS>
@@ -564,18 +607,26 @@ __device__ __forceinline__ int64_t gemm_range_start(const GemmParams& p, int64_t
 // 22.0 us); with what is left of the bookkeeping (ring positions, segment lengths, a division per role) as constants
 // there, int8 4096 x 4096 takes 24.42 us at M = 512 (24.58 without, 24.38 before there were segments), 18.6 at
 // M = 256 (18.8).
-template <int BITS, int NTOK, bool SEGS>
+// DUO: a pair of CTAs (a cluster of two) works on a tile of 256 features x 256 tokens with MMAs of cta_group::2: each CTA
+// dequantizes its 128 features into its own tensor memory and brings half of the tokens into its shared memory, one thread
+// of the first issues for both.  Half the activation bytes per SM, half the MMA instructions, and four stages fit instead of
+// three: K-step 1110 -> 1030 cycles with all SMs busy (the tensor core's own time is 1024).  The second CTA keeps barriers of its own;
+// its warp 1 passes every full stage on to the first CTA's barrier (an arrival with cluster scope instead of the default one
+// takes 180 cycles per step: a fence; what it would order, TMA bytes and tensor memory, other instructions order already).
+template <int BITS, int NTOK, bool SEGS, bool DUO>
 __global__ void __launch_bounds__(kGemmThreadsT, 1)
 gemm_tmem_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tmap) {
     constexpr int UNIT = BITS == 4 ? kUnitBytesQ4 : kUnitBytesQ8;
     constexpr int CODES = BITS == 4 ? kUnitCodesQ4 : kUnitCodesQ8;
-    constexpr int BSTAGE = NTOK * kKStep * 2;
-    constexpr int kNSTT = gemm_stages(NTOK);
+    constexpr int BSTAGE = gemm_bstage(NTOK, DUO);
+    constexpr int kNSTT = gemm_stages(NTOK, DUO);
+    constexpr int CS = DUO ? 2 : 1, BROWS = NTOK / CS;        // CTAs of a tile; its tokens in this CTA's shared memory
     constexpr int ISS = gemm_issuers(NTOK);
     constexpr uint32_t TMEM_COLS = 512;                       // ISS accumulators (NTOK columns each) + A ring, power of two
     constexpr uint32_t A_COL0 = ISS * NTOK;                   // A ring starts after the accumulators
     static_assert(ISS * NTOK + kNSTT * kAColsPerStage <= 512 && kNSTT >= 3,
                   "tensor memory holds the accumulators and the A ring");
+    static_assert(!DUO || ISS == 1, "the second CTA of a pair has one warp that passes its stages on");
     extern __shared__ uint8_t smem_raw[];
     if (p.dbg && blockIdx.x == 0 && threadIdx.x == 64) { p.dbg[300] = (unsigned long long)clock64(); p.dbg[304] = gtime_ns(); }
     __shared__ int s_abort;
@@ -593,7 +644,9 @@ gemm_tmem_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tmap) {
     // This CTA's range of the step sequence.  It is worked off in segments, one per tile it touches; step q of the
     // range (counted over all segments) uses ring stage q mod kNSTT.  Where tiles are shared the ranges are dealt out
     // from the back: a CTA then waits only for CTAs launched before it.
-    const int KS = p.ksteps, cta = SEGS || p.half > 0 ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x;
+    const int KS = p.ksteps, units = (int)gridDim.x / CS, unit = (int)blockIdx.x / CS;
+    const int cta = SEGS || p.half > 0 ? units - 1 - unit : unit;   // (DUO: the pair's number)
+    const uint32_t rank = DUO ? blockIdx.x & 1 : 0;                 // (its place in the cluster: clusters are two neighbours)
     int tile_first, k_first, steps_own;   // first tile, first step in it, number of steps
     if (p.half > 0) {
         tile_first = cta >> 1;
@@ -609,7 +662,7 @@ gemm_tmem_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tmap) {
         k_first = (int)(r0 - (uint32_t)tile_first * KS);
         steps_own = (int)((uint32_t)gemm_range_start(p, cta + 1) - r0);
     }
-    const int ft_first = tile_first / p.ttiles, tok_first = (tile_first - ft_first * p.ttiles) * NTOK;
+    const int fd = tile_first / p.ttiles, ft_first = fd * CS + (int)rank, tok_first = (tile_first - fd * p.ttiles) * NTOK;
 
     if (tid == 0) asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmap)) : "memory");
     if (warp >= 2 && warp < 2 + kDqWarps) {
@@ -626,7 +679,7 @@ gemm_tmem_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tmap) {
         }
     }
     if (tid < kNSTT) {
-        mbar_init(full + 8 * tid, kDqWarps / 2 + 1);
+        mbar_init(full + 8 * tid, kDqWarps / 2 + 1 + (DUO && rank == 0 ? 1 : 0));   // (+ 1: the other CTA's stage, passed on)
         mbar_init(empty + 8 * tid, 1);
     } else if (tid == kNSTT) {
         mbar_init(acc_full, ISS == 2 && (SEGS || steps_own >= 2) ? 2 : 1);   // one arrival per MMA issuer (that has steps) and segment
@@ -635,12 +688,19 @@ gemm_tmem_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tmap) {
     }
     if (tid <= kNSTT) asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     if (warp == 1) {
-        tmem_alloc(smem_u32(&s_tmem), TMEM_COLS);
-        tmem_relinquish();
+        if constexpr (DUO) {
+            tmem_alloc2(smem_u32(&s_tmem), TMEM_COLS);
+            tmem_relinquish2();
+        } else {
+            tmem_alloc(smem_u32(&s_tmem), TMEM_COLS);
+            tmem_relinquish();
+        }
     }
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     tc_fence_before();
     __syncthreads();
+    // (the other CTA's barriers: only the warps that arrive on them wait for it here, the others at the end)
+    if constexpr (DUO) cluster_arrive();
     tc_fence_after();
     const uint32_t tmem = s_tmem;
     unsigned long long* dbg = (p.dbg && blockIdx.x == 0) ? p.dbg : nullptr;
@@ -692,17 +752,23 @@ gemm_tmem_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tmap) {
                     if (!ok) break;
                     const uint32_t dst = sbase + s * BSTAGE;
                     mbar_expect_tx(full + 8 * s, BSTAGE);
-                    tma_load_2d(dst, &tmap, (k0 + ks) * kKStep, tok0, full + 8 * s);
-                    tma_load_2d(dst + NTOK * 128, &tmap, (k0 + ks) * kKStep + 64, tok0, full + 8 * s);
+                    tma_load_2d(dst, &tmap, (k0 + ks) * kKStep, tok0 + (int)rank * BROWS, full + 8 * s);
+                    tma_load_2d(dst + BROWS * 128, &tmap, (k0 + ks) * kKStep + 64, tok0 + (int)rank * BROWS, full + 8 * s);
                     ++issued;
                     if (++s == kNSTT) { s = 0; ph ^= 1u; }
                 }
                 if (!SEGS || (left -= n) == 0) break;
                 ++seg;
                 ++tile;
-                ft = tile / p.ttiles;
-                tok0 = (tile - ft * p.ttiles) * NTOK;
+                const int fd2 = tile / p.ttiles;
+                ft = fd2 * CS + (int)rank;
+                tok0 = (tile - fd2 * p.ttiles) * NTOK;
             }
+            if constexpr (DUO)   // the last arrivals from the pair's MMAs: none may find this CTA's shared memory gone
+                for (int i = 0; i < kNSTT && ok; ++i) {   // (stages never used pass at once)
+                    ok = mbar_block(empty + 8 * s, ph ^ 1u, abort_flag);
+                    if (++s == kNSTT) { s = 0; ph ^= 1u; }
+                }
             if (!ok) {  // let the copies already issued land before this CTA's shared memory goes away
                 for (int k = issued > kNSTT ? issued - kNSTT : 0; k < issued; ++k) {
                     const unsigned long long t0 = gtime_ns();
@@ -711,6 +777,27 @@ gemm_tmem_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tmap) {
                     }
                 }
             }
+        }
+    } else if (DUO && rank == 1 && warp == 1) {
+        // ---------------- the second CTA of a pair: its stages, passed on to the issuer ----------------
+        // (A further segment's first stage goes on only after this CTA's epilogue is done with the accumulators.)
+        bool ok = true;
+        int q = 0, seg = 0, left = steps_own;
+        cluster_wait();
+        for (int k0 = k_first; ok; k0 = 0) {
+            const int n = SEGS ? min(KS - k0, left) : steps_own;
+            if (SEGS && seg > 0) ok = __all_sync(0xffffffffu, mbar_spin(acc_free, (uint32_t)(seg - 1) & 1u, abort_flag));
+            for (int ks = 0; ks < n && ok; ++ks, ++q) {
+                const uint32_t bar = full + 8 * (q % kNSTT);
+                ok = __all_sync(0xffffffffu, mbar_spin(bar, (uint32_t)(q / kNSTT) & 1u, abort_flag));
+                if (!ok) break;
+                tc_fence_after();
+                tc_fence_before();
+                if (lane == 0) mbar_arrive_at(bar, 0);
+                __syncwarp();
+            }
+            if (!SEGS || (left -= n) == 0) break;
+            ++seg;
         }
     } else if (warp == 1 || (ISS == 2 && warp == 2 + kDqWarps)) {
         // ---------------- MMA issuers ----------------
@@ -723,12 +810,17 @@ gemm_tmem_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tmap) {
         // The whole warp runs the loop with identical values (the address arithmetic stays
         // warp-uniform) and lane 0 alone issues the tensor-core instructions.
         const int m = warp == 1 ? 0 : 1;
-        constexpr uint32_t idesc = idesc_f16(NTOK);
         const uint32_t leader = lane == 0;
+        constexpr uint32_t idesc = DUO ? idesc_f16_pair(NTOK) : idesc_f16(NTOK);
+        auto commit = [&](uint32_t bar) {
+            if constexpr (DUO) umma_commit2_if(bar, leader);
+            else umma_commit_if(bar, leader);
+        };
         const uint64_t d0 = smem_desc_sw128(sbase);
         const uint32_t d_lo = (uint32_t)d0, d_hi = (uint32_t)(d0 >> 32);
         const uint32_t dcol = tmem + (uint32_t)(m * NTOK);
         static_assert(kKStep == 128, "eight MMAs per step");
+        if constexpr (DUO) cluster_wait();
         bool any = false, ok = true;
         int q0 = 0, seg = 0, left = steps_own;
         for (int k0 = k_first; ok; k0 = 0) {
@@ -745,16 +837,16 @@ gemm_tmem_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tmap) {
                 if (s2 >= kNSTT) { s2 -= kNSTT; ph2 ^= 1u; }
                 const uint32_t a0 = tmem + A_COL0 + s * kAColsPerStage, b_lo = d_lo + (uint32_t)s * (BSTAGE >> 4);
                 // the block also tests the barrier of this issuer's next step (ks + ISS) early
-                const uint32_t n2 = umma_f16_ts_step<NTOK * 8>(dcol, a0, b_lo, d_hi, idesc, ks != first, leader, full + 8 * s2,
+                const uint32_t n2 = umma_f16_ts_step<BROWS * 8, DUO>(dcol, a0, b_lo, d_hi, idesc, ks != first, leader, full + 8 * s2,
                                                                ph2);
-                umma_commit_if(empty + 8 * s, leader);  // the stage is free once these MMAs have read it
+                commit(empty + 8 * s);  // the stage is free once these MMAs have read it
                 any = true;
                 if (ks + ISS < n && !n2) ok = mbar_spin(full + 8 * s2, ph2, abort_flag);
                 s = s2;
                 ph = ph2;
             }
             if (dbg && lane == 0) dbg[307 + 2 * m] = (unsigned long long)clock64();
-            if (any || (SEGS && ok)) umma_commit_if(acc_full, leader);   // (arrives at once where this issuer had no step)
+            if (any || (SEGS && ok)) commit(acc_full);   // (arrives at once where this issuer had no step)
             if (!ok && any) {  // gave up: the tensor core must be idle before tensor memory is freed
                 const unsigned long long t0 = gtime_ns();
                 while (!mbar_try(acc_full, (uint32_t)seg & 1u) && gtime_ns() - t0 < kWaitLimitNs) {
@@ -922,9 +1014,10 @@ gemm_tmem_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tmap) {
         int takes = 0;   // CTAs behind this one with steps of this tile
         if (!SEGS) takes = p.half > 0 && !giver;
         else if (!giver && n < KS)
-            while (cta + 1 + takes < (int)gridDim.x && gemm_range_start(p, cta + 1 + takes) < (int64_t)(tile + 1) * KS) ++takes;
+            while (cta + 1 + takes < units && gemm_range_start(p, cta + 1 + takes) < (int64_t)(tile + 1) * KS) ++takes;
         constexpr size_t kPart = (size_t)kDqWarps * CPW * 32;   // floats per CTA
-        float* part = p.part + cta * kPart + (size_t)dq * (CPW * 32);
+        const int slot = cta * CS + (int)rank;        // of this CTA's sums and flag
+        float* part = p.part + slot * kPart + (size_t)dq * (CPW * 32);
         if (ok && takes > 0) {
             int got = 1;
             if (lane == 0) {
@@ -932,7 +1025,7 @@ gemm_tmem_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tmap) {
                 for (int k = 1; k <= (SEGS ? takes : 1) && got; ++k) {
                     for (;;) {
                         int v;
-                        asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p.part_flags + cta + k) : "memory");
+                        asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p.part_flags + slot + k * CS) : "memory");
                         if (v != 0) break;
                         if (*abort_flag || gtime_ns() - t0 > kWaitLimitNs) {
                             *abort_flag = 1;
@@ -950,7 +1043,7 @@ gemm_tmem_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tmap) {
             const int sp = warp & 3;          // tensor-memory lanes 32*sp .. 32*sp + 31
             const int64_t f = (int64_t)ft * 128 + sp * 32 + lane;
             const float wdiv = p.wdiv;
-            constexpr int LD = 36;  // floats per token row of the staging tile (16-byte aligned rows)
+            constexpr int LD = kEpiLd;
             float* tile_s = reinterpret_cast<float*>(smem) + dq * (CH * LD);
 #pragma unroll
             for (int h = 0; h < NCH; ++h) {
@@ -978,7 +1071,7 @@ gemm_tmem_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tmap) {
                     continue;
                 }
                 for (int k = 1; k <= (SEGS ? takes : (takes > 0 ? 1 : 0)); ++k) {
-                    const float* from = part + k * kPart + (h * CH) * 32 + lane;
+                    const float* from = part + k * CS * kPart + (h * CH) * 32 + lane;
 #pragma unroll
                     for (int j = 0; j < CH; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) + __ldcg(from + j * 32));
                 }
@@ -1035,16 +1128,17 @@ gemm_tmem_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tmap) {
             asm volatile("bar.sync 6, %0;" ::"r"(kDqWarps * 32) : "memory");
             if (dq == 0 && lane == 0) {
                 if (!giver)
-                    for (int k = 1; k <= (SEGS ? takes : 1); ++k) p.part_flags[cta + k] = 0;
-                else if (ok) asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(p.part_flags + cta), "r"(1) : "memory");
+                    for (int k = 1; k <= (SEGS ? takes : 1); ++k) p.part_flags[slot + k * CS] = 0;
+                else if (ok) asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(p.part_flags + slot), "r"(1) : "memory");
             }
         }
         if (!SEGS || (left -= n) == 0) break;
         q0 += n;
         ++seg;
         ++tile;
-        ft = tile / p.ttiles;
-        tok0 = (tile - ft * p.ttiles) * NTOK;
+        const int fd2 = tile / p.ttiles;
+        ft = fd2 * CS + (int)rank;
+        tok0 = (tile - fd2 * p.ttiles) * NTOK;
         if (ok) {   // the accumulators and the activation stages are free for the next segment
             fence_async_smem();
             tc_fence_before();
@@ -1056,7 +1150,15 @@ gemm_tmem_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tmap) {
     if (dbg && tid == 64) { dbg[303] = (unsigned long long)clock64(); dbg[305] = gtime_ns(); }
     tc_fence_before();
     __syncthreads();
-    if (warp == 1) tmem_dealloc(tmem, TMEM_COLS);
+    if constexpr (DUO) {
+        if (warp != 1) cluster_wait();
+        __syncwarp();
+        cluster_sync();   // neither CTA leaves, nor frees its tensor memory, under the other's MMAs and arrivals
+    }
+    if (warp == 1) {
+        if constexpr (DUO) tmem_dealloc2(tmem, TMEM_COLS);
+        else tmem_dealloc(tmem, TMEM_COLS);
+    }
     if (tid == 0 && s_abort) atomicExch(p.status, 2);
 }
 
@@ -1066,11 +1168,44 @@ static int32_t gemm_attr() {
     if constexpr (NTOK <= 128)
         RSTQ_CUDA(cudaFuncSetAttribute(gemm_tc_kernel<BITS, NTOK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        kNST * (kAStage + NTOK * kKStep * 2) + 1024));
-    RSTQ_CUDA(cudaFuncSetAttribute(gemm_tmem_kernel<BITS, NTOK, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   gemm_stages(NTOK) * (NTOK * kKStep * 2) + 1024));
-    RSTQ_CUDA(cudaFuncSetAttribute(gemm_tmem_kernel<BITS, NTOK, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   gemm_stages(NTOK) * (NTOK * kKStep * 2) + 1024));
+    auto smem = [](auto kernel, int bytes) { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes); };
+    RSTQ_CUDA(smem(gemm_tmem_kernel<BITS, NTOK, false, false>, gemm_smem(NTOK, false)));
+    RSTQ_CUDA(smem(gemm_tmem_kernel<BITS, NTOK, true, false>, gemm_smem(NTOK, false)));
+    if constexpr (NTOK == 256) {
+        RSTQ_CUDA(smem(gemm_tmem_kernel<BITS, NTOK, false, true>, gemm_smem(NTOK, true)));
+        RSTQ_CUDA(smem(gemm_tmem_kernel<BITS, NTOK, true, true>, gemm_smem(NTOK, true)));
+    }
     return RSTQ_OK;
+}
+
+template <int BITS, int NTOK>
+static cudaError_t gemm_launch(const DeviceState& ds, const GemmParams& p, const CUtensorMap& tmap, int ctas, bool general, bool duo) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)ctas);
+    cfg.blockDim = dim3(kGemmThreadsT);
+    cfg.dynamicSmemBytes = gemm_smem(NTOK, duo);
+    cfg.stream = ds.stream;
+    cudaLaunchAttribute a[2];
+    int n = 0;
+    if (duo) {
+        a[n].id = cudaLaunchAttributeClusterDimension;
+        a[n].val.clusterDim.x = 2;
+        a[n].val.clusterDim.y = a[n].val.clusterDim.z = 1;
+        ++n;
+    }
+    if (ds.pdl) {
+        a[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        a[n].val.programmaticStreamSerializationAllowed = 1;
+        ++n;
+    }
+    cfg.attrs = a;
+    cfg.numAttrs = (unsigned)n;
+    if constexpr (NTOK == 256) {
+        if (duo) return general ? cudaLaunchKernelEx(&cfg, gemm_tmem_kernel<BITS, NTOK, true, true>, p, tmap)
+                                : cudaLaunchKernelEx(&cfg, gemm_tmem_kernel<BITS, NTOK, false, true>, p, tmap);
+    }
+    return general ? cudaLaunchKernelEx(&cfg, gemm_tmem_kernel<BITS, NTOK, true, false>, p, tmap)
+                   : cudaLaunchKernelEx(&cfg, gemm_tmem_kernel<BITS, NTOK, false, false>, p, tmap);
 }
 
 int32_t gemm_configure(DeviceState& ds) {
@@ -1141,7 +1276,7 @@ void gemm_plan(int64_t out, int64_t in, int64_t M, int sm_count, bool tmem_kerne
     if (M > 128 && tmem_kernel && wide != 1) {
         bool split_w = false;
         const int64_t c_wide = cycles(256, &split_w);
-        if (wide == 2 || c_wide < c_narrow) {
+        if (wide == 2 || wide >= 5 || c_wide < c_narrow) {
             ntok = 256;
             split = split_w;
         }
@@ -1160,13 +1295,26 @@ void gemm_plan(int64_t out, int64_t in, int64_t M, int sm_count, bool tmem_kerne
         bool s2 = false;
         const int64_t other = cycles(ntok, &s2);
         const bool pays = per <= 3 * ksteps_total && (per * c + fixed + kRangeCycles) * 100 < other * (s2 ? 100 : (ntok <= 64 ? 94 : 85));
-        if (steps < (1ll << 31) && (wide == 4 || pays)) {
+        if (steps < (1ll << 31) && (wide == 4 || wide == 6 || pays)) {
             *ranges_out = (int)G;
             split = false;
         }
     }
     *ntok_out = ntok;
     *split_out = split;
+}
+
+// 256-token tiles on pairs of CTAs?  A launch of clusters costs about 1.2 us more (both SMs of a pair have to be free of the
+// pre-pass), the K-step gains 7 %: where every SM has 80 of them to do.  In a burst / over 0.1 s, us: 70B-class MLP at
+// M = 256 (97 steps each) 103.3 -> 97.0 / 116.9 -> 112.1 and 104.7 -> 98.6 / 118.6 -> 114.9; int4 4096 x 8192 at M = 2048 (110)
+// 122.3 -> 113.5 / 135.1 -> 128.7; 7168 x 16384 at M = 512 (97) 103.8 -> 99.2 / 118.6 -> 114.4.  Below the line: 8192 x 8192 at
+// M = 512 (55) 54.5 -> 53.0 / 58.7 -> 60.0, 16384 x 6144 at M = 250 (41) 43.0 -> 41.2 / 43.7 -> 46.1.  Tiles of 128 tokens, as fast
+// in the kernel either way, only lose the launch (int8 4096 x 4096 at M = 512 21.5 -> 22.8).  An odd number of 128-feature
+// tiles idles a CTA of the last pair.
+static bool gemm_duo(int ntok, int64_t ftiles, int64_t ttiles, int64_t ksteps, int sm_count, int wide) {
+    if (ntok != 256) return false;
+    if (wide >= 5) return true;
+    return wide == 0 && ftiles * ttiles * ksteps >= 80ll * sm_count && ((ftiles & 1) == 0 || ftiles >= 9);
 }
 
 // y[M, out] = x[M, in] . dequant(W)^T on the tensor cores.  src: 0 = f32 x, 1 = bf16 x,
@@ -1194,6 +1342,7 @@ int32_t launch_gemm(rstq_ctx* ctx, DeviceState& ds, const rstq_weight* w, const 
     bool split = false;
     int ranges = 0;
     gemm_plan(w->out, w->in, M, ds.sm_count, a_in_tmem && acc32 != nullptr, (int)ctx->tune_gemm_wide, &ntok, &split, &ranges);
+    const bool duo = a_in_tmem && gemm_duo(ntok, ftiles, (M + ntok - 1) / ntok, (w->nb + 3) / 4, ds.sm_count, (int)ctx->tune_gemm_wide);
     // pre-pass: activations -> fp16 with one exponent per token row.  kind::f16 wants A and B of
     // one type (fp16 weights against bf16 activations raise "illegal instruction"), and fp16 on
     // both sides keeps three more mantissa bits of the weights than bf16 would.
@@ -1204,7 +1353,7 @@ int32_t launch_gemm(rstq_ctx* ctx, DeviceState& ds, const rstq_weight* w, const 
     CUtensorMap tmap;
     const cuuint64_t dims[2] = {(cuuint64_t)w->in, (cuuint64_t)M};
     const cuuint64_t strides[1] = {(cuuint64_t)w->in * 2};
-    const cuuint32_t box[2] = {64, (cuuint32_t)ntok};
+    const cuuint32_t box[2] = {64, (cuuint32_t)(duo ? ntok / 2 : ntok)};
     const cuuint32_t estr[2] = {1, 1};
     const CUresult cr = enc(&tmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, x16, dims, strides, box, estr,
                             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
@@ -1229,37 +1378,31 @@ int32_t launch_gemm(rstq_ctx* ctx, DeviceState& ds, const rstq_weight* w, const 
     p.out_dtype = out_dtype;
     p.dbg = ds.dbg;
     RSTQ_REQUIRE(ftiles * p.ttiles < (1ll << 30), RSTQ_E_LIMIT, "grid too large");
-    const int64_t tiles = ftiles * p.ttiles;
-    const int64_t ctas = ranges > 0 ? ranges : (split ? tiles * 2 : tiles);
+    // (units: thread blocks, or pairs of them on tiles of 256 features)
+    const int64_t cs = duo ? 2 : 1, tiles = (ftiles + cs - 1) / cs * p.ttiles;
+    const int64_t units = ranges > 0 ? std::max<int64_t>(1, std::min(ranges / cs, tiles * p.ksteps)) : (split ? tiles * 2 : tiles);
     p.half = split ? (p.ksteps + 1) / 2 : 0;
-    p.uq = ranges > 0 ? tiles * p.ksteps / ranges : p.ksteps;
-    p.ur = ranges > 0 ? tiles * p.ksteps % ranges : 0;
+    p.uq = ranges > 0 ? tiles * p.ksteps / units : p.ksteps;
+    p.ur = ranges > 0 ? tiles * p.ksteps % units : 0;
     p.part = acc32;   // [CTA][16 warps][columns per warp][32 lanes] f32: 128 * ntok floats each
     p.part_flags = ds.counters + ds.counters_len - kGemmSharers;
     const bool general = ranges > 0 || (w->nb & 3) != 0;
-    const dim3 grid((unsigned)ctas);
-    const size_t smem = a_in_tmem ? gemm_stages(ntok) * ((size_t)ntok * kKStep * 2) + 1024
-                                  : kNST * (kAStage + (size_t)ntok * kKStep * 2) + 1024;
-#define GT(B, N)                                                                                          \
-    le = general ? launch_pdl(gemm_tmem_kernel<B, N, true>, grid, dim3(kGemmThreadsT), smem, ds, p, tmap)  \
-                 : launch_pdl(gemm_tmem_kernel<B, N, false>, grid, dim3(kGemmThreadsT), smem, ds, p, tmap)
-#define GL(B, N)                 \
-    do {                         \
-        if (a_in_tmem) GT(B, N); \
-        else le = launch_pdl(gemm_tc_kernel<B, N>, grid, dim3(kGemmThreads), smem, ds, p, tmap); \
-    } while (0)
+    const int grid = (int)(units * cs);
+    const size_t smem1 = kNST * (kAStage + (size_t)ntok * kKStep * 2) + 1024;
+#define GL(B, N) \
+    le = a_in_tmem ? gemm_launch<B, N>(ds, p, tmap, grid, general, duo) \
+                   : launch_pdl(gemm_tc_kernel<B, N>, dim3((unsigned)grid), dim3(kGemmThreads), smem1, ds, p, tmap)
     if (w->bits == 4) {
         if (ntok == 32) GL(4, 32);
         else if (ntok == 64) GL(4, 64);
         else if (ntok == 128) GL(4, 128);
-        else GT(4, 256);
+        else le = gemm_launch<4, 256>(ds, p, tmap, grid, general, duo);
     } else {
         if (ntok == 32) GL(8, 32);
         else if (ntok == 64) GL(8, 64);
         else if (ntok == 128) GL(8, 128);
-        else GT(8, 256);
+        else le = gemm_launch<8, 256>(ds, p, tmap, grid, general, duo);
     }
-#undef GT
 #undef GL
     ctx->launches++;
     RSTQ_CUDA(le);

@@ -84,6 +84,12 @@ __device__ __forceinline__ bool mbar_block(uint32_t bar, uint32_t parity, volati
         if (mbar_try(bar, parity)) return true;
     return mbar_wait(bar, parity, abort_flag);
 }
+// An arrival on the barrier at the same address in CTA `rank` of the cluster.
+__device__ __forceinline__ void mbar_arrive_at(uint32_t bar, uint32_t rank) {
+    asm volatile(
+        "{ .reg .b32 a; mapa.shared::cluster.u32 a, %0, %1; mbarrier.arrive.shared::cluster.b64 _, [a]; }" ::"r"(bar), "r"(rank)
+        : "memory");
+}
 // Warp-wide wait that polls from lane 0 only, sleeping between polls: a producer warp that is
 // a long way ahead of its consumer then leaves the barrier unit and the issue slots to the
 // warps that are on the critical path.  All 32 lanes must call it; all get the same answer.

@@ -21,6 +21,22 @@ __device__ __forceinline__ void tmem_relinquish() {
 __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
+// The same for a pair of CTAs (a cluster of two): one warp of each takes part, both get the same columns.
+__device__ __forceinline__ void tmem_alloc2(uint32_t smem_dst, uint32_t ncols) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_dst), "r"(ncols) : "memory");
+}
+__device__ __forceinline__ void tmem_relinquish2() {
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_dealloc2(uint32_t taddr, uint32_t ncols) {
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_sync() {
+    cluster_arrive();
+    cluster_wait();
+}
 __device__ __forceinline__ void tc_fence_before() {
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
 }
@@ -86,6 +102,10 @@ __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t saddr) {
 __host__ __device__ constexpr uint32_t idesc_f16(int n) {
     return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
 }
+// A pair of CTAs: M = 256, its upper half in the second CTA; each CTA's shared memory holds half of the N rows of B.
+__host__ __device__ constexpr uint32_t idesc_f16_pair(int n) {
+    return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
+}
 // The same with bf16 A and B (both: the two must be of one type).
 __host__ __device__ constexpr uint32_t idesc_bf16(int n) { return idesc_f16(n) | (1u << 7) | (1u << 10); }
 
@@ -102,6 +122,15 @@ __device__ __forceinline__ void umma_commit_if(uint32_t bar, uint32_t leader) {
     asm volatile(
         "{ .reg .pred q; setp.ne.b32 q, %1, 0; "
         "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0]; }" ::"r"(bar),
+        "r"(leader)
+        : "memory");
+}
+
+// The pair's MMAs issued so far by this thread have completed: one arrival on the barrier at this address in both CTAs.
+__device__ __forceinline__ void umma_commit2_if(uint32_t bar, uint32_t leader) {
+    asm volatile(
+        "{ .reg .pred q; .reg .b16 m; setp.ne.b32 q, %1, 0; mov.b16 m, 3; "
+        "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], m; }" ::"r"(bar),
         "r"(leader)
         : "memory");
 }

@@ -42,3 +42,33 @@ def test_ranges_against_whole_tiles(ctx, bits, out, in_, M):
     ref = orc.matmul_dq_f64(c, s, 0 if bits == 4 else 1, x, M, in_, rows.size).reshape(M, rows.size)
     assert np.abs(y[4][:, rows] - ref).max() <= 1e-3 * np.abs(ref).max()
     bw.free()
+
+
+@pytest.mark.parametrize("bits", [4, 8])
+@pytest.mark.parametrize("out,in_,M", [(100, 160, 129), (300, 4128, 300), (2500, 1056, 200), (1000, 2080, 256), (1032, 8192, 515),
+                                       (256, 32, 257)])
+def test_tiles_on_pairs_of_sms_against_tiles_on_one(ctx, bits, out, in_, M):
+    """256-token tiles on pairs of SMs: an odd number of 128-feature tiles (one of a pair has none), tokens in the first SM's
+    half alone, tiles shared by two pairs, cut at any step, partial last K-steps, rows of one K-step.  Same products, same
+    sums as a 256-token tile on one SM; cut tiles differ as above."""
+    w = synth.normal(out + in_ + bits, out * in_, 0.02)
+    wq, ws = orc.quantize_weight(w, bits)
+    x = synth.normal(out + in_ + M, M * in_)
+    bw = ctx.bind_weight(wq, ws, out, in_, L.FMT_Q4_0 if bits == 4 else L.FMT_Q8_0, L.LAYOUT_ROWMAJOR)
+    y = {}
+    try:
+        for how in (2, 5, 6, 5):
+            ctx.tune(TUNE_GEMM_WIDE, how)
+            got = ctx.qmatmul_host(bw, x, M, L.F32, L.MODE_F).reshape(M, out).astype(np.float64)
+            assert how not in y or np.array_equal(got, y[how])
+            y[how] = got
+    finally:
+        ctx.tune(TUNE_GEMM_WIDE, 0)
+    top = np.abs(y[2]).max()
+    assert np.abs(y[5] - y[2]).max() <= 4 * 8e-6 * top and np.abs(y[6] - y[2]).max() <= 4 * 8e-6 * top
+    rows = np.unique(np.concatenate([np.arange(0, out, max(1, out // 64)), [out - 1]]))
+    c = np.ascontiguousarray(wq.reshape(out, -1)[rows]).ravel()
+    s = np.ascontiguousarray(ws.reshape(out, -1)[rows]).ravel()
+    ref = orc.matmul_dq_f64(c, s, 0 if bits == 4 else 1, x, M, in_, rows.size).reshape(M, rows.size)
+    assert np.abs(y[5][:, rows] - ref).max() <= 1e-3 * np.abs(ref).max()
+    bw.free()
