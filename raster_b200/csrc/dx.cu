@@ -851,7 +851,7 @@ int32_t launch_qlinear_q8_dx(rstq_ctx* ctx, DeviceState& ds, const float* dy, co
                  RSTQ_E_CUDA, "cuTensorMapEncodeTiled failed (m = %lld, in = %lld, out = %lld)", (long long)m, (long long)in,
                  (long long)out);
     if (!tma_scales) ms = mw;   // not used then
-    RSTQ_CUDA(launch_pdl(dx_prep_kernel, dim3((unsigned)(m + kDxParts)), dim3(opad > 4096 ? kDxPrepMax : 256), 0, ds, q));
+    RSTQ_CUDA(launch_pdl(dx_prep_kernel, dim3((unsigned)(m + kDxParts)), dim3(opad > 4096 ? kDxPrepMax : opad > 2048 ? 256 : 128), 0, ds, q));
     ctx->launches++;
     DxParams p{scales, q.rowexp, q.colmax, dx, ds.status, in, out, tma_scales, (int)m, (int)steps, (int)ttiles, split};
     RSTQ_CUDA(nt == 32   ? dx_launch<32>(ds, p, (int)tiles, mw, my, mh, ms)

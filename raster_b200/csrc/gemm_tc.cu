@@ -81,8 +81,8 @@ __device__ __forceinline__ void quant_dequant8(float (&v)[8]) {
 // SRC 2, 3: the int8 quantizer on the way (MODE_A8): code * scale of every element, without the quantizer's own
 // launch and its arrays' trip through memory (int4, 11000 x 4128, M = 100: 26.9 us a call with both kernels, 23.1
 // with one; 14336 x 4096, M = 64: 22.4 -> 19.9).
-template <int SRC>  // 0 = f32, 1 = bf16, 2 = f32 quantized here, 3 = bf16 quantized here
-__global__ void __launch_bounds__(256)
+template <int SRC, int T>  // 0 = f32, 1 = bf16, 2 = f32 quantized here, 3 = bf16 quantized here
+__global__ void __launch_bounds__(T)
 act_to_f16_kernel(const void* __restrict__ x, __half* __restrict__ x16,
                   float* __restrict__ rowscale, int64_t in) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -108,13 +108,13 @@ act_to_f16_kernel(const void* __restrict__ x, __half* __restrict__ x16,
     // Rows of up to 8192 elements stay in registers between the two passes (max, convert);
     // longer rows are read twice.
     constexpr int kKeep = 4;  // x 256 threads x 8 elements
-    const bool keep = in <= (int64_t)kKeep * 256 * 8;
+    const bool keep = in <= (int64_t)kKeep * T * 8;
     float held[kKeep][8];
     float mx = 0.f;
     if (keep) {
 #pragma unroll
         for (int i = 0; i < kKeep; ++i) {
-            const int64_t k = (int64_t)(i * 256 + threadIdx.x) * 8;
+            const int64_t k = (int64_t)(i * T + threadIdx.x) * 8;
             if (k < in) {
                 load8(k, held[i]);
 #pragma unroll
@@ -122,21 +122,21 @@ act_to_f16_kernel(const void* __restrict__ x, __half* __restrict__ x16,
             }
         }
     } else {
-        for (int64_t k = threadIdx.x * 8; k < in; k += 256 * 8) {
+        for (int64_t k = threadIdx.x * 8; k < in; k += T * 8) {
             float v[8];
             load8(k, v);
 #pragma unroll
             for (int j = 0; j < 8; ++j) mx = fmaxf(mx, fabsf(v[j]));
         }
     }
-    __shared__ float s_mx[8];
+    __shared__ float s_mx[T / 32];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
     if ((threadIdx.x & 31) == 0) s_mx[threadIdx.x >> 5] = mx;
     __syncthreads();
     mx = s_mx[0];
 #pragma unroll
-    for (int i = 1; i < 8; ++i) mx = fmaxf(mx, s_mx[i]);
+    for (int i = 1; i < T / 32; ++i) mx = fmaxf(mx, s_mx[i]);
     int e = 0;
     if (mx > 0.f && mx < 3.0e38f) {
         int ex;
@@ -156,11 +156,11 @@ act_to_f16_kernel(const void* __restrict__ x, __half* __restrict__ x16,
     if (keep) {
 #pragma unroll
         for (int i = 0; i < kKeep; ++i) {
-            const int64_t k = (int64_t)(i * 256 + threadIdx.x) * 8;
+            const int64_t k = (int64_t)(i * T + threadIdx.x) * 8;
             if (k < in) store8(k, held[i]);
         }
     } else {
-        for (int64_t k = threadIdx.x * 8; k < in; k += 256 * 8) {
+        for (int64_t k = threadIdx.x * 8; k < in; k += T * 8) {
             float v[8];
             load8(k, v);
             store8(k, v);
@@ -1223,16 +1223,25 @@ int32_t gemm_configure(DeviceState& ds) {
 }
 
 // x (src 0 = f32, 1 = bf16, 2 / 3 = f32 / bf16 through the int8 quantizer) -> fp16 rows x16 and 2^e per row
+template <int SRC>
+static cudaError_t act_launch(const DeviceState& ds, const void* x, void* x16, float* rowscale, int64_t M, int64_t in) {
+    const dim3 grid((unsigned)M);
+    auto go = [&](auto kernel, int t) { return launch_pdl(kernel, grid, dim3((unsigned)t), 0, ds, x, (__half*)x16, rowscale, in); };
+    // 32 elements per thread at most, so that a row stays in registers up to 32768 (8192 with 256 threads for any row,
+    // before): 4096 x 11008, M = 70, quantized on the way 34.0 -> 28.0 us a call, 8192 x 28672, M = 100 73.5 -> 66.0.  128 threads
+    // for short rows: 1000 x 1024, M = 2048 12.8 -> 12.0; at in = 4096 they lose (4096 x 4096, M = 512 22.2 -> 23.2), as 512 threads
+    // do at 6016 (3000 x 6016, M = 30 16.9 -> 17.5).
+    if (in <= 2048) return go(act_to_f16_kernel<SRC, 128>, 128);
+    if (in <= 8192) return go(act_to_f16_kernel<SRC, 256>, 256);
+    if (in <= 16384) return go(act_to_f16_kernel<SRC, 512>, 512);
+    return go(act_to_f16_kernel<SRC, 1024>, 1024);
+}
 static int32_t launch_act_to_f16(rstq_ctx* ctx, DeviceState& ds, const void* x, int src, void* x16,
                                  float* rowscale, int64_t M, int64_t in) {
-    cudaError_t le;
-    const dim3 grid((unsigned)M), block(256);
-    switch (src) {
-        case 0: le = launch_pdl(act_to_f16_kernel<0>, grid, block, 0, ds, x, (__half*)x16, rowscale, in); break;
-        case 1: le = launch_pdl(act_to_f16_kernel<1>, grid, block, 0, ds, x, (__half*)x16, rowscale, in); break;
-        case 2: le = launch_pdl(act_to_f16_kernel<2>, grid, block, 0, ds, x, (__half*)x16, rowscale, in); break;
-        default: le = launch_pdl(act_to_f16_kernel<3>, grid, block, 0, ds, x, (__half*)x16, rowscale, in);
-    }
+    const cudaError_t le = src == 0   ? act_launch<0>(ds, x, x16, rowscale, M, in)
+                           : src == 1 ? act_launch<1>(ds, x, x16, rowscale, M, in)
+                           : src == 2 ? act_launch<2>(ds, x, x16, rowscale, M, in)
+                                      : act_launch<3>(ds, x, x16, rowscale, M, in);
     ctx->launches++;
     RSTQ_CUDA(le);
     return RSTQ_OK;

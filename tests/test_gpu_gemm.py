@@ -195,3 +195,30 @@ def test_wide_token_tiles_match_the_narrow_ones(ctx, bits, M, out, in_):
         assert np.abs(ys[2].reshape(M, out)[:, r] - ref).max() <= 1e-3 * max(np.abs(ref).max(), 1e-30)
     for o in (w, bx, by):
         o.free()
+
+
+@pytest.mark.parametrize("in_", [2048, 2080, 8192, 8224, 16384, 16416, 32768, 32800])
+@pytest.mark.parametrize("mode,M,act", [(L.MODE_F, 19, L.F32), (L.MODE_F, 19, L.BF16), (L.MODE_A8, 65, L.F32)])
+def test_activation_rows_at_the_edges_of_the_pre_pass(ctx, mode, M, act, in_):
+    """The pre-pass takes 128, 256, 512 or 1024 threads per row, and reads rows above 32768 twice."""
+    out = 40
+    w = synth.normal(in_, out * in_, 0.02)
+    wq, ws = orc.quantize_weight(w, 8)
+    x = synth.normal(in_ + M, M * in_)
+    x[in_:2 * in_] *= 1e-3
+    x[2 * in_ - 1] = 7.0                      # the row's largest at its very end
+    if act == L.BF16:
+        x = synth.from_bf16_bits(synth.to_bf16_bits(x))
+    bw = ctx.bind_weight(wq, ws, out, in_, L.FMT_Q8_0, L.LAYOUT_ROWMAJOR)
+    bx, by = ctx.array_to_buffer(synth.to_bf16_bits(x) if act == L.BF16 else x), ctx.make_buffer(M * out, np.float32)
+    ctx.qmatmul(bw, bx, by, M, act, L.F32, mode)
+    ctx.sync()
+    y = by.download().reshape(M, out)
+    if mode == L.MODE_F:
+        ref = orc.matmul_dq_f64(wq, ws, 1, x, M, in_, out).reshape(M, out)
+    else:
+        xq, xs, xsum = orc.quantize_act_i8(x, M, in_)
+        ref = orc.matmul_a8_f64(wq, ws, 1, xq, xs, xsum, M, in_, out).reshape(M, out)
+    for rows in (slice(0, 1), slice(1, 2), slice(2, M)):
+        assert relerr(y[rows], ref[rows]) <= 1e-3
+    bx.free(), by.free(), bw.free()
