@@ -12,12 +12,18 @@
 
 namespace rstq {
 
-// One warp per block; lane k owns element k.  Bytes are gathered so that each
-// of eight lanes stores one 32-bit word.
+// Eight lanes per block, four blocks per warp: lane j of a block owns elements 4j .. 4j + 3, one word of codes.
+// What bounds it beside a decode kernel is where its thread blocks go: they start on the SMs that the launch before leaves
+// idle, the ones that find no room there wait for its thread blocks to leave, and the next decode kernel's thread blocks
+// start where they are not.  So few warps in small thread blocks: with a warp per block of 32 (four times as many warps) in
+// thread blocks of 256 threads int4 4096 x 11008 at 8 tokens took 12.63 us a call, now 9.99 (thread blocks of 256 threads
+// 10.66); 11008 x 4096 at 8 11.53 -> 10.76, 8192 x 8192 at 8 14.69 -> 12.13, int8 11008 x 4096 at 12 17.46 -> 16.56, 28672 x 8192 at 16
+// 45.75 -> 45.56.  Dynamic shared memory to spread the thread blocks over more SMs: between 5 % faster and 15 % slower.
 // BF16IN: x holds bf16 bit patterns (uint16_t); they are widened exactly, so the codes are those
 // the f32 quantizer gives for the widened values.
+constexpr int kQuantThreads = 64;
 template <bool BF16IN>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(kQuantThreads)
 quant_act_i8_kernel(const void* __restrict__ xv, int8_t* __restrict__ xq, float* __restrict__ xs,
                     int32_t* __restrict__ xsum, int64_t nblocks, uint8_t* __restrict__ img, int M, int nb, int zp,
                     int four_bit) {
@@ -25,22 +31,30 @@ quant_act_i8_kernel(const void* __restrict__ xv, int8_t* __restrict__ xq, float*
     // x may come from the kernel before this one, so wait for it
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31, j = lane & 7;
     const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t blk = warp; blk < nblocks; blk += nwarps) {
-        const float v = BF16IN ? __uint_as_float((uint32_t)reinterpret_cast<const uint16_t*>(xv)[blk * 32 + lane] << 16)
-                               : reinterpret_cast<const float*>(xv)[blk * 32 + lane];
-        int q, s;
+    for (int64_t blk0 = warp * 4; blk0 < nblocks; blk0 += nwarps * 4) {
+        const int64_t blk = blk0 + (lane >> 3);
+        const bool act = blk < nblocks;
+        float v[4] = {0.f, 0.f, 0.f, 0.f};
+        if (act && BF16IN) {
+            const uint2 r = reinterpret_cast<const uint2*>(xv)[blk * 8 + j];
+            v[0] = __uint_as_float(r.x << 16);
+            v[1] = __uint_as_float(r.x & 0xFFFF0000u);
+            v[2] = __uint_as_float(r.y << 16);
+            v[3] = __uint_as_float(r.y & 0xFFFF0000u);
+        } else if (act) {
+            const float4 r = reinterpret_cast<const float4*>(xv)[blk * 8 + j];
+            v[0] = r.x; v[1] = r.y; v[2] = r.z; v[3] = r.w;
+        }
+        uint32_t w;
+        int s;
         float scale;
-        quant_block32(v, &q, &s, &scale);
-        // pack four neighbouring codes into the word lane (lane & ~3) stores
-        uint32_t b = (uint32_t)(q & 0xFF);
-        uint32_t w = b << (8 * (lane & 3));
-        w |= __shfl_xor_sync(0xffffffffu, w, 1);
-        w |= __shfl_xor_sync(0xffffffffu, w, 2);
-        if ((lane & 3) == 0) reinterpret_cast<uint32_t*>(xq)[blk * 8 + (lane >> 2)] = w;
-        if (lane == 0) {
+        quant_block32_words(v, &w, &s, &scale);
+        if (!act) continue;
+        reinterpret_cast<uint32_t*>(xq)[blk * 8 + j] = w;
+        if (j == 0) {
             xs[blk] = scale;
             if (xsum) xsum[blk] = s;
         }
@@ -53,13 +67,11 @@ quant_act_i8_kernel(const void* __restrict__ xv, int8_t* __restrict__ xq, float*
             const int piece = ct / kGemvMaxM, c = ct - piece * kGemvMaxM;        // token inside its launch
             const int Mp = min(kGemvMaxM, M - piece * kGemvMaxM);                // tokens of that launch
             uint8_t* im = img + piece * act_image_stride(nb);
-            const int j = lane >> 2;                                            // word held by lanes 0, 4, .. 28
-            if ((lane & 3) == 0)
-                reinterpret_cast<uint32_t*>(im)[((int64_t)(b * Mp + c) * 4 + (j & 3)) * 2 + (j >> 2)] = w;
+            reinterpret_cast<uint32_t*>(im)[((int64_t)(b * Mp + c) * 4 + (j & 3)) * 2 + (j >> 2)] = w;
             const int Mz = (Mp + 1) & ~1;
             uint8_t* recs = im + (((int64_t)nb * Mp * 32 + 127) & ~127ll);
-            if (lane == 0) put_act_record(recs, b, Mz, c, scale, zp * s, four_bit);
-            if (lane == 1 && c == Mp - 1 && Mz > Mp) put_act_record(recs, b, Mz, Mp, 0.f, 0, four_bit);
+            if (j == 0) put_act_record(recs, b, Mz, c, scale, zp * s, four_bit);
+            if (j == 1 && c == Mp - 1 && Mz > Mp) put_act_record(recs, b, Mz, Mp, 0.f, 0, four_bit);
         }
     }
 }
@@ -123,13 +135,13 @@ int32_t launch_act_image(rstq_ctx* ctx, DeviceState& ds, const int8_t* xq, const
 int32_t launch_quant_act_i8(rstq_ctx* ctx, DeviceState& ds, const void* x, int8_t* xq, float* xs,
                             int32_t* xsum, int64_t M, int64_t in, int act_dtype, uint8_t* img, int zp, int bits) {
     const int64_t nblocks = M * (in / 32);
-    int64_t ctas = (nblocks + 7) / 8;  // 8 warps per CTA
-    const int64_t cap = (int64_t)ds.sm_count * 8;
+    int64_t ctas = (nblocks + kQuantThreads / 8 - 1) / (kQuantThreads / 8);
+    const int64_t cap = (int64_t)ds.sm_count * (2048 / kQuantThreads);
     if (ctas > cap) ctas = cap;
     if (ctas < 1) ctas = 1;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)ctas);
-    cfg.blockDim = dim3(256);
+    cfg.blockDim = dim3(kQuantThreads);
     cfg.stream = ds.stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;

@@ -306,7 +306,7 @@ __device__ __forceinline__ void stage_a8(const StreamParams& p, uint8_t* smem, i
 // Thread (b, tig) holds the eight elements its record needs; the four threads of a block are
 // neighbouring lanes (two shuffles for the maximum, two for the sum).  The codes come from f32
 // arithmetic whenever that provably gives the double result: t = x * fl32(127 / max) is within
-// 127 * 2^-22 of the double product, so a t further than 1e-3 from every k + 0.5 rounds the same way;
+// 127 * 2^-22 of the double product, so a t further than 5e-5 from every k + 0.5 rounds the same way;
 // anything closer, and blocks whose maximum is zero, tiny, huge or not finite, take the double path.
 // xs: fl32(max / 127) equals (float)((double)max / 127.0) for every f32 max -- the quotient of a
 // 24-bit integer by 127 cannot sit on a 25-bit midpoint, so rounding through double changes nothing.
@@ -378,7 +378,9 @@ __device__ __forceinline__ void stage_a8_quant(const StreamParams& p, const void
         // f32 shortcut: u = fma(x, 127 / max, 1.5 * 2^23) holds round-to-nearest(x * 127 / max) in its low
         // mantissa bits (two's complement in the low byte); the quotient is 2 ulp accurate, so the
         // product is within 4e-5 of the double one and every element whose remainder is further than
-        // 2e-4 from a tie rounds exactly as round_half_up of the double product does.
+        // 5e-5 from a tie rounds exactly as round_half_up of the double product does.  (Every block of
+        // a launch waits for the same few elements that take the double path: at 2e-4 four rows of 4096 in five had one, 11008 x 4096 and
+        // 4096 x 11008 7.22 and 8.28 us; at 5e-5 7.17 and 8.11.)
         uint32_t wa, wb;
         int sum;
         float xs = 0.f;
@@ -395,7 +397,7 @@ __device__ __forceinline__ void stage_a8_quant(const StreamParams& p, const void
                 amb = max_nan(amb, fabsf(frac));                     // a NaN takes the double path as well
                 ub[k] = __float_as_uint(u);
             }
-            exact = !(amb <= 0.5f - 2e-4f);
+            exact = !(amb <= 0.5f - 5e-5f);
             wa = __byte_perm(__byte_perm(ub[0], ub[1], 0x0040), __byte_perm(ub[2], ub[3], 0x0040), 0x5410);
             wb = __byte_perm(__byte_perm(ub[4], ub[5], 0x0040), __byte_perm(ub[6], ub[7], 0x0040), 0x5410);
         }

@@ -121,3 +121,44 @@ def test_elements_that_are_no_number_get_the_same_code_on_every_route(ctx, fmt, 
     assert np.array_equal(got[0], ctx.qmatmul_host(w, x)[0], equal_nan=True)
     for b in (bx, by, w):
         b.free()
+
+
+@pytest.mark.parametrize("blocks", [1, 2, 3, 4, 5, 7, 8, 9, 31, 33, 300])   # parts of a warp, of a thread block, several
+@pytest.mark.parametrize("act", [L.F32, L.BF16])
+def test_numbers_of_blocks_that_fill_no_warp(ctx, act, blocks):
+    """Eight lanes quantize a block, a thread block 64 / 8 of them: codes, scales and sums (f32), and through a product of two
+    to four tokens the image of odd and even numbers of tokens (both types), against the oracle."""
+    all_ = hard_blocks()
+    all_ = all_[np.abs(all_).max(1) <= 1e6]
+    rng = np.random.default_rng(blocks)
+    x = all_[rng.integers(0, len(all_), blocks)].ravel()
+    n = x.size
+    if act == L.F32:
+        bx = ctx.array_to_buffer(x)
+        q, s, z = ctx.make_buffer(n + 64, np.int8), ctx.make_buffer(blocks + 8, np.float32), ctx.make_buffer(blocks + 8, np.int32)
+        for b in (q, s, z):
+            b.fill_bytes(0x5A)
+        ctx.quant_act_i8(bx, q, s, z, 1, n)
+        ctx.sync()
+        oq, os_, oz = orc.quantize_act_i8(x, 1, n)
+        assert np.array_equal(q.download()[:n], oq) and (q.download()[n:] == 0x5A).all()
+        assert np.array_equal(s.download().view(np.uint32)[:blocks], os_.view(np.uint32)) and (s.download().view(np.uint32)[blocks:] == 0x5A5A5A5A).all()
+        assert np.array_equal(z.download()[:blocks], oz) and (z.download()[blocks:] == 0x5A5A5A5A).all()
+        for b in (bx, q, s, z):
+            b.free()
+    out = 40
+    wq, ws = orc.quantize_weight(rng.standard_normal(out * n).astype(np.float32), 4)
+    w = ctx.bind_weight(wq, ws, out, n, L.FMT_Q4_0, L.LAYOUT_ROWMAJOR)
+    for M in (2, 3, 4):
+        xm = all_[rng.integers(0, len(all_), M * blocks)].ravel()
+        bits = (xm.view(np.uint32) >> 16).astype(np.uint16)
+        if act == L.BF16:
+            xm = (bits.astype(np.uint32) << 16).view(np.float32)
+        bx, by = ctx.array_to_buffer(bits if act == L.BF16 else xm), ctx.make_buffer(M * out, np.float32)
+        ctx.qmatmul(w, bx, by, M, act, L.F32, L.MODE_A8)
+        ctx.sync()
+        ref = orc.matmul_a8_f64(wq, ws, 0, *orc.quantize_act_i8(xm, M, n), M, n, out).reshape(M, out)
+        got = by.download().reshape(M, out)
+        assert (np.abs(got - ref).max(1) <= 2e-6 * np.abs(ref).max(1)).all()
+        bx.free(), by.free()
+    w.free()
