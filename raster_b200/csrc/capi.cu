@@ -218,8 +218,8 @@ static int32_t run_f(rstq_ctx* ctx, rstq_weight* w, const void* x, void* y, int6
 
 // Q4_K: decode kernel over the sub-block scales (zero point 0), then the min term added to y.
 static int32_t run_q4k(rstq_ctx* ctx, rstq_weight* w, const int8_t* xq, const float* xs32, const int32_t* bsums,
-                       float* y, int64_t M, uint8_t* img_scratch = nullptr) {
-    int32_t rc = run_a8(ctx, w, xq, xs32, bsums, y, M, nullptr, nullptr, w->kq ? img_scratch : nullptr);
+                       float* y, int64_t M, uint8_t* img_scratch = nullptr, const uint8_t* img = nullptr) {
+    int32_t rc = run_a8(ctx, w, xq, xs32, bsums, y, M, nullptr, img, w->kq ? img_scratch : nullptr);
     if (rc != RSTQ_OK || w->kq) return rc;   // Q4_K units: the decode kernel added the min term itself
     return launch_q4k_min(ctx, ctx->devs[w->dev], w->mins, xs32, bsums, y, M, w->nb, w->out);
 }
@@ -269,9 +269,10 @@ int32_t matmul_device(rstq_ctx* ctx, rstq_weight* w, const void* x, void* y, int
         if (rc != RSTQ_OK) return rc;
         if (w->k6) {
             // units with a scale per 16 elements: code sums per 16, one decode launch, y as it is
-            rc = launch_quant_act_q8k(ctx, ds, (const float*)x, s.xq, nullptr, s.xs, s.xsum, M, w->in, 16);
+            uint8_t* img = ds.act_image ? s.img : nullptr;
+            rc = launch_quant_act_q8k(ctx, ds, (const float*)x, s.xq, nullptr, s.xs, s.xsum, M, w->in, 16, M > 1 ? img : nullptr, w->zp);
             if (rc != RSTQ_OK) return rc;
-            return run_a8(ctx, w, s.xq, s.xs, s.xsum, (float*)y, M, nullptr, nullptr, ds.act_image ? s.img : nullptr);
+            return run_a8(ctx, w, s.xq, s.xs, s.xsum, (float*)y, M, nullptr, M > 1 ? img : nullptr, img);
         }
         if ((rc = dev_reserve(ds, &ds.kq_scratch, &ds.kq_scratch_bytes, M * w->out * 4)) != RSTQ_OK) return rc;
         rc = launch_quant_act_q8k(ctx, ds, (const float*)x, s.xq, nullptr, s.xs, s.xsum, M, w->in, 32);
@@ -289,9 +290,11 @@ int32_t matmul_device(rstq_ctx* ctx, rstq_weight* w, const void* x, void* y, int
         ActScratch s;
         int32_t rc = act_scratch(ds, M, w->in, &s);
         if (rc != RSTQ_OK) return rc;
-        rc = launch_quant_act_q8k(ctx, ds, (const float*)x, s.xq, nullptr, s.xs, s.xsum, M, w->in, 32);
+        uint8_t* img = ds.act_image ? s.img : nullptr;
+        const bool lay_out = w->kq && M > 1;      // (units with the minima outside take none)
+        rc = launch_quant_act_q8k(ctx, ds, (const float*)x, s.xq, nullptr, s.xs, s.xsum, M, w->in, 32, lay_out ? img : nullptr, w->zp);
         if (rc != RSTQ_OK) return rc;
-        return run_q4k(ctx, w, s.xq, s.xs, s.xsum, (float*)y, M, ds.act_image ? s.img : nullptr);
+        return run_q4k(ctx, w, s.xq, s.xs, s.xsum, (float*)y, M, img, lay_out ? img : nullptr);
     }
     // Prefill shapes go to the tensor-core GEMM (fp16 operands, results within 1e-3 of the
     // reference).  A8 keeps its exact integer path up to M = 63: callers that chose the

@@ -1956,7 +1956,7 @@ int32_t launch_gemv_a8(rstq_ctx* ctx, DeviceState& ds, const GemvA8Args& a) {
         StreamPlan pl;
         // the quantizer's image of this launch's tokens: laid out per kGemvMaxM tokens, so it serves a launch
         // that starts at such a boundary and takes all that is left up to the next
-        const bool at_piece = a.img && a.uk == 0 && m0 % kGemvMaxM == 0 && (want > 1 || a.M == 1);
+        const bool at_piece = a.img && m0 % kGemvMaxM == 0 && (want > 1 || (a.M == 1 && a.uk == 0));
         const uint8_t* img = at_piece ? a.img + (m0 / kGemvMaxM) * act_image_stride(nb) : nullptr;
         const int rec_bytes = a.uk == 1 ? 8 : kActRecBytes;
         bool make = false;

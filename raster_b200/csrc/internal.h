@@ -233,7 +233,7 @@ int32_t launch_q6k_units(rstq_ctx* ctx, DeviceState& ds, const uint8_t* src, con
                          int64_t out, int64_t nb);
 // kquant.cu (Q4_K: q8_K activation quantizer, scale expansion, the min-term GEMV)
 int32_t launch_quant_act_q8k(rstq_ctx* ctx, DeviceState& ds, const float* x, int8_t* xq, float* xs, float* xs32,
-                             int32_t* bsums, int64_t rows, int64_t in, int sub);
+                             int32_t* bsums, int64_t rows, int64_t in, int sub, uint8_t* img = nullptr, int zp = 0);
 int32_t launch_expand_scales(rstq_ctx* ctx, DeviceState& ds, const float* xs, float* xs32, int64_t n32);
 int32_t launch_q6k_prep(rstq_ctx* ctx, DeviceState& ds, const float* xs, const int32_t* bsums16, float* xs32,
                         int32_t* bsum32, int64_t n32);

@@ -31,47 +31,101 @@ __device__ __forceinline__ int kq_round_half_up(double v) {
     return (int)f + ((v - f) >= 0.5 ? 1 : 0);
 }
 
-// One CTA of 256 threads per (row, super-block); thread t owns element t.
+// A warp per (row, super-block), lane l owns elements 8 l .. 8 l + 7; two warps per thread block (see quant_act_i8_kernel for
+// why small thread blocks).  Codes come from f32 arithmetic except next to a tie or where the largest magnitude is zero,
+// tiny, huge or not finite, as in quant_block32.
 // xs: [rows, nsb] (the reference's array) and / or xs32: [rows, nsb * 8], the super-block scale
 // repeated for each of its 32-element blocks (what the decode kernel reads); either may be null.
 // bsums: [rows, nsb * 256 / SUB].
+// img (or null): the same as the image of a decode launch above one token (act_image_kernel with uk 1 where SUB is 32, 2 where
+// it is 16), one per kGemvMaxM rows; zp: the units' zero point.  With a thread block of 256 threads in double per super-block
+// and act_image_kernel behind it, or the decode kernel staging the arrays itself, before -> now, us a call: Q4_K 4096 x 4096 at 16
+// tokens 13.70 -> 8.41, 8192 x 8192 at 8 19.45 -> 14.78, 11008 x 4096 at 2 11.64 -> 10.92; Q6_K 4096 x 11008 at 8 19.22 -> 16.26,
+// 4096 x 8192 at 5 15.73 -> 12.36.
+constexpr int kQ8kThreads = 64;
 template <int SUB>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(kQ8kThreads)
 quant_act_q8k_kernel(const float* __restrict__ x, int8_t* __restrict__ xq, float* __restrict__ xs,
-                     float* __restrict__ xs32, int32_t* __restrict__ bsums) {
-    __shared__ float s_mx[8];
+                     float* __restrict__ xs32, int32_t* __restrict__ bsums, int64_t count, uint8_t* __restrict__ img, int M, int nb,
+                     int zp) {
+    constexpr float kMagic = 12582912.0f;   // 2^23 + 2^22
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    const int64_t sb = blockIdx.x;  // row * nsb + super-block
-    const float v = x[sb * 256 + t];
-    float mx = fabsf(v);
+    const int lane = threadIdx.x & 31;
+    const int64_t sb = blockIdx.x * (int64_t)(kQ8kThreads / 32) + (threadIdx.x >> 5);  // row * nsb + super-block
+    if (sb >= count) return;
+    const float4 lo = reinterpret_cast<const float4*>(x)[sb * 64 + lane * 2], hi = reinterpret_cast<const float4*>(x)[sb * 64 + lane * 2 + 1];
+    const float v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+    float mx = fabsf(v[0]);
+#pragma unroll
+    for (int k = 1; k < 8; ++k) mx = fmaxf(mx, fabsf(v[k]));
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if (lane == 0) s_mx[warp] = mx;
-    __syncthreads();
-    mx = s_mx[0];
+    uint32_t w[2] = {0u, 0u};
+    float scale = 0.f;
+    bool exact = !(mx >= 1e-30f && mx <= 1e37f);
+    if (!exact) {
+        const float id = __fdividef(127.f, mx);
+        uint32_t u[8];
 #pragma unroll
-    for (int i = 1; i < 8; ++i) mx = fmaxf(mx, s_mx[i]);
-    const double d = (double)mx / 127.0;
-    const double id = d == 0.0 ? 0.0 : 1.0 / d;
-    int q = kq_round_half_up((double)v * id);
-    q = max(-127, min(127, q));
-    uint32_t w = (uint32_t)(q & 0xFF) << (8 * (lane & 3));
-    w |= __shfl_xor_sync(0xffffffffu, w, 1);
-    w |= __shfl_xor_sync(0xffffffffu, w, 2);
-    if ((lane & 3) == 0) reinterpret_cast<uint32_t*>(xq)[sb * 64 + (t >> 2)] = w;
-    int s = q;
+        for (int k = 0; k < 8; ++k) {
+            const float t = fmaf(v[k], id, kMagic);
+            exact |= !(fabsf(fmaf(v[k], id, kMagic - t)) <= 0.5f - 5e-5f);
+            u[k] = __float_as_uint(t);
+        }
 #pragma unroll
-    for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (SUB == 16) {
-        if ((lane & 15) == 0) bsums[sb * 16 + warp * 2 + (lane >> 4)] = s;
-    } else {
-        s += __shfl_xor_sync(0xffffffffu, s, 16);
-        if (lane == 0) bsums[sb * 8 + warp] = s;
+        for (int h = 0; h < 2; ++h)
+            w[h] = __byte_perm(__byte_perm(u[4 * h], u[4 * h + 1], 0x0040), __byte_perm(u[4 * h + 2], u[4 * h + 3], 0x0040), 0x5410);
+        scale = __fdiv_rn(mx, 127.f);
     }
-    if (xs && t == 0) xs[sb] = (float)d;
-    if (xs32 && t < 8) xs32[sb * 8 + t] = (float)d;
+    if (exact) {
+        const double d = (double)mx / 127.0;
+        const double id = d == 0.0 ? 0.0 : 1.0 / d;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            w[h] = 0u;
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                w[h] |= (uint32_t)(max(-127, min(127, kq_round_half_up((double)v[4 * h + k] * id))) & 0xFF) << (8 * k);
+        }
+        scale = (float)d;
+    }
+    reinterpret_cast<uint2*>(xq)[sb * 32 + lane] = make_uint2(w[0], w[1]);
+    int s16 = __dp4a((int)w[0], 0x01010101, __dp4a((int)w[1], 0x01010101, 0));
+    s16 += __shfl_xor_sync(0xffffffffu, s16, 1);                     // of the 16 elements of lanes l & ~1, + 1
+    const int other = __shfl_xor_sync(0xffffffffu, s16, 2), s32 = s16 + other;
+    const bool first = (lane & 3) == 0;                              // of the four lanes of a block of 32
+    if (SUB == 16) {
+        if ((lane & 1) == 0) bsums[sb * 16 + (lane >> 1)] = s16;
+    } else if (first) {
+        bsums[sb * 8 + (lane >> 2)] = s32;
+    }
+    if (xs && lane == 0) xs[sb] = scale;
+    if (xs32 && first) xs32[sb * 8 + (lane >> 2)] = scale;
+    if (img) {
+        const int nsb = nb >> 3, ct = (int)(sb / nsb), b = (int)(sb - (int64_t)ct * nsb) * 8 + (lane >> 2);   // token, block
+        const int piece = ct / kGemvMaxM, c = ct - piece * kGemvMaxM, Mp = min(kGemvMaxM, M - piece * kGemvMaxM), Mz = (Mp + 1) & ~1;
+        uint8_t* im = img + piece * act_image_stride(nb);
+        uint8_t* recs = im + (((int64_t)nb * Mp * 32 + 127) & ~127ll);
+        uint32_t* words = reinterpret_cast<uint32_t*>(im) + ((int64_t)b * Mp + c) * 8;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int j = (lane & 3) * 2 + h;
+            words[(j & 3) * 2 + (j >> 2)] = w[h];
+        }
+        if (first) {
+            const bool pad = c == Mp - 1 && Mz > Mp;
+            if (SUB == 32) {
+                int2* z = reinterpret_cast<int2*>(recs) + (int64_t)b * Mz + c;
+                z[0] = make_int2(__float_as_int(scale), __float_as_int(scale * (float)s32));
+                if (pad) z[1] = make_int2(0, 0);
+            } else {
+                int4* z = reinterpret_cast<int4*>(recs) + (int64_t)b * Mz + c;
+                z[0] = make_int4(__float_as_int(scale), zp * s16, zp * other, 0);
+                if (pad) z[1] = make_int4(0, 0, 0, 0);
+            }
+        }
+    }
 }
 
 // xs32[i] = xs[i / 8]: the reference's per-super-block scales laid out per 32-element block
@@ -157,10 +211,10 @@ pair_sum_kernel(const float2* __restrict__ t, float* __restrict__ y, int64_t n) 
 }
 
 template <typename K, typename... Args>
-static cudaError_t launch_pdl(K kernel, dim3 grid, const DeviceState& ds, Args... args) {
+static cudaError_t launch_pdl_t(K kernel, dim3 grid, int threads, const DeviceState& ds, Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
-    cfg.blockDim = dim3(256);
+    cfg.blockDim = dim3((unsigned)threads);
     cfg.stream = ds.stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -169,15 +223,22 @@ static cudaError_t launch_pdl(K kernel, dim3 grid, const DeviceState& ds, Args..
     cfg.numAttrs = ds.pdl ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
+template <typename K, typename... Args>
+static cudaError_t launch_pdl(K kernel, dim3 grid, const DeviceState& ds, Args... args) {
+    return launch_pdl_t(kernel, grid, 256, ds, args...);
+}
 
 int32_t launch_quant_act_q8k(rstq_ctx* ctx, DeviceState& ds, const float* x, int8_t* xq, float* xs, float* xs32,
-                             int32_t* bsums, int64_t rows, int64_t in, int sub) {
-    const int64_t ctas = rows * (in / 256);
-    RSTQ_REQUIRE(ctas >= 1 && ctas < (1ll << 31), RSTQ_E_LIMIT, "rows * in / 256 = %lld", (long long)ctas);
+                             int32_t* bsums, int64_t rows, int64_t in, int sub, uint8_t* img, int zp) {
+    constexpr int kWarps = kQ8kThreads / 32;
+    const int64_t n = rows * (in / 256), ctas = (n + kWarps - 1) / kWarps;
+    RSTQ_REQUIRE(n >= 1 && n < (1ll << 31), RSTQ_E_LIMIT, "rows * in / 256 = %lld", (long long)n);
+    const dim3 grid((unsigned)ctas);
+    const int nb = (int)(in / 32);
     if (sub == 16)
-        RSTQ_CUDA(launch_pdl(quant_act_q8k_kernel<16>, dim3((unsigned)ctas), ds, x, xq, xs, xs32, bsums));
+        RSTQ_CUDA(launch_pdl_t(quant_act_q8k_kernel<16>, grid, kQ8kThreads, ds, x, xq, xs, xs32, bsums, n, img, (int)rows, nb, zp));
     else
-        RSTQ_CUDA(launch_pdl(quant_act_q8k_kernel<32>, dim3((unsigned)ctas), ds, x, xq, xs, xs32, bsums));
+        RSTQ_CUDA(launch_pdl_t(quant_act_q8k_kernel<32>, grid, kQ8kThreads, ds, x, xq, xs, xs32, bsums, n, img, (int)rows, nb, zp));
     ctx->launches++;
     return RSTQ_OK;
 }

@@ -316,3 +316,66 @@ def test_operators_reproduce_k_quant_golden_vectors(ctx):
         assert relerr(by.download(), G[key]) <= 1e-5
     for o in (w4, w6, bx, by):
         o.free()
+
+
+def hard_super_blocks(n, seed):
+    """n super-blocks: maxima over f32's range, elements on and next to every k + 0.5 of their scale."""
+    rng = np.random.default_rng(seed)
+    tops = [0.0, 1e-38, 9.9e-31, 1.1e-30, 1e-5, 1.0, 127.0, 9e36, 1.1e37, 3.3e38]
+    x = np.empty((n, 256), np.float32)
+    for i in range(n):
+        top = np.float32(tops[rng.integers(0, len(tops))])
+        v = ((rng.integers(-127, 127, 256) + 0.5) * (np.float64(top) / 127.0)).astype(np.float32)
+        if rng.integers(0, 2):
+            v = np.nextafter(v, np.where(rng.integers(0, 2, 256) == 1, np.inf, -np.inf).astype(np.float32))
+        x[i] = rng.standard_normal(256).astype(np.float32) if i % 3 == 0 else np.clip(v, -top, top)
+        x[i, rng.integers(0, 256)] = top if i % 3 else np.float32(3.0)
+    return x.ravel()
+
+
+@pytest.mark.parametrize("rows,in_,sub", [(1, 256, 16), (1, 256, 32), (3, 256, 32), (7, 2304, 16), (40, 1280, 32)])
+def test_q8k_quantizer_at_ties_and_extremes(ctx, rows, in_, sub):
+    x = hard_super_blocks(rows * in_ // 256, rows + sub)
+    n, nsb = rows * in_, rows * in_ // 256
+    bx = ctx.array_to_buffer(x)
+    bq, bs, bb = ctx.make_buffer(n + 64, np.int8), ctx.make_buffer(nsb + 4, np.float32), ctx.make_buffer(n // sub + 16, np.int32)
+    for b in (bq, bs, bb):
+        b.fill_bytes(0x5A)
+    ctx.quant_act_q8k(bx, bq, bs, bb, rows, in_, sub)
+    ctx.sync()
+    gq, gs, gb = bq.download(), bs.download().view(np.uint32), bb.download()
+    xq, xs, bsums = orc.quantize_act_q8k(x, n, sub)
+    assert np.array_equal(gq[:n], xq) and np.array_equal(gs[:nsb], xs.view(np.uint32)) and np.array_equal(gb[:n // sub], bsums)
+    assert (gq[n:] == 0x5A).all() and (gs[nsb:] == 0x5A5A5A5A).all() and (gb[n // sub:] == 0x5A5A5A5A).all()
+    for b in (bx, bq, bs, bb):
+        b.free()
+
+
+@pytest.mark.parametrize("fmt", ["q4k", "q6k"])
+@pytest.mark.parametrize("out,in_", [(40, 256), (200, 2304), (96, 8192)])
+@pytest.mark.parametrize("M", [2, 3, 8, 9, 16, 17, 18, 35])   # odd and even, one and two token tiles, several launches, a last one of one token
+def test_kquant_tokens_laid_out_by_the_quantizer(ctx, fmt, out, in_, M):
+    """The quantizer writes what the decode launches read, one array per 16 tokens; a call with pre-quantized activations
+    after it uses its own."""
+    W, x, x2 = synth.normal(in_ + out, out * in_, 0.02), synth.normal(in_ + M, M * in_), synth.normal(in_ + M + 1, M * in_)
+    if fmt == "q4k":
+        e = orc.quantize_weight_q4k(W)
+        w, rows_of, sub = ctx.bind_weight_q4k(e, out, in_), oracle_rows, 32
+    else:
+        e = orc.quantize_weight_q6k(W)
+        w, rows_of, sub = ctx.bind_weight_q6k(e, out, in_), oracle_rows_q6k, 16
+    bx, by = ctx.array_to_buffer(x), ctx.make_buffer(M * out, np.float32)
+    by.fill_bytes(0xFF)
+    ctx.qmatmul(w, bx, by, M, L.F32, L.F32, L.MODE_A8)
+    ctx.sync()
+    got, ref = by.download().reshape(M, out), rows_of(e, x, M, in_, out).reshape(M, out)
+    assert (np.abs(got - ref).max(1) <= 1e-5 * np.abs(ref).max(1)).all()
+    q, s, z = ctx.make_buffer(M * in_, np.int8), ctx.make_buffer(M * in_ // 256, np.float32), ctx.make_buffer(M * in_ // sub, np.int32)
+    bx2 = ctx.array_to_buffer(x2)
+    ctx.quant_act_q8k(bx2, q, s, z, M, in_, sub)
+    ctx.qmatmul_prequant(w, q, s, z, by, M)
+    ctx.sync()
+    got, ref = by.download().reshape(M, out), rows_of(e, x2, M, in_, out).reshape(M, out)
+    assert (np.abs(got - ref).max(1) <= 1e-5 * np.abs(ref).max(1)).all()
+    for b in (bx, by, q, s, z, bx2, w):
+        b.free()
