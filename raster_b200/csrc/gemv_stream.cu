@@ -496,6 +496,28 @@ act_image_f_kernel(const void* __restrict__ x, uint2* __restrict__ img, int M, i
     }
 }
 
+// bf16 activations (one term): a thread lays out half a block of a token, 16 elements, in thread blocks of 64 (few warps in small
+// thread blocks, as quant_act_i8_kernel).  us a call, int4, with an entry of 8 bytes per thread in thread blocks of 256 before:
+// 70B-class MLP at 16 tokens 107.4 -> 105.2 for both matrices, 4096 x 11008 at 8 12.43 -> 11.16, 11008 x 4096 and 4096 x 11008 at 8
+// 29.2 -> 28.9.  (f32 terms lose up to 5 % that way; a tensor map on x instead of this kernel, a copy per chunk of 64-byte
+// rows: 4096 x 11008 at 8 10.8, but 28672 x 8192 at 8 38.9 -> 42.7.)
+constexpr int kImageFThreads = 64;
+__global__ void __launch_bounds__(kImageFThreads)
+act_image_bf16_kernel(const uint4* __restrict__ x, uint4* __restrict__ img, int M, int nb) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int64_t n = (int64_t)nb * 2 * M, step = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < n; o += step) {   // o = half block * M + token
+        const int64_t bh = o / M;
+        const uint4* src = x + ((o - bh * M) * nb * 2 + bh) * 2;
+        const uint4 a = src[0], b = src[1];
+        auto entry = [](uint32_t lo, uint32_t hi) { return make_uint2(__byte_perm(lo, hi, 0x5410), __byte_perm(lo, hi, 0x7632)); };
+        const uint2 e0 = entry(a.x, a.y), e1 = entry(a.z, a.w), e2 = entry(b.x, b.y), e3 = entry(b.z, b.w);
+        img[o * 2] = make_uint4(e0.x, e0.y, e1.x, e1.y);
+        img[o * 2 + 1] = make_uint4(e2.x, e2.y, e3.x, e3.y);
+    }
+}
+
 // ---- one unit (32 rows x one 32-element block) from the ring ------------------------
 // UK: unit kind beyond the plain one: 1 = Q4_K (32 minima behind the scales), 2 = Q6_K (8-bit codes, 64
 // scales: for row gid + 8i of the group the scales of elements 0..15 and 16..31 at floats (gid*4 + i)*2 + h)
@@ -2126,20 +2148,23 @@ int32_t launch_gemv_f(rstq_ctx* ctx, DeviceState& ds, const GemvFArgs& a) {
         if (pl.ring) {
             // the staged array of this launch's tokens, built by a kernel of its own; the decode kernel's copy
             // thread waits for that grid before the first slice, as it does for the quantizer in mode A8
-            const int64_t n = nb * 8 * C;
-            int64_t ctas = (n + 255) / 256;
-            if (ctas > (int64_t)ds.sm_count * 8) ctas = (int64_t)ds.sm_count * 8;
+            const bool bf = a.act_dtype == RSTQ_BF16;
+            const int threads = bf ? kImageFThreads : 256;
+            const int64_t n = bf ? nb * 2 * M : nb * 8 * C;
+            int64_t ctas = (n + threads - 1) / threads;
+            if (ctas > (int64_t)ds.sm_count * (2048 / threads)) ctas = (int64_t)ds.sm_count * (2048 / threads);
             cudaLaunchConfig_t cfg = {};
             cfg.gridDim = dim3((unsigned)ctas);
-            cfg.blockDim = dim3(256);
+            cfg.blockDim = dim3((unsigned)threads);
             cfg.stream = ds.stream;
             cudaLaunchAttribute attr[1];
             attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
             attr[0].val.programmaticStreamSerializationAllowed = 1;
             cfg.attrs = attr;
             cfg.numAttrs = ds.pdl ? 1 : 0;
-            RSTQ_CUDA(cudaLaunchKernelEx(&cfg, act_image_f_kernel, p.x, reinterpret_cast<uint2*>(a.img_scratch), M, T,
-                                         (int)nb, a.in, a.act_dtype));
+            if (bf) RSTQ_CUDA(cudaLaunchKernelEx(&cfg, act_image_bf16_kernel, (const uint4*)p.x, (uint4*)a.img_scratch, M, (int)nb));
+            else RSTQ_CUDA(cudaLaunchKernelEx(&cfg, act_image_f_kernel, p.x, reinterpret_cast<uint2*>(a.img_scratch), M, T,
+                                              (int)nb, a.in, a.act_dtype));
             ctx->launches++;
             p.img = a.img_scratch;
             p.slice1 = (uint32_t)(2 * C * 32);

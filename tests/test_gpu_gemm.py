@@ -222,3 +222,21 @@ def test_activation_rows_at_the_edges_of_the_pre_pass(ctx, mode, M, act, in_):
     for rows in (slice(0, 1), slice(1, 2), slice(2, M)):
         assert relerr(y[rows], ref[rows]) <= 1e-3
     bx.free(), by.free(), bw.free()
+
+
+@pytest.mark.parametrize("M,in_", [(3, 28704), (5, 16416), (13, 11040), (16, 8224)])   # half blocks that fill no thread block
+def test_bf16_tokens_laid_out_for_the_decode_ring(ctx, M, in_):
+    out = 40
+    w = synth.normal(in_, out * in_, 0.02)
+    wq, ws = orc.quantize_weight(w, 4)
+    bits = synth.to_bf16_bits(synth.normal(in_ + M, M * in_))
+    x = synth.from_bf16_bits(bits)
+    bw = ctx.bind_weight(wq, ws, out, in_, L.FMT_Q4_0, L.LAYOUT_ROWMAJOR)
+    bx, by = ctx.array_to_buffer(bits), ctx.make_buffer(M * out, np.float32)
+    by.fill_bytes(0xFF)
+    ctx.qmatmul(bw, bx, by, M, L.BF16, L.F32, L.MODE_F)
+    ctx.sync()
+    ref = orc.matmul_dq_f64(wq, ws, 0, x, M, in_, out).reshape(M, out)
+    got = by.download().reshape(M, out)
+    assert (np.abs(got - ref).max(1) <= 4e-6 * np.abs(ref).max(1)).all()   # exact products, f32 sums: TOL_A8 of test_gpu_parity
+    bx.free(), by.free(), bw.free()
