@@ -43,6 +43,24 @@ int32_t use_dev(rstq_ctx* ctx, int dev) {
     return RSTQ_OK;
 }
 
+static void drop_spare_weights(DeviceState& ds) {
+    for (auto& b : ds.spare_weights) cudaFree(b.first);
+    ds.spare_weights.clear();
+    ds.spare_bytes = 0;
+}
+// cudaMalloc; before it fails, the arrays kept for weights to come are given back
+static cudaError_t dev_malloc(DeviceState& ds, void** p, int64_t bytes) {
+    *p = nullptr;
+    cudaError_t e = cudaMalloc(p, (size_t)bytes);
+    if (e != cudaSuccess && !ds.spare_weights.empty()) {
+        cudaGetLastError();
+        drop_spare_weights(ds);
+        e = cudaMalloc(p, (size_t)bytes);
+    }
+    if (e != cudaSuccess) *p = nullptr;
+    return e;
+}
+
 // grow-only scratch helpers (never called while capturing)
 int32_t dev_reserve(DeviceState& ds, void** p, int64_t* have, int64_t need) {
     if (need <= *have) return RSTQ_OK;
@@ -56,7 +74,7 @@ int32_t dev_reserve(DeviceState& ds, void** p, int64_t* have, int64_t need) {
         *have = 0;
     }
     need = (need + 0xFFFFF) & ~0xFFFFFll;
-    RSTQ_CUDA(cudaMalloc(p, (size_t)need));
+    RSTQ_CUDA(dev_malloc(ds, p, need));
     *have = need;
     return RSTQ_OK;
 }
@@ -378,6 +396,35 @@ static cudaError_t put_products(rstq_ctx* ctx, DeviceState& ds, const ProductSca
     return cudaGetLastError();
 }
 static int64_t products_tmp_bytes(int64_t n, int per) { return ((n / per * 4 + 255) & ~255ll) + ((n + 255) & ~255ll); }
+// Device arrays of weights.  cudaMalloc and cudaFree of a 10 MB matrix take 0.4 .. 1.4 and 0.35 .. 1.2 ms, more than its copies, so
+// the arrays of weights that are gone serve the next ones of their size (a 4096 x 4096 int4 matrix that takes another one's
+// place: 3.6 -> 2.9 ms).  Up to kWeightKeep bytes per device are kept, and given back before an allocation fails and with
+// the context.  Like cudaFree, giving an array back waits for the whole device.  (A driver's memory pool instead is as fast
+// here, but matrices that lie in it stream 1 - 2 % slower at one token.)
+static cudaError_t weight_malloc(DeviceState& ds, void** p, int64_t bytes) {
+    for (size_t i = ds.spare_weights.size(); i-- > 0;)
+        if (ds.spare_weights[i].second == bytes) {
+            *p = ds.spare_weights[i].first;
+            ds.spare_weights.erase(ds.spare_weights.begin() + i);
+            ds.spare_bytes -= bytes;
+            return cudaSuccess;
+        }
+    return dev_malloc(ds, p, bytes);
+}
+// (the device is current)
+static void weight_release(DeviceState& ds, void* p, int64_t bytes) {
+    if (!p) return;
+    if (!ds.capturing && ds.spare_bytes + bytes <= kWeightKeep && cudaDeviceSynchronize() == cudaSuccess) {
+        try {
+            ds.spare_weights.emplace_back(p, bytes);
+            ds.spare_bytes += bytes;
+            return;
+        } catch (...) {      // no room for the note
+        }
+    }
+    cudaGetLastError();
+    cudaFree(p);
+}
 static void trim_bind_stage(DeviceState& ds, int64_t keep = kBindStageKeep) {
     if (ds.bind_stage_bytes <= keep) return;
     cudaFree(ds.bind_stage);
@@ -474,7 +521,7 @@ static int32_t bind_impl(rstq_ctx* ctx, rstq_weight** wout, const void* codes,
     }
     uint8_t* stage_c = (uint8_t*)ds.bind_stage;
     float* stage_s = (float*)(stage_c + scales_off);
-    cudaError_t e = cudaMalloc((void**)&w->data, (size_t)w->data_bytes);
+    cudaError_t e = weight_malloc(ds, (void**)&w->data, w->data_bytes);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(stage_c, hcodes, (size_t)codes_bytes, cudaMemcpyHostToDevice, ds.stream);
     if (e == cudaSuccess) {
@@ -488,7 +535,7 @@ static int32_t bind_impl(rstq_ctx* ctx, rstq_weight** wout, const void* codes,
     }
     trim_bind_stage(ds);
     if (e != cudaSuccess || rc != RSTQ_OK) {
-        if (w->data) cudaFree(w->data);
+        weight_release(ds, w->data, w->data_bytes);
         delete w;
         if (e != cudaSuccess) return cuda_fail(e, "weight bind", __FILE__, __LINE__);
         return rc;
@@ -624,6 +671,7 @@ int32_t rstq_shutdown(rstq_ctx* ctx) {
         if (ds.dbg_store) cudaFree(ds.dbg_store);
         if (ds.io_dev) cudaFree(ds.io_dev);
         if (ds.pinned) cudaFreeHost(ds.pinned);
+        drop_spare_weights(ds);
         if (ds.own_stream) cudaStreamDestroy(ds.own_stream);
     }
     cudaGetLastError();
@@ -799,7 +847,7 @@ int32_t rstq_alloc(rstq_ctx* ctx, rstq_buf** buf, int32_t dev, int64_t bytes) {
     int32_t rc = use_dev(ctx, dev);
     if (rc != RSTQ_OK) return rc;
     void* p = nullptr;
-    RSTQ_CUDA(cudaMalloc(&p, (size_t)bytes));
+    RSTQ_CUDA(dev_malloc(ctx->devs[dev], &p, bytes));
     rstq_buf* b = new (std::nothrow) rstq_buf{kBufMagic, ctx, dev, p, bytes, true};
     if (!b) {
         cudaFree(p);
@@ -933,8 +981,7 @@ int32_t rstq_weight_bind_q4k(rstq_ctx* ctx, rstq_weight** wout, const void* wq, 
         rstq_weight_free(w);
         return rc;
     }
-    cudaError_t e = cudaMalloc((void**)&w->mins, (size_t)n * 4);
-    if (e != cudaSuccess) w->mins = nullptr;
+    cudaError_t e = weight_malloc(ds, (void**)&w->mins, n * 4);
     if (e == cudaSuccess) e = put_products(ctx, ds, b, w->mins, n, ds.bind_stage);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ds.stream);
     trim_bind_stage(ds);
@@ -946,17 +993,17 @@ int32_t rstq_weight_bind_q4k(rstq_ctx* ctx, rstq_weight** wout, const void* wq, 
         // the minima move into the units (768 B): the decode kernel folds them, no third kernel
         const int64_t kbytes = (w->outp / 32) * w->nb * kUnitBytesQ4K;
         uint8_t* kdata = nullptr;
-        e = cudaMalloc((void**)&kdata, (size_t)kbytes);
+        e = weight_malloc(ds, (void**)&kdata, kbytes);
         if (e == cudaSuccess) {
             rc = launch_q4k_units(ctx, ds, w->data, w->mins, kdata, w->out, w->nb);
             if (rc == RSTQ_OK) e = cudaStreamSynchronize(ds.stream);
         }
         if (e != cudaSuccess || rc != RSTQ_OK) {
-            if (kdata) cudaFree(kdata);
+            weight_release(ds, kdata, kbytes);
             rstq_weight_free(w);
             return rc != RSTQ_OK ? rc : cuda_fail(e, "Q4_K units", __FILE__, __LINE__);
         }
-        cudaFree(w->data);
+        weight_release(ds, w->data, w->data_bytes);
         w->data = kdata;
         w->data_bytes = kbytes;
         w->kq = true;
@@ -993,7 +1040,7 @@ int32_t rstq_weight_bind_q6k(rstq_ctx* ctx, rstq_weight** wout, const void* wq, 
         float* d16 = (float*)ds.bind_stage;
         const int64_t kbytes = (w->outp / 32) * w->nb * kUnitBytesQ6K;
         uint8_t* kdata = nullptr;
-        cudaError_t e = cudaMalloc((void**)&kdata, (size_t)kbytes);
+        cudaError_t e = weight_malloc(ds, (void**)&kdata, kbytes);
         if (e == cudaSuccess) e = put_products(ctx, ds, s16, d16, n16, (char*)ds.bind_stage + d16_bytes);
         if (e == cudaSuccess) {
             rc = launch_q6k_units(ctx, ds, w->data, d16, kdata, out, w->nb);
@@ -1001,11 +1048,11 @@ int32_t rstq_weight_bind_q6k(rstq_ctx* ctx, rstq_weight** wout, const void* wq, 
         }
         trim_bind_stage(ds);
         if (e != cudaSuccess || rc != RSTQ_OK) {
-            if (kdata) cudaFree(kdata);
+            weight_release(ds, kdata, kbytes);
             rstq_weight_free(w);
             return rc != RSTQ_OK ? rc : cuda_fail(e, "Q6_K units", __FILE__, __LINE__);
         }
-        cudaFree(w->data);
+        weight_release(ds, w->data, w->data_bytes);
         w->data = kdata;
         w->data_bytes = kbytes;
         w->zp = 32;
@@ -1056,17 +1103,17 @@ int32_t rstq_weight_clone(rstq_weight* src, rstq_weight** wout) {
     w->raw_scales = nullptr;
     w->mins = nullptr;
     const size_t min_bytes = (size_t)(src->out * src->nb * 4);
-    cudaError_t e = cudaMalloc((void**)&w->data, (size_t)w->data_bytes);
+    cudaError_t e = weight_malloc(ds, (void**)&w->data, w->data_bytes);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(w->data, src->data, (size_t)w->data_bytes, cudaMemcpyDeviceToDevice,
                             ds.stream);
-    if (e == cudaSuccess && src->mins) e = cudaMalloc((void**)&w->mins, min_bytes);
+    if (e == cudaSuccess && src->mins) e = weight_malloc(ds, (void**)&w->mins, (int64_t)min_bytes);
     if (e == cudaSuccess && src->mins)
         e = cudaMemcpyAsync(w->mins, src->mins, min_bytes, cudaMemcpyDeviceToDevice, ds.stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ds.stream);
     if (e != cudaSuccess) {
-        if (w->data) cudaFree(w->data);
-        if (w->mins) cudaFree(w->mins);
+        weight_release(ds, w->data, w->data_bytes);
+        weight_release(ds, w->mins, (int64_t)min_bytes);
         delete w;
         return cuda_fail(e, "weight clone", __FILE__, __LINE__);
     }
@@ -1084,10 +1131,10 @@ int32_t rstq_weight_free(rstq_weight* w) {
     if (ds.last_decode_w == w) ds.last_decode_w = nullptr;
     cudaSetDevice(ds.ordinal);
     if (!ds.capturing) cudaStreamSynchronize(ds.stream);
-    cudaFree(w->data);
+    weight_release(ds, w->data, w->data_bytes);
+    weight_release(ds, w->mins, w->out * w->nb * 4);
     if (w->raw_codes) cudaFree(w->raw_codes);
     if (w->raw_scales) cudaFree(w->raw_scales);
-    if (w->mins) cudaFree(w->mins);
     cudaGetLastError();
     w->magic = 0;
     delete w;
@@ -1439,8 +1486,8 @@ int32_t rstq_qlinear_q8_dx(rstq_ctx* ctx, const float* dy, const void* codes, co
     if ((rc = use_dev(ctx, w->dev)) != RSTQ_OK) return rc;
     if (!w->raw_codes) {  // the transposed product reads W as the reference stores it
         const int64_t cb = out * in, sb = out * (in / 32) * 4;
-        RSTQ_CUDA(cudaMalloc((void**)&w->raw_codes, (size_t)cb));
-        RSTQ_CUDA(cudaMalloc((void**)&w->raw_scales, (size_t)sb));
+        RSTQ_CUDA(dev_malloc(ds, (void**)&w->raw_codes, cb));
+        RSTQ_CUDA(dev_malloc(ds, (void**)&w->raw_scales, sb));
         RSTQ_CUDA(cudaMemcpyAsync(w->raw_codes, codes, (size_t)cb, cudaMemcpyHostToDevice, ds.stream));
         RSTQ_CUDA(cudaMemcpyAsync(w->raw_scales, scales, (size_t)sb, cudaMemcpyHostToDevice, ds.stream));
         RSTQ_CUDA(cudaStreamSynchronize(ds.stream));

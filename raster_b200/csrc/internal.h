@@ -115,6 +115,9 @@ struct DeviceState {
     std::vector<void*> kept;       // outgrown blocks that such a graph may name: freed with the context
     void* bind_stage = nullptr;    // the host arrays of the weight being bound, before they are re-tiled (at most
     int64_t bind_stage_bytes = 0;  // kBindStageKeep bytes are kept between binds)
+    // arrays of weights that are gone, kept for the next one of the same size: at most kWeightKeep bytes
+    std::vector<std::pair<void*, int64_t>> spare_weights;
+    int64_t spare_bytes = 0;
     int* status = nullptr;         // device status word: nonzero after a bounded wait ran out
     // Instantiated graphs hold the scratch addresses of the launches they recorded.  While any is
     // alive, scratch that has to grow is parked here instead of freed, so a replay never touches
@@ -127,6 +130,7 @@ struct DeviceState {
 };
 
 constexpr int64_t kBindStageKeep = 64ll << 20;
+constexpr int64_t kWeightKeep = 64ll << 20;
 
 }  // namespace rstq
 

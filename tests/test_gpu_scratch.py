@@ -80,3 +80,54 @@ def test_backward_recorded_in_a_graph_of_the_caller(ctx):
         ctx.set_stream(None)
     for b in bufs + big + other:
         b.free()
+
+
+def quant_arrays(n, seed):
+    rng = np.random.default_rng(seed)
+    return rng.integers(0, 256, n * n // 2, dtype=np.uint8), (rng.standard_normal(n * n // 32) * 0.01).astype(np.float32)
+
+
+def dense(codes, scales, n):
+    b = codes.reshape(-1, 16)
+    return (np.concatenate([b & 15, b >> 4], 1).astype(np.float64) - 8) * scales[:, None].astype(np.float64)
+
+
+def test_an_array_that_serves_the_next_weight_of_its_size_holds_that_weight(ctx):
+    """A weight takes the place of one that is gone, with a product of the old one still under way when that is freed; one of
+    another size does not, and two alive at once have an array each."""
+    n = 2048
+    x = np.random.default_rng(1).standard_normal(n).astype(np.float32)
+    bx = ctx.array_to_buffer(x)
+    w, ys = None, []
+    for seed in range(6):
+        a = quant_arrays(n, seed)
+        if w is not None:
+            ctx.qmatmul(w, bx, ys[-1][1], 1, L.F32, L.F32, L.MODE_F)
+            w.free()                                  # waits for the product
+        w = ctx.bind_weight(*a, n, n, L.FMT_Q4_0, L.LAYOUT_ROWMAJOR)
+        ys.append((a, ctx.make_buffer(n, np.float32)))
+    other = ctx.bind_weight(*quant_arrays(1024, 9), 1024, 1024, L.FMT_Q4_0, L.LAYOUT_ROWMAJOR)
+    twin = ctx.bind_weight(*ys[0][0], n, n, L.FMT_Q4_0, L.LAYOUT_ROWMAJOR)
+    ctx.qmatmul(w, bx, ys[-1][1], 1, L.F32, L.F32, L.MODE_F)
+    ctx.sync()
+    for a, by in ys:
+        ref = dense(*a, n).reshape(n, n) @ x.astype(np.float64)
+        assert np.abs(by.download() - ref).max() <= 2e-5 * np.abs(ref).max()
+    for b in (w, other, twin, bx, *(y for _, y in ys)):
+        b.free()
+
+
+def test_arrays_of_weights_that_are_gone_are_bounded_and_go_with_the_context():
+    torch.cuda.synchronize()
+    c = Context(("cuda:0",))
+    try:
+        c.bind_weight(*quant_arrays(512, 0), 512, 512, L.FMT_Q4_0, L.LAYOUT_ROWMAJOR).free()
+        start = torch.cuda.mem_get_info()[0]
+        for n in (4096, 4224, 4352, 4480, 4608, 4736, 4864, 4992, 5120, 8192, 14336):   # 10 .. 129 MB
+            c.bind_weight(*quant_arrays(n, n), n, n, L.FMT_Q4_0, L.LAYOUT_ROWMAJOR).free()
+        # at most 64 MB of arrays and 64 MB of staging stay, in allocations of 2 MB
+        assert start - torch.cuda.mem_get_info()[0] <= (64 + 64 + 32) << 20
+    finally:
+        before = torch.cuda.mem_get_info()[0]
+        c.close()
+    assert torch.cuda.mem_get_info()[0] - before >= 40 << 20
