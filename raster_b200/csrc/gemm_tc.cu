@@ -189,6 +189,7 @@ struct GemmParams {
     int* part_flags;        // one word per CTA, zero between launches: set when its `part` is complete
     float wmul, wdiv;       // 2^ew applied to the block scales, 2^-ew applied to the result
     int out_dtype;
+    int cols;               // pairs of CTAs: columns of a tile that are computed (a multiple of 16)
     unsigned long long* dbg;  // optional timeline of CTA 0 (see RSTQ_TUNE_TIMELINE), or null
 };
 
@@ -664,6 +665,11 @@ gemm_tmem_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tmap) {
     }
     const int fd = tile_first / p.ttiles, ft_first = fd * CS + (int)rank, tok_first = (tile_first - fd * p.ttiles) * NTOK;
 
+    // DUO: the columns of a tile that hold tokens, in sixteens, where one tile takes all tokens: narrower MMAs.  (The rest of its
+    // columns is never written, and what is read there goes nowhere.  int4 28672 x 8192 at M = 160 91.4 -> 85.6 us, 8192 x 28672 at
+    // M = 200 94.6 -> 91.8.  Worked out per tile, for several, full tiles lose 1.4 %.)
+    const int cols = DUO ? p.cols : NTOK;
+
     if (tid == 0) asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmap)) : "memory");
     if (warp >= 2 && warp < 2 + kDqWarps) {
         // the first weights this warp will load: ask for them now, so that the HBM round trip
@@ -741,6 +747,7 @@ gemm_tmem_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tmap) {
                     for (int k2 = 0; k2 < 8 + kPfSteps; k2 += 4) request(k2);
                     ok = mbar_block(acc_free, (uint32_t)(seg - 1) & 1u, abort_flag);
                 }
+                const int row0 = tok0 + (DUO ? (int)rank * (cols / 2) : 0);   // a pair's second CTA holds the upper half of the columns
                 for (int ks = 0; ks < n && ok; ++ks) {
                     // weight requests: none before the wait above (they would compete for HBM with the
                     // pre-pass this kernel waits for) nor before the first activation tiles are on their
@@ -752,8 +759,8 @@ gemm_tmem_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tmap) {
                     if (!ok) break;
                     const uint32_t dst = sbase + s * BSTAGE;
                     mbar_expect_tx(full + 8 * s, BSTAGE);
-                    tma_load_2d(dst, &tmap, (k0 + ks) * kKStep, tok0 + (int)rank * BROWS, full + 8 * s);
-                    tma_load_2d(dst + BROWS * 128, &tmap, (k0 + ks) * kKStep + 64, tok0 + (int)rank * BROWS, full + 8 * s);
+                    tma_load_2d(dst, &tmap, (k0 + ks) * kKStep, row0, full + 8 * s);
+                    tma_load_2d(dst + BROWS * 128, &tmap, (k0 + ks) * kKStep + 64, row0, full + 8 * s);
                     ++issued;
                     if (++s == kNSTT) { s = 0; ph ^= 1u; }
                 }
@@ -811,7 +818,7 @@ gemm_tmem_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tmap) {
         // warp-uniform) and lane 0 alone issues the tensor-core instructions.
         const int m = warp == 1 ? 0 : 1;
         const uint32_t leader = lane == 0;
-        constexpr uint32_t idesc = DUO ? idesc_f16_pair(NTOK) : idesc_f16(NTOK);
+        const uint32_t idesc = DUO ? idesc_f16_pair(cols) : idesc_f16(NTOK);
         auto commit = [&](uint32_t bar) {
             if constexpr (DUO) umma_commit2_if(bar, leader);
             else umma_commit_if(bar, leader);
@@ -1385,6 +1392,7 @@ int32_t launch_gemm(rstq_ctx* ctx, DeviceState& ds, const rstq_weight* w, const 
     p.wmul = ldexpf(1.0f, w->gemm_exp + (a_in_tmem ? kSubnormalShift : 0));
     p.wdiv = ldexpf(1.0f, -w->gemm_exp + (a_in_tmem ? 24 - kSubnormalShift : 0));
     p.out_dtype = out_dtype;
+    p.cols = p.ttiles == 1 ? (int)std::min<int64_t>(ntok, (M + 15) & ~15ll) : ntok;
     p.dbg = ds.dbg;
     RSTQ_REQUIRE(ftiles * p.ttiles < (1ll << 30), RSTQ_E_LIMIT, "grid too large");
     // (units: thread blocks, or pairs of them on tiles of 256 features)
