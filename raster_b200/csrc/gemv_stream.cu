@@ -1655,23 +1655,32 @@ struct StreamPlan {
     int64_t in_flight() const { return (int64_t)(NS - 1) * cu; }   // units on their way while one chunk is consumed
 };
 
-// Measured on B200 at 14 shapes from 512x4096 to 28672x8192 (int4 and int8, M = 1..8): whole
-// groups were faster every time, by 3 % (64 groups) to 37 % (Llama-7B shapes), even with only 32 of
-// 148 SMs holding a CTA.  The equal-range split is kept for matrices so flat that a handful of
-// CTAs would each have to stream many megabytes.
-// Two token tiles (9 .. 16 tokens): the loop is bound by the consumers, so SMs left without a thread block cost
-// their share: 70B-class matrices (7 groups per block, 128 of 148 SMs busy) gain 3 - 6 % from the equal-range
-// split, the 7B shapes (3 groups per block) still lose 7 - 15 % to its hand-overs.
-static bool whole_groups_pay(int64_t groups, int64_t nb, int64_t k, int64_t Gw, int sm_count, int unit, int nt) {
-    (void)groups;
-    const int64_t bytes_per_cta = k * nb * unit;
-    if (nt >= 2 && Gw * 8 < sm_count * 7 && bytes_per_cta >= (1ll << 20)) return false;
-    return !(Gw * 2 < sm_count && bytes_per_cta > (4ll << 20));
+// Which loop a launch runs: one token of MODE_A8, several, or MODE_F.
+enum StreamLoop { LOOP_ONE, LOOP_A8, LOOP_F };
+
+// Whole groups leave SMs idle when the groups do not divide evenly over them; an equal-range split feeds all of
+// them and pays a hand-over of partial sums (a few us at the end) instead.  What decides is the difference of the
+// two: the bytes by which the equal split shortens each CTA's stream.  Measured on B200 over 7 formats and modes,
+// 300 .. 28672 rows, K = 4096 .. 28672, M = 1 .. 16 (time of whole groups / of equal ranges):
+//   MODE_F, and several tokens of K-quant units: 0.86 - 1.03 below 144 KB (0.99 - 1.01 next to it), 1.00 - 1.09 at
+//   150 - 230 KB, 1.1 - 1.5 at 300 - 600 KB, up to 2.8 above.
+//   Several tokens of plain units (MODE_A8): 0.77 - 1.06 below 288 KB, 1.02 - 1.24 at 300 - 400 KB, up to 1.9 above;
+//   9 .. 16 tokens lie a little better and take 1 MB per CTA with an eighth of the SMs idle as well (70B-class
+//   matrices gain 3 - 6 %, the 7B shapes still lose 7 - 15 %).
+//   One token (MODE_A8; its whole groups stream without any of the reduction's barriers): 0.80 - 1.13 below
+//   576 KB, 1.1 - 1.9 above it, and no line in the units' format.
+static bool whole_groups_pay(int64_t nb, int64_t k, int64_t Gw, int sm_count, int bits, int nt, StreamLoop loop) {
+    const int64_t per_cta = k * nb * unit_bytes(bits);
+    const int64_t saved = per_cta - per_cta * Gw / sm_count;
+    if (nt >= 2 && Gw * 8 < sm_count * 7 && per_cta >= (1ll << 20)) return false;
+    const bool kq = bits == 5 || bits == 6;
+    const int64_t line = loop == LOOP_ONE ? 576 : (loop == LOOP_F || kq ? 144 : 288);
+    return saved <= line << 10;
 }
 
 // How the units of a weight are cut over the CTAs of a launch: G ranges, CTA c owns uq (+1 if c < ur).
 static void split_units(const DeviceState& ds, int bits, int64_t groups, int64_t nb, int* Gout, int64_t* uq,
-                        int64_t* ur, int nt = 1) {
+                        int64_t* ur, int nt, StreamLoop loop) {
     const int kChunkUnits = chunk_units_of(bits);
     const int64_t U = groups * nb;
     int64_t G = (U + kChunkUnits - 1) / kChunkUnits;  // at least one chunk of work per CTA
@@ -1685,7 +1694,7 @@ static void split_units(const DeviceState& ds, int bits, int64_t groups, int64_t
     const int64_t k = (groups + ds.sm_count - 1) / ds.sm_count;   // groups per CTA
     const int64_t Gw = (groups + k - 1) / k;
     bool whole = ds.gemv_plan == 2;
-    if (ds.gemv_plan == 0) whole = whole_groups_pay(groups, nb, k, Gw, ds.sm_count, unit_bytes(bits), nt);
+    if (ds.gemv_plan == 0) whole = whole_groups_pay(nb, k, Gw, ds.sm_count, bits, nt, loop);
     if (whole && groups >= 1) {
         *Gout = (int)Gw;
         *uq = k * nb;
@@ -1696,13 +1705,13 @@ static void split_units(const DeviceState& ds, int bits, int64_t groups, int64_t
 // cu: units per chunk (0: the full chunk of the unit kind).  ring: act_bytes / act2_bytes are the bytes PER UNIT
 // of a chunk's slice of the activation image, which rides in the ring stage behind the weights.
 static StreamPlan plan_stream(const DeviceState& ds, int bits, int NT, int64_t groups, int64_t nb,
-                              int64_t act_bytes, int64_t act2_bytes, bool onecol = false, int cu = 0,
+                              int64_t act_bytes, int64_t act2_bytes, StreamLoop loop, int cu = 0,
                               bool ring = false) {
     StreamPlan pl{};
     if (cu <= 0) cu = chunk_units_of(bits);
     const int chunk = cu * unit_bytes(bits);
     // reduction buffers ([warp][lane] at M = 1; [warp][value][lane] otherwise, two that alternate for one tile of tokens)
-    const int64_t red = onecol ? (int64_t)(kParkGroups + 1) * kParkStride * 4 : (NT == 1 ? 2 : 1) * (int64_t)kCW * NT * 8 * 32 * 4;
+    const int64_t red = loop == LOOP_ONE ? (int64_t)(kParkGroups + 1) * kParkStride * 4 : (NT == 1 ? 2 : 1) * (int64_t)kCW * NT * 8 * 32 * 4;
     int64_t a1 = (act_bytes + 127) & ~127ll, a2 = (act2_bytes + 127) & ~127ll;
     int64_t stage = chunk, room;
     if (ring) {
@@ -1717,7 +1726,7 @@ static StreamPlan plan_stream(const DeviceState& ds, int bits, int NT, int64_t g
     if (ns > RSTQ_NSMAX) ns = RSTQ_NSMAX;
     pl.fits = ns >= 2;
     if (!pl.fits) return pl;
-    split_units(ds, bits, groups, nb, &pl.G, &pl.uq, &pl.ur, onecol ? 1 : NT);
+    split_units(ds, bits, groups, nb, &pl.G, &pl.uq, &pl.ur, NT, loop);
     pl.NS = (int)ns;
     pl.cu = cu;
     pl.ring = ring;
@@ -1827,14 +1836,15 @@ static void fill_common(StreamParams& p, const DeviceState& ds, const StreamPlan
 // every thread block's range); larger matrices are HBM-bound anyway and must not flood the L2.
 constexpr int64_t kNextPrefetchBytes = 48ll << 20;
 
-static void fill_next(StreamParams& p, const DeviceState& ds, const NextWeight& n) {
+static void fill_next(StreamParams& p, const DeviceState& ds, const NextWeight& n, StreamLoop loop) {
     p.nx_w = nullptr;
     if (!n.data || n.groups < 1 || n.nb < 1) return;
     p.nx_w = n.data;
     p.nx_unit = unit_bytes(n.bits);
     p.nx_U = n.groups * n.nb;
     // (the next launch is taken to have this one's token tiles: a decode loop runs its matrices with one M)
-    split_units(ds, n.bits, n.groups, n.nb, &p.nx_G, &p.nx_uq, &p.nx_ur, p.M * (p.T > 0 ? p.T : 1) <= 8 ? 1 : 2);
+    split_units(ds, n.bits, n.groups, n.nb, &p.nx_G, &p.nx_uq, &p.nx_ur, p.M * (p.T > 0 ? p.T : 1) <= 8 ? 1 : 2,
+                loop);
     const int64_t per_cta = kNextPrefetchBytes / p.nx_G / p.nx_unit;
     p.nx_pf_units = per_cta < 1 ? 1 : per_cta;
 }
@@ -1865,12 +1875,12 @@ static cudaError_t launch_stream_x(const DeviceState& ds, const StreamPlan& pl, 
 // Largest token count <= want whose staged activations fit next to a ring of >= 2 chunks.
 template <typename BytesFn>
 static int fit_tokens(const DeviceState& ds, int bits, int64_t groups, int64_t nb, int want, BytesFn f,
-                      StreamPlan* out, bool a8 = false) {
+                      StreamPlan* out, bool a8) {
     for (int m = want; m >= 1; --m) {
         int NT;
         int64_t a1, a2;
         f(m, &NT, &a1, &a2);
-        StreamPlan pl = plan_stream(ds, bits, NT, groups, nb, a1, a2, a8 && m == 1);
+        StreamPlan pl = plan_stream(ds, bits, NT, groups, nb, a1, a2, a8 ? (m == 1 ? LOOP_ONE : LOOP_A8) : LOOP_F);
         if (pl.fits) {
             *out = pl;
             return m;
@@ -1903,7 +1913,7 @@ static int plan_a8_piece(const DeviceState& ds, int uk, int bits, int64_t groups
         // one token of a row so long that its staged record leaves no room for two ring stages (4-bit units:
         // K > ~57 K): the general kernel with the image riding the ring serves it
         if (M < 1 && (have_img || can_make) && ds.act_ring != 1 && ds.act_ring != 4) {
-            const StreamPlan r = plan_stream(ds, ukind, 1, groups, nb, 32, 2 * rec_bytes, false, chunk_units_of(ukind), true);
+            const StreamPlan r = plan_stream(ds, ukind, 1, groups, nb, 32, 2 * rec_bytes, LOOP_A8, chunk_units_of(ukind), true);
             if (r.fits) {
                 *pl = r;
                 M = 1;
@@ -1915,9 +1925,9 @@ static int plan_a8_piece(const DeviceState& ds, int uk, int bits, int64_t groups
     const int full = chunk_units_of(ukind), half = full / 2, NTw = want <= 8 ? 1 : 2;
     const int64_t b1 = (int64_t)want * 32, b2 = (int64_t)((want + 1) & ~1) * rec_bytes;
     const bool imgs = have_img || can_make;
-    const StreamPlan res_h = plan_stream(ds, ukind, NTw, groups, nb, nb * b1, nb * b2, false, half);
-    const StreamPlan ring_f = imgs ? plan_stream(ds, ukind, NTw, groups, nb, b1, b2, false, full, true) : StreamPlan{};
-    const StreamPlan ring_h = imgs ? plan_stream(ds, ukind, NTw, groups, nb, b1, b2, false, half, true) : StreamPlan{};
+    const StreamPlan res_h = plan_stream(ds, ukind, NTw, groups, nb, nb * b1, nb * b2, LOOP_A8, half);
+    const StreamPlan ring_f = imgs ? plan_stream(ds, ukind, NTw, groups, nb, b1, b2, LOOP_A8, full, true) : StreamPlan{};
+    const StreamPlan ring_h = imgs ? plan_stream(ds, ukind, NTw, groups, nb, b1, b2, LOOP_A8, half, true) : StreamPlan{};
     const StreamPlan* pick = nullptr;
     switch (ds.act_ring) {
         case 1: break;
@@ -2024,7 +2034,7 @@ int32_t launch_gemv_a8(rstq_ctx* ctx, DeviceState& ds, const GemvA8Args& a) {
             p.img_z_off = (p.img_b_bytes + 127u) & ~127u;
         }
         if (a.tp) p.tp = *a.tp;
-        if (m0 + M >= a.M) fill_next(p, ds, a.next);   // the last piece of this call: what comes next is another weight
+        if (m0 + M >= a.M) fill_next(p, ds, a.next, M == 1 ? LOOP_ONE : LOOP_A8);   // the last piece of this call: what comes next is another weight
         cudaError_t le = cudaSuccess;
 #define LAUNCH(...)                                                                  \
     le = a.tp ? launch_stream(gemv_stream_kernel<__VA_ARGS__, true>, ds, pl, p)      \
@@ -2081,18 +2091,18 @@ static int plan_f_piece(const DeviceState& ds, int bits, int64_t groups, int64_t
         *a1 = nb * 2 * C * 32;
         *a2 = 0;
     };
-    int m = fit_tokens(ds, bits, groups, nb, want, bytes, pl);
+    int m = fit_tokens(ds, bits, groups, nb, want, bytes, pl, false);
     if (m < 1 && *max_terms == 3) {
         *max_terms = 2;  // a very long row: two bf16 terms (16 significant bits) per element
-        m = fit_tokens(ds, bits, groups, nb, want, bytes, pl);
+        m = fit_tokens(ds, bits, groups, nb, want, bytes, pl, false);
     }
     if (m < want && ring_ok && ds.act_ring != 1 && ds.act_ring != 4) {
         for (int mm = want; mm > m; --mm) {   // the most tokens whose columns of terms ride the ring
             const int C = mm * terms(mm);
             if (C > 16) continue;
             const int NT = C <= 8 ? 1 : 2, full = chunk_units_of(bits);
-            StreamPlan r = plan_stream(ds, bits, NT, groups, nb, 2 * C * 32, 0, false, full, true);
-            if (!r.fits || ds.act_ring == 3) r = plan_stream(ds, bits, NT, groups, nb, 2 * C * 32, 0, false, full / 2, true);
+            StreamPlan r = plan_stream(ds, bits, NT, groups, nb, 2 * C * 32, 0, LOOP_F, full, true);
+            if (!r.fits || ds.act_ring == 3) r = plan_stream(ds, bits, NT, groups, nb, 2 * C * 32, 0, LOOP_F, full / 2, true);
             if (r.fits) {
                 *pl = r;
                 m = mm;
@@ -2171,7 +2181,7 @@ int32_t launch_gemv_f(rstq_ctx* ctx, DeviceState& ds, const GemvFArgs& a) {
             p.slice2 = 0;
         }
         if (a.tp) p.tp = *a.tp;
-        if (m0 + M >= a.M) fill_next(p, ds, a.next);   // the last piece of this call: what comes next is another weight
+        if (m0 + M >= a.M) fill_next(p, ds, a.next, LOOP_F);   // the last piece of this call: what comes next is another weight
         cudaError_t le = cudaSuccess;
         if (a.bits == 4) {
             if (NT == 1) LAUNCH(4, 1, MODE_F, false);

@@ -807,3 +807,67 @@ def test_host_array_cache_notices_new_contents_at_an_old_address(ctx):
     dy = synth.normal(4, m * out)
     dx = train.qlinear_q8_dx(dy, codes, scales, m, in_, out, ctx)
     assert relerr(dx, orc.qlinear_q8_dx(dy, codes, scales, m, in_, out)) <= TOL_F
+
+
+# (out, in, format, mode, M, act, equal ranges?): either side of each line of the rule.  What an equal split saves a
+# thread block, in KB: (1 - blocks/148) x its whole groups x units x the unit's 640 / 1152 / 768 / 1280 bytes.
+@pytest.mark.parametrize("out,in_,fmt,mode,M,act,equal", [
+    (72, 8192, "q4_0", "f", 3, "bf16", 1), (72, 7168, "q4_0", "f", 3, "bf16", 0),      # 157 and 137, line 144
+    (72, 4608, "q8_0", "f", 12, "bf16", 1), (72, 4096, "q8_0", "f", 12, "bf16", 0),    # 159 and 141
+    (72, 8192, "q4_0", "f", 2, "f32", 1),
+    (40, 6656, "q4k", "a8", 4, "f32", 1), (40, 5888, "q4k", "a8", 11, "f32", 0),       # 154 and 136
+    (40, 4096, "q6k", "a8", 9, "f32", 1), (40, 3584, "q6k", "a8", 2, "f32", 0),        # 158 and 138
+    (72, 16384, "q4_0", "a8", 3, "f32", 1), (72, 14336, "q4_0", "a8", 12, "f32", 0),   # 313 and 274, line 288
+    (72, 8704, "q8_0", "a8", 2, "f32", 1), (72, 8192, "q8_0", "a8", 16, "f32", 0),     # 300 and 282
+    (72, 32768, "q4_0", "a8", 1, "f32", 1), (72, 28672, "q4_0", "a8", 1, "f32", 0),    # 627 and 548, line 576
+    (40, 16896, "q8_0", "a8", 1, "bf16", 1), (40, 16384, "q8_0", "a8", 1, "bf16", 0),  # 586 and 568
+    (40, 25600, "q4k", "a8", 1, "f32", 1), (40, 16384, "q6k", "a8", 1, "f32", 1), (40, 14336, "q6k", "a8", 1, "f32", 0),
+])
+def test_flat_matrices_take_equal_ranges_where_they_save_enough(ctx, out, in_, fmt, mode, M, act, equal):
+    """A matrix of few 32-row groups leaves SMs idle when thread blocks take whole groups; above a line of bytes saved
+    the default split is equal ranges.  The default gives the bits of the split it should have taken, and both splits
+    lie within the kernel's bound of the oracle's sums (MODE_F: of an f64 product over the dequantized weight)."""
+    rng = np.random.default_rng(out + in_ + M)
+    x = synth.normal(in_ + M, M * in_)
+    if act == "bf16":
+        xb = synth.to_bf16_bits(x)
+        x = synth.from_bf16_bits(xb)
+        bx, adt = ctx.array_to_buffer(xb), L.BF16
+    else:
+        bx, adt = ctx.array_to_buffer(x), L.F32
+    W = synth.normal(out, out * in_, 0.02)
+    if fmt in ("q4k", "q6k"):
+        sub = 32 if fmt == "q4k" else 16
+        e = orc.quantize_weight_q4k(W) if fmt == "q4k" else orc.quantize_weight_q6k(W)
+        w = (ctx.bind_weight_q4k if fmt == "q4k" else ctx.bind_weight_q6k)(e, out, in_)
+        dot = orc.qmatmul_q4k if fmt == "q4k" else orc.qmatmul_q6k
+        ref, tol = [], 1e-5
+        for m in range(M):
+            xq, xs, bsums = orc.quantize_act_q8k(x[m * in_:(m + 1) * in_], in_, sub)
+            ref.append(dot(xq, xs, bsums, e, in_, out)[1])
+        ref = np.stack(ref)
+    else:
+        bits = 4 if fmt == "q4_0" else 8
+        wq, ws = orc.quantize_weight(W, bits)
+        w = ctx.bind_weight(wq, ws, out, in_, FMT[bits][1], L.LAYOUT_ROWMAJOR)
+        if mode == "a8":
+            xq, xs, xsum = orc.quantize_act_i8(x, M, in_)
+            ref, tol = orc.matmul_a8_f64(wq, ws, FMT[bits][2], xq, xs, xsum, M, in_, out), TOL_A8
+        else:
+            ref, tol = orc.matmul_dq_f64(wq, ws, FMT[bits][2], x, M, in_, out), TOL_F
+    by = ctx.make_buffer(M * out, np.float32)
+    ys = {}
+    try:
+        for plan in (0, 1, 2):
+            ctx.tune(L.TUNE_GEMV_PLAN, plan)
+            by.fill_bytes(0xFF)
+            ctx.qmatmul(w, bx, by, M, adt, L.F32, L.MODE_F if mode == "f" else L.MODE_A8)
+            ctx.sync()
+            ys[plan] = by.download()
+            assert relerr(ys[plan], ref) <= tol, plan
+    finally:
+        ctx.tune(L.TUNE_GEMV_PLAN, 0)
+    assert np.array_equal(ys[0].view(np.uint32), ys[1 if equal else 2].view(np.uint32))
+    assert not np.array_equal(ys[1], ys[2])     # (the two splits add in different orders, so the line above tells them apart)
+    for o in (w, bx, by):
+        o.free()
