@@ -161,7 +161,8 @@ RSTQ_API int32_t rstq_init(const int32_t* devices, rstq_ctx** ctx, int32_t ndev)
 RSTQ_API int32_t rstq_shutdown(rstq_ctx* ctx);
 /* How the prefill GEMM (M above the decode kernel's range) would tile a call on a device of sm_count SMs
  * at the default settings: plan2[0] = tokens per tile (32, 64, 128 or 256), plan2[1] = thread blocks per
- * tile (2 = each takes half of K; the second hands its sums to the first; 1 also where whole tiles would leave
+ * tile (2 = K is cut: over two, the second hands its sums to the first, or over as many more as the SMs hold where
+ * the tiles are few and K is long; 1 also where whole tiles would leave
  * most SMs idle in the last wave and the thread blocks take equal ranges of all tiles' K instead: rstq_gemm_ranges).  Pure host arithmetic: no
  * device, no context.  No counterpart in the reference (its GEMM is one work-item per output). */
 RSTQ_API int32_t rstq_gemm_plan(int32_t* plan2, int64_t out, int64_t in, int64_t m, int32_t sm_count);

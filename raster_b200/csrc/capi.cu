@@ -683,7 +683,8 @@ int32_t rstq_shutdown(rstq_ctx* ctx) {
 static int32_t plan_of(int64_t out, int64_t in, int64_t m, int32_t sm_count, int* ntok, bool* split, int* ranges) {
     RSTQ_REQUIRE(out >= 1 && in >= 32 && in % 32 == 0 && m >= 1 && sm_count >= 1, RSTQ_E_SHAPE,
                  "out = %lld, in = %lld, m = %lld, sm_count = %d", (long long)out, (long long)in, (long long)m, sm_count);
-    gemm_plan(out, in, m, sm_count, true, 0, ntok, split, ranges);
+    int parts = 0;
+    gemm_plan(out, in, m, sm_count, true, 0, ntok, split, ranges, &parts);
     return RSTQ_OK;
 }
 int32_t rstq_gemm_plan(int32_t* plan2, int64_t out, int64_t in, int64_t m, int32_t sm_count) {

@@ -184,6 +184,7 @@ struct GemmParams {
     // [range_start(c), range_start(c + 1)) of it
     int64_t uq, ur;         // uq steps each, the first ur CTAs one more
     int half;               // > 0 instead: two CTAs per tile, the first runs the tile's first `half` steps
+    int parts;              // > 0 instead: that many CTAs per tile, each an equal part of its steps
     float* part;            // a range that begins inside a tile leaves that tile's f32 sums here ([CTA][warp][column]
                             // [lane]); the CTA that holds the tile's first step adds them to its own and stores y
     int* part_flags;        // one word per CTA, zero between launches: set when its `part` is complete
@@ -600,6 +601,10 @@ struct RawT<8> {
 static __device__ __align__(16) uint8_t g_zero_unit[kUnitBytesQ8];   // never written
 __device__ __forceinline__ int64_t gemm_range_start(const GemmParams& p, int64_t c) {
     if (p.half > 0) return (c >> 1) * p.ksteps + (c & 1) * p.half;
+    if (p.parts > 0) {
+        const uint32_t t = (uint32_t)c / (uint32_t)p.parts;
+        return t * p.ksteps + ((uint32_t)c - t * p.parts) * p.ksteps / p.parts;
+    }
     return c * p.uq + (c < p.ur ? c : p.ur);
 }
 
@@ -653,7 +658,7 @@ gemm_tmem_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tmap) {
         tile_first = cta >> 1;
         k_first = (cta & 1) * p.half;
         steps_own = (cta & 1) ? KS - p.half : p.half;
-    } else if (!SEGS || (p.uq == KS && p.ur == 0)) {
+    } else if (!SEGS || (p.uq == KS && p.ur == 0 && p.parts == 0)) {
         tile_first = cta;
         k_first = 0;
         steps_own = KS;
@@ -1020,30 +1025,31 @@ gemm_tmem_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tmap) {
         const bool giver = (SEGS || p.half > 0) && k0 > 0;
         int takes = 0;   // CTAs behind this one with steps of this tile
         if (!SEGS) takes = p.half > 0 && !giver;
+        else if (p.parts > 0) takes = giver ? 0 : p.parts - 1;
         else if (!giver && n < KS)
             while (cta + 1 + takes < units && gemm_range_start(p, cta + 1 + takes) < (int64_t)(tile + 1) * KS) ++takes;
         constexpr size_t kPart = (size_t)kDqWarps * CPW * 32;   // floats per CTA
         const int slot = cta * CS + (int)rank;        // of this CTA's sums and flag
         float* part = p.part + slot * kPart + (size_t)dq * (CPW * 32);
         if (ok && takes > 0) {
+            // (a lane per flag: one after the other they cost a trip to L2 each, 850 cycles)
             int got = 1;
-            if (lane == 0) {
-                const unsigned long long t0 = gtime_ns();
-                for (int k = 1; k <= (SEGS ? takes : 1) && got; ++k) {
-                    for (;;) {
-                        int v;
-                        asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p.part_flags + slot + k * CS) : "memory");
-                        if (v != 0) break;
-                        if (*abort_flag || gtime_ns() - t0 > kWaitLimitNs) {
-                            *abort_flag = 1;
-                            got = 0;
-                            break;
-                        }
-                        __nanosleep(64);
+            const unsigned long long t0 = gtime_ns();
+            for (int k = 1 + lane; k <= (SEGS ? takes : 1) && got; k += 32) {
+                for (;;) {
+                    int v;
+                    asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p.part_flags + slot + k * CS) : "memory");
+                    if (v != 0) break;
+                    if (*abort_flag || gtime_ns() - t0 > kWaitLimitNs) {
+                        *abort_flag = 1;
+                        got = 0;
+                        break;
                     }
+                    __nanosleep(64);
                 }
             }
-            ok = __shfl_sync(0xffffffffu, got, 0) != 0;
+            __syncwarp();
+            ok = __all_sync(0xffffffffu, got);
         }
         if (ok) {
             tc_fence_after();
@@ -1133,10 +1139,10 @@ gemm_tmem_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tmap) {
             // grid has completed).  All sixteen warps meet here whether or not a wait ran out.
             if (giver && ok) __threadfence();
             asm volatile("bar.sync 6, %0;" ::"r"(kDqWarps * 32) : "memory");
-            if (dq == 0 && lane == 0) {
+            if (dq == 0) {
                 if (!giver)
-                    for (int k = 1; k <= (SEGS ? takes : 1); ++k) p.part_flags[slot + k * CS] = 0;
-                else if (ok) asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(p.part_flags + slot), "r"(1) : "memory");
+                    for (int k = 1 + lane; k <= (SEGS ? takes : 1); k += 32) p.part_flags[slot + k * CS] = 0;
+                else if (ok && lane == 0) asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(p.part_flags + slot), "r"(1) : "memory");
             }
         }
         if (!SEGS || (left -= n) == 0) break;
@@ -1255,7 +1261,7 @@ static int32_t launch_act_to_f16(rstq_ctx* ctx, DeviceState& ds, const void* x, 
 }
 
 // Token-tile width and split along K of a prefill GEMM on a device of `sm_count` SMs: whichever of
-// 128- / 256-wide tiles, one or two CTAs per tile, needs the fewest cycles over the waves of CTAs
+// 128- / 256-wide tiles, one, two or more CTAs per tile, needs the fewest cycles over the waves of CTAs
 // the grid makes.  `tmem_kernel`: the call runs gemm_tmem_kernel with a pair scratch (wide tiles and
 // the split exist only there); `wide`: RSTQ_TUNE_GEMM_WIDE.
 // (measured: a 128-wide K-step 690 cycles; a 256-wide one 1140 with 64 CTAs running, 1240 with 96,
@@ -1273,28 +1279,53 @@ static int32_t launch_act_to_f16(rstq_ctx* ctx, DeviceState& ds, const void* x, 
 // 5120 x 13824 at M = 300 65.9 -> 67.3.  More than four tiles per range:
 // 11008 x 4096 at M = 1024 and 2048, as fast either way.)
 constexpr int64_t kRangeCycles = 13000;
+// (More than two CTAs per tile, where the tiles are few: equal parts of a tile's steps, one segment each.  The first part's CTA
+// waits for all the others' flags at once and adds their sums in order: beside a pair's hand-over about 1500 cycles for the
+// kernel that knows segments, and 10 x (tokens of the tile) - 100 per part, which is reading it from L2.  With seven eighths of
+// the SMs taken the last CTAs queue behind the pre-pass (6000 x 4096 over 141 of them: M = 64 15.5 -> 16.5 us).  Two CTAs per
+// tile, or ranges -> parts, int4 / int8 with bf16 tokens, us: 1024 x 16384 at M = 32 23.4 -> 14.6 (16 parts), 1608 x 9248 at M = 17
+// 17.9 -> 13.1, 4096 x 11008 at M = 64 24.3 -> 22.1, at M = 128 28.3 -> 24.8, 4096 x 4096 at M = 32 13.9 -> 12.1 (four), 2592 x 4064 at
+// M = 128 17.3 -> 15.8.  On the other side: 1024 x 4096 at M = 128 over 8 parts 16.7, over 16 21.6 (pairs 15.8, four 15.2); 2048 x 2048
+// at M = 128 13.6 over three, 12.8 over two; 512 x 1024, K too short to cut, 8.2 whole and 9.1 over four.  256-token tiles are left as they are.
+// Ranges instead of parts where they save 2500 cycles' steps: 4096 x 16384 at M = 32 24.2 against 25.2 over four, but
+// 4096 x 8192 19.4 against 18.2.)
+constexpr int64_t kPartsCycles = 3000, kPartsFull = 2000, kMaxParts = 64, kPartsToRange = 2500;
 void gemm_plan(int64_t out, int64_t in, int64_t M, int sm_count, bool tmem_kernel, int wide, int* ntok_out,
-               bool* split_out, int* ranges_out) {
+               bool* split_out, int* ranges_out, int* parts_out) {
     const int64_t ftiles = (out + 127) / 128, sm = sm_count > 0 ? sm_count : 1;
     const int64_t ksteps_total = (in / 32 + 3) / 4;
-    auto cycles = [&](int nt, bool* split) {
+    auto cycles = [&](int nt, bool* split, int* parts) {
         const int64_t tiles = ftiles * ((M + nt - 1) / nt);
         *split = tmem_kernel && tiles * 2 <= sm && tiles * 2 <= kGemmSharers &&
                  tiles * 2 * 128 * nt * 4 <= kPairScratchBytes && ksteps_total >= 16 && wide != 3;
         const int64_t ctas = *split ? tiles * 2 : tiles, active = ctas < sm ? ctas : sm;
         const int64_t c = nt == 256 ? 1140 + (active > 64 ? (active - 64) * 31 / 10 : 0) : 690;
         const int64_t fixed = nt == 256 ? 9000 : 8000;
-        return *split ? (ksteps_total + 1) / 2 * c + 1500 + fixed : (tiles + sm - 1) / sm * (ksteps_total * c + fixed);
+        int64_t best = *split ? (ksteps_total + 1) / 2 * c + 1500 + fixed : (tiles + sm - 1) / sm * (ksteps_total * c + fixed);
+        *parts = 0;
+        for (int64_t k = 3; *split && nt <= 128 && k <= ksteps_total && k <= kMaxParts; ++k) {
+            const int64_t n = tiles * k;
+            if (n > sm || n > kGemmSharers || n * 128 * nt * 4 > kPairScratchBytes) break;
+            const int64_t t = (ksteps_total + k - 1) / k * c + kPartsCycles + (n * 8 > sm * 7 ? kPartsFull : 0) + (k - 1) * (nt * 10 - 100) + fixed;
+            if (t < best) {
+                best = t;
+                *parts = (int)k;
+            }
+        }
+        return best;
     };
     int ntok = M <= 32 ? 32 : (M <= 64 ? 64 : 128);
     bool split = false;
-    const int64_t c_narrow = cycles(ntok, &split);
+    int parts = 0;
+    const int64_t c_narrow = cycles(ntok, &split, &parts);
     if (M > 128 && tmem_kernel && wide != 1) {
         bool split_w = false;
-        const int64_t c_wide = cycles(256, &split_w);
+        int parts_w = 0;
+        const int64_t c_wide = cycles(256, &split_w, &parts_w);
         if (wide == 2 || wide >= 5 || c_wide < c_narrow) {
             ntok = 256;
             split = split_w;
+            parts = parts_w;
         }
     }
     // Equal ranges of the step sequence on all SMs instead of whole tiles (or pairs) per thread block: no SM waits
@@ -1309,15 +1340,19 @@ void gemm_plan(int64_t out, int64_t in, int64_t M, int sm_count, bool tmem_kerne
         const int64_t per = (steps + G - 1) / G;
         const int64_t c = ntok == 256 ? 1140 + (G > 64 ? (G - 64) * 31 / 10 : 0) : 690, fixed = ntok == 256 ? 9000 : 8000;
         bool s2 = false;
-        const int64_t other = cycles(ntok, &s2);
-        const bool pays = per <= 3 * ksteps_total && (per * c + fixed + kRangeCycles) * 100 < other * (s2 ? 100 : (ntok <= 64 ? 94 : 85));
+        int p2 = 0;
+        const int64_t other = cycles(ntok, &s2, &p2);
+        const bool pays = p2 > 0 ? per * c + kPartsToRange + (ksteps_total / per - p2) * (ntok * 10 - 100) < (ksteps_total + p2 - 1) / p2 * c
+                                 : per <= 3 * ksteps_total && (per * c + fixed + kRangeCycles) * 100 < other * (s2 ? 100 : (ntok <= 64 ? 94 : 85));
         if (steps < (1ll << 31) && (wide == 4 || wide == 6 || pays)) {
             *ranges_out = (int)G;
             split = false;
+            parts = 0;
         }
     }
     *ntok_out = ntok;
-    *split_out = split;
+    *split_out = split || parts > 0;
+    *parts_out = parts;
 }
 
 // 256-token tiles on pairs of CTAs?  A launch of clusters costs about 1.2 us more (both SMs of a pair have to be free of the
@@ -1356,8 +1391,8 @@ int32_t launch_gemm(rstq_ctx* ctx, DeviceState& ds, const rstq_weight* w, const 
     const int64_t ftiles = (w->out + 127) / 128;
     int ntok = 128;
     bool split = false;
-    int ranges = 0;
-    gemm_plan(w->out, w->in, M, ds.sm_count, a_in_tmem && acc32 != nullptr, (int)ctx->tune_gemm_wide, &ntok, &split, &ranges);
+    int ranges = 0, parts = 0;
+    gemm_plan(w->out, w->in, M, ds.sm_count, a_in_tmem && acc32 != nullptr, (int)ctx->tune_gemm_wide, &ntok, &split, &ranges, &parts);
     const bool duo = a_in_tmem && gemm_duo(ntok, ftiles, (M + ntok - 1) / ntok, (w->nb + 3) / 4, ds.sm_count, (int)ctx->tune_gemm_wide);
     // pre-pass: activations -> fp16 with one exponent per token row.  kind::f16 wants A and B of
     // one type (fp16 weights against bf16 activations raise "illegal instruction"), and fp16 on
@@ -1397,13 +1432,14 @@ int32_t launch_gemm(rstq_ctx* ctx, DeviceState& ds, const rstq_weight* w, const 
     RSTQ_REQUIRE(ftiles * p.ttiles < (1ll << 30), RSTQ_E_LIMIT, "grid too large");
     // (units: thread blocks, or pairs of them on tiles of 256 features)
     const int64_t cs = duo ? 2 : 1, tiles = (ftiles + cs - 1) / cs * p.ttiles;
-    const int64_t units = ranges > 0 ? std::max<int64_t>(1, std::min(ranges / cs, tiles * p.ksteps)) : (split ? tiles * 2 : tiles);
-    p.half = split ? (p.ksteps + 1) / 2 : 0;
+    const int64_t units = ranges > 0 ? std::max<int64_t>(1, std::min(ranges / cs, tiles * p.ksteps)) : (parts > 0 ? tiles * parts : (split ? tiles * 2 : tiles));
+    p.half = split && parts == 0 ? (p.ksteps + 1) / 2 : 0;
+    p.parts = parts;
     p.uq = ranges > 0 ? tiles * p.ksteps / units : p.ksteps;
     p.ur = ranges > 0 ? tiles * p.ksteps % units : 0;
     p.part = acc32;   // [CTA][16 warps][columns per warp][32 lanes] f32: 128 * ntok floats each
     p.part_flags = ds.counters + ds.counters_len - kGemmSharers;
-    const bool general = ranges > 0 || (w->nb & 3) != 0;
+    const bool general = ranges > 0 || parts > 0 || (w->nb & 3) != 0;
     const int grid = (int)(units * cs);
     const size_t smem1 = kNST * (kAStage + (size_t)ntok * kKStep * 2) + 1024;
 #define GL(B, N) \

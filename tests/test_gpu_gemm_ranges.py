@@ -72,3 +72,31 @@ def test_tiles_on_pairs_of_sms_against_tiles_on_one(ctx, bits, out, in_, M):
     ref = orc.matmul_dq_f64(c, s, 0 if bits == 4 else 1, x, M, in_, rows.size).reshape(M, rows.size)
     assert np.abs(y[5][:, rows] - ref).max() <= 1e-3 * np.abs(ref).max()
     bw.free()
+
+
+@pytest.mark.parametrize("bits", [4, 8])
+@pytest.mark.parametrize("out,in_,M", [(100, 2080, 20), (40, 20000, 17), (300, 4128, 40), (1000, 16384, 30), (2500, 4128, 100),
+                                       (130, 8192, 128), (250, 2048, 64), (600, 8224, 200)])
+def test_few_tiles_cut_over_many_thread_blocks(ctx, bits, out, in_, M):
+    """A call of few tiles: each cut over as many thread blocks as its K-steps are worth (3 .. 52 here), tiles of 32, 64 and
+    128 tokens, parts of unequal length, a partial last K-step.  As whole tiles up to the order of the additions; three calls
+    in a row (each finds the flags of the one before taken down) give the same bits."""
+    w = synth.normal(out + in_ + bits, out * in_, 0.02)
+    wq, ws = orc.quantize_weight(w, bits)
+    x = synth.normal(out + in_ + M, M * in_)
+    bw = ctx.bind_weight(wq, ws, out, in_, L.FMT_Q4_0 if bits == 4 else L.FMT_Q8_0, L.LAYOUT_ROWMAJOR)
+    try:
+        y = [ctx.qmatmul_host(bw, x, M, L.F32, L.MODE_F).reshape(M, out).astype(np.float64) for _ in range(3)]
+        ctx.tune(TUNE_GEMM_WIDE, 3)
+        whole = ctx.qmatmul_host(bw, x, M, L.F32, L.MODE_F).reshape(M, out).astype(np.float64)
+    finally:
+        ctx.tune(TUNE_GEMM_WIDE, 0)
+    assert np.array_equal(y[0], y[1]) and np.array_equal(y[0], y[2])
+    assert not np.array_equal(y[0], whole)                         # (it was cut)
+    assert np.abs(y[0] - whole).max() <= 4 * 8e-6 * np.abs(whole).max()
+    rows = np.unique(np.concatenate([np.arange(0, out, max(1, out // 64)), [out - 1]]))
+    c = np.ascontiguousarray(wq.reshape(out, -1)[rows]).ravel()
+    s = np.ascontiguousarray(ws.reshape(out, -1)[rows]).ravel()
+    ref = orc.matmul_dq_f64(c, s, 0 if bits == 4 else 1, x, M, in_, rows.size).reshape(M, rows.size)
+    assert np.abs(y[0][:, rows] - ref).max() <= 1e-3 * np.abs(ref).max()
+    bw.free()
