@@ -822,6 +822,8 @@ def test_host_array_cache_notices_new_contents_at_an_old_address(ctx):
     (72, 32768, "q4_0", "a8", 1, "f32", 1), (72, 28672, "q4_0", "a8", 1, "f32", 0),    # 627 and 548, line 576
     (40, 16896, "q8_0", "a8", 1, "bf16", 1), (40, 16384, "q8_0", "a8", 1, "bf16", 0),  # 586 and 568
     (40, 25600, "q4k", "a8", 1, "f32", 1), (40, 16384, "q6k", "a8", 1, "f32", 1), (40, 14336, "q6k", "a8", 1, "f32", 0),
+    # one group on 64 (4 bits) and 128 (8 bits) thread blocks: its finisher takes 63 and 127 hand-overs, more than a warp has lanes
+    (32, 131072, "q4_0", "a8", 3, "f32", 1), (32, 131072, "q8_0", "f", 2, "bf16", 1), (32, 131072, "q4_0", "f", 12, "bf16", 1),
 ])
 def test_flat_matrices_take_equal_ranges_where_they_save_enough(ctx, out, in_, fmt, mode, M, act, equal):
     """A matrix of few 32-row groups leaves SMs idle when thread blocks take whole groups; above a line of bytes saved
