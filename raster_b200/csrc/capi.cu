@@ -680,28 +680,41 @@ int32_t rstq_shutdown(rstq_ctx* ctx) {
     return RSTQ_OK;
 }
 
-static int32_t plan_of(int64_t out, int64_t in, int64_t m, int32_t sm_count, int* ntok, bool* split, int* ranges) {
+static int32_t plan_of(int64_t out, int64_t in, int64_t m, int32_t sm_count, int64_t wide, GemmPlan* pl) {
     RSTQ_REQUIRE(out >= 1 && in >= 32 && in % 32 == 0 && m >= 1 && sm_count >= 1, RSTQ_E_SHAPE,
                  "out = %lld, in = %lld, m = %lld, sm_count = %d", (long long)out, (long long)in, (long long)m, sm_count);
-    int parts = 0;
-    gemm_plan(out, in, m, sm_count, true, 0, ntok, split, ranges, &parts);
+    *pl = gemm_plan(out, in, m, sm_count, true, (int)wide);
     return RSTQ_OK;
 }
 int32_t rstq_gemm_plan(int32_t* plan2, int64_t out, int64_t in, int64_t m, int32_t sm_count) {
     RSTQ_REQUIRE(plan2, RSTQ_E_INVALID, "null argument");
-    int ntok = 0, ranges = 0;
-    bool split = false;
-    const int32_t rc = plan_of(out, in, m, sm_count, &ntok, &split, &ranges);
+    GemmPlan pl;
+    const int32_t rc = plan_of(out, in, m, sm_count, 0, &pl);
     if (rc != RSTQ_OK) return rc;
-    plan2[0] = ntok;
-    plan2[1] = split ? 2 : 1;
+    plan2[0] = pl.ntok;
+    plan2[1] = pl.parts > 1 ? 2 : 1;
     return RSTQ_OK;
 }
 int32_t rstq_gemm_ranges(int32_t* out_ranges, int64_t out, int64_t in, int64_t m, int32_t sm_count) {
     RSTQ_REQUIRE(out_ranges, RSTQ_E_INVALID, "null argument");
-    int ntok = 0;
-    bool split = false;
-    return plan_of(out, in, m, sm_count, &ntok, &split, out_ranges);
+    GemmPlan pl;
+    const int32_t rc = plan_of(out, in, m, sm_count, 0, &pl);
+    if (rc != RSTQ_OK) return rc;
+    *out_ranges = pl.ranges > 0 ? (int32_t)pl.grid : 0;
+    return RSTQ_OK;
+}
+int32_t rstq_gemm_layout(int64_t* layout5, int64_t out, int64_t in, int64_t m, int32_t sm_count, int64_t wide) {
+    RSTQ_REQUIRE(layout5, RSTQ_E_INVALID, "null argument");
+    RSTQ_REQUIRE(wide >= 0 && wide <= 6, RSTQ_E_INVALID, "256-token tile selector 0..6");
+    GemmPlan pl;
+    const int32_t rc = plan_of(out, in, m, sm_count, wide, &pl);
+    if (rc != RSTQ_OK) return rc;
+    layout5[0] = pl.ntok;
+    layout5[1] = pl.parts;
+    layout5[2] = pl.ranges;
+    layout5[3] = pl.duo ? 1 : 0;
+    layout5[4] = pl.grid;
+    return RSTQ_OK;
 }
 
 int32_t rstq_decode_plan(int32_t* plan6, int32_t mode, int32_t bits, int64_t out, int64_t in, int64_t m, int32_t act_dtype,

@@ -1260,6 +1260,18 @@ static int32_t launch_act_to_f16(rstq_ctx* ctx, DeviceState& ds, const void* x, 
     return RSTQ_OK;
 }
 
+// 256-token tiles on pairs of CTAs?  A launch of clusters costs about 1.2 us more (both SMs of a pair have to be free of the
+// pre-pass), the K-step gains 7 %: where every SM has 80 of them to do.  In a burst / over 0.1 s, us: 70B-class MLP at
+// M = 256 (97 steps each) 103.3 -> 97.0 / 116.9 -> 112.1 and 104.7 -> 98.6 / 118.6 -> 114.9; int4 4096 x 8192 at M = 2048 (110)
+// 122.3 -> 113.5 / 135.1 -> 128.7; 7168 x 16384 at M = 512 (97) 103.8 -> 99.2 / 118.6 -> 114.4.  Below the line: 8192 x 8192 at
+// M = 512 (55) 54.5 -> 53.0 / 58.7 -> 60.0, 16384 x 6144 at M = 250 (41) 43.0 -> 41.2 / 43.7 -> 46.1.  Tiles of 128 tokens, as fast
+// in the kernel either way, only lose the launch (int8 4096 x 4096 at M = 512 21.5 -> 22.8).  An odd number of 128-feature
+// tiles idles a CTA of the last pair.
+static bool gemm_duo(int64_t ftiles, int64_t ttiles, int64_t ksteps, int sm_count, int wide) {
+    if (wide >= 5) return true;
+    return wide == 0 && ftiles * ttiles * ksteps >= 80ll * sm_count && ((ftiles & 1) == 0 || ftiles >= 9);
+}
+
 // Token-tile width and split along K of a prefill GEMM on a device of `sm_count` SMs: whichever of
 // 128- / 256-wide tiles, one, two or more CTAs per tile, needs the fewest cycles over the waves of CTAs
 // the grid makes.  `tmem_kernel`: the call runs gemm_tmem_kernel with a pair scratch (wide tiles and
@@ -1290,22 +1302,23 @@ constexpr int64_t kRangeCycles = 13000;
 // Ranges instead of parts where they save 2500 cycles' steps: 4096 x 16384 at M = 32 24.2 against 25.2 over four, but
 // 4096 x 8192 19.4 against 18.2.)
 constexpr int64_t kPartsCycles = 3000, kPartsFull = 2000, kMaxParts = 64, kPartsToRange = 2500;
-void gemm_plan(int64_t out, int64_t in, int64_t M, int sm_count, bool tmem_kernel, int wide, int* ntok_out,
-               bool* split_out, int* ranges_out, int* parts_out) {
+GemmPlan gemm_plan(int64_t out, int64_t in, int64_t M, int sm_count, bool tmem_kernel, int wide) {
     const int64_t ftiles = (out + 127) / 128, sm = sm_count > 0 ? sm_count : 1;
     const int64_t ksteps_total = (in / 32 + 3) / 4;
-    auto cycles = [&](int nt, bool* split, int* parts) {
-        const int64_t tiles = ftiles * ((M + nt - 1) / nt);
-        *split = tmem_kernel && tiles * 2 <= sm && tiles * 2 <= kGemmSharers &&
-                 tiles * 2 * 128 * nt * 4 <= kPairScratchBytes && ksteps_total >= 16 && wide != 3;
-        const int64_t ctas = *split ? tiles * 2 : tiles, active = ctas < sm ? ctas : sm;
-        const int64_t c = nt == 256 ? 1140 + (active > 64 ? (active - 64) * 31 / 10 : 0) : 690;
+    // cs: CTAs of a tile, 1 or 2 (a pair, on a tile of two feature tiles: an odd number of them leaves a CTA of the last pair idle)
+    auto tiles_of = [&](int nt, int cs) { return (ftiles + cs - 1) / cs * ((M + nt - 1) / nt); };
+    // CTAs that may share tiles: a slot of the scratch (128 x nt sums) and a flag for every one, and all of them on the device at once
+    auto sharers = [&](int nt) { return std::min({sm, (int64_t)kGemmSharers, kPairScratchBytes / (128 * 4 * nt)}); };
+    auto step_cycles = [&](int nt, int64_t active) { return nt == 256 ? 1140 + (active > 64 ? (active - 64) * 31 / 10 : 0) : (int64_t)690; };
+    auto cycles = [&](int nt, int cs, int* parts) {
+        const int64_t tiles = tiles_of(nt, cs), places = std::max<int64_t>(1, sm / cs), cap = sharers(nt) / cs;
+        const bool split = tmem_kernel && tiles * 2 <= cap && ksteps_total >= 16 && wide != 3;
+        const int64_t ctas = (split ? tiles * 2 : tiles) * cs, c = step_cycles(nt, ctas < sm ? ctas : sm);
         const int64_t fixed = nt == 256 ? 9000 : 8000;
-        int64_t best = *split ? (ksteps_total + 1) / 2 * c + 1500 + fixed : (tiles + sm - 1) / sm * (ksteps_total * c + fixed);
-        *parts = 0;
-        for (int64_t k = 3; *split && nt <= 128 && k <= ksteps_total && k <= kMaxParts; ++k) {
+        int64_t best = split ? (ksteps_total + 1) / 2 * c + 1500 + fixed : (tiles + places - 1) / places * (ksteps_total * c + fixed);
+        *parts = split ? 2 : 1;
+        for (int64_t k = 3; split && nt <= 128 && k <= ksteps_total && k <= kMaxParts && tiles * k <= cap; ++k) {
             const int64_t n = tiles * k;
-            if (n > sm || n > kGemmSharers || n * 128 * nt * 4 > kPairScratchBytes) break;
             const int64_t t = (ksteps_total + k - 1) / k * c + kPartsCycles + (n * 8 > sm * 7 ? kPartsFull : 0) + (k - 1) * (nt * 10 - 100) + fixed;
             if (t < best) {
                 best = t;
@@ -1314,58 +1327,50 @@ void gemm_plan(int64_t out, int64_t in, int64_t M, int sm_count, bool tmem_kerne
         }
         return best;
     };
-    int ntok = M <= 32 ? 32 : (M <= 64 ? 64 : 128);
-    bool split = false;
-    int parts = 0;
-    const int64_t c_narrow = cycles(ntok, &split, &parts);
+    GemmPlan pl{};
+    pl.ntok = M <= 32 ? 32 : (M <= 64 ? 64 : 128);
+    int64_t best = cycles(pl.ntok, 1, &pl.parts);
     if (M > 128 && tmem_kernel && wide != 1) {
-        bool split_w = false;
-        int parts_w = 0;
-        const int64_t c_wide = cycles(256, &split_w, &parts_w);
-        if (wide == 2 || wide >= 5 || c_wide < c_narrow) {
-            ntok = 256;
-            split = split_w;
-            parts = parts_w;
+        int parts = 1;
+        const int64_t c = cycles(256, 1, &parts);
+        if (wide == 2 || wide >= 5 || c < best) {
+            pl.ntok = 256;
+            pl.parts = parts;
+            best = c;
         }
     }
     // Equal ranges of the step sequence on all SMs instead of whole tiles (or pairs) per thread block: no SM waits
     // for the last wave, at the price of a second segment per thread block (an epilogue, a refill of the pipeline,
     // a hand-over).
-    *ranges_out = 0;
     if (tmem_kernel && wide != 3) {
-        const int64_t tiles = ftiles * ((M + ntok - 1) / ntok), steps = tiles * ksteps_total;
-        const int64_t fit = kPairScratchBytes / (128 * 4 * ntok), cap = fit < kGemmSharers ? fit : kGemmSharers;
-        int64_t G = sm < cap ? sm : cap;
-        G = G < steps ? G : steps;
-        const int64_t per = (steps + G - 1) / G;
-        const int64_t c = ntok == 256 ? 1140 + (G > 64 ? (G - 64) * 31 / 10 : 0) : 690, fixed = ntok == 256 ? 9000 : 8000;
-        bool s2 = false;
-        int p2 = 0;
-        const int64_t other = cycles(ntok, &s2, &p2);
-        const bool pays = p2 > 0 ? per * c + kPartsToRange + (ksteps_total / per - p2) * (ntok * 10 - 100) < (ksteps_total + p2 - 1) / p2 * c
-                                 : per <= 3 * ksteps_total && (per * c + fixed + kRangeCycles) * 100 < other * (s2 ? 100 : (ntok <= 64 ? 94 : 85));
-        if (steps < (1ll << 31) && (wide == 4 || wide == 6 || pays)) {
-            *ranges_out = (int)G;
-            split = false;
-            parts = 0;
+        const int64_t steps = tiles_of(pl.ntok, 1) * ksteps_total, G = std::min(sharers(pl.ntok), steps);
+        const int64_t per = (steps + G - 1) / G, c = step_cycles(pl.ntok, G), fixed = pl.ntok == 256 ? 9000 : 8000;
+        const int p2 = pl.parts;
+        const bool pays = p2 > 2 ? per * c + kPartsToRange + (ksteps_total / per - p2) * (pl.ntok * 10 - 100) < (ksteps_total + p2 - 1) / p2 * c
+                                 : per <= 3 * ksteps_total && (per * c + fixed + kRangeCycles) * 100 < best * (p2 == 2 ? 100 : (pl.ntok <= 64 ? 94 : 85));
+        if (steps < (1ll << 30) && (wide == 4 || wide == 6 || pays)) {
+            pl.ranges = (int)G;
+            pl.parts = 1;
         }
     }
-    *ntok_out = ntok;
-    *split_out = split || parts > 0;
-    *parts_out = parts;
-}
-
-// 256-token tiles on pairs of CTAs?  A launch of clusters costs about 1.2 us more (both SMs of a pair have to be free of the
-// pre-pass), the K-step gains 7 %: where every SM has 80 of them to do.  In a burst / over 0.1 s, us: 70B-class MLP at
-// M = 256 (97 steps each) 103.3 -> 97.0 / 116.9 -> 112.1 and 104.7 -> 98.6 / 118.6 -> 114.9; int4 4096 x 8192 at M = 2048 (110)
-// 122.3 -> 113.5 / 135.1 -> 128.7; 7168 x 16384 at M = 512 (97) 103.8 -> 99.2 / 118.6 -> 114.4.  Below the line: 8192 x 8192 at
-// M = 512 (55) 54.5 -> 53.0 / 58.7 -> 60.0, 16384 x 6144 at M = 250 (41) 43.0 -> 41.2 / 43.7 -> 46.1.  Tiles of 128 tokens, as fast
-// in the kernel either way, only lose the launch (int8 4096 x 4096 at M = 512 21.5 -> 22.8).  An odd number of 128-feature
-// tiles idles a CTA of the last pair.
-static bool gemm_duo(int ntok, int64_t ftiles, int64_t ttiles, int64_t ksteps, int sm_count, int wide) {
-    if (ntok != 256) return false;
-    if (wide >= 5) return true;
-    return wide == 0 && ftiles * ttiles * ksteps >= 80ll * sm_count && ((ftiles & 1) == 0 || ftiles >= 9);
+    int units = pl.ranges > 0 ? pl.ranges : 0;
+    if (pl.ntok == 256 && tmem_kernel && gemm_duo(ftiles, tiles_of(256, 1) / ftiles, ksteps_total, (int)sm, wide)) {
+        // what pairs need, by their own count of tiles; where a pair's places do not allow the cut that the plan has, the cut goes if
+        // pairs are asked for, and else the pairs
+        int parts = 1;
+        cycles(256, 2, &parts);
+        if (pl.ranges > 0) {
+            units = (int)std::max<int64_t>(1, std::min<int64_t>(pl.ranges / 2, tiles_of(256, 2) * ksteps_total));
+            pl.duo = true;
+        } else if (wide >= 5 || parts == pl.parts) {
+            pl.parts = parts;
+            pl.duo = true;
+        }
+    }
+    const int cs = pl.duo ? 2 : 1;
+    if (pl.ranges > 0) pl.ranges = units;
+    pl.grid = (pl.ranges > 0 ? pl.ranges : tiles_of(pl.ntok, cs) * pl.parts) * cs;
+    return pl;
 }
 
 // y[M, out] = x[M, in] . dequant(W)^T on the tensor cores.  src: 0 = f32 x, 1 = bf16 x,
@@ -1388,12 +1393,12 @@ int32_t launch_gemm(rstq_ctx* ctx, DeviceState& ds, const rstq_weight* w, const 
     // fewest cycles over the waves of CTAs it makes on this device is taken (4096 features: M <= 256: 128
     // wide, split; M = 512: 128 wide, one wave of 128 tiles; M = 768: 256 wide, one wave of 96 tiles
     // instead of two of 192; M >= 1024: 256 wide).
-    const int64_t ftiles = (w->out + 127) / 128;
-    int ntok = 128;
-    bool split = false;
-    int ranges = 0, parts = 0;
-    gemm_plan(w->out, w->in, M, ds.sm_count, a_in_tmem && acc32 != nullptr, (int)ctx->tune_gemm_wide, &ntok, &split, &ranges, &parts);
-    const bool duo = a_in_tmem && gemm_duo(ntok, ftiles, (M + ntok - 1) / ntok, (w->nb + 3) / 4, ds.sm_count, (int)ctx->tune_gemm_wide);
+    const GemmPlan pl = gemm_plan(w->out, w->in, M, ds.sm_count, a_in_tmem && acc32 != nullptr, (int)ctx->tune_gemm_wide);
+    const int ntok = pl.ntok;
+    const bool duo = pl.duo, shared = pl.parts > 1 || pl.ranges > 0;
+    // (as gemm_plan has it: a slot of the sums' scratch and a flag for every CTA)
+    RSTQ_REQUIRE(!shared || (pl.grid <= kGemmSharers && pl.grid * 128 * ntok * 4 <= kPairScratchBytes), RSTQ_E_LIMIT,
+                 "%lld thread blocks share tiles of %d tokens", (long long)pl.grid, ntok);
     // pre-pass: activations -> fp16 with one exponent per token row.  kind::f16 wants A and B of
     // one type (fp16 weights against bf16 activations raise "illegal instruction"), and fp16 on
     // both sides keeps three more mantissa bits of the weights than bf16 would.
@@ -1429,18 +1434,17 @@ int32_t launch_gemm(rstq_ctx* ctx, DeviceState& ds, const rstq_weight* w, const 
     p.out_dtype = out_dtype;
     p.cols = p.ttiles == 1 ? (int)std::min<int64_t>(ntok, (M + 15) & ~15ll) : ntok;
     p.dbg = ds.dbg;
-    RSTQ_REQUIRE(ftiles * p.ttiles < (1ll << 30), RSTQ_E_LIMIT, "grid too large");
+    RSTQ_REQUIRE(pl.grid < (1ll << 30), RSTQ_E_LIMIT, "grid too large");
     // (units: thread blocks, or pairs of them on tiles of 256 features)
-    const int64_t cs = duo ? 2 : 1, tiles = (ftiles + cs - 1) / cs * p.ttiles;
-    const int64_t units = ranges > 0 ? std::max<int64_t>(1, std::min(ranges / cs, tiles * p.ksteps)) : (parts > 0 ? tiles * parts : (split ? tiles * 2 : tiles));
-    p.half = split && parts == 0 ? (p.ksteps + 1) / 2 : 0;
-    p.parts = parts;
-    p.uq = ranges > 0 ? tiles * p.ksteps / units : p.ksteps;
-    p.ur = ranges > 0 ? tiles * p.ksteps % units : 0;
+    const int64_t cs = duo ? 2 : 1, steps = ((w->out + 127) / 128 + cs - 1) / cs * p.ttiles * p.ksteps;
+    p.half = pl.parts == 2 ? (p.ksteps + 1) / 2 : 0;
+    p.parts = pl.parts > 2 ? pl.parts : 0;
+    p.uq = pl.ranges > 0 ? steps / pl.ranges : p.ksteps;
+    p.ur = pl.ranges > 0 ? steps % pl.ranges : 0;
     p.part = acc32;   // [CTA][16 warps][columns per warp][32 lanes] f32: 128 * ntok floats each
     p.part_flags = ds.counters + ds.counters_len - kGemmSharers;
-    const bool general = ranges > 0 || parts > 0 || (w->nb & 3) != 0;
-    const int grid = (int)(units * cs);
+    const bool general = pl.ranges > 0 || pl.parts > 2 || (w->nb & 3) != 0;
+    const int grid = (int)pl.grid;
     const size_t smem1 = kNST * (kAStage + (size_t)ntok * kKStep * 2) + 1024;
 #define GL(B, N) \
     le = a_in_tmem ? gemm_launch<B, N>(ds, p, tmap, grid, general, duo) \

@@ -336,9 +336,15 @@ int64_t gemv_f_image_bytes(int64_t in);
 int32_t decode_plan(int mode, int bits, int64_t out, int64_t in, int64_t M, int act_dtype, int sm_count, int32_t* res);
 int32_t gemv_configure(DeviceState& ds);  // shared-memory attributes, once per device
 // gemm_tc.cu
-// gemm_tc.cu: token-tile width (32 / 64 / 128 / 256) and whether two CTAs share a tile, for a device of sm_count SMs
-void gemm_plan(int64_t out, int64_t in, int64_t M, int sm_count, bool tmem_kernel, int wide, int* ntok_out,
-               bool* split_out, int* ranges_out, int* parts_out);
+// gemm_tc.cu: how a call is cut into tiles on a device of sm_count SMs (wide: RSTQ_TUNE_GEMM_WIDE)
+struct GemmPlan {
+    int ntok;       // tokens per tile: 32, 64, 128 or 256
+    int parts;      // CTAs (duo: pairs of them) per tile, each with a part of its K-steps; 1 = whole tiles
+    int ranges;     // > 0 instead: so many CTAs (pairs), each with an equal range of all tiles' K-steps
+    bool duo;       // tiles of 256 features on pairs of CTAs
+    int64_t grid;   // CTAs
+};
+GemmPlan gemm_plan(int64_t out, int64_t in, int64_t M, int sm_count, bool tmem_kernel, int wide);
 int32_t launch_gemm(rstq_ctx* ctx, DeviceState& ds, const rstq_weight* w, const void* x, int src, void* y,
                     int out_dtype, int64_t M, void* x16, float* rowscale, float* acc32);
 int32_t gemm_configure(DeviceState& ds);

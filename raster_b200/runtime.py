@@ -36,6 +36,14 @@ def gemm_ranges(out: int, in_: int, m: int, sm_count: int = 148) -> int:
     return n.value
 
 
+def gemm_layout(out: int, in_: int, m: int, sm_count: int = 148, wide: int = 0) -> dict:
+    """All of that call's layout at a setting of RSTQ_TUNE_GEMM_WIDE (rstq_gemm_layout): tokens per tile, thread blocks per tile,
+    ranges (with pairs of SMs both count pairs) and thread blocks of the launch."""
+    v = (C.c_int64 * 5)()
+    L.check(L.load().rstq_gemm_layout(v, out, in_, m, sm_count, wide))
+    return {"tile_tokens": v[0], "per_tile": v[1], "ranges": v[2], "pairs": bool(v[3]), "blocks": v[4]}
+
+
 def decode_plan(mode: int, bits: int, out: int, in_: int, m: int, act_dtype: int = L.F32, sm_count: int = 148) -> dict:
     """What the first decode launch of a call would be (rstq_decode_plan: host arithmetic, no device): tokens it
     takes, ring stages, units per chunk, whether the activations ride the weight ring, dynamic shared memory,

@@ -117,6 +117,34 @@ def test_gemm_ranges_where_whole_tiles_leave_sms_idle():
     assert L.load().rstq_gemm_ranges(None, 4096, 4096, 64, 148) == L.E_INVALID
 
 
+@pytest.mark.parametrize("wide", range(7))
+def test_thread_blocks_that_share_gemm_tiles_have_a_slot_each(wide):
+    """The scratch of shared tiles holds 160 slots of 128 x 256 sums and there are 256 flags, whatever the selector; pairs of SMs
+    round an odd number of feature tiles up, which counts: 300 x 4096 at M = 6000 is 72 tiles of 256 tokens, and 48 pairs of
+    feature tiles with a slot for each of their 96 thread blocks and part."""
+    from raster_b200 import runtime as R
+    shapes = [(300, 4096, 6000), (384, 2048, 6144), (128, 2048, 18944), (1032, 4096, 2048), (1100, 8192, 2048), (100, 4096, 37000)]
+    shapes += [(out, in_, m) for out in (1, 32, 129, 300, 1000, 1152, 4096, 11008, 28672) for in_ in (32, 160, 2048, 4128, 28672)
+               for m in (17, 33, 64, 100, 129, 300, 512, 2048, 6000, 20000)]
+    for sm in (20, 74, 132, 148, 160, 296):
+        for out, in_, m in shapes:
+            v = R.gemm_layout(out, in_, m, sm, wide)
+            ft, tt, cs = -(-out // 128), -(-m // v["tile_tokens"]), 2 if v["pairs"] else 1
+            assert v["blocks"] == cs * (v["ranges"] or -(-ft // cs) * tt * v["per_tile"])
+            if v["per_tile"] > 1 or v["ranges"]:
+                assert v["blocks"] <= min(sm, 256) and v["blocks"] * v["tile_tokens"] <= 160 * 256
+            assert v["pairs"] <= (v["tile_tokens"] == 256)
+            if wide >= 5 and m > 128:
+                assert v["pairs"]
+    assert R.gemm_layout(28672, 8192, 256) == {"tile_tokens": 256, "per_tile": 1, "ranges": 74, "pairs": True, "blocks": 148}
+    assert R.gemm_layout(1000, 16384, 30)["per_tile"] > 2
+    lib = L.load()
+    assert lib.rstq_gemm_layout(None, 4096, 4096, 64, 148, 0) == L.E_INVALID
+    v = (C.c_int64 * 5)()
+    assert lib.rstq_gemm_layout(v, 4096, 100, 64, 148, 0) == L.E_SHAPE
+    assert lib.rstq_gemm_layout(v, 4096, 4096, 64, 148, 7) == L.E_INVALID
+
+
 def test_decode_plan_is_host_arithmetic_and_always_fits_shared_memory():
     """rstq_decode_plan needs no device: what the first decode launch of a call would be.  One token keeps its
     activations resident; several tokens of MODE_A8 ride the weight ring in one launch whatever K is (three
