@@ -1260,18 +1260,6 @@ static int32_t launch_act_to_f16(rstq_ctx* ctx, DeviceState& ds, const void* x, 
     return RSTQ_OK;
 }
 
-// 256-token tiles on pairs of CTAs?  A launch of clusters costs about 1.2 us more (both SMs of a pair have to be free of the
-// pre-pass), the K-step gains 7 %: where every SM has 80 of them to do.  In a burst / over 0.1 s, us: 70B-class MLP at
-// M = 256 (97 steps each) 103.3 -> 97.0 / 116.9 -> 112.1 and 104.7 -> 98.6 / 118.6 -> 114.9; int4 4096 x 8192 at M = 2048 (110)
-// 122.3 -> 113.5 / 135.1 -> 128.7; 7168 x 16384 at M = 512 (97) 103.8 -> 99.2 / 118.6 -> 114.4.  Below the line: 8192 x 8192 at
-// M = 512 (55) 54.5 -> 53.0 / 58.7 -> 60.0, 16384 x 6144 at M = 250 (41) 43.0 -> 41.2 / 43.7 -> 46.1.  Tiles of 128 tokens, as fast
-// in the kernel either way, only lose the launch (int8 4096 x 4096 at M = 512 21.5 -> 22.8).  An odd number of 128-feature
-// tiles idles a CTA of the last pair.
-static bool gemm_duo(int64_t ftiles, int64_t ttiles, int64_t ksteps, int sm_count, int wide) {
-    if (wide >= 5) return true;
-    return wide == 0 && ftiles * ttiles * ksteps >= 80ll * sm_count && ((ftiles & 1) == 0 || ftiles >= 9);
-}
-
 // Token-tile width and split along K of a prefill GEMM on a device of `sm_count` SMs: whichever of
 // 128- / 256-wide tiles, one, two or more CTAs per tile, needs the fewest cycles over the waves of CTAs
 // the grid makes.  `tmem_kernel`: the call runs gemm_tmem_kernel with a pair scratch (wide tiles and
@@ -1302,6 +1290,17 @@ constexpr int64_t kRangeCycles = 13000;
 // Ranges instead of parts where they save 2500 cycles' steps: 4096 x 16384 at M = 32 24.2 against 25.2 over four, but
 // 4096 x 8192 19.4 against 18.2.)
 constexpr int64_t kPartsCycles = 3000, kPartsFull = 2000, kMaxParts = 64, kPartsToRange = 2500;
+// (256-token tiles on pairs of CTAs, where every SM has 80 K-steps to do: a K-step takes 7 % less, a launch of clusters about 1.2 us more
+// (both SMs of a pair have to be free of the pre-pass), a tile 1800 cycles more, and the tiles are counted in twos: an odd number of
+// feature tiles idles a CTA of the last pair, and may need a wave that single CTAs do not.  In a burst / over 0.1 s, us: 70B-class
+// MLP at M = 256 (97 steps each) 103.3 -> 97.0 / 116.9 -> 112.1 and 104.7 -> 98.6 / 118.6 -> 114.9; int4 4096 x 8192 at M = 2048 (110)
+// 122.3 -> 113.5 / 135.1 -> 128.7; 7168 x 16384 at M = 512 (97) 103.8 -> 99.2 / 118.6 -> 114.4.  Fewer steps: 8192 x 8192 at
+// M = 512 (55) 54.5 -> 53.0 / 58.7 -> 60.0, 16384 x 6144 at M = 250 (41) 43.0 -> 41.2 / 43.7 -> 46.1.  Where pairs take a wave more: 6272 x 11008 at
+// M = 768 (147 tiles) 98 -> 132, 2688 x 10752 at M = 1792 107 -> 137, 4736 x 5120 at M = 2048 (two waves, three) 101 -> 115, 6272 x 5632 at M = 1536
+// 108 -> 122.  Short rows, where the tile's own cycles decide: 28672 x 1056 at M = 2048 201 -> 206, 28280 x 2112 at M = 1177 188 -> 189,
+// 28672 x 2048 at M = 1024 149 -> 148.  40 others of 80 .. 180 steps: 0.93 .. 0.99.  Tiles of 128 tokens, as fast
+// in the kernel either way, only lose the launch (int8 4096 x 4096 at M = 512 21.5 -> 22.8).)
+constexpr int64_t kPairSteps = 80, kPairStep = 93, kPairFixed = 1800;
 GemmPlan gemm_plan(int64_t out, int64_t in, int64_t M, int sm_count, bool tmem_kernel, int wide) {
     const int64_t ftiles = (out + 127) / 128, sm = sm_count > 0 ? sm_count : 1;
     const int64_t ksteps_total = (in / 32 + 3) / 4;
@@ -1313,8 +1312,8 @@ GemmPlan gemm_plan(int64_t out, int64_t in, int64_t M, int sm_count, bool tmem_k
     auto cycles = [&](int nt, int cs, int* parts) {
         const int64_t tiles = tiles_of(nt, cs), places = std::max<int64_t>(1, sm / cs), cap = sharers(nt) / cs;
         const bool split = tmem_kernel && tiles * 2 <= cap && ksteps_total >= 16 && wide != 3;
-        const int64_t ctas = (split ? tiles * 2 : tiles) * cs, c = step_cycles(nt, ctas < sm ? ctas : sm);
-        const int64_t fixed = nt == 256 ? 9000 : 8000;
+        const int64_t ctas = (split ? tiles * 2 : tiles) * cs, c = step_cycles(nt, ctas < sm ? ctas : sm) * (cs == 2 ? kPairStep : 100) / 100;
+        const int64_t fixed = (nt == 256 ? 9000 : 8000) + (cs == 2 ? kPairFixed : 0);
         int64_t best = split ? (ksteps_total + 1) / 2 * c + 1500 + fixed : (tiles + places - 1) / places * (ksteps_total * c + fixed);
         *parts = split ? 2 : 1;
         for (int64_t k = 3; split && nt <= 128 && k <= ksteps_total && k <= kMaxParts && tiles * k <= cap; ++k) {
@@ -1353,22 +1352,21 @@ GemmPlan gemm_plan(int64_t out, int64_t in, int64_t M, int sm_count, bool tmem_k
             pl.parts = 1;
         }
     }
-    int units = pl.ranges > 0 ? pl.ranges : 0;
-    if (pl.ntok == 256 && tmem_kernel && gemm_duo(ftiles, tiles_of(256, 1) / ftiles, ksteps_total, (int)sm, wide)) {
-        // what pairs need, by their own count of tiles; where a pair's places do not allow the cut that the plan has, the cut goes if
-        // pairs are asked for, and else the pairs
-        int parts = 1;
-        cycles(256, 2, &parts);
+    // Pairs, by their own count of tiles, places and slots
+    if (pl.ntok == 256 && tmem_kernel && (wide >= 5 || (wide == 0 && tiles_of(256, 1) * ksteps_total >= kPairSteps * sm && ((ftiles & 1) == 0 || ftiles >= 9)))) {
         if (pl.ranges > 0) {
-            units = (int)std::max<int64_t>(1, std::min<int64_t>(pl.ranges / 2, tiles_of(256, 2) * ksteps_total));
-            pl.duo = true;
-        } else if (wide >= 5 || parts == pl.parts) {
-            pl.parts = parts;
-            pl.duo = true;
+            const int64_t steps = tiles_of(256, 2) * ksteps_total, G = std::max<int64_t>(1, std::min<int64_t>(pl.ranges / 2, steps));
+            const int64_t one = tiles_of(256, 1) * ksteps_total, per1 = (one + pl.ranges - 1) / pl.ranges;
+            pl.duo = wide >= 5 || (steps + G - 1) / G * kPairStep < per1 * 100;
+            if (pl.duo) pl.ranges = (int)G;
+        } else {
+            int parts = 1;
+            const int64_t c = cycles(256, 2, &parts);
+            pl.duo = wide >= 5 || c < best;
+            if (pl.duo) pl.parts = parts;
         }
     }
     const int cs = pl.duo ? 2 : 1;
-    if (pl.ranges > 0) pl.ranges = units;
     pl.grid = (pl.ranges > 0 ? pl.ranges : tiles_of(pl.ntok, cs) * pl.parts) * cs;
     return pl;
 }

@@ -145,6 +145,24 @@ def test_thread_blocks_that_share_gemm_tiles_have_a_slot_each(wide):
     assert lib.rstq_gemm_layout(v, 4096, 4096, 64, 148, 7) == L.E_INVALID
 
 
+def test_pairs_of_sms_take_no_more_waves_than_single_ones():
+    """Whole 256-token tiles run on pairs only where their number, feature tiles rounded up to two, needs no wave more."""
+    from raster_b200 import runtime as R
+    for out, in_, m in [(6272, 11008, 768), (6145, 10752, 600), (2688, 10752, 1792), (3712, 11008, 1280), (4736, 10752, 1024),
+                        (4736, 5120, 2048), (6272, 5632, 1536), (28672, 1056, 2048), (28280, 2112, 1177)]:
+        v = R.gemm_layout(out, in_, m)
+        assert v["tile_tokens"] == 256 and not v["pairs"]
+    for out, in_, m in [(28672, 8192, 256), (8192, 28672, 256), (4096, 8192, 2048), (7168, 16384, 512), (5968, 5824, 1500), (2400, 14464, 1410)]:
+        assert R.gemm_layout(out, in_, m)["pairs"]
+    for out in range(1100, 28672, 331):
+        for in_ in (1056, 4096, 8192, 16384):
+            for m in (200, 256, 512, 700, 1024, 1500, 2048):
+                v = R.gemm_layout(out, in_, m)
+                if v["pairs"] and not v["ranges"]:
+                    ft, tt = -(-out // 128), -(-m // 256)
+                    assert -(-(-(-ft // 2) * tt) // 74) <= -(-ft * tt // 148)
+
+
 def test_decode_plan_is_host_arithmetic_and_always_fits_shared_memory():
     """rstq_decode_plan needs no device: what the first decode launch of a call would be.  One token keeps its
     activations resident; several tokens of MODE_A8 ride the weight ring in one launch whatever K is (three
