@@ -51,7 +51,7 @@
 (defrstq sync*               "rstq_sync"           I [P I])          ; ctx dev
 (defrstq gemm-plan*          "rstq_gemm_plan"      I [P L L L I])    ; plan2 out in m sm-count
 (defrstq gemm-ranges*        "rstq_gemm_ranges"    I [P L L L I])    ; ranges out in m sm-count
-(defrstq gemm-layout*        "rstq_gemm_layout"    I [P L L L I L])  ; layout5 out in m sm-count wide
+(defrstq gemm-layout*        "rstq_gemm_layout"    I [P L L L I L])  ; layout6 out in m sm-count wide
 (defrstq decode-plan*        "rstq_decode_plan"    I [P I I L L L I I])  ; plan6 mode bits out in m act-dtype sm-count
 (defrstq tune*               "rstq_tune"           I [P I L])        ; ctx key value
 (defrstq device-info*        "rstq_device_info"    I [P P I])        ; ctx out4 dev

@@ -169,11 +169,12 @@ RSTQ_API int32_t rstq_gemm_plan(int32_t* plan2, int64_t out, int64_t in, int64_t
 /* In how many equal ranges of all tiles' K-steps (thread blocks) that call would run; 0 = as whole tiles, or two thread
  * blocks per tile (rstq_gemm_plan).  Pure host arithmetic as well. */
 RSTQ_API int32_t rstq_gemm_ranges(int32_t* ranges, int64_t out, int64_t in, int64_t m, int32_t sm_count);
-/* All of that call's layout, at a setting of RSTQ_TUNE_GEMM_WIDE: layout5[0] = tokens per tile, [1] = thread blocks per tile
+/* All of that call's layout, at a setting of RSTQ_TUNE_GEMM_WIDE: layout6[0] = tokens per tile, [1] = thread blocks per tile
  * (1 = whole tiles), [2] = ranges (0 = none), [3] = 1 where a tile has 256 features and [1] and [2] count pairs of thread
- * blocks on neighbouring SMs, [4] = thread blocks of the launch.  Where tiles are shared ([1] > 1 or [2] > 0) these are at most
+ * blocks on neighbouring SMs, [4] = thread blocks of the launch, [5] = columns of a tile that are computed (on pairs
+ * a multiple of 32).  Where tiles are shared ([1] > 1 or [2] > 0) these are at most
  * sm_count, at most 256, and have a slot each in a scratch of 160 x 128 x 256 sums.  Pure host arithmetic. */
-RSTQ_API int32_t rstq_gemm_layout(int64_t* layout5, int64_t out, int64_t in, int64_t m, int32_t sm_count, int64_t wide);
+RSTQ_API int32_t rstq_gemm_layout(int64_t* layout6, int64_t out, int64_t in, int64_t m, int32_t sm_count, int64_t wide);
 /* What the FIRST decode launch of rstq_qmatmul (mode, bits 4 / 8, act_dtype) on an out x in weight with m tokens
  * would be at the default settings on a device of sm_count SMs: plan6[0] = tokens it takes (up to 16; 0 = a
  * row of activations does not fit at all), [1] = ring stages, [2] = units per chunk, [3] = 1 when the

@@ -703,17 +703,18 @@ int32_t rstq_gemm_ranges(int32_t* out_ranges, int64_t out, int64_t in, int64_t m
     *out_ranges = pl.ranges > 0 ? (int32_t)pl.grid : 0;
     return RSTQ_OK;
 }
-int32_t rstq_gemm_layout(int64_t* layout5, int64_t out, int64_t in, int64_t m, int32_t sm_count, int64_t wide) {
-    RSTQ_REQUIRE(layout5, RSTQ_E_INVALID, "null argument");
+int32_t rstq_gemm_layout(int64_t* layout6, int64_t out, int64_t in, int64_t m, int32_t sm_count, int64_t wide) {
+    RSTQ_REQUIRE(layout6, RSTQ_E_INVALID, "null argument");
     RSTQ_REQUIRE(wide >= 0 && wide <= 6, RSTQ_E_INVALID, "256-token tile selector 0..6");
     GemmPlan pl;
     const int32_t rc = plan_of(out, in, m, sm_count, wide, &pl);
     if (rc != RSTQ_OK) return rc;
-    layout5[0] = pl.ntok;
-    layout5[1] = pl.parts;
-    layout5[2] = pl.ranges;
-    layout5[3] = pl.duo ? 1 : 0;
-    layout5[4] = pl.grid;
+    layout6[0] = pl.ntok;
+    layout6[1] = pl.parts;
+    layout6[2] = pl.ranges;
+    layout6[3] = pl.duo ? 1 : 0;
+    layout6[4] = pl.grid;
+    layout6[5] = pl.cols;
     return RSTQ_OK;
 }
 

@@ -190,7 +190,7 @@ struct GemmParams {
     int* part_flags;        // one word per CTA, zero between launches: set when its `part` is complete
     float wmul, wdiv;       // 2^ew applied to the block scales, 2^-ew applied to the result
     int out_dtype;
-    int cols;               // pairs of CTAs: columns of a tile that are computed (a multiple of 16)
+    int cols;               // columns of a tile that are computed (pairs of CTAs: a multiple of 32)
     unsigned long long* dbg;  // optional timeline of CTA 0 (see RSTQ_TUNE_TIMELINE), or null
 };
 
@@ -670,7 +670,7 @@ gemm_tmem_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tmap) {
     }
     const int fd = tile_first / p.ttiles, ft_first = fd * CS + (int)rank, tok_first = (tile_first - fd * p.ttiles) * NTOK;
 
-    // DUO: the columns of a tile that hold tokens, in sixteens, where one tile takes all tokens: narrower MMAs.  (The rest of its
+    // DUO: the columns of a tile that hold tokens, in thirty-twos (N of an MMA of cta_group::2 with M = 256), where one tile takes all tokens: narrower MMAs.  (The rest of its
     // columns is never written, and what is read there goes nowhere.  int4 28672 x 8192 at M = 160 91.4 -> 85.6 us, 8192 x 28672 at
     // M = 200 94.6 -> 91.8.  Worked out per tile, for several, full tiles lose 1.4 %.)
     const int cols = DUO ? p.cols : NTOK;
@@ -1367,6 +1367,7 @@ GemmPlan gemm_plan(int64_t out, int64_t in, int64_t M, int sm_count, bool tmem_k
         }
     }
     const int cs = pl.duo ? 2 : 1;
+    pl.cols = pl.duo && M < 256 ? (int)((M + 31) & ~31ll) : pl.ntok;
     pl.grid = (pl.ranges > 0 ? pl.ranges : tiles_of(pl.ntok, cs) * pl.parts) * cs;
     return pl;
 }
@@ -1430,7 +1431,7 @@ int32_t launch_gemm(rstq_ctx* ctx, DeviceState& ds, const rstq_weight* w, const 
     p.wmul = ldexpf(1.0f, w->gemm_exp + (a_in_tmem ? kSubnormalShift : 0));
     p.wdiv = ldexpf(1.0f, -w->gemm_exp + (a_in_tmem ? 24 - kSubnormalShift : 0));
     p.out_dtype = out_dtype;
-    p.cols = p.ttiles == 1 ? (int)std::min<int64_t>(ntok, (M + 15) & ~15ll) : ntok;
+    p.cols = pl.cols;
     p.dbg = ds.dbg;
     RSTQ_REQUIRE(pl.grid < (1ll << 30), RSTQ_E_LIMIT, "grid too large");
     // (units: thread blocks, or pairs of them on tiles of 256 features)

@@ -342,6 +342,7 @@ struct GemmPlan {
     int parts;      // CTAs (duo: pairs of them) per tile, each with a part of its K-steps; 1 = whole tiles
     int ranges;     // > 0 instead: so many CTAs (pairs), each with an equal range of all tiles' K-steps
     bool duo;       // tiles of 256 features on pairs of CTAs
+    int cols;       // columns of a tile that its MMAs compute: fewer than ntok on pairs of CTAs whose one tile takes all tokens
     int64_t grid;   // CTAs
 };
 GemmPlan gemm_plan(int64_t out, int64_t in, int64_t M, int sm_count, bool tmem_kernel, int wide);

@@ -38,10 +38,10 @@ def gemm_ranges(out: int, in_: int, m: int, sm_count: int = 148) -> int:
 
 def gemm_layout(out: int, in_: int, m: int, sm_count: int = 148, wide: int = 0) -> dict:
     """All of that call's layout at a setting of RSTQ_TUNE_GEMM_WIDE (rstq_gemm_layout): tokens per tile, thread blocks per tile,
-    ranges (with pairs of SMs both count pairs) and thread blocks of the launch."""
-    v = (C.c_int64 * 5)()
+    ranges (with pairs of SMs both count pairs), thread blocks of the launch and columns computed per tile."""
+    v = (C.c_int64 * 6)()
     L.check(L.load().rstq_gemm_layout(v, out, in_, m, sm_count, wide))
-    return {"tile_tokens": v[0], "per_tile": v[1], "ranges": v[2], "pairs": bool(v[3]), "blocks": v[4]}
+    return {"tile_tokens": v[0], "per_tile": v[1], "ranges": v[2], "pairs": bool(v[3]), "blocks": v[4], "columns": v[5]}
 
 
 def decode_plan(mode: int, bits: int, out: int, in_: int, m: int, act_dtype: int = L.F32, sm_count: int = 148) -> dict:

@@ -125,7 +125,7 @@ def test_thread_blocks_that_share_gemm_tiles_have_a_slot_each(wide):
     from raster_b200 import runtime as R
     shapes = [(300, 4096, 6000), (384, 2048, 6144), (128, 2048, 18944), (1032, 4096, 2048), (1100, 8192, 2048), (100, 4096, 37000)]
     shapes += [(out, in_, m) for out in (1, 32, 129, 300, 1000, 1152, 4096, 11008, 28672) for in_ in (32, 160, 2048, 4128, 28672)
-               for m in (17, 33, 64, 100, 129, 300, 512, 2048, 6000, 20000)]
+               for m in (17, 33, 64, 100, 129, 161, 176, 240, 300, 512, 2048, 6000, 20000)]
     for sm in (20, 74, 132, 148, 160, 296):
         for out, in_, m in shapes:
             v = R.gemm_layout(out, in_, m, sm, wide)
@@ -134,13 +134,15 @@ def test_thread_blocks_that_share_gemm_tiles_have_a_slot_each(wide):
             if v["per_tile"] > 1 or v["ranges"]:
                 assert v["blocks"] <= min(sm, 256) and v["blocks"] * v["tile_tokens"] <= 160 * 256
             assert v["pairs"] <= (v["tile_tokens"] == 256)
+            # an MMA of cta_group::2 with M = 256 takes N in thirty-twos
+            assert v["columns"] == (min(-(-m // 32) * 32, 256) if v["pairs"] else v["tile_tokens"])
             if wide >= 5 and m > 128:
                 assert v["pairs"]
-    assert R.gemm_layout(28672, 8192, 256) == {"tile_tokens": 256, "per_tile": 1, "ranges": 74, "pairs": True, "blocks": 148}
+    assert R.gemm_layout(28672, 8192, 256) == {"tile_tokens": 256, "per_tile": 1, "ranges": 74, "pairs": True, "blocks": 148, "columns": 256}
     assert R.gemm_layout(1000, 16384, 30)["per_tile"] > 2
     lib = L.load()
     assert lib.rstq_gemm_layout(None, 4096, 4096, 64, 148, 0) == L.E_INVALID
-    v = (C.c_int64 * 5)()
+    v = (C.c_int64 * 6)()
     assert lib.rstq_gemm_layout(v, 4096, 100, 64, 148, 0) == L.E_SHAPE
     assert lib.rstq_gemm_layout(v, 4096, 4096, 64, 148, 7) == L.E_INVALID
 

@@ -46,10 +46,10 @@ def test_ranges_against_whole_tiles(ctx, bits, out, in_, M):
 
 @pytest.mark.parametrize("bits", [4, 8])
 @pytest.mark.parametrize("out,in_,M", [(100, 160, 129), (300, 4128, 300), (2500, 1056, 200), (1000, 2080, 256), (1032, 8192, 515),
-                                       (256, 32, 257), (300, 2048, 6000)])
+                                       (256, 32, 257), (300, 2048, 6000), (700, 1056, 176), (300, 2080, 240), (256, 160, 161)])
 def test_tiles_on_pairs_of_sms_against_tiles_on_one(ctx, bits, out, in_, M):
     """256-token tiles on pairs of SMs: an odd number of 128-feature tiles (one of a pair has none), tokens in the first SM's
-    half alone, tiles shared by two pairs, cut at any step, partial last K-steps, rows of one K-step.  Same products, same
+    half alone, widths (of 160, 192 and 256 columns) that the tokens do not fill, tiles shared by two pairs, cut at any step, partial last K-steps, rows of one K-step.  Same products, same
     sums as a 256-token tile on one SM; cut tiles differ as above.  300 x 2048 at M = 6000: 72 tiles, cut in two on single SMs,
     would be 96 pairs so, more than there are places or scratch for, and stay whole on pairs."""
     w = synth.normal(out + in_ + bits, out * in_, 0.02)
