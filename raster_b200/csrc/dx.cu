@@ -13,20 +13,23 @@
 //   pairs of fp16     W' = H + 2^-11 L, dy = h + 2^-11 l:  H h + 2^-11 (H l + L h)                             3 MMAs
 //   triples of bf16   W' = W1 + W2 + W3, dy = Y1 + Y2 + Y3:  W1 Y1 + (W1 Y2 + W2 Y1) + (W1 Y3 + W2 Y2 + W3 Y1)  6 MMAs
 //
-// A pair holds 23 bits.  Its second term is kept 2^11 larger than it is, in a sum of its own, and a power of two per token
-// row and per 32-column block brings the largest of them close to fp16's, so an element down to 2^-27 of its row's largest
-// (a scale down to 2^-20 of its column block's) has all of them: the tiles whose rows and column blocks hold nothing
+// A pair holds an f32 to within one unit of its last place (11 bits, a sign, 11 bits), a weight to within three: its scale is a
+// pair itself, times the code in packed fp16.  Its second term is kept 2^11 larger than it is, in a sum of its own, and a power of
+// two per token row and per 32-column block brings the largest of them close to fp16's, so an element down to 2^-27 of its row's
+// largest (a scale down to 2^-20 of its column block's) is held so: the tiles whose rows and column blocks hold nothing
 // smaller but zeros, and no infinity, take pairs.  Triples hold all 24 bits at any spread (2^-90 is tested); a tile with
 // one such row or column block takes them.  dx_prep_kernel writes both forms of dy and says which rows are which.
 //
-// The sums on the tensor core decide the error, not the products.  2-norm against the f64 product, over that of the product,
-// triples / pairs: 4096 x 4096, m = 512 9.2e-6 / 4.9e-6 (pairs add half as often to the first sum), m = 64 9.7e-7 / 6.5e-7
-// (even and odd steps have sums of their own), 1024 x 1024, m = 16 4.5e-7 / 3.6e-7.
+// The sums on the tensor core decide the error of a long sum, its products that of a short one.  2-norm against the f64 product,
+// over that of the product, triples / pairs: 4096 x 4096, m = 512 9.2e-6 / 4.9e-6 (pairs add half as often to the first sum), m = 64
+// 9.7e-7 / 6.5e-7 (even and odd steps have sums of their own), 1024 x 1024, m = 16 4.5e-7 / 3.5e-7; sums over 256, 192, 128, 64, 32 rows
+// up to 64 tokens 2.2e-7 / 2.1e-7, 1.7 / 1.9, 1.1 / 1.4, 0.68 / 1.4, 0.53 / 1.1; more tokens, over 64 rows 1.7 / 1.4, over 32 1.09 / 1.11.
+// So sums that short are triples: pairs are nowhere further from the f64 product (dx_pair_rows).
 //
 // What bounds it: the tensor core at the power cap, for pairs nominally 768 cycles per 64 rows of a 128 x 128 tile; with the
-// conversions taken out the same MMAs take 1050, with them 1160.  us per call back to back, all tiles triples (before) ->
-// pairs: 4096 x 4096, m = 512 91.9 -> 58.9, m = 64 29.4 -> 25.8; 1024 x 1024, m = 16 16.6 -> 15.1; 11008 x 2048, m = 300
-// 135 -> 82.7.  With a row of small elements per tile, so triples: 91.6, 30.0, 17.4 (dy waits for the tile's form), 126.
+// conversions taken out the same MMAs take 1050, with them 1160.  us per call back to back, all tiles triples -> pairs
+// where they hold: 4096 x 4096, m = 512 98.4 -> 62.5, m = 64 29.0 -> 25.5; 1024 x 1024, m = 16 16.3 -> 15.0; 11008 x 2048, m = 300
+// 135 -> 82.8.  With a row of small elements per tile, so triples: 91.6, 30.0, 17.4 (dy waits for the tile's form), 126 (92.0, 29.2, 16.6 without pairs).
 #include <type_traits>
 
 #include "internal.h"
@@ -103,6 +106,7 @@ constexpr int kDxPrepMax = 512;     // threads per block of the pre-pass, at mos
 constexpr float kDxPairMin = 0.00390625f;
 constexpr int kDxPairExp = 5;
 constexpr float kDxLow = 2048.0f;   // what the second terms of pairs are larger by
+__host__ __device__ constexpr int dx_pair_rows(int nt) { return nt <= 64 ? 256 : 64; }   // shorter sums: triples
 __device__ __forceinline__ float dx_nonzero(float v) { return v == 0.f ? __int_as_float(0x7F800000) : fabsf(v); }
 __device__ __forceinline__ void dx_block_range(float& mx, float& mn, float (*red)[kDxPrepMax / 32]) {
 #pragma unroll
@@ -567,7 +571,7 @@ dx_tmem_kernel(const DxParams p, const __grid_constant__ CUtensorMap map_w, cons
         float down, down2;   // the block's scales are used times 2^-ce, the largest in [2^12, 2^13)
         const int ce = dx_exponent(mx, 13, &down, &down2);
         const bool infinite = isinf(mx);   // a scale of this column block (of the whole matrix)
-        const bool any_wide = __any_sync(0xffffffffu, row_wide) || infinite || mn * down * down2 < kDxPairMin;
+        const bool any_wide = p.out < dx_pair_rows(NT) || __any_sync(0xffffffffu, row_wide) || infinite || mn * down * down2 < kDxPairMin;
         if (lane == 0) {
             s_colexp[blk] = ce;   // (the four warps of a block of columns agree)
             if (any_wide) s_wide = 1;
@@ -662,9 +666,12 @@ dx_tmem_kernel(const DxParams p, const __grid_constant__ CUtensorMap map_w, cons
         } else {
             down *= 1.0f / (1 << kDxPairExp);      // (no scale of such a block comes near f32's limits on the way)
             stages(std::true_type{}, [&](const uint32_t (&w)[2][4], const uint32_t (&sc)[2][4], uint32_t dst) {
-                // Two rows at a time in packed fp16, scale = s1 + 2^-11 s2: H = code * s1 rounded, what the rounding left
-                // is exact (a multiple of s1's last place, at most 2^6 of them), L = 2^11 times that + code * s2 rounded
-                // once.  Seven instructions per two weights; from f32 products it was 14.
+                // Two rows at a time in packed fp16, scale = s1 + 2^-11 s2: H = code * (s1 + 2^-11 s2) to within a little more than half a
+                // step (the second product is rounded, and absorbed), what it left of code * s1 is exact (a multiple of s1's
+                // last place, below 2^8 of them), L = 2^11 times that + code * s2 rounded once.  (Eight instructions per two weights.
+                // Without the second product in H, L is up to three times as large and rounded as much more: weights off
+                // by up to 9 units of 2^-24, 1.21 rms, now 4.0 and 0.95; from f32 products it would be
+                // 3.0 and 0.83, but fourteen instructions.  4096 x 4096, m = 512: 62.3, 62.5 and 67.4 us.)
                 uint32_t v1[2][8], v2[2][8];
 #pragma unroll
                 for (int g = 0; g < 2; ++g)
@@ -672,6 +679,7 @@ dx_tmem_kernel(const DxParams p, const __grid_constant__ CUtensorMap map_w, cons
                     for (int h = 0; h < 2; ++h) {       // rows 2t + 8h, 2t + 8h + 1
                         const uint32_t s1 = __byte_perm(sc[g][2 * h], sc[g][2 * h + 1], 0x5410);
                         const uint32_t s2 = __byte_perm(sc[g][2 * h], sc[g][2 * h + 1], 0x7632);
+                        const uint32_t s3 = hmul2_u32(s2, 0x10001000u);   // 2^-11 s2
 #pragma unroll
                         for (int q = 0; q < 2; ++q) {   // columns 4 gid + 2q, + 2q + 1
                             const uint32_t both = __byte_perm(w[g][2 * h], w[g][2 * h + 1], q ? 0x7362 : 0x5140);
@@ -679,7 +687,7 @@ dx_tmem_kernel(const DxParams p, const __grid_constant__ CUtensorMap map_w, cons
                             for (int c = 0; c < 2; ++c) {
                                 // under the upper byte of 1024 the code + 128 is 1152 + code
                                 const uint32_t n = hadd2_u32(__byte_perm(both, 0x64u, c ? 0x4342 : 0x4140), 0xE480E480u);
-                                const uint32_t hi = hmul2_u32(n, s1);
+                                const uint32_t hi = hfma2_u32(n, s1, hmul2_u32(n, s3));
                                 const uint32_t left = hfma2_u32(n, s1, hi ^ 0x80008000u);
                                 const int e = g * 4 + c * 2 + h;
                                 v1[q][e] = hi;
@@ -713,21 +721,20 @@ dx_tmem_kernel(const DxParams p, const __grid_constant__ CUtensorMap map_w, cons
             }
             tmem_ld_wait();
             if constexpr (NT <= 64) {
-                if (wide || k1 - k0 > 1) {   // triples: the third sum; pairs: the sums of the odd steps, if there are any
-                    uint32_t c[CH];
+                // triples: the third sum; pairs: the sums of the odd steps (a block has eight of them at least, or the whole of four)
+                uint32_t c[CH];
 #pragma unroll
-                    for (int j = 0; j < CH; j += 8) tmem_ld8(ta + 2 * NT + j, *reinterpret_cast<uint32_t(*)[8]>(&c[j]));
+                for (int j = 0; j < CH; j += 8) tmem_ld8(ta + 2 * NT + j, *reinterpret_cast<uint32_t(*)[8]>(&c[j]));
+                tmem_ld_wait();
+                uint32_t (&to)[CH] = wide ? b : a;
+#pragma unroll
+                for (int j = 0; j < CH; ++j) to[j] = __float_as_uint(__uint_as_float(to[j]) + __uint_as_float(c[j]));
+                if (!wide) {
+#pragma unroll
+                    for (int j = 0; j < CH; j += 8) tmem_ld8(ta + 3 * NT + j, *reinterpret_cast<uint32_t(*)[8]>(&c[j]));
                     tmem_ld_wait();
-                    uint32_t (&to)[CH] = wide ? b : a;
 #pragma unroll
-                    for (int j = 0; j < CH; ++j) to[j] = __float_as_uint(__uint_as_float(to[j]) + __uint_as_float(c[j]));
-                    if (!wide) {
-#pragma unroll
-                        for (int j = 0; j < CH; j += 8) tmem_ld8(ta + 3 * NT + j, *reinterpret_cast<uint32_t(*)[8]>(&c[j]));
-                        tmem_ld_wait();
-#pragma unroll
-                        for (int j = 0; j < CH; ++j) b[j] = __float_as_uint(__uint_as_float(b[j]) + __uint_as_float(c[j]));
-                    }
+                    for (int j = 0; j < CH; ++j) b[j] = __float_as_uint(__uint_as_float(b[j]) + __uint_as_float(c[j]));
                 }
             }
             const float low = wide ? 1.0f : 1.0f / kDxLow;

@@ -133,7 +133,8 @@ def test_dx_recorded_without_a_first_call(ctx):
         b.free()
 
 
-@pytest.mark.parametrize("m,in_,out", [(5, 96, 64), (40, 160, 128), (64, 256, 200), (300, 256, 320)])   # one step, even and odd steps
+@pytest.mark.parametrize("m,in_,out", [(5, 96, 64), (40, 160, 128), (64, 256, 200),              # short sums: triples in any case
+                                       (300, 256, 320), (300, 160, 64), (5, 96, 256), (40, 160, 320), (64, 256, 300)])
 @pytest.mark.parametrize("what,below", [("dy", 26), ("dy", 27), ("dy", 28), ("scales", 19), ("scales", 20), ("scales", 21)])
 def test_dx_pairs_and_triples_on_both_sides_of_the_line(ctx, what, below, m, in_, out):
     """Rows whose smallest element, blocks whose smallest scale lies about where pairs of fp16 stop holding it whole, in
@@ -151,6 +152,29 @@ def test_dx_pairs_and_triples_on_both_sides_of_the_line(ctx, what, below, m, in_
     dx = run(ctx, m, in_, out, dy.ravel(), codes.ravel(), scales.ravel())
     w = codes.astype(np.float64) * np.repeat(scales.astype(np.float64), 32, axis=1)
     d = dy.astype(np.float64)
-    # A product of pairs: 6 * 2^-24 for the weight (second term up to 1.5 times the first's half step, its rounding and
-    # that of the second term of the scale), 2 * 2^-24 for dy, 6 * 2^-24 for the product of the second terms, left out.
+    # A product of pairs: 6 * 2^-24 for the weight (4 for the rounding of its second term, which may be a little more than
+    # half a step of the first, 2 for that of the scale's), 2 * 2^-24 for dy, 6 * 2^-24 for the product of the second terms, left out.
     assert np.all(np.abs(dx - d @ w) <= (14 * 2.0 ** -24 + (out / 8 + 12) * 2.0 ** -23) * (np.abs(d) @ np.abs(w)))
+
+
+@pytest.mark.parametrize("m,out,units", [(64, 512, 6), (40, 260, 6), (200, 512, 6), (64, 255, 1), (5, 64, 1), (200, 63, 1)])
+def test_dx_holds_weights_and_elements_of_dy(ctx, m, out, units):
+    """Sums of one term, which round nothing: dy with one 1 per row gives the weights, codes of 1 and scales of 1 in one row
+    give the elements of dy back.  A weight as a pair of fp16 is off by 6 * 2^-24 of itself at most (see above), an element of dy by 2;
+    short sums are triples, and only the f32 product of code and scale rounds: 1 * 2^-24."""
+    in_ = 4096
+    rng = np.random.default_rng(out)
+    codes = rng.integers(-128, 128, (out, in_)).astype(np.int8)
+    scales = np.exp2(rng.uniform(-6, 0, (out, in_ // 32))).astype(np.float32)
+    rows = rng.integers(0, out, m)
+    dy = np.zeros((m, out), np.float32)
+    dy[np.arange(m), rows] = 1
+    dx = run(ctx, m, in_, out, dy.ravel(), codes.ravel(), scales.ravel())
+    w = (codes.astype(np.float64) * np.repeat(scales.astype(np.float64), 32, axis=1))[rows]
+    assert np.all(np.abs(dx - w) <= (units * (1 + 2.0 ** -10) * 2.0 ** -24) * np.abs(w))
+    dy = (rng.uniform(0.01, 1, (m, out)) * rng.choice([-1, 1], (m, out))).astype(np.float32)
+    codes[:], scales[:] = 0, 1
+    codes[rows[0]] = 1
+    dx = run(ctx, m, in_, out, dy.ravel(), codes.ravel(), scales.ravel())
+    d = dy[:, rows[:1]].astype(np.float64)
+    assert np.all(np.abs(dx - d) <= (2 * (1 + 2.0 ** -10) * 2.0 ** -24 if units > 1 else 0) * np.abs(d))
