@@ -399,8 +399,10 @@ static int64_t products_tmp_bytes(int64_t n, int per) { return ((n / per * 4 + 2
 // Device arrays of weights.  cudaMalloc and cudaFree of a 10 MB matrix take 0.4 .. 1.4 and 0.35 .. 1.2 ms, more than its copies, so
 // the arrays of weights that are gone serve the next ones of their size (a 4096 x 4096 int4 matrix that takes another one's
 // place: 3.6 -> 2.9 ms).  Up to kWeightKeep bytes per device are kept, and given back before an allocation fails and with
-// the context.  Like cudaFree, giving an array back waits for the whole device.  (A driver's memory pool instead is as fast
-// here, but matrices that lie in it stream 1 - 2 % slower at one token.)
+// the context.  What used an array was launched on the context's own stream, so that is waited for, and no more: a wait for the whole
+// device would spoil a capture that the caller has under way elsewhere.  Once a stream of the caller's may have a launch or a recorded
+// graph of theirs (ds.lent), arrays go to cudaFree, which waits for all of it, and are not kept.  (A driver's memory pool
+// instead is as fast here, but matrices that lie in it stream 1 - 2 % slower at one token.)
 static cudaError_t weight_malloc(DeviceState& ds, void** p, int64_t bytes) {
     for (size_t i = ds.spare_weights.size(); i-- > 0;)
         if (ds.spare_weights[i].second == bytes) {
@@ -414,7 +416,7 @@ static cudaError_t weight_malloc(DeviceState& ds, void** p, int64_t bytes) {
 // (the device is current)
 static void weight_release(DeviceState& ds, void* p, int64_t bytes) {
     if (!p) return;
-    if (!ds.capturing && ds.spare_bytes + bytes <= kWeightKeep && cudaDeviceSynchronize() == cudaSuccess) {
+    if (!ds.capturing && !ds.lent && ds.spare_bytes + bytes <= kWeightKeep && cudaStreamSynchronize(ds.stream) == cudaSuccess) {
         try {
             ds.spare_weights.emplace_back(p, bytes);
             ds.spare_bytes += bytes;
@@ -896,6 +898,7 @@ int32_t rstq_stream_set(rstq_ctx* ctx, void* stream, int32_t dev) {
     RSTQ_CUDA(cudaStreamSynchronize(ds.stream));
     if (stream) {
         ds.stream = (cudaStream_t)stream;
+        ds.lent = true;
     } else {
         ds.stream = ds.own_stream;
     }

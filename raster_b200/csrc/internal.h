@@ -115,6 +115,7 @@ struct DeviceState {
     std::vector<void*> kept;       // outgrown blocks that such a graph may name: freed with the context
     void* bind_stage = nullptr;    // the host arrays of the weight being bound, before they are re-tiled (at most
     int64_t bind_stage_bytes = 0;  // kBindStageKeep bytes are kept between binds)
+    bool lent = false;             // a stream of the caller's has been used: it may have launches or graphs that name weights
     // arrays of weights that are gone, kept for the next one of the same size: at most kWeightKeep bytes
     std::vector<std::pair<void*, int64_t>> spare_weights;
     int64_t spare_bytes = 0;

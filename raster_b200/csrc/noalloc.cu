@@ -76,11 +76,12 @@ extern "C" int32_t rstq_qmatmul_prequant_noalloc(rstq_weight* w, const void* xq,
                  "out = %lld rows exceeds the fixed scratch of this entry point (%d rows)",
                  (long long)w->out, kNaMaxGroups * 32);
     rstq_ctx* ctx = w->ctx;
-    const DeviceState& real = ctx->devs[w->dev];
+    DeviceState& real = ctx->devs[w->dev];
     RSTQ_REQUIRE(real.ordinal >= 0 && real.ordinal < 64 && real.sm_count <= kNaMaxCtas, RSTQ_E_LIMIT,
                  "device outside the fixed limits of this entry point");
     RSTQ_CUDA(cudaSetDevice(real.ordinal));
     const cudaStream_t st = stream ? (cudaStream_t)stream : real.stream;
+    if (stream) real.lent = true;
     int32_t rc = na_setup(real.ordinal, st);
     if (rc != RSTQ_OK) return rc;
     // Same launcher, same kernel; only the scratch and the stream differ.

@@ -1,4 +1,6 @@
 """Device memory that outlives a call: what is kept, what is given back, and what a recorded graph may still name."""
+import threading
+
 import numpy as np
 import pytest
 import torch
@@ -131,3 +133,58 @@ def test_arrays_of_weights_that_are_gone_are_bounded_and_go_with_the_context():
         before = torch.cuda.mem_get_info()[0]
         c.close()
     assert torch.cuda.mem_get_info()[0] - before >= 40 << 20
+
+
+@pytest.mark.parametrize("where", ["this thread", "another thread"])
+def test_a_weight_is_freed_while_the_caller_captures_elsewhere(where):
+    """The caller records a graph of their own (relaxed mode) on a stream that the context knows nothing of; freeing a weight and
+    binding the next one meanwhile leaves it intact."""
+    c = Context(("cuda:0",))
+    try:
+        w = c.bind_weight(*quant_arrays(512, 0), 512, 512, L.FMT_Q4_0, L.LAYOUT_ROWMAJOR)
+        x = c.array_to_buffer(np.ones(512, np.float32))
+        y = c.make_buffer(512, np.float32)
+        a = torch.zeros(64, device="cuda")
+        graph, done = torch.cuda.CUDAGraph(), []
+
+        def swap():
+            c.qmatmul(w, x, y, 1, L.F32, L.F32, L.MODE_F)
+            w.free()
+            done.append(1)
+
+        torch.cuda.synchronize()
+        with torch.cuda.stream(torch.cuda.Stream()):
+            graph.capture_begin(capture_error_mode="relaxed")
+            a.add_(1)
+            if where == "this thread":
+                swap()
+            else:
+                t = threading.Thread(target=swap)
+                t.start()
+                t.join()
+            a.add_(1)
+            graph.capture_end()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert done == [1] and a.eq(2).all()
+        ref = dense(*quant_arrays(512, 0), 512).reshape(512, 512).sum(1)
+        assert np.abs(y.download() - ref).max() <= 2e-5 * np.abs(ref).max()
+    finally:
+        c.close()
+
+
+def test_arrays_are_not_kept_once_a_stream_was_lent():
+    """On a stream of the caller's a graph that names the weight may be in flight: its array goes to cudaFree, which waits."""
+    c = Context(("cuda:0",))
+    try:
+        n = 4096
+        c.bind_weight(*quant_arrays(n, 0), n, n, L.FMT_Q4_0, L.LAYOUT_ROWMAJOR).free()
+        with torch.cuda.stream(torch.cuda.Stream()):
+            c.set_stream(torch.cuda.current_stream().cuda_stream)
+            w = c.bind_weight(*quant_arrays(n, 1), n, n, L.FMT_Q4_0, L.LAYOUT_ROWMAJOR)
+            before = torch.cuda.mem_get_info()[0]
+            w.free()
+            assert torch.cuda.mem_get_info()[0] - before >= 8 << 20
+            c.set_stream(None)
+    finally:
+        c.close()
