@@ -48,8 +48,7 @@ static void drop_spare_weights(DeviceState& ds) {
     ds.spare_weights.clear();
     ds.spare_bytes = 0;
 }
-// cudaMalloc; before it fails, the arrays kept for weights to come are given back
-static cudaError_t dev_malloc(DeviceState& ds, void** p, int64_t bytes) {
+cudaError_t dev_malloc(DeviceState& ds, void** p, int64_t bytes) {
     *p = nullptr;
     cudaError_t e = cudaMalloc(p, (size_t)bytes);
     if (e != cudaSuccess && !ds.spare_weights.empty()) {
@@ -103,8 +102,7 @@ int32_t dx_reserve(DeviceState& ds, int64_t need) {
         ds.dx_named = false;
         cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
         RSTQ_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
-        const cudaError_t e = cudaMalloc(&ds.dx_scratch, (size_t)need);
-        if (e != cudaSuccess) ds.dx_scratch = nullptr;
+        const cudaError_t e = dev_malloc(ds, &ds.dx_scratch, need);
         RSTQ_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
         RSTQ_CUDA(e);
         ds.dx_scratch_bytes = need;

@@ -362,6 +362,8 @@ int32_t matmul_device(rstq_ctx* ctx, rstq_weight* w, const void* x, void* y, int
                       int out_dtype, int mode, const TpFuse* tp = nullptr);
 // capi.cu: grow-only device scratch (refuses to grow during graph capture; the outgrown block is
 // freed at once, or parked until the last live graph of the device is destroyed)
+// cudaMalloc; before it fails, the arrays kept for weights to come are given back (*p is null after a failure)
+cudaError_t dev_malloc(DeviceState& ds, void** p, int64_t bytes);
 int32_t dev_reserve(DeviceState& ds, void** p, int64_t* have, int64_t need);
 int32_t dx_reserve(DeviceState& ds, int64_t need);   // ds.dx_scratch, during a capture as well
 int32_t dev_release_scratch(DeviceState& ds, void* p);

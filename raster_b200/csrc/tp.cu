@@ -280,7 +280,7 @@ int32_t rstq_tp_create_local(rstq_ctx* ctx, const int32_t* devs, rstq_tp** tps, 
     };
     for (int r = 0; r < nranks; ++r) {
         cudaError_t e = cudaSetDevice(ctx->devs[devs[r]].ordinal);
-        if (e == cudaSuccess) e = cudaMalloc(&regions[r], (size_t)bytes);
+        if (e == cudaSuccess) e = dev_malloc(ctx->devs[devs[r]], &regions[r], bytes);
         if (e == cudaSuccess) e = cudaMemset(regions[r], 0, (size_t)bytes);
         if (e == cudaSuccess) e = cudaDeviceSynchronize();
         if (e != cudaSuccess) {
@@ -346,7 +346,7 @@ int32_t rstq_tp_qmatmul(rstq_tp* tp, rstq_weight* w, rstq_buf* x, rstq_buf* y, i
         if ((rc = dev_release_scratch(ds, tp->tmp)) != RSTQ_OK) return rc;  // parked while a graph may name it
         tp->tmp = nullptr;
         tp->tmp_bytes = 0;
-        RSTQ_CUDA(cudaMalloc(&tp->tmp, (size_t)need));
+        RSTQ_CUDA(dev_malloc(ds, &tp->tmp, need));
         tp->tmp_bytes = need;
     }
     // Decode shapes: the exchange runs in the tail of the matmul kernel itself (one launch).

@@ -188,3 +188,28 @@ def test_arrays_are_not_kept_once_a_stream_was_lent():
             c.set_stream(None)
     finally:
         c.close()
+
+
+@pytest.mark.parametrize("who", ["buffer", "backward"])
+def test_kept_arrays_are_given_back_before_an_allocation_fails(who):
+    """An allocation that the device cannot hold is an error, not before the arrays kept for weights to come are free again; the
+    backward call fails on its scratch (10 bytes per element of dy), ahead of any launch."""
+    c = Context(("cuda:0",))
+    try:
+        n = 8192
+        a = c.make_buffer(1 << 20, np.float32)
+        c.bind_weight(*quant_arrays(n, 0), n, n, L.FMT_Q4_0, L.LAYOUT_ROWMAJOR).free()     # 42 MB
+        before = torch.cuda.mem_get_info()[0]
+        if who == "buffer":
+            with pytest.raises(L.RstqError):
+                c.make_buffer(1 << 40, np.uint8)
+        else:
+            m, out = 1 << 20, 1 << 15
+            dy = c.wrap_buffer(a.device_ptr, m * out, np.float32)
+            codes, scales = c.wrap_buffer(a.device_ptr, out * 32, np.int8), c.wrap_buffer(a.device_ptr, out, np.float32)
+            dx = c.wrap_buffer(a.device_ptr, m * 32, np.float32)
+            with pytest.raises(L.RstqError):
+                c.qlinear_q8_dx_device(dy, codes, scales, dx, m, 32, out)
+        assert torch.cuda.mem_get_info()[0] - before >= 40 << 20
+    finally:
+        c.close()
