@@ -396,8 +396,8 @@ static cudaError_t put_products(rstq_ctx* ctx, DeviceState& ds, const ProductSca
 static int64_t products_tmp_bytes(int64_t n, int per) { return ((n / per * 4 + 255) & ~255ll) + ((n + 255) & ~255ll); }
 // Device arrays of weights.  cudaMalloc and cudaFree of a 10 MB matrix take 0.4 .. 1.4 and 0.35 .. 1.2 ms, more than its copies, so
 // the arrays of weights that are gone serve the next ones of their size (a 4096 x 4096 int4 matrix that takes another one's
-// place: 3.6 -> 2.9 ms).  Up to kWeightKeep bytes per device are kept, and given back before an allocation fails and with
-// the context.  What used an array was launched on the context's own stream, so that is waited for, and no more: a wait for the whole
+// place: 3.6 -> 2.9 ms).  Up to kWeightKeep bytes per device are kept, the longest kept ones making room for others, and given
+// back before an allocation fails and with the context.  What used an array was launched on the context's own stream, so that is waited for, and no more: a wait for the whole
 // device would spoil a capture that the caller has under way elsewhere.  Once a stream of the caller's may have a launch or a recorded
 // graph of theirs (ds.lent), arrays go to cudaFree, which waits for all of it, and are not kept.  (A driver's memory pool
 // instead is as fast here, but matrices that lie in it stream 1 - 2 % slower at one token.)
@@ -414,7 +414,13 @@ static cudaError_t weight_malloc(DeviceState& ds, void** p, int64_t bytes) {
 // (the device is current)
 static void weight_release(DeviceState& ds, void* p, int64_t bytes) {
     if (!p) return;
-    if (!ds.capturing && !ds.lent && ds.spare_bytes + bytes <= kWeightKeep && cudaStreamSynchronize(ds.stream) == cudaSuccess) {
+    if (!ds.capturing && !ds.lent && bytes <= kWeightKeep && cudaStreamSynchronize(ds.stream) == cudaSuccess) {
+        size_t old = 0;
+        for (; ds.spare_bytes + bytes > kWeightKeep; ++old) {
+            ds.spare_bytes -= ds.spare_weights[old].second;
+            cudaFree(ds.spare_weights[old].first);
+        }
+        ds.spare_weights.erase(ds.spare_weights.begin(), ds.spare_weights.begin() + old);
         try {
             ds.spare_weights.emplace_back(p, bytes);
             ds.spare_bytes += bytes;

@@ -213,3 +213,21 @@ def test_kept_arrays_are_given_back_before_an_allocation_fails(who):
         assert torch.cuda.mem_get_info()[0] - before >= 40 << 20
     finally:
         c.close()
+
+
+def test_arrays_of_sizes_that_do_not_come_back_make_room():
+    """64 MB of other sizes are held; a size that comes again is kept and serves the next one all the same."""
+    c = Context(("cuda:0",))
+    try:
+        def bind(n):
+            return c.bind_weight(*quant_arrays(n, n), n, n, L.FMT_Q4_0, L.LAYOUT_ROWMAJOR)
+        bind(8192).free()                                          # 42 MB, and the staging
+        bind(5632).free()                                          # 20 MB: 62 of 64 MB are held
+        bind(4096).free()                                          # 10 MB
+        before = torch.cuda.mem_get_info()[0]
+        w = bind(4096)
+        assert torch.cuda.mem_get_info()[0] == before              # (it took the array that was kept)
+        w.free()
+        assert torch.cuda.mem_get_info()[0] == before              # (and gave it back to be kept)
+    finally:
+        c.close()
