@@ -161,13 +161,13 @@ RSTQ_API int32_t rstq_init(const int32_t* devices, rstq_ctx** ctx, int32_t ndev)
 RSTQ_API int32_t rstq_shutdown(rstq_ctx* ctx);
 /* How the prefill GEMM (M above the decode kernel's range) would tile a call on a device of sm_count SMs
  * at the default settings: plan2[0] = tokens per tile (32, 64, 128 or 256), plan2[1] = thread blocks per
- * tile (2 = K is cut: over two, the second hands its sums to the first, or over as many more as the SMs hold where
- * the tiles are few and K is long; 1 also where whole tiles would leave
- * most SMs idle in the last wave and the thread blocks take equal ranges of all tiles' K instead: rstq_gemm_ranges).  Pure host arithmetic: no
+ * tile: 1 = one has the whole tile, 2 = its K is cut, over two thread blocks or over more where the tiles are few and K is
+ * long (rstq_gemm_layout: over how many), the first of which adds the others' sums to its own; 1 also where thread blocks take
+ * equal ranges of all tiles' K (rstq_gemm_ranges) and where a pair has the tile (rstq_gemm_layout).  Pure host arithmetic: no
  * device, no context.  No counterpart in the reference (its GEMM is one work-item per output). */
 RSTQ_API int32_t rstq_gemm_plan(int32_t* plan2, int64_t out, int64_t in, int64_t m, int32_t sm_count);
-/* In how many equal ranges of all tiles' K-steps (thread blocks) that call would run; 0 = as whole tiles, or two thread
- * blocks per tile (rstq_gemm_plan).  Pure host arithmetic as well. */
+/* In how many equal ranges of all tiles' K-steps (thread blocks) that call would run; 0 = as whole tiles, or as
+ * parts of them (rstq_gemm_plan).  Pure host arithmetic as well. */
 RSTQ_API int32_t rstq_gemm_ranges(int32_t* ranges, int64_t out, int64_t in, int64_t m, int32_t sm_count);
 /* All of that call's layout, at a setting of RSTQ_TUNE_GEMM_WIDE: layout6[0] = tokens per tile, [1] = thread blocks per tile
  * (1 = whole tiles), [2] = ranges (0 = none), [3] = 1 where a tile has 256 features and [1] and [2] count pairs of thread

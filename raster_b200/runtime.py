@@ -23,7 +23,7 @@ _ptr_cache: dict = {}   # id(array) -> (weak reference to it, its address): hot 
 
 def gemm_plan(out: int, in_: int, m: int, sm_count: int = 148) -> dict:
     """How the prefill GEMM would tile a call on a device of sm_count SMs (rstq_gemm_plan: host arithmetic, no
-    device): tokens per tile and thread blocks per tile (2: K is cut, over two or more)."""
+    device): tokens per tile and thread blocks per tile (2: K is cut, over two or more: gemm_layout)."""
     plan = (C.c_int32 * 2)()
     L.check(L.load().rstq_gemm_plan(plan, out, in_, m, sm_count))
     return {"tile_tokens": plan[0], "blocks_per_tile": plan[1]}

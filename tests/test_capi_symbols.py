@@ -139,7 +139,11 @@ def test_thread_blocks_that_share_gemm_tiles_have_a_slot_each(wide):
             if wide >= 5 and m > 128:
                 assert v["pairs"]
     assert R.gemm_layout(28672, 8192, 256) == {"tile_tokens": 256, "per_tile": 1, "ranges": 74, "pairs": True, "blocks": 148, "columns": 256}
-    assert R.gemm_layout(1000, 16384, 30)["per_tile"] > 2
+    # the calls of few tiles that the GPU tests run, on both sides of the lines
+    for out, in_, m, parts in [(100, 2080, 20, 9), (40, 20000, 17, 23), (40, 65536, 17, 43), (300, 4128, 40, 7), (1000, 16384, 30, 16),
+                               (2500, 4128, 100, 5), (130, 8192, 128, 6), (250, 2048, 64, 2), (600, 8224, 200, 6), (2048, 2048, 128, 2),
+                               (4096, 4096, 256, 2), (512, 1024, 32, 1)]:
+        assert R.gemm_layout(out, in_, m, 148)["per_tile"] == parts or wide, (out, in_, m)
     lib = L.load()
     assert lib.rstq_gemm_layout(None, 4096, 4096, 64, 148, 0) == L.E_INVALID
     v = (C.c_int64 * 6)()

@@ -76,10 +76,10 @@ def test_tiles_on_pairs_of_sms_against_tiles_on_one(ctx, bits, out, in_, M):
 
 
 @pytest.mark.parametrize("bits", [4, 8])
-@pytest.mark.parametrize("out,in_,M", [(100, 2080, 20), (40, 20000, 17), (300, 4128, 40), (1000, 16384, 30), (2500, 4128, 100),
+@pytest.mark.parametrize("out,in_,M", [(100, 2080, 20), (40, 20000, 17), (40, 65536, 17), (300, 4128, 40), (1000, 16384, 30), (2500, 4128, 100),
                                        (130, 8192, 128), (250, 2048, 64), (600, 8224, 200)])
 def test_few_tiles_cut_over_many_thread_blocks(ctx, bits, out, in_, M):
-    """A call of few tiles: each cut over as many thread blocks as its K-steps are worth (3 .. 52 here), tiles of 32, 64 and
+    """A call of few tiles: each cut over as many thread blocks as its K-steps are worth (2 .. 43 here), tiles of 32, 64 and
     128 tokens, parts of unequal length, a partial last K-step.  As whole tiles up to the order of the additions; three calls
     in a row (each finds the flags of the one before taken down) give the same bits."""
     w = synth.normal(out + in_ + bits, out * in_, 0.02)
