@@ -94,7 +94,9 @@ def test_few_tiles_cut_over_many_thread_blocks(ctx, bits, out, in_, M):
         ctx.tune(TUNE_GEMM_WIDE, 0)
     assert np.array_equal(y[0], y[1]) and np.array_equal(y[0], y[2])
     assert not np.array_equal(y[0], whole)                         # (it was cut)
-    assert np.abs(y[0] - whole).max() <= 4 * 8e-6 * np.abs(whole).max()
+    # (rows of 65536, 4096 additions of 16 products, no random walk of 260: each off by 2^-23 of a running value, about max|y| at most)
+    bound = 4 * 8e-6 if in_ <= 32768 else in_ / 16 * 2.0 ** -23
+    assert np.abs(y[0] - whole).max() <= bound * np.abs(whole).max()
     rows = np.unique(np.concatenate([np.arange(0, out, max(1, out // 64)), [out - 1]]))
     c = np.ascontiguousarray(wq.reshape(out, -1)[rows]).ravel()
     s = np.ascontiguousarray(ws.reshape(out, -1)[rows]).ravel()
