@@ -105,9 +105,9 @@ act_to_f16_kernel(const void* __restrict__ x, __half* __restrict__ x16,
         }
         if (SRC >= 2) quant_dequant8(v);
     };
-    // Rows of up to 8192 elements stay in registers between the two passes (max, convert);
+    // Rows of up to 32 T elements (32768: act_launch) stay in registers between the two passes (max, convert);
     // longer rows are read twice.
-    constexpr int kKeep = 4;  // x 256 threads x 8 elements
+    constexpr int kKeep = 4;  // x T threads x 8 elements
     const bool keep = in <= (int64_t)kKeep * T * 8;
     float held[kKeep][8];
     float mx = 0.f;
@@ -1243,8 +1243,11 @@ static cudaError_t act_launch(const DeviceState& ds, const void* x, void* x16, f
     // 32 elements per thread at most, so that a row stays in registers up to 32768 (8192 with 256 threads for any row,
     // before): 4096 x 11008, M = 70, quantized on the way 34.0 -> 28.0 us a call, 8192 x 28672, M = 100 73.5 -> 66.0.  128 threads
     // for short rows: 1000 x 1024, M = 2048 12.8 -> 12.0; at in = 4096 they lose (4096 x 4096, M = 512 22.2 -> 23.2), as 512 threads
-    // do at 6016 (3000 x 6016, M = 30 16.9 -> 17.5).
-    if (in <= 2048) return go(act_to_f16_kernel<SRC, 128>, 128);
+    // do at 6016 (3000 x 6016, M = 30 16.9 -> 17.5).  Where the quantizer is on the way a thread has more to do, and fewer of
+    // them pay only once 256 for each row do not run at once, eight rows per SM: int8 7520 x 1632, 128 / 256 threads, M = 74 12.5 / 12.1, M = 150
+    // 14.3 / 13.6, M = 600 26.5 / 25.9, M = 1200 40.4 / 41.5; 2000 x 2048, M = 600 16.0 / 15.1, M = 2000 24.7 / 26.4; 4096 x 1024, M = 300
+    // 10.6 / 10.3, M = 1200 24.9 / 26.3.  Without it 128 are as fast or faster at every M (M = 150 11.8 / 12.7, M = 20 10.2 / 10.2).
+    if (in <= 2048 && (SRC < 2 || M > 8 * ds.sm_count)) return go(act_to_f16_kernel<SRC, 128>, 128);
     if (in <= 8192) return go(act_to_f16_kernel<SRC, 256>, 256);
     if (in <= 16384) return go(act_to_f16_kernel<SRC, 512>, 512);
     return go(act_to_f16_kernel<SRC, 1024>, 1024);

@@ -201,6 +201,17 @@ def test_wide_token_tiles_match_the_narrow_ones(ctx, bits, M, out, in_):
 @pytest.mark.parametrize("mode,M,act", [(L.MODE_F, 19, L.F32), (L.MODE_F, 19, L.BF16), (L.MODE_A8, 65, L.F32)])
 def test_activation_rows_at_the_edges_of_the_pre_pass(ctx, mode, M, act, in_):
     """The pre-pass takes 128, 256, 512 or 1024 threads per row, and reads rows above 32768 twice."""
+    check_pre_pass(ctx, mode, M, act, in_)
+
+
+@pytest.mark.parametrize("in_", [32, 1056, 2048, 2080])
+@pytest.mark.parametrize("rows,act", [(0, L.F32), (1, L.F32), (1, L.BF16)])
+def test_quantized_rows_on_both_sides_of_the_pre_pass_line(ctx, rows, act, in_):
+    """Short rows that are quantized on the way: 256 threads up to eight rows per SM, 128 above."""
+    check_pre_pass(ctx, L.MODE_A8, 8 * ctx.device_info()["sm_count"] + rows, act, in_)
+
+
+def check_pre_pass(ctx, mode, M, act, in_):
     out = 40
     w = synth.normal(in_, out * in_, 0.02)
     wq, ws = orc.quantize_weight(w, 8)
