@@ -105,8 +105,7 @@ act_to_f16_kernel(const void* __restrict__ x, __half* __restrict__ x16,
         }
         if (SRC >= 2) quant_dequant8(v);
     };
-    // Rows of up to 32 T elements (32768: act_launch) stay in registers between the two passes (max, convert);
-    // longer rows are read twice.
+    // Rows of up to 32 T elements stay in registers between the two passes (max, convert); longer rows are read twice.
     constexpr int kKeep = 4;  // x T threads x 8 elements
     const bool keep = in <= (int64_t)kKeep * T * 8;
     float held[kKeep][8];
@@ -1249,7 +1248,13 @@ static cudaError_t act_launch(const DeviceState& ds, const void* x, void* x16, f
     // 10.6 / 10.3, M = 1200 24.9 / 26.3.  Without it 128 are as fast or faster at every M (M = 150 11.8 / 12.7, M = 20 10.2 / 10.2).
     if (in <= 2048 && (SRC < 2 || M > 8 * ds.sm_count)) return go(act_to_f16_kernel<SRC, 128>, 128);
     if (in <= 8192) return go(act_to_f16_kernel<SRC, 256>, 256);
-    if (in <= 16384) return go(act_to_f16_kernel<SRC, 512>, 512);
+    // Many rows: an SM holds one block of 1024 threads or two of 512, so that loads of the next rows wait for the last ones' reductions;
+    // bf16 rows are then read twice by four blocks of 256 per SM sooner (1024 features, 256 / 512 threads: in = 16384, M = 2000 87.6 / 93.4,
+    // M = 1000 50.8 / 52.5, M = 520 35.8 / 36.1, M = 300 29.3 / 28.2; f32 102.7 / 102.0 at 2000, quantized 123.5 / 112.1), and others by
+    // 512 threads instead of 1024 (in = 20000, M = 2000 f32 130.4 / 140.7; M = 520 47.9 / 48.6, M = 300 34.4 / 34.5, quantized 40.4 / 38.9).
+    const int64_t sm = ds.sm_count;
+    if (SRC == 1 && M > 4 * sm) return go(act_to_f16_kernel<SRC, 256>, 256);
+    if (in <= 16384 || M > (SRC >= 2 ? 3 : 2) * sm) return go(act_to_f16_kernel<SRC, 512>, 512);
     return go(act_to_f16_kernel<SRC, 1024>, 1024);
 }
 static int32_t launch_act_to_f16(rstq_ctx* ctx, DeviceState& ds, const void* x, int src, void* x16,

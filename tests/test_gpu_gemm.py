@@ -211,6 +211,14 @@ def test_quantized_rows_on_both_sides_of_the_pre_pass_line(ctx, rows, act, in_):
     check_pre_pass(ctx, L.MODE_A8, 8 * ctx.device_info()["sm_count"] + rows, act, in_)
 
 
+@pytest.mark.parametrize("mode,act,in_,per_sm", [(L.MODE_F, L.BF16, 8224, 4), (L.MODE_F, L.BF16, 16416, 4), (L.MODE_F, L.BF16, 16416, 2),
+                                                 (L.MODE_F, L.F32, 16416, 2), (L.MODE_A8, L.F32, 16416, 3)])
+@pytest.mark.parametrize("rows", [0, 1])
+def test_long_rows_on_both_sides_of_the_pre_pass_lines(ctx, mode, act, in_, per_sm, rows):
+    """Long rows take fewer threads each where there are more than a few per SM, and are then read twice."""
+    check_pre_pass(ctx, mode, per_sm * ctx.device_info()["sm_count"] + rows, act, in_)
+
+
 def check_pre_pass(ctx, mode, M, act, in_):
     out = 40
     w = synth.normal(in_, out * in_, 0.02)
