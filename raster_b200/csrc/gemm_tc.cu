@@ -62,7 +62,7 @@ __device__ __forceinline__ void quant_dequant8(float (&v)[8]) {
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             code[j] = fmaf(v[j], id, kMagic) - kMagic;
-            exact |= !(fabsf(fmaf(v[j], id, -code[j])) <= 0.5f - 5e-5f);
+            exact |= !(fabsf(fmaf(v[j], id, -code[j])) <= kQuantSure);
         }
         if (!exact) {
 #pragma unroll

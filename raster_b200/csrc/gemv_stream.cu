@@ -36,6 +36,7 @@
 
 #include "internal.h"
 #include "mma_helpers.cuh"
+#include "quant_helpers.cuh"
 #include "sync_helpers.cuh"
 
 // Timing probes and the per-chunk stamps of CTA 0 exist only in builds made with -DRSTQ_PROBES=1
@@ -397,7 +398,7 @@ __device__ __forceinline__ void stage_a8_quant(const StreamParams& p, const void
                 amb = max_nan(amb, fabsf(frac));                     // a NaN takes the double path as well
                 ub[k] = __float_as_uint(u);
             }
-            exact = !(amb <= 0.5f - 5e-5f);
+            exact = !(amb <= kQuantSure);
             wa = __byte_perm(__byte_perm(ub[0], ub[1], 0x0040), __byte_perm(ub[2], ub[3], 0x0040), 0x5410);
             wb = __byte_perm(__byte_perm(ub[4], ub[5], 0x0040), __byte_perm(ub[6], ub[7], 0x0040), 0x5410);
         }
@@ -479,7 +480,7 @@ __device__ __forceinline__ void stage_f(const StreamParams& p, uint8_t* smem, in
 // The same array in global memory, for launches whose activations ride the weight ring (StreamParams::ring):
 // block-major, so the entries of a chunk's K blocks are one contiguous slice.
 __global__ void __launch_bounds__(256)
-act_image_f_kernel(const void* __restrict__ x, uint2* __restrict__ img, int M, int T, int nb, int64_t in, int act_dtype) {
+act_image_f_kernel(const void* __restrict__ x, uint2* __restrict__ img, int M, int T, int nb, int64_t in) {   // (f32 activations)
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const int C = M * T;
@@ -492,7 +493,7 @@ act_image_f_kernel(const void* __restrict__ x, uint2* __restrict__ img, int M, i
         const int h = (int)(bh & 1);
         const int64_t b = bh >> 1;
         const int m = c / T, t = c - m * T;
-        img[o] = f_entry(x, act_dtype, (int64_t)m * in + b * 32 + h * 16 + tg * 4, t);
+        img[o] = f_entry(x, RSTQ_F32, (int64_t)m * in + b * 32 + h * 16 + tg * 4, t);
     }
 }
 
@@ -2192,7 +2193,7 @@ int32_t launch_gemv_f(rstq_ctx* ctx, DeviceState& ds, const GemvFArgs& a) {
             cfg.numAttrs = ds.pdl ? 1 : 0;
             if (bf) RSTQ_CUDA(cudaLaunchKernelEx(&cfg, act_image_bf16_kernel, (const uint4*)p.x, (uint4*)a.img_scratch, M, (int)nb));
             else RSTQ_CUDA(cudaLaunchKernelEx(&cfg, act_image_f_kernel, p.x, reinterpret_cast<uint2*>(a.img_scratch), M, T,
-                                              (int)nb, a.in, a.act_dtype));
+                                              (int)nb, a.in));
             ctx->launches++;
             p.img = a.img_scratch;
             p.slice1 = (uint32_t)(2 * C * 32);

@@ -21,15 +21,11 @@
 // is a small f32 GEMV over the per-sub-block minima  b = db*bq  ([out, in/32] floats, a quarter
 // of the code bytes), added to y by q4k_min_kernel.  The q8_K activation quantizer
 // (quantize-act-q8k, src/raster/compiler/backend/cpu/quant.clj:172-193; device form
-// quant-act-q8k-gpu!, kernels_k.clj:93-134) is one kernel here: a CTA per super-block.
+// quant-act-q8k-gpu!, kernels_k.clj:93-134) is one kernel here: a warp per super-block.
 #include "internal.h"
+#include "quant_helpers.cuh"
 
 namespace rstq {
-
-__device__ __forceinline__ int kq_round_half_up(double v) {
-    const double f = floor(v);
-    return (int)f + ((v - f) >= 0.5 ? 1 : 0);
-}
 
 // A warp per (row, super-block), lane l owns elements 8 l .. 8 l + 7; two warps per thread block (see quant_act_i8_kernel for
 // why small thread blocks).  Codes come from f32 arithmetic except next to a tie or where the largest magnitude is zero,
@@ -70,7 +66,7 @@ quant_act_q8k_kernel(const float* __restrict__ x, int8_t* __restrict__ xq, float
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
             const float t = fmaf(v[k], id, kMagic);
-            exact |= !(fabsf(fmaf(v[k], id, kMagic - t)) <= 0.5f - 5e-5f);
+            exact |= !(fabsf(fmaf(v[k], id, kMagic - t)) <= kQuantSure);
             u[k] = __float_as_uint(t);
         }
 #pragma unroll
@@ -86,7 +82,7 @@ quant_act_q8k_kernel(const float* __restrict__ x, int8_t* __restrict__ xq, float
             w[h] = 0u;
 #pragma unroll
             for (int k = 0; k < 4; ++k)
-                w[h] |= (uint32_t)(max(-127, min(127, kq_round_half_up((double)v[4 * h + k] * id))) & 0xFF) << (8 * k);
+                w[h] |= (uint32_t)(max(-127, min(127, quant_round_half_up((double)v[4 * h + k] * id))) & 0xFF) << (8 * k);
         }
         scale = (float)d;
     }

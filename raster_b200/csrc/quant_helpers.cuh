@@ -15,7 +15,9 @@ __device__ __forceinline__ int quant_round_half_up(double v) {
 // double product, so where t is further than 5e-5 from every k + 0.5, rounding t to nearest gives the same code; u = fma(x, id,
 // 1.5 * 2^23) holds that code in its low bits.  xs = fl32(mx / 127) equals (float)((double)mx / 127.0): the quotient
 // of a 24-bit integer by 127 is no midpoint.  Blocks whose maximum is zero, tiny, huge or infinite, and elements
-// near a tie or not a number, take the double path.
+// near a tie or not a number, take the double path.  (The decode kernel, the pre-pass and the super-block quantizer, which hold
+// their elements in other places, go by the same margin.)
+constexpr float kQuantSure = 0.5f - 5e-5f;
 // (An SM does 64 double operations per clock, and a decode step's 4096-element norm quantizes its row on one SM: two
 // divisions per lane were half a microsecond of each such launch.  7B-class MLP at 8 tokens, whose quantizer
 // kernels ran them too: 23.3 -> 22.6 us; a step of four 7B layers 227 -> 224 us.)
@@ -29,7 +31,7 @@ __device__ __forceinline__ void quant_block32(float v, int* q, int* sum, float* 
     if (!exact) {
         const float id = __fdividef(127.f, mx);
         const float u = fmaf(v, id, kMagic);
-        exact = !(fabsf(fmaf(v, id, kMagic - u)) <= 0.5f - 5e-5f);
+        exact = !(fabsf(fmaf(v, id, kMagic - u)) <= kQuantSure);
         code = __float_as_int(u) - __float_as_int(kMagic);
         *xs = __fdiv_rn(mx, 127.f);
     }
@@ -59,7 +61,7 @@ __device__ __forceinline__ void quant_block32_words(const float (&v)[4], uint32_
         for (int k = 0; k < 4; ++k) {
             const float t = fmaf(v[k], id, kMagic);
             const float frac = fabsf(fmaf(v[k], id, kMagic - t));
-            exact |= !(frac <= 0.5f - 5e-5f);
+            exact |= !(frac <= kQuantSure);
             u[k] = __float_as_uint(t);
         }
         w = __byte_perm(__byte_perm(u[0], u[1], 0x0040), __byte_perm(u[2], u[3], 0x0040), 0x5410);
