@@ -13,8 +13,8 @@
 //   pairs of fp16     W' = H + 2^-11 L, dy = h + 2^-11 l:  H h + 2^-11 (H l + L h)                             3 MMAs
 //   triples of bf16   W' = W1 + W2 + W3, dy = Y1 + Y2 + Y3:  W1 Y1 + (W1 Y2 + W2 Y1) + (W1 Y3 + W2 Y2 + W3 Y1)  6 MMAs
 //
-// A pair holds an f32 to within one unit of its last place (11 bits, a sign, 11 bits), a weight to within three: its scale is a
-// pair itself, times the code in packed fp16.  Its second term is kept 2^11 larger than it is, in a sum of its own, and a power of
+// A pair (11 bits, a sign, 11 bits) holds an element of dy to 2 * 2^-24 of itself, one unit of f32's last place, and a weight to
+// 6 * 2^-24 (4.0 seen, 0.95 rms): its scale is a pair itself, times the code in packed fp16.  The second term is kept 2^11 larger than it is, in a sum of its own, and a power of
 // two per token row and per 32-column block brings the largest of them close to fp16's, so an element down to 2^-27 of its row's
 // largest (a scale down to 2^-20 of its column block's) is held so: the tiles whose rows and column blocks hold nothing
 // smaller but zeros, and no infinity, take pairs.  Triples hold all 24 bits at any spread (2^-90 is tested); a tile with

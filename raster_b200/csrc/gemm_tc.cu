@@ -670,8 +670,9 @@ gemm_tmem_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tmap) {
     const int fd = tile_first / p.ttiles, ft_first = fd * CS + (int)rank, tok_first = (tile_first - fd * p.ttiles) * NTOK;
 
     // DUO: the columns of a tile that hold tokens, in thirty-twos (N of an MMA of cta_group::2 with M = 256), where one tile takes all tokens: narrower MMAs.  (The rest of its
-    // columns is never written, and what is read there goes nowhere.  int4 28672 x 8192 at M = 160 91.4 -> 85.6 us, 8192 x 28672 at
-    // M = 200 94.6 -> 91.8.  Worked out per tile, for several, full tiles lose 1.4 %.)
+    // columns is never written, and what is read there goes nowhere.  int4 28672 x 8192 at M = 160 91.4 -> 85.6 us; in
+    // sixteens M = 200 would be 208 columns and 104.2 us at 8192 x 28672, it is 224 and 105.0.  Worked out per tile, for several, full
+    // tiles lose 1.4 %.)
     const int cols = DUO ? p.cols : NTOK;
 
     if (tid == 0) asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmap)) : "memory");
